@@ -383,3 +383,155 @@ def tolerance(case):
     if op == "train":
         return {"rel": 0.02, "max": 0.4}
     return {"rel": 0.02, "max": 0.2}
+
+
+# ------------------------------------------------------------------------------------------------
+# the same outputs in 64 bits, in plain torch
+# ------------------------------------------------------------------------------------------------
+_QUINTIC = ((4.0848, -6.8946, 2.9270), (3.9505, -6.3029, 2.6377), (3.7418, -5.5913, 2.3037),
+            (2.8769, -3.1427, 1.2046), (2.8366, -3.0525, 1.2012))
+_POLAR = ((8.156554524902461, -22.48329292557795, 15.878769915207462),
+          (4.042929935166739, -2.808917465908714, 0.5000178451051316),
+          (3.8916678022926607, -2.772484153217685, 0.5060648178503393),
+          (3.285753657755655, -2.3681294933425376, 0.46449024233003106),
+          (2.3465413258596377, -1.7097828382687081, 0.42323551169305323))
+_AOL = ((4.6051, -9.6552, 5.6769), (4.7505, -6.0861, 2.1790), (2.7763, -2.3190, 0.5523),
+        (2.4231, -2.2861, 0.8193))
+
+
+def _ortho64(G, driver, eps):
+    """Newton-Schulz iteration of one matrix; the Gram driver is the same iteration reordered."""
+    X = G.double()
+    tall = X.size(0) > X.size(1)
+    X = X.mT if tall else X
+    coeffs, mult = (_QUINTIC, 1.0) if driver == "quintic" else (_POLAR, 1.02)
+    if driver == "aol":
+        coeffs = _AOL
+        X = X * (X @ X.mT).abs().sum(dim=-1, keepdim=True).clamp_min(eps).rsqrt()
+    else:
+        X = X / (X.norm() * mult + eps)
+    for a, b, c in coeffs:
+        A = X @ X.mT
+        X = a * X + (b * A + c * (A @ A)) @ X
+    return X.mT if tall else X
+
+
+def _split(flat, shapes):
+    views, at = [], 0
+    for s in shapes:
+        n = math.prod(s)
+        views.append(flat[at:at + n].view(s))
+        at += -(-n // 128) * 128
+    return views
+
+
+def _update64(case, out, shapes, grads, steps):
+    """One optimizer step on the flat fp64 buffers ``out`` (weights and state), in place."""
+    mats, scals = shapes
+    w, m = _split(out["weights_matrix"], mats), _split(out["momentum_matrix"], mats)
+    v = None
+    if case["algorithm"] == "normuon":
+        key = next(k for k in out if k.startswith("variance") and k.endswith("_matrix"))
+        v = _split(out[key], [(r, 1) for r, _ in mats])
+    for i, (rows, cols) in enumerate(mats):
+        W, M, G = w[i], m[i], grads[i].double()
+        ratio = math.sqrt(rows / cols)
+        if case["algorithm"] == "dion2":
+            dim = 0 if rows <= cols else 1
+            M.add_(G)
+            k = math.ceil(case["fraction"] * M.size(dim))
+            sel = M.abs().sum(dim=1 - dim).topk(k).indices.sort().values
+            U = _ortho64(M.index_select(dim, sel), "polar", 1e-8)
+            full = torch.zeros_like(M).index_copy_(dim, sel, U)
+            M.index_copy_(dim, sel, M.index_select(dim, sel) * MU)
+        else:
+            M.mul_(MU).add_(G)
+            full = _ortho64(MU * M + G, "polar", 1e-8)
+            if v is not None:
+                before = full.norm()
+                v[i].lerp_(full.square().mean(dim=1, keepdim=True), 0.05)
+                full = full / (v[i].sqrt() + 1e-8)
+                full = full * (before / full.norm())
+        W.mul_(1 - LR * WD).sub_(full, alpha=LR * ratio)
+    w, m = _split(out["weights_scalar"], scals), _split(out["momentum_scalar"], scals)
+    for i in range(len(scals)):
+        W, M, G = w[i], m[i], grads[len(mats) + i].double()
+        if case["scalar"] == "lion":
+            lr = SCALAR_LR if i == 0 else SCALAR_LR / math.sqrt(case["width"])
+            W.sub_(torch.lerp(M, G, 0.1).sign_(), alpha=lr)
+            M.lerp_(G, 0.05)
+        else:
+            V = _split(out["variance_scalar"], scals)[i]
+            M.lerp_(G, 0.1)
+            V.lerp_(G.square(), 0.05)
+            W.sub_(SCALAR_LR * (M / (1 - 0.9 ** steps))
+                   / ((V / (1 - 0.95 ** steps)).sqrt_() + 1e-8))
+    return out
+
+
+def _norm64(x, eps):
+    return x * (x.square().mean(dim=-1, keepdim=True) + eps).rsqrt()
+
+
+def _hidden64(weights, embedding, ids, heads):
+    """Residual stream of the GPT after its last norm; norms use the epsilon of their input's
+    data type (fp32 residual stream, bf16 queries and keys)."""
+    x = embedding[ids]
+    B, T, C = x.shape
+    D = C // heads
+    inv = 10000.0 ** (-torch.arange(0, D, 2, device="cuda", dtype=torch.float64) / D)
+    ang = torch.outer(torch.arange(T, device="cuda", dtype=torch.float64), inv)
+    cos, sin = ang.cos(), ang.sin()
+
+    def rope(t):
+        a, b = t[..., :D // 2], t[..., D // 2:]
+        return _norm64(torch.cat([a * cos + b * sin, b * cos - a * sin], dim=-1), 2.0 ** -7)
+
+    mask = torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1)
+    for q, k, v, o, fc, proj in weights:
+        h = _norm64(x, 2.0 ** -23)
+        q, k, v = ((h @ W.mT).view(B, T, heads, D).transpose(1, 2) for W in (q, k, v))
+        s = (rope(q) @ rope(k).mT / math.sqrt(D)).masked_fill(mask, -math.inf)
+        y = (s.softmax(dim=-1) @ v).transpose(1, 2).reshape(B, T, C)
+        x = x + y @ o.mT
+        x = x + (_norm64(x, 2.0 ** -23) @ fc.mT).relu().square() @ proj.mT
+    return _norm64(x, 2.0 ** -23)
+
+
+def _weights64(model, grad):
+    mats = [p.detach().double().requires_grad_(grad) for p in model.transformer.h.parameters()]
+    scals = [p.detach().double().requires_grad_(grad)
+             for p in (model.transformer.wte.weight, model.lm_head.weight)]
+    return mats, scals, [mats[i:i + 6] for i in range(0, len(mats), 6)]
+
+
+def exact(case, seed):
+    op = case["op"]
+    if case.get("algorithm") in ("dion", "nordion2"):
+        return None   # a sketch drawn on the device; rows selected and normalized together
+    state = prepare(case, seed)
+    if op == "ortho":
+        G = state["G"]
+        one = lambda g: _ortho64(g, case["driver"],  # noqa: E731
+                                 1e-7 if case["driver"] in ("quintic", "aol") else 1e-6)
+        return one(G) if G.ndim == 2 else torch.stack([one(g) for g in G])
+    if op == "optimizer":
+        grads = [p.grad for p in state["params"]]
+        out = {k: t.double() for k, t in state["outputs"].items()}
+        return _update64(case, out, _shapes(case), grads, 101)
+    mats, scals, blocks = _weights64(state["model"], op == "train")
+    if op == "logits":
+        h = _hidden64(blocks, scals[0], state["x"], case["heads"])
+        return (h if "y" in state else h[:, -1:]) @ scals[1].mT
+    total, rows = 0.0, max(1, 4096 // case["tokens"])
+    count = state["y"].numel()
+    for x, y in zip(state["x"].split(rows), state["y"].split(rows)):
+        h = _hidden64(blocks, scals[0], x, case["heads"])
+        loss = torch.nn.functional.cross_entropy((h @ scals[1].mT).flatten(0, 1), y.flatten(),
+                                                 reduction="sum") / count
+        loss.backward()
+        total = total + loss.detach()
+    out = {k: t.double() for k, t in state["outputs"].items()}
+    shapes = [tuple(p.shape) for p in mats], [tuple(p.shape) for p in scals]
+    grads = [p.grad for p in mats + scals]
+    return {"loss": total, **_update64(case, out, shapes, grads, 1)}
