@@ -11,7 +11,7 @@
 // barrier; no multicast).  The leader CTA's MMA thread issues the instructions for the pair and
 // releases stages / publishes accumulators in both CTAs with a cluster-multicast tcgen05.commit.
 // Each CTA drains its own half (128 TMEM lanes) of the accumulator in its epilogue warps, 64 columns
-// at a time through shared memory: D arrives by TMA (prefetched two sub-tiles ahead), each thread
+// at a time through shared memory: D arrives by TMA (prefetched three sub-tiles ahead), each thread
 // combines its row in place in the 128-byte-swizzled buffer, and the buffer leaves by TMA store.
 // In symmetric mode only tiles on or above the diagonal are computed; an off-diagonal tile also
 // writes a transposed copy of each sub-tile that a second TMA store places at the mirrored
@@ -29,17 +29,27 @@ constexpr int BM2 = 128;   // rows per CTA (256 per pair)
 constexpr int BN2 = 256;   // columns per pair (128 loaded by each CTA)
 constexpr int BK2 = 64;
 constexpr int kThreads2 = 192;
-constexpr int kStagesSym = 5;     // symmetric mode also stages transposed sub-tiles
-constexpr int kStagesPlain = 6;
+// Shared memory is split between operand stages (32 KB), D/C sub-tile buffers and transposed
+// sub-tile buffers (16 KB each).  With two D/C buffers the chain "store has read the buffer -> next
+// D arrives -> combine" bounded a tile at 10 us whatever K was (update of 64 matrices 768 x 3072,
+// K = 768: 324 us).  Four buffers keep three sub-tiles of D in flight while the next tile
+// multiplies, which is worth more than the sixth stage (256 us; K = 2048: 326 -> 321 us, K = 4096
+// unchanged; polynomial at K = 768: 81 -> 72.5 us).
+//   plain             5 stages + 4 D/C
+//   symmetric, no D   5 stages + 2 D/C + 2 transposed
+//   symmetric, D      4 stages + 4 D/C + 2 transposed
+struct CfgPlain { static constexpr int kStages = 5, kDC = 4, kT = 0; };
+struct CfgSym { static constexpr int kStages = 5, kDC = 2, kT = 2; };
+struct CfgSymD { static constexpr int kStages = 4, kDC = 4, kT = 2; };
 constexpr int kABytes2 = BM2 * BK2 * 2;          // 16 KB
 constexpr int kBBytes2 = (BN2 / 2) * BK2 * 2;    // 16 KB
 constexpr int kStageBytes2 = kABytes2 + kBBytes2;
 constexpr int kSubCols = 64;                       // epilogue sub-tile: 128 rows x 64 columns
-constexpr int kEpiBufs = 2;
 constexpr int kEpiBufBytes = BM2 * kSubCols * 2;    // 16 KB: two 64 x 64 boxes of bf16
-// stages | kEpiBufs D/C buffers | kEpiBufs transposed buffers (symmetric mode) | alignment slack
-constexpr int dyn_bytes2(int stages, bool sym) {
-  return stages * kStageBytes2 + (sym ? 2 : 1) * kEpiBufs * kEpiBufBytes + 1024;
+// stages | D/C buffers | transposed buffers (symmetric mode) | alignment slack
+template <class CFG>
+constexpr int dyn_bytes2() {
+  return CFG::kStages * kStageBytes2 + (CFG::kDC + CFG::kT) * kEpiBufBytes + 1024;
 }
 constexpr uint32_t kTmemCols2 = 2 * BN2;
 
@@ -202,8 +212,10 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void*
 __device__ __forceinline__ void bulk_commit_group() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
-__device__ __forceinline__ void bulk_wait_group_read_all() {
-  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+// Waits until all but the latest N committed stores have read their shared memory.
+template <int N>
+__device__ __forceinline__ void bulk_wait_group_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void bulk_wait_group_all() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -230,11 +242,12 @@ __device__ __forceinline__ float ipow2(float s, int p) {
   return r;
 }
 
-template <bool A_MN, bool B_MN, int kStages2>
+template <bool A_MN, bool B_MN, class CFG>
 __global__ void __launch_bounds__(kThreads2, 1)
 ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                 const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_d,
                 const Gemm2Args p) {
+  constexpr int kStages2 = CFG::kStages, kDC = CFG::kDC, kT = CFG::kT;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -242,7 +255,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   __shared__ __align__(8) uint64_t empty_bar[kStages2];   // one copy per CTA
   __shared__ __align__(8) uint64_t tfull_bar[2];          // one copy per CTA
   __shared__ __align__(8) uint64_t tempty_bar[2];         // used in the leader CTA
-  __shared__ __align__(8) uint64_t dfull_bar[kEpiBufs];   // D sub-tiles, one copy per CTA
+  __shared__ __align__(8) uint64_t dfull_bar[kDC];        // D sub-tiles, one copy per CTA
   __shared__ uint32_t tmem_base_slot;
 
   const int warp = threadIdx.x >> 5;
@@ -261,7 +274,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       mbar_init(&tfull_bar[a], 1);
       mbar_init(&tempty_bar[a], 8);  // four epilogue warps in each CTA of the pair
     }
-    for (int a = 0; a < kEpiBufs; ++a) mbar_init(&dfull_bar[a], 1);
+    for (int a = 0; a < kDC; ++a) mbar_init(&dfull_bar[a], 1);
     fence_barrier_init();
     fence_proxy_async();
     prefetch_tmap(&map_a);
@@ -402,9 +415,12 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   } else {
     // ------------------------------ epilogue (both CTAs) ----------------------------------
     // The 128 x 256 half-tile of this CTA is drained in sub-tiles of 64 columns.  D arrives by
-    // TMA into a shared-memory buffer (prefetched two sub-tiles ahead), each thread combines
+    // TMA into a shared-memory buffer (prefetched kDC - 1 sub-tiles ahead), each thread combines
     // its row in place, and the buffer leaves by TMA store; with `sym`, off-diagonal tiles also
     // write a transposed copy that a second TMA store places at the mirrored position.
+    // Before the barrier of sub-tile g the elected thread makes sure that the stores of
+    // sub-tile g-1 (without D: of the one whose buffer sub-tile g+1 will write) have read their
+    // buffers; they have had the arithmetic of sub-tile g to do so.
     const int lane_grp = warp & 3;
     const int row_in_tile = lane_grp * 32 + lane;
     const bool elected = (warp == 2 && lane == 0);
@@ -413,7 +429,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const uint32_t row_off = (uint32_t)(row_in_tile >> 6) * 8192u + (uint32_t)(row_in_tile & 63) * 128u;
     const uint32_t row_sw = (uint32_t)(row_in_tile & 7);
     uint8_t* dc_base = smem + kStages2 * kStageBytes2;
-    uint8_t* t_base = dc_base + kEpiBufs * kEpiBufBytes;
+    uint8_t* t_base = dc_base + kDC * kEpiBufBytes;
 
     // Iterator over the sub-tiles this pair will process, in order (used for the D prefetch).
     int pf_t = first_tile, pf_s = 0;
@@ -438,14 +454,14 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       d_issued = g + 1;
       int b, r0, c0;
       pf_coords(b, r0, c0);
-      const uint32_t buf = g % kEpiBufs;
+      const uint32_t buf = g % kDC;
       uint8_t* dst = dc_base + buf * kEpiBufBytes;
       mbar_expect_tx(&dfull_bar[buf], kEpiBufBytes);
       tma_load_3d(dst, &map_d, &dfull_bar[buf], c0, r0, b);
       tma_load_3d(dst + 8192, &map_d, &dfull_bar[buf], c0, r0 + 64, b);
     };
     if (elected && has_d) {
-      for (uint32_t g0 = 0; g0 < 2 && pf_valid(); ++g0) {
+      for (uint32_t g0 = 0; g0 < kDC - 1 && pf_valid(); ++g0) {
         issue_d(g0);
         pf_advance();
       }
@@ -496,12 +512,12 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll 1
       for (int s = 0; s < nsub; ++s, ++g) {
         const int c0 = tt.y * BN2 + s * kSubCols;
-        const uint32_t buf = g % kEpiBufs;
+        const uint32_t buf = g % kDC;
         uint8_t* dc = dc_base + buf * kEpiBufBytes;
-        uint8_t* tb = t_base + buf * kEpiBufBytes;
+        uint8_t* tb = kT ? t_base + (g % (kT ? kT : 1)) * kEpiBufBytes : nullptr;
         if (has_d && mine_ok) {
           mine_ok = __all_sync(0xffffffffu,
-                               mbar_wait_bounded(&dfull_bar[buf], (g / kEpiBufs) & 1));
+                               mbar_wait_bounded(&dfull_bar[buf], (g / kDC) & 1));
           if (!mine_ok && lane == 0) atomicExch(p.status, kStatusTimeoutFull);
         }
         if (mine_ok) {
@@ -554,7 +570,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
             for (int e = 0; e < 4; ++e) pk[e] = pack_bf16x2(vj[2 * e], vj[2 * e + 1]);
             *cell = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            if (mirror) {
+            if (kT && mirror) {
               // Transposed copy: element (row, c0 + c) goes to row c, column `row` of two
               // 64 x 64 boxes (128-byte swizzled like every other buffer).
               const uint32_t tcol = (uint32_t)(row_in_tile >> 6) * 8192u +
@@ -570,6 +586,15 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             }
           }
           fence_proxy_async();
+        }
+        if (elected) {
+          // (remote: nothing was committed; the barrier that ends a sub-tile freed its buffer)
+          if (has_d || kT) bulk_wait_group_read<0>();
+          else bulk_wait_group_read<kDC - 2>();
+          if (mine_ok && has_d && pf_valid()) {
+            issue_d(g + kDC - 1);
+            pf_advance();
+          }
         }
         // Every epilogue thread reaches this barrier (all waits above are bounded); it also
         // tells whether any of them gave up.
@@ -604,27 +629,18 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               }
             }
           }
-          epi_barrier_plain();   // the buffer has been read: it may take the next D sub-tile
-          if (elected && has_d && pf_valid()) {
-            issue_d(g + 2);
-            pf_advance();
-          }
+          fence_proxy_async();
+          epi_barrier_plain();   // the buffer has been read: it may take another D sub-tile
           continue;
         }
         if (elected) {
           if (row0 < p.M) tma_store_3d(&map_c, dc, c0, row0, b);
           if (row0 + 64 < p.M) tma_store_3d(&map_c, dc + 8192, c0, row0 + 64, b);
-          if (mirror) {
+          if (kT && mirror) {
             if (row0 < p.N) tma_store_3d(&map_c, tb, row0, c0, b);
             if (row0 + 64 < p.N) tma_store_3d(&map_c, tb + 8192, row0 + 64, c0, b);
           }
           bulk_commit_group();
-          // Once the stores have read their buffers, these are free for sub-tile g+2.
-          bulk_wait_group_read_all();
-          if (has_d && pf_valid()) {
-            issue_d(g + 2);
-            pf_advance();
-          }
         }
       }
       aslot ^= 1;
@@ -635,7 +651,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       // After a timeout: let the D copies still in flight land before the CTA exits.
       if (!ok)
         for (uint32_t x = g; x < d_issued; ++x)
-          mbar_wait_bounded(&dfull_bar[x % kEpiBufs], (x / kEpiBufs) & 1);
+          mbar_wait_bounded(&dfull_bar[x % kDC], (x / kDC) & 1);
     }
   }
 
@@ -685,13 +701,13 @@ static int make_map2(CUtensorMap* map, const void* ptr, int batch, int rows, int
   return encode_bf16_3d(enc, map, ptr, dims, strides, box);  // cached when opted in
 }
 
-template <bool A_MN, bool B_MN, int STAGES>
+template <bool A_MN, bool B_MN, class CFG>
 static int launch2(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc,
                    const CUtensorMap& md, const Gemm2Args& args, cudaStream_t stream) {
   static bool configured = false;
   static int max_clusters = 0;
-  auto kernel = ns_gemm2_kernel<A_MN, B_MN, STAGES>;
-  constexpr int kDynBytes2 = dyn_bytes2(STAGES, STAGES == kStagesSym);
+  auto kernel = ns_gemm2_kernel<A_MN, B_MN, CFG>;
+  constexpr int kDynBytes2 = dyn_bytes2<CFG>();
   if (!configured) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynBytes2) !=
         cudaSuccess)
@@ -734,6 +750,18 @@ static int launch2(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorM
     return -4;
   }
   return 0;
+}
+
+template <class CFG>
+static int launch2_mode(int a_mn, int b_mn, const CUtensorMap& ma, const CUtensorMap& mb,
+                        const CUtensorMap& mc, const CUtensorMap& md, const Gemm2Args& args,
+                        cudaStream_t stream) {
+  switch ((a_mn ? 2 : 0) | (b_mn ? 1 : 0)) {
+    case 0: return launch2<false, false, CFG>(ma, mb, mc, md, args, stream);
+    case 1: return launch2<false, true, CFG>(ma, mb, mc, md, args, stream);
+    case 2: return launch2<true, false, CFG>(ma, mb, mc, md, args, stream);
+    default: return launch2<true, true, CFG>(ma, mb, mc, md, args, stream);
+  }
 }
 
 }  // namespace dion
@@ -827,21 +855,9 @@ DION_EXPORT int dion_ns_gemm2_ex(const void* A, long long lda, long long strideA
   a.epi = epi;
   if (epi == kEpiMul2Sqrt && D == nullptr) return -16;
   if (epi == kEpiRelu2 && D != nullptr) return -16;
-  const int mode = (a_mn ? 2 : 0) | (b_mn ? 1 : 0);
-  if (sym) {
-    switch (mode) {
-      case 0: return launch2<false, false, kStagesSym>(ma, mb, mc, md, a, s);
-      case 1: return launch2<false, true, kStagesSym>(ma, mb, mc, md, a, s);
-      case 2: return launch2<true, false, kStagesSym>(ma, mb, mc, md, a, s);
-      default: return launch2<true, true, kStagesSym>(ma, mb, mc, md, a, s);
-    }
-  }
-  switch (mode) {
-    case 0: return launch2<false, false, kStagesPlain>(ma, mb, mc, md, a, s);
-    case 1: return launch2<false, true, kStagesPlain>(ma, mb, mc, md, a, s);
-    case 2: return launch2<true, false, kStagesPlain>(ma, mb, mc, md, a, s);
-    default: return launch2<true, true, kStagesPlain>(ma, mb, mc, md, a, s);
-  }
+  if (sym && D) return launch2_mode<CfgSymD>(a_mn, b_mn, ma, mb, mc, md, a, s);
+  if (sym) return launch2_mode<CfgSym>(a_mn, b_mn, ma, mb, mc, md, a, s);
+  return launch2_mode<CfgPlain>(a_mn, b_mn, ma, mb, mc, md, a, s);
 }
 
 DION_EXPORT int dion_ns_gemm2(const void* A, long long lda, long long strideA, int a_mn,
