@@ -28,13 +28,18 @@ namespace dion {
 constexpr int BM2 = 128;   // rows per CTA (256 per pair)
 constexpr int BN2 = 256;   // columns per pair (128 loaded by each CTA)
 constexpr int BK2 = 64;
-constexpr int kThreads2 = 192;
+constexpr int kEpiGroups = 2;                       // groups of four epilogue warps
+constexpr int kThreads2 = 64 + kEpiGroups * 128;
+// Two groups of four warps drain a tile, each every second 64-column sub-tile through buffers of
+// its own.  One group alone needs 1.2 us per sub-tile (1.8 us with D: TMEM read, arithmetic,
+// shared-memory round trip, barrier, TMA store), 4.7 / 7.2 us a tile, more than the 3.3 us that
+// K = 768 multiplies for; two need 3.6 / 5.3 us (update of 64 matrices 768 x 3072: 256 -> 233 us,
+// 48 x 768^3: 62 -> 54 us, polynomial 64 x 768^3: 72.5 -> 65.7 us; K >= 2048 unchanged).
 // Shared memory is split between operand stages (32 KB), D/C sub-tile buffers and transposed
-// sub-tile buffers (16 KB each).  With two D/C buffers the chain "store has read the buffer -> next
-// D arrives -> combine" bounded a tile at 10 us whatever K was (update of 64 matrices 768 x 3072,
-// K = 768: 324 us).  Four buffers keep three sub-tiles of D in flight while the next tile
-// multiplies, which is worth more than the sixth stage (256 us; K = 2048: 326 -> 321 us, K = 4096
-// unchanged; polynomial at K = 768: 81 -> 72.5 us).
+// sub-tile buffers (16 KB each, half of them for each group).  A buffer is written again only after
+// its store has read it and, with D, the next D has arrived: with D a group has two buffers, so
+// that one D sub-tile is always in flight, at the expense of an operand stage (with two buffers in
+// all, the same update took 324 us).
 //   plain             5 stages + 4 D/C
 //   symmetric, no D   5 stages + 2 D/C + 2 transposed
 //   symmetric, D      4 stages + 4 D/C + 2 transposed
@@ -103,9 +108,9 @@ __device__ __forceinline__ float ld_volatile_f32_2(const float* p) {
   asm volatile("ld.volatile.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
   return v;
 }
-// Barrier over the 128 epilogue threads without a predicate (barrier 2).
-__device__ __forceinline__ void epi_barrier_plain() {
-  asm volatile("barrier.cta.sync.aligned 2, 128;" ::: "memory");
+// Barrier over the 128 threads of an epilogue group without a predicate (barriers 3 and 4).
+__device__ __forceinline__ void epi_barrier_plain(int group) {
+  asm volatile("barrier.cta.sync.aligned %0, 128;" ::"r"(3 + group) : "memory");
 }
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -220,18 +225,18 @@ __device__ __forceinline__ void bulk_wait_group_read() {
 __device__ __forceinline__ void bulk_wait_group_all() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
-// Barrier over the 128 epilogue threads (barrier 1) that also ANDs a predicate.
-__device__ __forceinline__ bool epi_barrier_and(bool mine) {
+// Barrier over the 128 threads of an epilogue group (barriers 1 and 2) that also ANDs a predicate.
+__device__ __forceinline__ bool epi_barrier_and(int group, bool mine) {
   uint32_t out;
   asm volatile(
       "{\n"
       ".reg .pred p, q;\n"
       "setp.ne.u32 q, %1, 0;\n"
-      "barrier.cta.red.and.pred.aligned p, 1, 128, q;\n"
+      "barrier.cta.red.and.pred.aligned p, %2, 128, q;\n"
       "selp.u32 %0, 1, 0, p;\n"
       "}\n"
       : "=r"(out)
-      : "r"((uint32_t)mine)
+      : "r"((uint32_t)mine), "r"(1 + group)
       : "memory");
   return out != 0;
 }
@@ -247,7 +252,9 @@ __global__ void __launch_bounds__(kThreads2, 1)
 ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                 const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_d,
                 const Gemm2Args p) {
-  constexpr int kStages2 = CFG::kStages, kDC = CFG::kDC, kT = CFG::kT;
+  constexpr int kStages2 = CFG::kStages, kDC = CFG::kDC;
+  constexpr int kGDC = CFG::kDC / kEpiGroups, kGT = CFG::kT / kEpiGroups;  // buffers per group
+  constexpr bool kSingle = kGT == 1 || kGDC == 1;   // a buffer is written by every sub-tile
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -272,7 +279,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 8);  // four epilogue warps in each CTA of the pair
+      mbar_init(&tempty_bar[a], 8 * kEpiGroups);  // every epilogue warp of both CTAs
     }
     for (int a = 0; a < kDC; ++a) mbar_init(&dfull_bar[a], 1);
     fence_barrier_init();
@@ -414,25 +421,34 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   } else {
     // ------------------------------ epilogue (both CTAs) ----------------------------------
-    // The 128 x 256 half-tile of this CTA is drained in sub-tiles of 64 columns.  D arrives by
-    // TMA into a shared-memory buffer (prefetched kDC - 1 sub-tiles ahead), each thread combines
-    // its row in place, and the buffer leaves by TMA store; with `sym`, off-diagonal tiles also
-    // write a transposed copy that a second TMA store places at the mirrored position.
-    // Before the barrier of sub-tile g the elected thread makes sure that the stores of
-    // sub-tile g-1 (without D: of the one whose buffer sub-tile g+1 will write) have read their
-    // buffers; they have had the arithmetic of sub-tile g to do so.
+    // The 128 x 256 half-tile of this CTA is drained in sub-tiles of 64 columns, alternately by
+    // the two groups of warps.  D arrives by TMA into a shared-memory buffer (prefetched), each
+    // thread combines its row in place, and the buffer leaves by TMA store; with `sym`,
+    // off-diagonal tiles also write a transposed copy that a second TMA store places at the
+    // mirrored position.  g counts the sub-tiles of this group.
+    const int grp = (warp - 2) >> 2;
     const int lane_grp = warp & 3;
     const int row_in_tile = lane_grp * 32 + lane;
-    const bool elected = (warp == 2 && lane == 0);
+    const bool elected = (warp == 2 + 4 * grp && lane == 0);
     const bool has_d = p.D != nullptr;
     const int epi = p.epi;
     const uint32_t row_off = (uint32_t)(row_in_tile >> 6) * 8192u + (uint32_t)(row_in_tile & 63) * 128u;
     const uint32_t row_sw = (uint32_t)(row_in_tile & 7);
-    uint8_t* dc_base = smem + kStages2 * kStageBytes2;
-    uint8_t* t_base = dc_base + kDC * kEpiBufBytes;
+    uint8_t* dc_base = smem + kStages2 * kStageBytes2 + grp * kGDC * kEpiBufBytes;
+    uint8_t* t_base = smem + kStages2 * kStageBytes2 + kDC * kEpiBufBytes + grp * kGT * kEpiBufBytes;
+    uint64_t* dfull = dfull_bar + grp * kGDC;
 
-    // Iterator over the sub-tiles this pair will process, in order (used for the D prefetch).
-    int pf_t = first_tile, pf_s = 0;
+    // Iterator over the sub-tiles this group will process, in order (used for the D prefetch).
+    // Only the last column of tiles can be narrower than 256 columns.
+    int pf_t = first_tile, pf_s = grp;
+    auto pf_skip = [&]() {   // to the next sub-tile of this group that exists
+      while (pf_t < p.total_tiles) {
+        const int2 tt = p.tiles[pf_t % p.tiles_per_mat];
+        if (pf_s < 4 && tt.y * BN2 + pf_s * kSubCols < p.N) break;
+        pf_s = grp;
+        pf_t += tile_step;
+      }
+    };
     auto pf_valid = [&]() { return pf_t < p.total_tiles; };
     auto pf_coords = [&](int& b, int& r0, int& c0) {
       b = pf_t / p.tiles_per_mat;
@@ -441,38 +457,34 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       c0 = tt.y * BN2 + pf_s * kSubCols;
     };
     auto pf_advance = [&]() {
-      const int b = pf_t / p.tiles_per_mat;
-      const int2 tt = p.tiles[pf_t - b * p.tiles_per_mat];
-      ++pf_s;
-      if (pf_s >= 4 || tt.y * BN2 + pf_s * kSubCols >= p.N) {
-        pf_s = 0;
-        pf_t += tile_step;
-      }
+      pf_s += kEpiGroups;
+      pf_skip();
     };
+    if (elected && has_d) pf_skip();
     uint32_t d_issued = 0;  // D sub-tiles requested so far (elected thread)
     auto issue_d = [&](uint32_t g) {
       d_issued = g + 1;
       int b, r0, c0;
       pf_coords(b, r0, c0);
-      const uint32_t buf = g % kDC;
+      const uint32_t buf = g % kGDC;
       uint8_t* dst = dc_base + buf * kEpiBufBytes;
-      mbar_expect_tx(&dfull_bar[buf], kEpiBufBytes);
-      tma_load_3d(dst, &map_d, &dfull_bar[buf], c0, r0, b);
-      tma_load_3d(dst + 8192, &map_d, &dfull_bar[buf], c0, r0 + 64, b);
+      mbar_expect_tx(&dfull[buf], kEpiBufBytes);
+      tma_load_3d(dst, &map_d, &dfull[buf], c0, r0, b);
+      tma_load_3d(dst + 8192, &map_d, &dfull[buf], c0, r0 + 64, b);
     };
     if (elected && has_d) {
-      for (uint32_t g0 = 0; g0 < kDC - 1 && pf_valid(); ++g0) {
+      for (uint32_t g0 = 0; g0 < kGDC && pf_valid(); ++g0) {
         issue_d(g0);
         pf_advance();
       }
     }
 
     uint32_t aslot = 0, aphase = 0;
-    uint32_t g = 0;  // running sub-tile count
+    uint32_t g = 0;  // running sub-tile count of this group
     bool ok = true;
     bool all_sources_ready = false;
     const bool remote = p.remote_c[0] != 0;
-    const int epi_tid = (warp - 2) * 32 + lane;   // 0..127
+    const int epi_tid = ((warp - 2) & 3) * 32 + lane;   // 0..127
     for (int t = first_tile; t < p.total_tiles && ok; t += tile_step) {
       const int b = t / p.tiles_per_mat;
       const int2 tt = p.tiles[t - b * p.tiles_per_mat];
@@ -509,35 +521,53 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const bool mirror = p.sym && tt.y > tt.x;
       int nsub = (p.N - tt.y * BN2 + kSubCols - 1) / kSubCols;
       nsub = nsub > 4 ? 4 : nsub;
+      // After this group's last read of the accumulator: hand the TMEM slot back to the MMA thread.
+      auto release_accumulator = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[aslot]), 0));
+      };
+      if (grp >= nsub && mine_ok) release_accumulator();   // a narrow tile: nothing to drain here
+      if (grp >= nsub) ok = epi_barrier_and(grp, mine_ok);
 #pragma unroll 1
-      for (int s = 0; s < nsub; ++s, ++g) {
+      for (int s = grp; s < nsub; s += kEpiGroups, ++g) {
         const int c0 = tt.y * BN2 + s * kSubCols;
-        const uint32_t buf = g % kDC;
+        const uint32_t buf = g % kGDC;
         uint8_t* dc = dc_base + buf * kEpiBufBytes;
-        uint8_t* tb = kT ? t_base + (g % (kT ? kT : 1)) * kEpiBufBytes : nullptr;
+        uint8_t* tb = kGT ? t_base + (g % (kGT ? kGT : 1)) * kEpiBufBytes : nullptr;
+        if (elected && (has_d || kSingle)) {
+          // The stores of sub-tile g-1 have read their buffers: the next D may land there.
+          bulk_wait_group_read<0>();
+          if (mine_ok && has_d && g > 0 && pf_valid()) {
+            issue_d(g + kGDC - 1);
+            pf_advance();
+          }
+        }
         if (has_d && mine_ok) {
           mine_ok = __all_sync(0xffffffffu,
-                               mbar_wait_bounded(&dfull_bar[buf], (g / kDC) & 1));
+                               mbar_wait_bounded(&dfull[buf], (g / kGDC) & 1));
           if (!mine_ok && lane == 0) atomicExch(p.status, kStatusTimeoutFull);
         }
+        // 32 columns at a time: 64 accumulators in registers would spill at 320 threads.
+        float v[32];
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(lane_grp * 32) << 16) +
+                               aslot * BN2 + s * kSubCols;
         if (mine_ok) {
-          float v[kSubCols];
-          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(lane_grp * 32) << 16) +
-                                 aslot * BN2 + s * kSubCols;
           tmem_ld_32x32(taddr, v);
-          tmem_ld_32x32(taddr + 32, v + 32);
           tmem_ld_wait();
-          if (s == nsub - 1) {
-            // Last read of this accumulator: hand the TMEM slot back to the MMA thread.
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[aslot]), 0));
-          }
+        }
+        if (kSingle) epi_barrier_plain(grp);   // ... and so may this sub-tile
+        if (mine_ok) {
           uint8_t* rowp = dc + row_off;
 #pragma unroll
           for (int j = 0; j < kSubCols / 8; ++j) {
+            if (j == 4) {
+              tmem_ld_32x32(taddr + 32, v);
+              tmem_ld_wait();
+              if (s + kEpiGroups >= nsub) release_accumulator();
+            }
             uint4* cell = reinterpret_cast<uint4*>(rowp + (((uint32_t)j ^ row_sw) << 4));
-            float* vj = v + j * 8;
+            float* vj = v + (j & 3) * 8;
             if (has_d) {
               const uint4 u = *cell;
               const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -570,7 +600,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
             for (int e = 0; e < 4; ++e) pk[e] = pack_bf16x2(vj[2 * e], vj[2 * e + 1]);
             *cell = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            if (kT && mirror) {
+            if (kGT && mirror) {
               // Transposed copy: element (row, c0 + c) goes to row c, column `row` of two
               // 64 x 64 boxes (128-byte swizzled like every other buffer).
               const uint32_t tcol = (uint32_t)(row_in_tile >> 6) * 8192u +
@@ -587,18 +617,11 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           }
           fence_proxy_async();
         }
-        if (elected) {
-          // (remote: nothing was committed; the barrier that ends a sub-tile freed its buffer)
-          if (has_d || kT) bulk_wait_group_read<0>();
-          else bulk_wait_group_read<kDC - 2>();
-          if (mine_ok && has_d && pf_valid()) {
-            issue_d(g + kDC - 1);
-            pf_advance();
-          }
-        }
+        // Two buffers and no D: sub-tile g+1 overwrites what the store of g-1 reads.
+        if (elected && !has_d && !kSingle) bulk_wait_group_read<0>();
         // Every epilogue thread reaches this barrier (all waits above are bounded); it also
         // tells whether any of them gave up.
-        ok = epi_barrier_and(mine_ok);
+        ok = epi_barrier_and(grp, mine_ok);
         if (!ok) break;
         if (remote) {
           // Rows leave for the ranks that own them: 16-byte stores over NVLink, eight
@@ -630,13 +653,13 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             }
           }
           fence_proxy_async();
-          epi_barrier_plain();   // the buffer has been read: it may take another D sub-tile
+          epi_barrier_plain(grp);   // the buffer has been read: it may take another D sub-tile
           continue;
         }
         if (elected) {
           if (row0 < p.M) tma_store_3d(&map_c, dc, c0, row0, b);
           if (row0 + 64 < p.M) tma_store_3d(&map_c, dc + 8192, c0, row0 + 64, b);
-          if (kT && mirror) {
+          if (kGT && mirror) {
             if (row0 < p.N) tma_store_3d(&map_c, tb, row0, c0, b);
             if (row0 + 64 < p.N) tma_store_3d(&map_c, tb + 8192, row0 + 64, c0, b);
           }
@@ -651,7 +674,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       // After a timeout: let the D copies still in flight land before the CTA exits.
       if (!ok)
         for (uint32_t x = g; x < d_issued; ++x)
-          mbar_wait_bounded(&dfull_bar[x % kDC], (x / kDC) & 1);
+          mbar_wait_bounded(&dfull[x % kGDC], (x / kGDC) & 1);
     }
   }
 

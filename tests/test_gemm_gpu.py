@@ -128,6 +128,26 @@ def test_pair_symmetric(shape):
     assert (C - C.mT).abs().max().item() == 0.0
 
 
+@pytest.mark.parametrize("sym", [False, True])
+@pytest.mark.parametrize("n", [256 + 8, 256 + 64, 256 + 72, 256 + 192, 512 + 136])
+def test_pair_narrow_last_tile(n, sym):
+    """Last tile of 1 to 4 epilogue sub-tiles (the second group of warps may have none), more tiles
+    than CTA pairs, with an addend.  bf16 output of fp32 sums: half an ulp (2^-9) of the value."""
+    from dion_b200.ops import gemm
+    torch.manual_seed(3)
+    b, K = 40, 104
+    X = torch.randn(b, n, K, device="cuda").bfloat16()
+    Y = X if sym else torch.randn(b, 384, K, device="cuda").bfloat16()
+    D = torch.randn(b, Y.size(1), n, device="cuda").bfloat16()
+    if sym:
+        D = (D + D.mT).contiguous()
+    C = gemm.ns_gemm(Y, X, D=D, alpha=0.25, beta=-1.5, sym=sym, pair=True)
+    torch.cuda.synchronize()
+    gemm.check_status()
+    ref = 0.25 * (Y.float() @ X.float().mT) - 1.5 * D.float()
+    assert _rel_err(C, ref) < 2.0 ** -8
+
+
 def test_pair_km_a_operand():
     """A given as [K, M] (tall Gram matrix X^T X without a transposed copy)."""
     from dion_b200.ops import gemm
