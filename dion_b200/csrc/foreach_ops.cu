@@ -808,6 +808,50 @@ sumsq_kernel(const __nv_bfloat16* X, long long numel, float* out) {
   if (threadIdx.x == 0) atomicAdd(&out[t], s);
 }
 
+// Newton-Schulz input of a dense fp32 or bf16 batch G [B][m][n]: rounded to bf16 into
+// X [B][mp][np] (mp >= m, np >= n multiples of 8, the padding zero), and the squares of the rounded
+// values added to ss[b].  One pass, bound by memory; it stands for a cast, a zero fill, a strided
+// copy and a norm pass (6 x 997 x 1531 fp32: 41 -> 9 us).
+__global__ void __launch_bounds__(kThreads)
+ns_prepare_kernel(const void* G, int g_dt, int m, int n, __nv_bfloat16* X, int mp, int np,
+                  float* ss) {
+  const int b = blockIdx.y;
+  const long long per = (long long)mp * np;
+  const long long gofs = (long long)b * m * n;
+  __nv_bfloat16* x = X + (long long)b * per;
+  const bool vec = (n & 7) == 0 && aligned16(G);
+  float acc = 0.f;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const long long i = (long long)blockIdx.x * kChunk + h * (kThreads * 8) + threadIdx.x * 8;
+    if (i >= per) continue;
+    const int r = (int)(i / np), c = (int)(i - (long long)r * np);
+    const long long g = gofs + (long long)r * n + c;
+    float v[8];
+    if (r < m && vec && c < n) {
+      if (g_dt == DT_BF16) {
+        ld8b(G, g, v);
+      } else {
+        const float4 a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(G) + g);
+        const float4 d = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(G) + g + 4);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = d.x; v[5] = d.y; v[6] = d.z; v[7] = d.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = (r < m && c + k < n) ? ld(G, g_dt, g + k) : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      v[k] = round_to(v[k], DT_BF16);
+      acc += v[k] * v[k];
+    }
+    st8b(x, i, v);
+  }
+  const float s = block_sum(acc);
+  if (threadIdx.x == 0) atomicAdd(&ss[b], s);
+}
+
 // scale[t] = 1 / (sqrt(sumsq[t]) * mult + eps)
 __global__ void finalize_scale_kernel(const float* sumsq, float* scale, int n, float mult,
                                       float eps) {
@@ -974,6 +1018,19 @@ DION_EXPORT int dion_sumsq(const void* X, int n, long long numel, float* out, vo
   if (n <= 0 || numel <= 0) return 0;
   dim3 grid((unsigned)((numel + kChunk - 1) / kChunk), (unsigned)n);
   sumsq_kernel<<<grid, kThreads, 0, S(stream)>>>(static_cast<const __nv_bfloat16*>(X), numel, out);
+  return rc();
+}
+
+// G: dense [batch, m, n] fp32 (0) or bf16 (1); X: bf16 [batch, mp, np], 16-byte aligned, mp and np
+// multiples of 8; ss: fp32 [batch], accumulated into.
+DION_EXPORT int dion_ns_prepare(const void* G, int g_dt, int batch, int m, int n, void* X, int mp,
+                                int np, float* ss, void* stream) {
+  if (batch <= 0 || m <= 0 || n <= 0) return 0;
+  if (mp < m || np < n || (np & 7) || batch > 65535 || (reinterpret_cast<uintptr_t>(X) & 15))
+    return -2;
+  dim3 grid((unsigned)(((long long)mp * np + kChunk - 1) / kChunk), (unsigned)batch);
+  ns_prepare_kernel<<<grid, kThreads, 0, S(stream)>>>(G, g_dt, m, n,
+                                                      static_cast<__nv_bfloat16*>(X), mp, np, ss);
   return rc();
 }
 

@@ -900,11 +900,12 @@ DION_EXPORT int dion_ns_gemm2(const void* A, long long lda, long long strideA, i
 //   B  = b * A + c * A A        symmetric
 //   X' = s * (a * X + B X)      (X B for tall matrices)
 // with the input scale s applied in the first iteration only, ping-ponging between the buffers
-// X and Xalt.  All operands are dense [batch, rows, cols] bf16.  The result of the last
-// iteration lies in Xalt when `iters` is odd, else in X.  This only saves the host the 3 * iters
+// X (X2 from the second iteration on, when given: X is then only read) and Xalt.  All operands are
+// dense [batch, rows, cols] bf16.  The result of the last
+// iteration lies in Xalt when `iters` is odd, else in X (X2).  This only saves the host the 3 * iters
 // trips through the Python front end; the launches are the same as issued one by one.
-DION_EXPORT int dion_ns_iterate2(void* X, void* Xalt, void* A, void* Bm, int batch, int m, int n,
-                                 const float* coeffs, int iters, const float* scale,
+DION_EXPORT int dion_ns_iterate2(void* X, void* Xalt, void* X2, void* A, void* Bm, int batch, int m,
+                                 int n, const float* coeffs, int iters, const float* scale,
                                  const void* tiles_gg, int n_tiles_gg, const void* tiles_mn,
                                  int n_tiles_mn, int* status, void* stream) {
   const int tall = m > n;
@@ -932,7 +933,7 @@ DION_EXPORT int dion_ns_iterate2(void* X, void* Xalt, void* A, void* Bm, int bat
                          sc, p1, p1, 0, tiles_mn, n_tiles_mn, 0, status, stream);
     }
     if (rc != 0) return rc;
-    void* t = cur; cur = nxt; nxt = t;
+    void* t = cur; cur = nxt; nxt = it == 0 && X2 != nullptr ? X2 : t;
   }
   return 0;
 }

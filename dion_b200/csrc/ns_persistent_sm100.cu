@@ -47,8 +47,8 @@ struct PersistArgs {
   Phase ph[kMaxPhases];
   int n_phases;
   int batch;
-  __nv_bfloat16* buf[4];       // X, Xalt, A, Bm
-  long long ld[4], stride[4];
+  __nv_bfloat16* buf[5];       // X, Xalt, A, Bm, X2
+  long long ld[5], stride[5];
   const int2* tiles;
   const float* scale;          // one fp32 per matrix or nullptr
   unsigned int* counter;       // grid barrier, zero at launch; left at zero
@@ -422,14 +422,15 @@ static int make_map_p(CUtensorMap* map, const void* ptr, int batch, int rows, in
 }  // namespace dion
 
 // All iterations (a, b, c) = coeffs[3*i .. 3*i+2] of the Newton-Schulz loop on the dense bf16 batch
-// X [batch, m, n] in one cooperative launch.  Xalt [batch, m, n], A and Bm [batch, g, g]
+// X [batch, m, n] in one cooperative launch.  Xalt and X2 [batch, m, n], A and Bm [batch, g, g]
 // (g = min(m, n)) are work buffers; `counter` points to two zero-initialised unsigned ints in
 // device memory that the kernel leaves at zero.  tiles_all: (tile_m, tile_n) pairs in units of
 // 128 x 128, first the n_tiles_gg tiles on or above the diagonal of the symmetric g x g products,
-// then the n_tiles_mn tiles of the m x n update.  The result lies in Xalt when `iters` is odd, else in X.  Returns 0 on success,
+// then the n_tiles_mn tiles of the m x n update.  The result lies in Xalt when
+// `iters` is odd, else in X, or in X2 where that is given (X is then only read).  Returns 0 on success,
 // -20 when the grid cannot be co-resident (the caller then uses the per-GEMM launches).
-DION_EXPORT int dion_ns_persistent(void* X, void* Xalt, void* A, void* Bm, int batch, int m, int n,
-                                   const float* coeffs, int iters, const float* scale,
+DION_EXPORT int dion_ns_persistent(void* X, void* Xalt, void* X2, void* A, void* Bm, int batch, int m,
+                                   int n, const float* coeffs, int iters, const float* scale,
                                    const void* tiles_all, int n_tiles_gg, int n_tiles_mn,
                                    unsigned int* counter, int num_sms, int* status,
                                    void* stream) {
@@ -437,26 +438,29 @@ DION_EXPORT int dion_ns_persistent(void* X, void* Xalt, void* A, void* Bm, int b
   if (batch <= 0 || m <= 0 || n <= 0 || iters <= 0) return 0;
   if (3 * iters > kMaxPhases) return -10;
   if ((m & 7) || (n & 7)) return -10;
-  for (void* ptr : {X, Xalt, A, Bm})
+  for (void* ptr : {X, Xalt, X2, A, Bm})
     if (reinterpret_cast<uintptr_t>(ptr) & 15) return -10;
   const int tall = m > n;
   const int g = tall ? n : m;
   PersistArgs a;
-  // maps: 0 X K-major, 1 X MN-major, 2 Xalt K-major, 3 Xalt MN-major, 4 A K-major, 5 Bm K-major
+  // maps: 0 X K-major, 1 X MN-major, 2 Xalt K-major, 3 Xalt MN-major, 4 A K-major, 5 Bm K-major,
+  // 6 X2 K-major, 7 X2 MN-major
   if (make_map_p(&a.maps[0], X, batch, m, n, PBK, PBM) != 0) return -12;
   if (make_map_p(&a.maps[1], X, batch, m, n, 64, PBK) != 0) return -12;
   if (make_map_p(&a.maps[2], Xalt, batch, m, n, PBK, PBM) != 0) return -12;
   if (make_map_p(&a.maps[3], Xalt, batch, m, n, 64, PBK) != 0) return -12;
   if (make_map_p(&a.maps[4], A, batch, g, g, PBK, PBM) != 0) return -12;
   if (make_map_p(&a.maps[5], Bm, batch, g, g, PBK, PBM) != 0) return -12;
-  a.maps[6] = a.maps[0];
-  a.maps[7] = a.maps[0];
+  if (X2 == nullptr) X2 = X;
+  if (make_map_p(&a.maps[6], X2, batch, m, n, PBK, PBM) != 0) return -12;
+  if (make_map_p(&a.maps[7], X2, batch, m, n, 64, PBK) != 0) return -12;
   a.buf[0] = static_cast<__nv_bfloat16*>(X);
   a.buf[1] = static_cast<__nv_bfloat16*>(Xalt);
   a.buf[2] = static_cast<__nv_bfloat16*>(A);
   a.buf[3] = static_cast<__nv_bfloat16*>(Bm);
-  a.ld[0] = a.ld[1] = n;
-  a.stride[0] = a.stride[1] = (long long)m * n;
+  a.buf[4] = static_cast<__nv_bfloat16*>(X2);
+  a.ld[0] = a.ld[1] = a.ld[4] = n;
+  a.stride[0] = a.stride[1] = a.stride[4] = (long long)m * n;
   a.ld[2] = a.ld[3] = g;
   a.stride[2] = a.stride[3] = (long long)g * g;
   a.batch = batch;
@@ -468,16 +472,18 @@ DION_EXPORT int dion_ns_persistent(void* X, void* Xalt, void* A, void* Bm, int b
   int max_tiles = 0;
   for (int it = 0; it < iters; ++it) {
     const float ca = coeffs[3 * it], cb = coeffs[3 * it + 1], cc = coeffs[3 * it + 2];
-    const int cur = it & 1, nxt = cur ^ 1;   // buffer index of X / X'
+    // buffer index of X and X': 0 -> 1 -> 4 -> 1 ...; their K-major maps (the MN-major one follows)
+    const int cur = it == 0 ? 0 : (it & 1) ? 1 : 4, nxt = (it & 1) ? 4 : 1;
+    const int cur_map = cur == 0 ? 0 : cur == 1 ? 2 : 6;
     const int p2 = (it == 0 && scale) ? 2 : 0, p1 = (it == 0 && scale) ? 1 : 0;
     Phase& gram = a.ph[3 * it];
     gram = Phase{};
     if (!tall) {  // X [g, K=n] against itself
-      gram.map_a = gram.map_b = cur == 0 ? 0 : 2;
+      gram.map_a = gram.map_b = cur_map;
       gram.a_mn = gram.b_mn = 0;
       gram.K = n;
     } else {      // X read as [K=m, g] on both sides
-      gram.map_a = gram.map_b = cur == 0 ? 1 : 3;
+      gram.map_a = gram.map_b = cur_map + 1;
       gram.a_mn = gram.b_mn = 1;
       gram.K = m;
     }
@@ -499,9 +505,9 @@ DION_EXPORT int dion_ns_persistent(void* X, void* Xalt, void* A, void* Bm, int b
     upd = Phase{};
     if (!tall) {  // X' = a X + B X, X given as [K, N]
       upd.map_a = 5; upd.a_mn = 0;
-      upd.map_b = cur == 0 ? 1 : 3; upd.b_mn = 1;
+      upd.map_b = cur_map + 1; upd.b_mn = 1;
     } else {      // X' = a X + X B, B symmetric: given as [N, K]
-      upd.map_a = cur == 0 ? 0 : 2; upd.a_mn = 0;
+      upd.map_a = cur_map; upd.a_mn = 0;
       upd.map_b = 5; upd.b_mn = 0;
     }
     upd.M = m; upd.N = n; upd.K = g;

@@ -303,12 +303,12 @@ topk_select_kernel(const float* norms, int num, int k, long long* idx_out, int* 
 // Row gather + error feedback.  grid = (k, n); U[t][j][:] = bf16(M[t][idx[j]][:]);
 // M[t][idx[j]][:] *= ef (skipped when ef_apply == 0).  M pointers from ptrs[n + t].
 // With u_ptrs the destination of matrix t is u_ptrs[t] (possibly another GPU's peer-mapped
-// memory) instead of U + t*u_stride; with ss_ptrs the sum of squares of the bf16 values of each
-// gathered row is added to *ss_ptrs[t].
+// memory) instead of U + t*u_stride; with ss_ptrs (ss) the sum of squares of the bf16 values of
+// each gathered row is added to *ss_ptrs[t] (ss[t]).
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const long long* ptrs, int n, int cols, int m_dt, const long long* idx, int k,
                    __nv_bfloat16* U, long long u_stride, float ef, int ef_apply,
-                   const long long* u_ptrs, const long long* ss_ptrs) {
+                   const long long* u_ptrs, const long long* ss_ptrs, float* ss) {
   __shared__ float red[8];
   const int j = blockIdx.x, t = blockIdx.y;
   void* M = reinterpret_cast<void*>(ptrs[n + t]);
@@ -344,35 +344,50 @@ gather_rows_kernel(const long long* ptrs, int n, int cols, int m_dt, const long 
       if (ef_apply) stv(M, m_dt, off + c, m * ef);
     }
   }
-  if (ss_ptrs) {
+  if (ss_ptrs || ss) {
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
       float s = 0.f;
       for (int w = 0; w < 8; ++w) s += red[w];
-      atomicAdd(reinterpret_cast<float*>(ss_ptrs[t]), s);
+      atomicAdd(ss ? ss + t : reinterpret_cast<float*>(ss_ptrs[t]), s);
     }
   }
 }
 
-// Column gather: U[t][r][j] = bf16(M[t][r][idx[j]]); M *= ef at the selected columns.
+// Column gather: U[t][r][j] = bf16(M[t][r][idx[j]]); M *= ef at the selected columns; with ss the
+// squares of the gathered bf16 values are added to ss[t].
 // grid = (ceil(rows/8), n); 256 threads = 8 rows x 32 column lanes.
 __global__ void __launch_bounds__(256)
 gather_cols_kernel(const long long* ptrs, int n, int rows, int cols, int m_dt,
                    const long long* idx, int k, __nv_bfloat16* U, long long u_stride, float ef,
-                   int ef_apply) {
+                   int ef_apply, float* ss) {
+  __shared__ float red[8];
   const int t = blockIdx.y;
   const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (r >= rows) return;
   void* M = reinterpret_cast<void*>(ptrs[n + t]);
   const long long* id = idx + (long long)t * k;
   __nv_bfloat16* u = U + (long long)t * u_stride + (long long)r * k;
-  for (int j = threadIdx.x & 31; j < k; j += 32) {
+  float acc = 0.f;
+  for (int j = threadIdx.x & 31; j < k && r < rows; j += 32) {
     const long long e = (long long)r * cols + id[j];
     const float m = ldv(M, m_dt, e);
-    u[j] = __float2bfloat16_rn(m);
+    const __nv_bfloat16 b = __float2bfloat16_rn(m);
+    u[j] = b;
+    const float f = __bfloat162float(b);
+    acc += f * f;
     if (ef_apply) stv(M, m_dt, e, m * ef);
+  }
+  if (ss) {
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float s = 0.f;
+      for (int w = 0; w < 8; ++w) s += red[w];
+      atomicAdd(&ss[t], s);
+    }
   }
 }
 
@@ -426,21 +441,21 @@ DION_EXPORT int dion_topk_select(const float* norms, int n, int num, int k, long
 DION_EXPORT int dion_gather_ef(const void* ptrs, int n, int rows, int cols, int m_dt,
                                const long long* idx, int k, int select_rows, void* U,
                                long long u_stride, float ef, int ef_apply, const void* u_ptrs,
-                               const void* ss_ptrs, void* stream) {
+                               const void* ss_ptrs, float* ss, void* stream) {
   if (n <= 0 || k <= 0) return 0;
   if (select_rows) {
     dim3 grid(k, n);
     gather_rows_kernel<<<grid, 256, 0, S(stream)>>>(
         static_cast<const long long*>(ptrs), n, cols, m_dt, idx, k,
         static_cast<__nv_bfloat16*>(U), u_stride, ef, ef_apply,
-        static_cast<const long long*>(u_ptrs), static_cast<const long long*>(ss_ptrs));
+        static_cast<const long long*>(u_ptrs), static_cast<const long long*>(ss_ptrs), ss);
   } else {
     if (u_ptrs != nullptr || ss_ptrs != nullptr) return -3;
     dim3 grid((rows + 7) / 8, n);
     gather_cols_kernel<<<grid, 256, 0, S(stream)>>>(static_cast<const long long*>(ptrs), n, rows,
                                                     cols, m_dt, idx, k,
                                                     static_cast<__nv_bfloat16*>(U), u_stride, ef,
-                                                    ef_apply);
+                                                    ef_apply, ss);
   }
   return rc();
 }

@@ -512,6 +512,20 @@ def sumsq(X: Tensor, out: Optional[Tensor] = None) -> Tensor:
     return out
 
 
+def ns_prepare(G: Tensor, mp: int, np_: int) -> Tuple[Tensor, Tensor]:
+    """``(X, ss)`` of a dense CUDA batch ``G [B, m, n]`` (fp32 or bf16): ``X [B, mp, np_]`` is ``G``
+    rounded to bf16 with zeros beyond it, ``ss [B]`` the fp32 sums of squares of ``X``."""
+    B, m, n = G.shape
+    X = torch.empty((B, mp, np_), dtype=torch.bfloat16, device=G.device)
+    ss = torch.zeros(B, dtype=torch.float32, device=G.device)
+    _check(
+        _backend.lib("foreach_ops").dion_ns_prepare(
+            _c(G.data_ptr()), _DT[G.dtype], B, m, n, _c(X.data_ptr()), mp, np_, _c(ss.data_ptr()),
+            _stream(G.device)),
+        "dion_ns_prepare")
+    return X, ss
+
+
 def aol_rescale_(X: Tensor, A: Tensor, eps: float) -> None:
     """AOL rescaling in place: with ``s_i = rsqrt(max(sum_j |A_ij|, eps))`` of the Gram matrix
     ``A = X X^T`` (``[B, m, m]``), ``X <- diag(s) X`` and ``A <- diag(s) A diag(s)``

@@ -368,12 +368,13 @@ def iterate_in_one_call(X: Tensor, batch: int, m: int, n: int) -> bool:
             and _choose_config(m, n, g, batch, False, True, dev)[0])
 
 
-def ns_iterate(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs, scale: Optional[Tensor]
-               ) -> Tensor:
+def ns_iterate(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs, scale: Optional[Tensor],
+               X2: Optional[Tensor] = None) -> Tensor:
     """All iterations ``(a, b, c) in coeffs`` of ``X <- aX + (bA + cA^2)X`` with ``A = X X^T``
     (right-multiplied forms for tall ``X``) issued by one call into the library; ``scale`` (one
-    fp32 per matrix) normalizes the input inside the first iteration.  ``X`` is overwritten;
-    returns whichever of ``X`` / ``Xalt`` holds the result."""
+    fp32 per matrix) normalizes the input inside the first iteration.  ``X`` is overwritten unless
+    ``X2`` takes its place from the second iteration on; returns whichever of ``X`` (``X2``) /
+    ``Xalt`` holds the result."""
     batch, m, n = X.shape
     dev = X.device
     g = min(m, n)
@@ -384,14 +385,14 @@ def ns_iterate(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs, scale: Op
         assert scale.dtype == torch.float32 and scale.numel() >= batch
     st = status_tensor(dev)
     rc = _backend.lib("ns_gemm2_sm100").dion_ns_iterate2(
-        _p(X), _p(Xalt), _p(A), _p(Bm), ctypes.c_int(batch), ctypes.c_int(m), ctypes.c_int(n),
-        flat, ctypes.c_int(len(coeffs)), _p(scale), _p(tiles_gg), ctypes.c_int(tiles_gg.size(0)),
+        _p(X), _p(Xalt), _p(X2), _p(A), _p(Bm), ctypes.c_int(batch), ctypes.c_int(m),
+        ctypes.c_int(n), flat, ctypes.c_int(len(coeffs)), _p(scale), _p(tiles_gg), ctypes.c_int(tiles_gg.size(0)),
         _p(tiles_mn), ctypes.c_int(tiles_mn.size(0)), _p(st),
         ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
     if rc != 0:
         raise RuntimeError(f"dion_ns_iterate2 failed with code {rc}")
     _backend.add_launches(3 * len(coeffs))
-    return Xalt if len(coeffs) % 2 else X
+    return Xalt if len(coeffs) % 2 else (X if X2 is None else X2)
 
 
 _persist_tiles: Dict[Tuple, Tensor] = {}
@@ -435,10 +436,11 @@ def persistent_fits(X: Tensor, batch: int, m: int, n: int, iters: int) -> bool:
 
 
 def ns_persistent(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs,
-                  scale: Optional[Tensor]) -> Optional[Tensor]:
+                  scale: Optional[Tensor], X2: Optional[Tensor] = None) -> Optional[Tensor]:
     """All iterations in one cooperative launch (csrc/ns_persistent_sm100.cu).  Returns the
     buffer that holds the result, or None when the launch could not be made co-resident (the
-    caller falls back to per-GEMM launches; nothing has been written then)."""
+    caller falls back to per-GEMM launches; nothing has been written then).  ``X2`` as in
+    :func:`ns_iterate`."""
     batch, m, n = X.shape
     dev = X.device
     g = min(m, n)
@@ -456,12 +458,12 @@ def ns_persistent(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs,
     flat = (ctypes.c_float * (3 * len(coeffs)))(*[float(v) for abc in coeffs for v in abc])
     st = status_tensor(dev)
     rc = _backend.lib("ns_persistent_sm100").dion_ns_persistent(
-        _p(X), _p(Xalt), _p(A), _p(Bm), ctypes.c_int(batch), ctypes.c_int(m), ctypes.c_int(n),
-        flat, ctypes.c_int(len(coeffs)), _p(scale), _p(tiles), ctypes.c_int(n_gg),
+        _p(X), _p(Xalt), _p(X2), _p(A), _p(Bm), ctypes.c_int(batch), ctypes.c_int(m),
+        ctypes.c_int(n), flat, ctypes.c_int(len(coeffs)), _p(scale), _p(tiles), ctypes.c_int(n_gg),
         ctypes.c_int(n_mn), _p(counter), ctypes.c_int(sm_count(dev)), _p(st),
         ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
     if rc == -20:
         return None
     if rc != 0:
         raise RuntimeError(f"dion_ns_persistent failed with code {rc}")
-    return Xalt if len(coeffs) % 2 else X
+    return Xalt if len(coeffs) % 2 else (X if X2 is None else X2)

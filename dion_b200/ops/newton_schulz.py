@@ -132,11 +132,13 @@ def _gram_torch(G: Tensor, coeffs: Coeffs, norm_mult: float, epsilon: float,
 # CUDA implementations on the tcgen05 GEMM
 # ------------------------------------------------------------------------------------------------
 def _prepare_cuda(G: Tensor, allow_tall: bool = False):
-    """-> (X [B, m, n] bf16 contiguous with m, n multiples of 8, restore).  Tall inputs are
-    transposed to wide unless ``allow_tall`` (the caller then iterates in right-multiply form)."""
+    """-> (X [B, m, n] bf16 contiguous with m, n multiples of 8, sums of squares [B] or None,
+    restore).  Tall inputs are transposed to wide unless ``allow_tall`` (the caller then iterates
+    in right-multiply form).  ``X`` may be ``G`` itself: it is to be read only.  The sums are there
+    where one pass could round, pad and add up."""
     G = unwrap(G)  # a pending functional collective must complete before its address is used
     shape = G.shape
-    X = G.to(torch.bfloat16)
+    X = G
     if X.ndim == 2:
         X = X.unsqueeze(0)
     elif X.ndim > 3:
@@ -147,14 +149,20 @@ def _prepare_cuda(G: Tensor, allow_tall: bool = False):
     m, n = X.size(-2), X.size(-1)
     mp, np_ = (m + 7) // 8 * 8, (n + 7) // 8 * 8
     padded = (mp, np_) != (m, n)
-    if padded:
-        Xp = torch.zeros((X.size(0), mp, np_), dtype=torch.bfloat16, device=X.device)
-        Xp[:, :m, :n] = X
-        X = Xp
-    elif not X.is_contiguous() or X.data_ptr() % 16:
-        X = X.contiguous()
-    elif X.data_ptr() == G.data_ptr():
-        X = X.clone()  # the iteration ping-pongs into its input buffer
+    ss: Optional[Tensor] = None
+    if (not padded and X.dtype == torch.bfloat16 and X.is_contiguous()
+            and X.data_ptr() % 16 == 0):
+        pass
+    elif X.is_contiguous() and X.dtype in (torch.float32, torch.bfloat16) and X.size(0) < 65536:
+        X, ss = F.ns_prepare(X, mp, np_)
+    else:
+        X = X.to(torch.bfloat16)
+        if padded:
+            Xp = torch.zeros((X.size(0), mp, np_), dtype=torch.bfloat16, device=X.device)
+            Xp[:, :m, :n] = X
+            X = Xp
+        elif not X.is_contiguous() or X.data_ptr() % 16:
+            X = X.clone(memory_format=torch.contiguous_format)
 
     def restore(Y: Tensor) -> Tensor:
         if padded:
@@ -163,32 +171,39 @@ def _prepare_cuda(G: Tensor, allow_tall: bool = False):
             Y = Y.mT
         return Y.reshape(shape)
 
-    return X, restore
+    return X, ss, restore
 
 
-def _norm_scale(X: Tensor, norm_mult: float, epsilon: float) -> Tensor:
-    ss = F.sumsq(X)
+def _norm_scale(X: Tensor, norm_mult: float, epsilon: float, ss: Optional[Tensor]) -> Tensor:
+    if ss is None:
+        ss = F.sumsq(X)
     return F.finalize_scale(ss, norm_mult, epsilon, out=ss)
 
 
-def _iterate_cuda(X: Tensor, coeffs: Coeffs, scale: Optional[Tensor], hooks=None) -> Tensor:
+def _iterate_cuda(X: Tensor, coeffs: Coeffs, scale: Optional[Tensor], hooks=None,
+                  overwrite: bool = False, alloc: Optional[Callable] = None) -> Tensor:
     """Newton-Schulz iterations on ``X [B, m, n]``.  Wide or square matrices use the left form
     ``A = X X^T, X' = aX + (bA + cA^2) X``; tall ones the right form ``A = X^T X,
     X' = aX + X (bA + cA^2)``, reading ``X`` as an MN-major operand so that neither needs a
-    transposed copy.  ``hooks`` (fused exchange) may supply per-launch coupling to other GPUs:
+    transposed copy.  ``X`` is only read unless ``overwrite`` lends it to the iteration, which
+    otherwise goes to and fro between two buffers of its own; these come from ``alloc(like)``
+    where the caller wants the result in memory of its own.  ``hooks`` (fused exchange) may supply per-launch coupling to other GPUs:
     ``hooks.first_gram()``, ``hooks.after_first_iteration()``, ``hooks.last_update()``."""
     B_, m, n = X.shape
     tall = m > n
     g = n if tall else m
     A = torch.empty((B_, g, g), dtype=torch.bfloat16, device=X.device)
     Bm = torch.empty_like(A)
-    C = torch.empty_like(X)
-    if hooks is None and gemm.persistent_fits(X, B_, m, n, len(coeffs)):
-        done = gemm.ns_persistent(X, C, A, Bm, coeffs, scale)
-        if done is not None:
-            return done
-    if hooks is None and gemm.iterate_in_one_call(X, B_, m, n):
-        return gemm.ns_iterate(X, C, A, Bm, coeffs, scale)
+    alloc = alloc or torch.empty_like
+    C = alloc(X)
+    if hooks is None:
+        X2 = X if overwrite else alloc(X) if len(coeffs) > 1 else None
+        if gemm.persistent_fits(X, B_, m, n, len(coeffs)):
+            done = gemm.ns_persistent(X, C, A, Bm, coeffs, scale, X2)
+            if done is not None:
+                return done
+        if gemm.iterate_in_one_call(X, B_, m, n):
+            return gemm.ns_iterate(X, C, A, Bm, coeffs, scale, X2)
     last = len(coeffs) - 1
     for it, (a, b, c) in enumerate(coeffs):
         sc = scale if it == 0 else None
@@ -215,6 +230,8 @@ def _iterate_cuda(X: Tensor, coeffs: Coeffs, scale: Optional[Tensor], hooks=None
             # the input belongs to the exchange and is handed back to the peers: from here on
             # ping-pong between private buffers only
             X, C = C, torch.empty_like(C)
+        elif it == 0:
+            X, C = C, X2
         else:
             X, C = C, X
     return None if (hooks is not None) else X
@@ -222,17 +239,37 @@ def _iterate_cuda(X: Tensor, coeffs: Coeffs, scale: Optional[Tensor], hooks=None
 
 def _ns_cuda(G: Tensor, coeffs: Coeffs, norm_mult: float, epsilon: float) -> Tensor:
     with trace.span("newton_schulz"):
-        X, restore = _prepare_cuda(G, allow_tall=True)
-        scale = _norm_scale(X, norm_mult, epsilon)
+        X, ss, restore = _prepare_cuda(G, allow_tall=True)
+        scale = _norm_scale(X, norm_mult, epsilon, ss)
         return restore(_iterate_cuda(X, coeffs, scale))
 
 
+def buffer_form(ns_func: Optional[Callable], X_shape, device: torch.device) -> bool:
+    """Whether :func:`orthogonalize_buffer` stands in for ``ns_func`` on such a batch."""
+    return (getattr(ns_func, "ns_spec", None) is not None and device.type == "cuda"
+            and len(X_shape) == 3 and all(X_shape) and X_shape[1] % 8 == 0 and X_shape[2] % 8 == 0)
+
+
+@torch.no_grad()
+def orthogonalize_buffer(ns_func: Callable, X: Tensor, epsilon, sumsq: Tensor,
+                         alloc: Callable) -> Tensor:
+    """``ns_func(X, epsilon)`` for a caller that owns ``X`` (dense bf16, see :func:`buffer_form`;
+    overwritten), knows its sums of squares (fp32 ``[B]``, overwritten) and wants the result in ``X``
+    or in a buffer from ``alloc(like)``: no copy and no norm pass."""
+    coeffs, mult = ns_func.ns_spec
+    with trace.span("newton_schulz"):
+        scale = F.finalize_scale(sumsq, float(mult), _eps(epsilon), out=sumsq)
+        return _iterate_cuda(X, coeffs, scale, overwrite=True, alloc=alloc)
+
+
 def _aol_cuda(G: Tensor, epsilon: float) -> Tensor:
-    X, restore = _prepare_cuda(G)
+    X, _, restore = _prepare_cuda(G)
+    if X.data_ptr() == G.data_ptr():
+        X = X.clone()
     B_, m, n = X.shape
     A = torch.empty((B_, m, m), dtype=torch.bfloat16, device=X.device)
     gemm.ns_gemm(X, X, out=A, sym=True)
-    # X is private to this call (see _prepare_cuda), so the rescale may work in place: two
+    # X is private to this call, so the rescale may work in place: two
     # launches, the row scales and then X and A rescaled together.
     F.aol_rescale_(X, A, epsilon)
     a, b, c = AOL_COEFFS[0]
@@ -240,13 +277,13 @@ def _aol_cuda(G: Tensor, epsilon: float) -> Tensor:
     C = torch.empty_like(X)
     gemm.ns_gemm(A, A, out=Bm, sym=True, D=A, alpha=c, beta=b)
     gemm.ns_gemm(Bm, X, out=C, b_is_kn=True, D=X, alpha=1.0, beta=a)
-    return restore(_iterate_cuda(C, AOL_COEFFS[1:], None))
+    return restore(_iterate_cuda(C, AOL_COEFFS[1:], None, overwrite=True, alloc=lambda _: X))
 
 
 def _gram_cuda(G: Tensor, coeffs: Coeffs, norm_mult: float, epsilon: float,
                resets: Sequence[int]) -> Tensor:
-    X, restore = _prepare_cuda(G)
-    scale = _norm_scale(X, norm_mult, epsilon)
+    X, ss, restore = _prepare_cuda(G)
+    scale = _norm_scale(X, norm_mult, epsilon, ss)
     B_, m, n = X.shape
     dev = X.device
     R = torch.empty((B_, m, m), dtype=torch.bfloat16, device=dev)

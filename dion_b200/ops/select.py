@@ -49,6 +49,8 @@ def dion2_select(
     apply_ef: bool = True,
     out_addresses: Optional[List[int]] = None,
     sumsq_addresses: Optional[List[int]] = None,
+    out: Optional[Tensor] = None,
+    sumsq: Optional[Tensor] = None,
 ) -> Tuple[Tensor, Tensor, Optional[Tensor]]:
     """``M += G`` (skipped when ``G`` is None), pick the ``k`` rows (``select_dim=-2``) or columns
     (``-1``) of each matrix with the largest L1 norm, return them as a dense bf16 stack and scale
@@ -57,7 +59,8 @@ def dion2_select(
     Returns ``(U, indices, maps)``: ``U`` is ``[N, k, cols]`` or ``[N, rows, k]``; ``indices`` is
     ``[N, k]`` int64 (unordered); ``maps`` is ``[N, num_slices]`` int32 giving each slice's
     position in ``U`` or -1 (None on the PyTorch path).  ``N`` counts 2-D matrices, so a
-    parameter with batch dimensions contributes several."""
+    parameter with batch dimensions contributes several.  ``out`` (dense bf16, the shape of ``U``)
+    receives ``U``; ``sumsq`` (``[N]`` fp32) is increased by the squares of its entries."""
     Mm = _as_matrices(M)
     Gm = _as_matrices(G) if G is not None else None
     N = len(Mm)
@@ -95,14 +98,16 @@ def dion2_select(
                                       _c(idx.data_ptr()), k, 1, _c(0), ctypes.c_longlong(0),
                                       ctypes.c_float(float(ef_decay)), int(bool(apply_ef)),
                                       _c(dst[0].data_ptr()),
-                                      _c(dst[1].data_ptr() if sumsq_addresses else 0),
+                                      _c(dst[1].data_ptr() if sumsq_addresses else 0), _c(0),
                                       _stream(dev)), "dion_gather_ef")
             return None, idx, maps
-        U = torch.empty(out_shape, dtype=torch.bfloat16, device=dev)
+        U = torch.empty(out_shape, dtype=torch.bfloat16, device=dev) if out is None else out
         _check(lib.dion_gather_ef(_c(ptrs.data_ptr()), N, rows, cols, m_dt, _c(idx.data_ptr()), k,
                                   int(select_dim == -2), _c(U.data_ptr()),
                                   ctypes.c_longlong(U[0].numel()), ctypes.c_float(float(ef_decay)),
-                                  int(bool(apply_ef)), _c(0), _c(0), _stream(dev)),
+                                  int(bool(apply_ef)), _c(0), _c(0),
+                                  _c(sumsq.data_ptr() if sumsq is not None else 0),
+                                  _stream(dev)),
                "dion_gather_ef")
         return U, idx, maps
 
@@ -110,7 +115,8 @@ def dion2_select(
     if Gm is not None:
         torch._foreach_add_(Mm, [g.to(Mm[0].dtype) for g in Gm])
     if k == 0 or num == 0:
-        U = torch.zeros(out_shape, dtype=torch.bfloat16, device=dev)
+        U = torch.zeros(out_shape, dtype=torch.bfloat16, device=dev) if out is None \
+            else out.zero_()
         return U, torch.empty((N, 0), dtype=torch.int64, device=dev), None
     stacked = torch.stack(Mm)
     norm_dim = -1 if select_dim == -2 else -2
@@ -124,7 +130,10 @@ def dion2_select(
     if apply_ef:
         for m, ie, s in zip(Mm, idx_exp.unbind(0), sel.unbind(0)):
             m.scatter_(select_dim, ie, s * ef_decay)
-    return sel.to(torch.bfloat16), idx, None
+    U = sel.to(torch.bfloat16) if out is None else out.copy_(sel)
+    if sumsq is not None:
+        sumsq.add_(U.to(torch.float32).square().sum(dim=(-2, -1)))
+    return U, idx, None
 
 
 def scatter_selected(src: Tensor, idx: Tensor, num: int, select_dim: int) -> Tensor:

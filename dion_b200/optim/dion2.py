@@ -203,13 +203,19 @@ def dion2_update_megabatch_async(
         fx.release()
         yield
         return
-    U_sel, idx, maps = dion2_select(Gl, Ml, k_topk, select_dim, float(ef_decay))
     batch_shape = Ml[0].shape[:-2]
-    sel_shape = tuple(batch_shape) + tuple(U_sel.shape[-2:])
+    rows, cols = Ml[0].shape[-2:]
+    sel_shape = tuple(batch_shape) + ((k_topk, cols) if select_dim == -2 else (rows, k_topk))
     plan = MegabatchPlan(sel_shape, N, Ml[0].device, comm_dim, device_rank, world_size,
                          process_group, global_comm_dim_size=global_dim,
                          local_comm_size=k if comm_dim is not None else None, arena=arena)
-    plan.load(U_sel.reshape((N,) + sel_shape).unbind(0))
+    dense = plan.whole_input() if k_topk > 0 else None
+    sub = dense.view((-1,) + sel_shape[-2:]) if dense is not None else None
+    U_sel, idx, maps = dion2_select(
+        Gl, Ml, k_topk, select_dim, float(ef_decay), out=sub,
+        sumsq=plan.input_sumsq(newton_schulz_func) if sub is not None else None)
+    if sub is None:
+        plan.load(U_sel.reshape((N,) + sel_shape).unbind(0))
     U = yield from plan.run(newton_schulz_func, flatten, epsilon)
     if num_select == 0:
         return  # empty shard: nothing of these parameters lives on this rank

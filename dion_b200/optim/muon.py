@@ -196,7 +196,8 @@ def muon_update_megabatch_async(
         global_comm_dim_size=global_comm_size(X[0], comm_dim), split_sizes=split_sizes,
         arena=arena)
     # Momentum update; the bf16 Newton-Schulz input lands in the exchange buffer.
-    F.muon_pre(Gl, Ml, float(momentum), nesterov, out=plan.input_views())
+    F.muon_pre(Gl, Ml, float(momentum), nesterov, out=plan.input_views(),
+               sumsq=plan.input_sumsq(newton_schulz_func, split_sizes))
     U = yield from plan.run(newton_schulz_func, flatten, epsilon, split_sizes, split_scales)
     F.muon_post(Xl, contiguous_list(U), lr, weight_decay, ratio, cautious_wd)
 

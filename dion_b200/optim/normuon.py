@@ -166,7 +166,8 @@ def normuon_update_megabatch_async(
         Ml[0].shape, len(X), Ml[0].device, comm_dim, device_rank, world_size, process_group,
         global_comm_dim_size=global_rows, split_sizes=split_sizes,
         arena=arena)
-    F.muon_pre(Gl, Ml, float(momentum), nesterov, out=plan.input_views())
+    F.muon_pre(Gl, Ml, float(momentum), nesterov, out=plan.input_views(),
+               sumsq=plan.input_sumsq(newton_schulz_func, split_sizes))
     U = yield from plan.run(newton_schulz_func, flatten, epsilon, split_sizes, split_scales)
     # Row blocks keep their own Frobenius norm only where whole matrices are local.
     norm_split = split_sizes if (comm_dim is None or process_group is None) else None

@@ -26,6 +26,7 @@ import torch.distributed as dist
 from torch import Tensor
 from torch.distributed import ProcessGroup
 
+from ..ops import newton_schulz as NS
 from ..utils.arena import StepArena, alloc as _alloc
 from .async_runtime import run_to_completion
 
@@ -160,6 +161,7 @@ class MegabatchPlan:
             shp[comm_dim] = padded
             self.padded_shape = tuple(shp)
         self._send: Optional[Tensor] = None
+        self._sumsq: Optional[Tensor] = None
 
     # -- producer side ------------------------------------------------------------------------
     def _alloc_send(self) -> Tensor:
@@ -190,6 +192,25 @@ class MegabatchPlan:
             lo = self.rank * self.per_rank
             return [s[i - lo] if lo <= i < lo + self.per_rank else None for i in range(self.n)]
         return [s[i] for i in range(self.n)]
+
+    def whole_input(self) -> Optional[Tensor]:
+        """The buffer that takes the Newton-Schulz inputs, ``[n, *local_shape]``, for a producer
+        that writes all of them at once; None where they go to several ranks."""
+        if self.mode != "single":
+            return None
+        self._send = self._alloc_send()
+        return self._send
+
+    def input_sumsq(self, newton_schulz_func: Callable, split_sizes=None) -> Optional[Tensor]:
+        """Zeroed fp32 ``[n]`` for the sums of squares of the inputs if :meth:`run` can use them
+        (whole 2-D matrices of this rank and a driver of this package), else None.  The producer
+        then has to fill it."""
+        if (self.mode != "single" or split_sizes is not None or len(self.local_shape) != 2
+                or not NS.buffer_form(newton_schulz_func, (self.n,) + self.local_shape,
+                                      self.device)):
+            return None
+        self._sumsq = _alloc(self.arena, (self.n,), torch.float32, self.device, zero=True)
+        return self._sumsq
 
     def load(self, U: Sequence[Tensor]) -> None:
         """Copy already computed inputs into the exchange buffer."""
@@ -222,6 +243,11 @@ class MegabatchPlan:
             X, newton_schulz_func, flatten, epsilon, split_sizes, split_scales)
 
         if self.mode == "single":
+            ss, self._sumsq = self._sumsq, None
+            if ss is not None:
+                return NS.orthogonalize_buffer(
+                    newton_schulz_func, send, epsilon, ss,
+                    lambda like: _alloc(self.arena, like.shape, like.dtype, like.device))
             return self._stable(ns(send))
 
         if self.mode == "replicated":

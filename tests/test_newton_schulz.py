@@ -44,6 +44,58 @@ def test_cpu_matches_reference(ref_dion):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("form", ["dense", "odd", "two_dims", "four_dims", "transposed", "columns",
+                                  "off_by_one", "one_row"])
+@pytest.mark.parametrize("variant", ["polar_express", "aol", "gram"])
+def test_cuda_input_forms(variant, form, dtype):
+    """The input is read in place or in one rounding / padding pass, whatever its order and
+    strides, and is never written."""
+    fn = {"polar_express": NS.polar_express, "aol": NS.newton_schulz_aol,
+          "gram": NS.gram_newton_schulz}[variant]
+    torch.manual_seed(0)
+    G = {"dense": lambda: torch.randn(3, 96, 200), "odd": lambda: torch.randn(3, 101, 57),
+         "two_dims": lambda: torch.randn(136, 264), "four_dims": lambda: torch.randn(2, 2, 64, 72),
+         "transposed": lambda: torch.randn(3, 200, 96), "columns": lambda: torch.randn(3, 96, 300),
+         "off_by_one": lambda: torch.randn(3 * 96 * 200 + 1),
+         "one_row": lambda: torch.randn(2, 1, 40)}[form]().to("cuda", dtype)
+    if form == "transposed":
+        G = G.mT
+    elif form == "columns":
+        G = G[:, :, 50:250]
+    elif form == "off_by_one":
+        G = G[1:].view(3, 96, 200)
+    before = G.clone()
+    got = fn(G)
+    assert torch.equal(G, before) and got.shape == G.shape and got.dtype == torch.bfloat16
+    m, n = G.shape[-2:]
+    dense = torch.zeros(*G.shape[:-2], -(-m // 8) * 8, -(-n // 8) * 8, device="cuda",
+                        dtype=torch.bfloat16)
+    dense[..., :m, :n] = G
+    ref = fn(dense)[..., :m, :n]
+    rel = (got.float() - ref.float()).norm() / ref.float().norm()
+    # the same products on the same bf16 input; only the last bits of the input's norm may differ,
+    # which moves single roundings (2^-9) of fifteen products
+    assert rel.item() < 2e-2, rel.item()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (5, 13, 29), (2, 64, 65), (3, 100, 96), (2, 517, 1031)])
+def test_prepare_rounds_pads_and_sums(shape, dtype):
+    from dion_b200.ops import foreach as F
+    torch.manual_seed(0)
+    G = torch.randn(*shape, device="cuda").to(dtype)
+    mp, np_ = (shape[1] + 7) // 8 * 8, (shape[2] + 7) // 8 * 8
+    X, ss = F.ns_prepare(G, mp, np_)
+    ref = torch.zeros(shape[0], mp, np_, device="cuda", dtype=torch.bfloat16)
+    ref[:, :shape[1], :shape[2]] = G
+    assert torch.equal(X, ref)
+    exact = ref.double().square().sum(dim=(1, 2))
+    assert ((ss - exact).abs() <= 1e-5 * exact).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("variant", ["quintic", "classic", "polar_express", "aol", "gram"])
 @pytest.mark.parametrize("shape", [(6, 768, 768), (2, 768, 3072), (2, 3072, 768), (3, 192, 768),
                                    (1, 100, 52), (256, 256)])
