@@ -24,6 +24,7 @@ import torch.nn.functional as tF
 from torch.distributed.device_mesh import DeviceMesh
 
 from . import functional as Fn
+from . import inference
 
 
 @dataclass
@@ -171,19 +172,23 @@ class GPT(nn.Module):
 
     def forward(self, idx: torch.Tensor, targets: Optional[torch.Tensor] = None,
                 return_logits: bool = False):
-        wte = self.transformer.wte
-        x = Fn.embedding(idx, wte.weight) if _is_plain(wte) else wte(idx)
-        h = None
-        for block in self.transformer.h:
-            x, h = block(x, h)
-        x = h if h is not None else Fn.rms_norm(x)  # final norm rides on the last residual add
+        x = None
+        if not torch.is_grad_enabled():
+            x = inference.hidden_states(self, idx, (Block, CausalSelfAttention, MLP, Rotary))
+        if x is None:
+            wte = self.transformer.wte
+            x = Fn.embedding(idx, wte.weight) if _is_plain(wte) else wte(idx)
+            h = None
+            for block in self.transformer.h:
+                x, h = block(x, h)
+            x = h if h is not None else Fn.rms_norm(x)  # final norm rides on the last residual add
         if targets is not None:
             logits = _linear(self.lm_head, x)
             if return_logits:
                 return logits.float()
             return Fn.cross_entropy(logits.view(-1, logits.size(-1)), targets.view(-1),
                                     ignore_index=-1)
-        logits = self.lm_head(x[:, [-1], :]).float()
+        logits = self.lm_head(x[:, -1:, :] if x.size(1) else x[:, [-1], :]).float()
         return logits if return_logits else None
 
     def compile(self) -> None:  # kept for call-site compatibility; there is nothing to trace

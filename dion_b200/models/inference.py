@@ -1,0 +1,161 @@
+"""The GPT's blocks without gradients (``generate``, scoring under ``torch.no_grad``) as two native
+calls per block around the attention (``csrc/infer_ops.cu``).
+
+The general forward of ``gpt.py`` goes through modules and autograd functions, about fifteen calls
+and 400 us of host time per block, which for a short prompt is six times what the device needs.  The
+path here takes the same weights, hooks nothing and keeps nothing between calls (next-token logits of
+GPT-160M for 128 tokens: 4838 -> 1182 us); whatever it does not recognise (see
+:func:`hidden_states`) takes the general forward.
+"""
+from __future__ import annotations
+
+import ctypes
+from typing import Optional
+
+import torch
+import torch.nn.functional as tF
+from torch import Tensor
+from torch.nn.modules import module as _nn_module
+
+from ..ops import _backend, gemm
+from ..utils.tensors import is_plain_tensor
+
+
+class _Gemm(ctypes.Structure):
+    _fields_ = [("tiles", ctypes.c_void_p), ("n_tiles", ctypes.c_int), ("bn", ctypes.c_int)]
+
+
+class _Infer(ctypes.Structure):
+    """Mirrors ``DionInfer`` in csrc/infer_ops.cu."""
+
+    _fields_ = ([(n, ctypes.c_void_p) for n in
+                 ("gemm2", "gemm", "norm", "rope", "relu2", "x0", "x1", "h", "w", "qkv", "qo", "ko",
+                  "o", "act", "rstd", "status")]
+                + [(n, ctypes.c_int) for n in ("B", "T", "H", "D", "F", "w_dt", "sms")]
+                + [("eps_x", ctypes.c_float), ("eps_qk", ctypes.c_float), ("cfg", _Gemm * 4)])
+
+
+_entries: Optional[tuple] = None
+
+
+def _entry_points() -> tuple:
+    """Addresses of the kernels' entry points in the other libraries."""
+    global _entries
+    if _entries is None:
+        def at(lib, name):
+            return ctypes.cast(getattr(_backend.lib(lib)._dll, name), ctypes.c_void_p).value
+        _entries = (at("ns_gemm2_sm100", "dion_ns_gemm2_ex"), at("ns_gemm_sm100", "dion_ns_gemm_ex"),
+                    at("model_ops", "dion_rmsnorm_fwd"), at("model_ops", "dion_rope_qknorm_fwd"),
+                    at("model_ops", "dion_relu2_fwd"))
+    return _entries
+
+
+def _unhooked(m) -> bool:
+    return not (m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__)
+
+
+def _observed() -> bool:
+    """Something watches or rewrites operators, modules or values: it has to see them."""
+    return bool(_nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks
+                or torch.jit.is_tracing() or torch.compiler.is_compiling()
+                or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
+                or torch._C._functorch.peek_interpreter_stack() is not None
+                or torch.autograd.forward_ad._current_level >= 0)
+
+
+def _block_weights(block, types, C: int):
+    """The block's six weights if its modules may be bypassed, else None."""
+    Block, Attention, MLP = types[:3]
+    attn, mlp = block.attn, block.mlp
+    if not (type(block) is Block and type(attn) is Attention and type(mlp) is MLP
+            and _unhooked(block) and _unhooked(attn) and _unhooked(mlp)):
+        return None
+    linears = (attn.c_q, attn.c_k, attn.c_v, attn.c_proj, mlp.c_fc, mlp.c_proj)
+    ws = tuple(m.weight for m in linears)
+    F = ws[4].size(0)
+    shapes = ((C, C),) * 4 + ((F, C), (C, F))
+    for m, w, s in zip(linears, ws, shapes):
+        if not (_unhooked(m) and m.bias is None and is_plain_tensor(w) and w.is_cuda
+                and w.shape == s and w.dtype == ws[0].dtype and w.is_contiguous()
+                and w.data_ptr() % 16 == 0):
+            return None
+    return ws
+
+
+def _config(rows: int, N: int, K: int, dev: torch.device) -> _Gemm:
+    pair, bn = gemm._choose_config(rows, N, K, 1, False, gemm.pair_default(), dev)
+    tiles = gemm.tile_table(rows, N, 256 if pair else bn, False, dev, bm=256 if pair else 128)
+    return _Gemm(tiles.data_ptr(), tiles.size(0), 0 if pair else bn)
+
+
+def hidden_states(model, idx: Tensor, types) -> Optional[Tensor]:
+    """``[B, T, C]`` bf16: the residual stream after the last block, normalized.  None unless
+    gradients are off, bf16 autocast is on, the model is a plain GPT (no hooks, no shards, no
+    replaced modules; fp32 embedding; dense fp32 or bf16 weights of one dtype) on the GPU of
+    ``idx``, and nothing observes operators."""
+    wte = model.transformer.wte
+    table = wte.weight
+    C = table.size(1)
+    blocks = model.transformer.h
+    if (torch.is_grad_enabled() or not idx.is_cuda or not is_plain_tensor(idx) or idx.ndim != 2
+            or idx.numel() == 0 or len(blocks) == 0
+            or not torch.is_autocast_enabled("cuda")
+            or torch.get_autocast_dtype("cuda") != torch.bfloat16
+            or not is_plain_tensor(table) or table.dtype != torch.float32
+            or table.device != idx.device or C % 8 or C > 4096 or not _unhooked(wte)
+            or _observed()):
+        return None
+    B, T = idx.shape
+    H = blocks[0].attn.n_head
+    D = C // H
+    if D not in (32, 64, 128, 256):
+        return None
+    weights = [_block_weights(b, types, C) for b in blocks]
+    first = weights[0]
+    if first is None or first[0].dtype not in (torch.float32, torch.bfloat16):
+        return None
+    F = first[4].size(0)
+    if F % 8 or any(w is None or w[4].size(0) != F or w[0].dtype != first[0].dtype
+                    or w[0].device != idx.device for w in weights) \
+            or any(b.attn.n_head != H for b in blocks):
+        return None
+    dev, rows = idx.device, B * T
+    tables = []
+    for b in blocks:
+        if type(b.attn.rotary) is not types[3] or not _unhooked(b.attn.rotary):
+            return None
+        cos, sin = b.attn.rotary(idx)
+        if any(not t.is_contiguous() or t.dtype != torch.bfloat16 or t.shape != (T, D // 2)
+               or t.device != dev for t in (cos, sin)):
+            return None
+        tables.append((cos, sin))
+    x = tF.embedding(idx, table)
+    x1 = torch.empty_like(x)
+    bf16 = lambda *s: torch.empty(s, dtype=torch.bfloat16, device=dev)  # noqa: E731
+    h, qkv, o, act = bf16(B, T, C), bf16(B, T, 3, H, D), bf16(rows, C), bf16(rows, F)
+    q, k = bf16(B, T, H, D), bf16(B, T, H, D)
+    w = bf16(4 * C * C + 2 * C * F)
+    rstd = torch.empty(2 * rows * H, dtype=torch.float32, device=dev)
+    p = _Infer(*_entry_points(), x.data_ptr(), x1.data_ptr(), h.data_ptr(), w.data_ptr(),
+               qkv.data_ptr(), q.data_ptr(), k.data_ptr(), o.data_ptr(), act.data_ptr(),
+               rstd.data_ptr(), gemm.status_tensor(dev).data_ptr(), B, T, H, D, F,
+               0 if first[0].dtype == torch.float32 else 1, gemm.sm_count(dev),
+               float(torch.finfo(torch.float32).eps), float(torch.finfo(torch.bfloat16).eps))
+    for i, (n, kk) in enumerate(((3 * C, C), (C, C), (F, C), (C, F))):
+        p.cfg[i] = _config(rows, n, kk, dev)
+    lib = _backend.lib("infer_ops")
+    ref = ctypes.byref(p)
+    ptr = ctypes.c_void_p
+    stream = ptr(torch.cuda.current_stream(dev).cuda_stream)
+    rc = _backend.lib("model_ops").dion_rmsnorm_fwd(
+        ptr(x.data_ptr()), 0, ptr(0), 0, ptr(0), ptr(h.data_ptr()), 1, ptr(rstd.data_ptr()),
+        ctypes.c_longlong(rows), C, ctypes.c_float(p.eps_x), stream)
+    qT, kT, vT = q.transpose(1, 2), k.transpose(1, 2), qkv[:, :, 2].transpose(1, 2)
+    for (cos, sin), ws in zip(tables, weights):
+        rc |= lib.dion_infer_block_in(ref, *(ptr(t.data_ptr()) for t in ws), ptr(cos.data_ptr()),
+                                      ptr(sin.data_ptr()), stream)
+        y = tF.scaled_dot_product_attention(qT, kT, vT, is_causal=True).transpose(1, 2).contiguous()
+        rc |= lib.dion_infer_block_out(ref, ptr(y.data_ptr()), stream)
+    if rc != 0:
+        raise RuntimeError("a kernel launch of the inference path failed")
+    return h

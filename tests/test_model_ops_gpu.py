@@ -258,3 +258,34 @@ def test_add_rms_norm(D):
     assert (h.float() - hr).abs().max().item() < 3e-2
     assert (x.grad - xr.grad).abs().max().item() < 2e-2  # g2 passed through bf16 h
     assert (d.grad.float() - dr.grad).abs().max().item() < 5e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,T,heads,dim", [(1, 1, 2, 64), (1, 37, 4, 64), (3, 128, 2, 128), (2, 300, 3, 32)])
+def test_blocks_without_gradients_match_the_general_forward(B, T, heads, dim, dtype):
+    """Row counts below, at and above a tile of both product kernels.  Both sides round every
+    product to bf16 (2^-9 each, over two blocks); the fused relu^2 skips one of the roundings."""
+    from dion_b200.models import inference
+    from dion_b200.models.gpt import GPT, GPTConfig
+    from dion_b200.ops import _backend
+    torch.manual_seed(0)
+    model = GPT(GPTConfig(sequence_len=T, vocab_size=512, n_layer=2, n_head=heads,
+                          n_embd=heads * dim)).cuda()
+    model.init_weights()
+    model.transformer.h.to(dtype)
+    ids = torch.randint(0, 512, (B, T), device="cuda")
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        ref = model(ids, ids, return_logits=True).detach()
+        with torch.no_grad():
+            _backend.reset_launch_count()
+            got = model(ids, ids, return_logits=True)
+            assert _backend.launch_count() >= 17
+            last = model(ids, return_logits=True)
+            seen = []
+            hook = model.transformer.h[1].mlp.c_fc.register_forward_hook(lambda *a: seen.append(1))
+            hooked = model(ids, ids, return_logits=True)
+            hook.remove()
+    assert seen
+    for x in (got, hooked):
+        assert ((x - ref).norm() / ref.norm()).item() < 2e-2
+    assert ((last[:, 0] - ref[:, -1]).norm() / ref[:, -1].norm()).item() < 2e-2
