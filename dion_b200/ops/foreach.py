@@ -252,14 +252,17 @@ def adamw(
         if state_steps is not None:
             lists.append(state_steps)
         tb = build_table(lists, [x.numel() for x in X], tag="adamw")
+        corr = torch.empty(2 * n, dtype=torch.float32, device=dev) if state_steps is not None \
+            else None
         _check(
             _backend.lib("foreach_ops").dion_adamw(
-                _c(tb.device_tensor.data_ptr()), ctypes.c_longlong(tb.n_chunks), n,
+                _c(tb.device_tensor.data_ptr()), ctypes.c_longlong(tb.n_chunks),
                 _c(lr_t.data_ptr()), _c(wd_t.data_ptr() if wd_t is not None else 0),
                 ctypes.c_float(wd_f), ctypes.c_float(beta1), ctypes.c_float(beta2),
                 ctypes.c_float(epsilon), int(bool(cautious_wd)),
                 _DT[X[0].dtype], _DT[G[0].dtype], _DT[M[0].dtype], _DT[V[0].dtype],
-                int(state_steps is not None), ctypes.c_float(float(step or 0)), _stream(dev)),
+                int(state_steps is not None), ctypes.c_float(float(step or 0)),
+                _c(corr.data_ptr() if corr is not None else 0), _stream(dev)),
             "dion_adamw")
         return
     # PyTorch path
