@@ -9,8 +9,8 @@
 //                            X' = s (a X + B X)   (X B for tall X)
 //
 // with the input scale s applied in the first iteration only, X and X' ping-ponging between two
-// buffers.  The phases are the same tcgen05 GEMMs as in ns_gemm_sm100.cu (128 x 128 tiles, TMA
-// producer warp, one MMA thread, four epilogue warps, TMEM accumulators) and are separated by a
+// buffers.  The phases are the same tcgen05 GEMMs as in ns_gemm_sm100.cu (128 x 128 or
+// 128 x 64 tiles, TMA producer warp, one MMA thread, eight epilogue warps, TMEM accumulators) and are separated by a
 // grid-wide barrier: the CTAs are launched cooperatively (all resident), count themselves in on
 // a global counter and spin, bounded, until everybody has arrived.  A phase reads what the
 // previous one wrote through L2 only: operand tiles by TMA after a proxy fence, the epilogue's
@@ -22,11 +22,17 @@
 
 namespace dion {
 
-constexpr int PBM = 128, PBN = 128, PBK = 64;
-constexpr int kPThreads = 192;
-constexpr int kPStages = 6;
-constexpr int kPStageBytes = (PBM + PBN) * PBK * 2;   // 32 KB
-constexpr int kPDynBytes = kPStages * kPStageBytes + 1024;
+constexpr int PBM = 128, PBK = 64;
+// Two groups of four epilogue warps share a tile's columns.  A phase is a chain of latencies (barrier,
+// first TMA, products, addend, stores), so its addend is fetched while the products run, and where
+// 128 x 64 tiles still fit the SMs they replace 128 x 128 ones: a CTA then loads 288 instead of
+// 384 KB per phase at K = 768.  Five iterations on one 768 x 768 matrix: 224 -> 166 us, 256 x 256:
+// 171 -> 113 us; with 128 x 128 tiles 1 x 768 x 3072: 290 -> 272 us.
+constexpr int kPGroups = 2;
+constexpr int kPThreads = 64 + 128 * kPGroups;
+__host__ __device__ constexpr int p_stage_bytes(int bn) { return (PBM + bn) * PBK * 2; }   // 32 KB / 24 KB
+__host__ __device__ constexpr int p_stages(int bn) { return bn == 128 ? 6 : 8; }
+__host__ __device__ constexpr int p_dyn_bytes(int bn) { return p_stages(bn) * p_stage_bytes(bn) + 1024; }
 constexpr int kMaxPhases = 24;   // eight iterations; keeps the launch parameters under 4 KB
 
 // One GEMM of the loop.  Buffers and tensor maps are referred to by index.
@@ -81,13 +87,15 @@ __device__ __forceinline__ float ld_cg_bf16(const __nv_bfloat16* p) {
   return __bfloat162float(__ushort_as_bfloat16(v));
 }
 
-// Barrier over the four epilogue warps (named barrier 1).
+// Barrier over all epilogue warps (named barrier 1).
 __device__ __forceinline__ void epi_sync() {
-  asm volatile("barrier.cta.sync.aligned 1, 128;" ::: "memory");
+  asm volatile("barrier.cta.sync.aligned 1, %0;" ::"n"(128 * kPGroups) : "memory");
 }
 
+template <int PBN>
 __global__ void __launch_bounds__(kPThreads, 1)
 ns_persistent_kernel(const __grid_constant__ PersistArgs p) {
+  constexpr int kPStages = p_stages(PBN), kPStageBytes = p_stage_bytes(PBN);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -110,7 +118,7 @@ ns_persistent_kernel(const __grid_constant__ PersistArgs p) {
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 4);
+      mbar_init(&tempty_bar[a], 4 * kPGroups);
     }
     mbar_init(&phase_bar, 1);
     grid_ok = 1;
@@ -158,8 +166,11 @@ ns_persistent_kernel(const __grid_constant__ PersistArgs p) {
             uint8_t* sa = smem + stage * kPStageBytes;
             uint8_t* sb = sa + PBM * PBK * 2;
             mbar_expect_tx(&full_bar[stage], kPStageBytes);
-            if (!g.a_mn) {
-              tma_load_3d(sa, ma, &full_bar[stage], kb * PBK, tt.x * PBM, b);
+            if (!g.a_mn) {   // K-major maps have boxes of PBN rows
+#pragma unroll
+              for (int c = 0; c < PBM / PBN; ++c)
+                tma_load_3d(sa + c * (PBN * 128), ma, &full_bar[stage], kb * PBK,
+                            tt.x * PBM + c * PBN, b);
             } else {
 #pragma unroll
               for (int c = 0; c < PBM / 64; ++c)
@@ -235,6 +246,8 @@ ns_persistent_kernel(const __grid_constant__ PersistArgs p) {
     // ------------------------------ epilogue ----------------------------------
     const int lane_grp = warp & 3;
     const int row_in_tile = lane_grp * 32 + lane;
+    const int grp = (warp - 2) >> 2;
+    constexpr int kCols = PBN / kPGroups;      // columns of a tile that this group drains
     const bool leader = (warp == 2 && lane == 0);
     uint32_t aslot = 0, aphase = 0;
     bool ok = true;
@@ -247,31 +260,40 @@ ns_persistent_kernel(const __grid_constant__ PersistArgs p) {
       for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
         const int b = t / g.tiles_per_mat;
         const int2 tt = p.tiles[g.tile_ofs + t - b * g.tiles_per_mat];
-        if (!mbar_wait_bounded(&tfull_bar[aslot], aphase)) {
-          if (lane == 0) atomicExch(p.status, kStatusTimeoutTmemFull);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
         float s = 1.f;
         if (p.scale != nullptr && (g.alpha_pow | g.beta_pow)) s = p.scale[b];
         const float alpha = g.alpha * ipow_p(s, g.alpha_pow);
         const float beta = g.beta * ipow_p(s, g.beta_pow);
         const int r = tt.x * PBM + row_in_tile;
         const int warp_row0 = tt.x * PBM + lane_grp * 32;
+        const int col0 = tt.y * PBN + grp * kCols;
         const bool row_ok = r < g.M;
         __nv_bfloat16* Cb = p.buf[g.c_buf] + (long long)b * sc_;
         __nv_bfloat16* Crow = Cb + (long long)r * ldc;
         const __nv_bfloat16* Drow =
             g.d_buf >= 0 ? p.buf[g.d_buf] + (long long)b * sd_ + (long long)r * ldd : nullptr;
-#pragma unroll 1
-        for (int ch = 0; ch < PBN / 32; ++ch) {
-          const int c0 = tt.y * PBN + ch * 32;
+        // The addend of whole 32-column pieces, fetched while the products run.
+        uint4 dv[kCols / 8];
+        if (Drow != nullptr && row_ok) {
+#pragma unroll
+          for (int q = 0; q < kCols / 8; ++q)
+            if (col0 + (q / 4) * 32 + 32 <= g.N) dv[q] = ld_cg_u4(Drow + col0 + q * 8);
+        }
+        if (!mbar_wait_bounded(&tfull_bar[aslot], aphase)) {
+          if (lane == 0) atomicExch(p.status, kStatusTimeoutTmemFull);
+          ok = false;
+          break;
+        }
+        __syncwarp();
+        tc_fence_after();
+#pragma unroll
+        for (int ch = 0; ch < kCols / 32; ++ch) {
+          const int c0 = col0 + ch * 32;
           if (c0 >= g.N) continue;
           if (g.sym && c0 + 31 < warp_row0) continue;   // wholly below the diagonal
           float v[32];
           tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(lane_grp * 32) << 16) + aslot * PBN +
-                            ch * 32,
+                            grp * kCols + ch * 32,
                         v);
           tmem_ld_wait();
           if (!row_ok) continue;
@@ -280,7 +302,7 @@ ns_persistent_kernel(const __grid_constant__ PersistArgs p) {
             if (full) {
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
-                const uint4 u = ld_cg_u4(Drow + c0 + q * 8);
+                const uint4 u = dv[ch * 4 + q];
                 const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -341,8 +363,8 @@ ns_persistent_kernel(const __grid_constant__ PersistArgs p) {
         asm volatile("fence.proxy.async;" ::: "memory");
         epi_sync();                        // every epilogue thread of this CTA has stored
         if (leader) {
-          __threadfence();
-          atomicAdd(p.counter, 1u);
+          // Releases the stores of all epilogue threads, which the barrier ordered before it.
+          asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.counter) : "memory");
           const unsigned want = gridDim.x * (unsigned)(ph + 1);
           WaitBudget budget;
           bool arrived = true;
@@ -351,7 +373,6 @@ ns_persistent_kernel(const __grid_constant__ PersistArgs p) {
               arrived = false;
               break;
             }
-            __nanosleep(32);
           }
           if (!arrived) {
             atomicExch(p.status, kStatusTimeoutGrid);
@@ -421,20 +442,56 @@ static int make_map_p(CUtensorMap* map, const void* ptr, int batch, int rows, in
 
 }  // namespace dion
 
+namespace dion {
+
+template <int PBN>
+static int launch_persistent(PersistArgs& a, int max_tiles, int num_sms, cudaStream_t stream) {
+  static bool configured = false;
+  static int max_blocks = 0;
+  auto kernel = ns_persistent_kernel<PBN>;
+  constexpr int kDyn = p_dyn_bytes(PBN);
+  if (!configured) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDyn) !=
+        cudaSuccess)
+      return -3;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPThreads, kDyn) !=
+            cudaSuccess ||
+        per_sm < 1)
+      return -20;
+    max_blocks = per_sm * num_sms;
+    configured = true;
+  }
+  int grid = max_tiles < num_sms ? max_tiles : num_sms;
+  if (grid > max_blocks) grid = max_blocks;
+  if (grid <= 0) return 0;
+  void* kargs[] = {&a};
+  cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kernel), dim3(grid),
+                                              dim3(kPThreads), kargs, kDyn, stream);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return e == cudaErrorCooperativeLaunchTooLarge ? -20 : -4;
+  }
+  return 0;
+}
+
+}  // namespace dion
+
 // All iterations (a, b, c) = coeffs[3*i .. 3*i+2] of the Newton-Schulz loop on the dense bf16 batch
 // X [batch, m, n] in one cooperative launch.  Xalt and X2 [batch, m, n], A and Bm [batch, g, g]
 // (g = min(m, n)) are work buffers; `counter` points to two zero-initialised unsigned ints in
 // device memory that the kernel leaves at zero.  tiles_all: (tile_m, tile_n) pairs in units of
-// 128 x 128, first the n_tiles_gg tiles on or above the diagonal of the symmetric g x g products,
+// 128 x bn, first the n_tiles_gg tiles on or above the diagonal of the symmetric g x g products,
 // then the n_tiles_mn tiles of the m x n update.  The result lies in Xalt when
 // `iters` is odd, else in X, or in X2 where that is given (X is then only read).  Returns 0 on success,
 // -20 when the grid cannot be co-resident (the caller then uses the per-GEMM launches).
 DION_EXPORT int dion_ns_persistent(void* X, void* Xalt, void* X2, void* A, void* Bm, int batch, int m,
                                    int n, const float* coeffs, int iters, const float* scale,
                                    const void* tiles_all, int n_tiles_gg, int n_tiles_mn,
-                                   unsigned int* counter, int num_sms, int* status,
+                                   unsigned int* counter, int num_sms, int bn, int* status,
                                    void* stream) {
   using namespace dion;
+  if (bn != 64 && bn != 128) return -10;
   if (batch <= 0 || m <= 0 || n <= 0 || iters <= 0) return 0;
   if (3 * iters > kMaxPhases) return -10;
   if ((m & 7) || (n & 7)) return -10;
@@ -445,14 +502,14 @@ DION_EXPORT int dion_ns_persistent(void* X, void* Xalt, void* X2, void* A, void*
   PersistArgs a;
   // maps: 0 X K-major, 1 X MN-major, 2 Xalt K-major, 3 Xalt MN-major, 4 A K-major, 5 Bm K-major,
   // 6 X2 K-major, 7 X2 MN-major
-  if (make_map_p(&a.maps[0], X, batch, m, n, PBK, PBM) != 0) return -12;
+  if (make_map_p(&a.maps[0], X, batch, m, n, PBK, bn) != 0) return -12;
   if (make_map_p(&a.maps[1], X, batch, m, n, 64, PBK) != 0) return -12;
-  if (make_map_p(&a.maps[2], Xalt, batch, m, n, PBK, PBM) != 0) return -12;
+  if (make_map_p(&a.maps[2], Xalt, batch, m, n, PBK, bn) != 0) return -12;
   if (make_map_p(&a.maps[3], Xalt, batch, m, n, 64, PBK) != 0) return -12;
-  if (make_map_p(&a.maps[4], A, batch, g, g, PBK, PBM) != 0) return -12;
-  if (make_map_p(&a.maps[5], Bm, batch, g, g, PBK, PBM) != 0) return -12;
+  if (make_map_p(&a.maps[4], A, batch, g, g, PBK, bn) != 0) return -12;
+  if (make_map_p(&a.maps[5], Bm, batch, g, g, PBK, bn) != 0) return -12;
   if (X2 == nullptr) X2 = X;
-  if (make_map_p(&a.maps[6], X2, batch, m, n, PBK, PBM) != 0) return -12;
+  if (make_map_p(&a.maps[6], X2, batch, m, n, PBK, bn) != 0) return -12;
   if (make_map_p(&a.maps[7], X2, batch, m, n, 64, PBK) != 0) return -12;
   a.buf[0] = static_cast<__nv_bfloat16*>(X);
   a.buf[1] = static_cast<__nv_bfloat16*>(Xalt);
@@ -519,29 +576,6 @@ DION_EXPORT int dion_ns_persistent(void* X, void* Xalt, void* X2, void* A, void*
     if (tg > max_tiles) max_tiles = tg;
     if (tm > max_tiles) max_tiles = tm;
   }
-  static bool configured = false;
-  static int max_blocks = 0;
-  if (!configured) {
-    if (cudaFuncSetAttribute(ns_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kPDynBytes) != cudaSuccess)
-      return -3;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ns_persistent_kernel, kPThreads,
-                                                      kPDynBytes) != cudaSuccess || per_sm < 1)
-      return -20;
-    max_blocks = per_sm * num_sms;
-    configured = true;
-  }
-  int grid = max_tiles < num_sms ? max_tiles : num_sms;
-  if (grid > max_blocks) grid = max_blocks;
-  if (grid <= 0) return 0;
-  void* kargs[] = {&a};
-  cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(ns_persistent_kernel),
-                                              dim3(grid), dim3(kPThreads), kargs, kPDynBytes,
-                                              static_cast<cudaStream_t>(stream));
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return e == cudaErrorCooperativeLaunchTooLarge ? -20 : -4;
-  }
-  return 0;
+  return bn == 64 ? launch_persistent<64>(a, max_tiles, num_sms, static_cast<cudaStream_t>(stream))
+                  : launch_persistent<128>(a, max_tiles, num_sms, static_cast<cudaStream_t>(stream));
 }

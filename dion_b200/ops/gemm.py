@@ -435,6 +435,13 @@ def persistent_fits(X: Tensor, batch: int, m: int, n: int, iters: int) -> bool:
     return tiles <= persistent_waves() * sm_count(X.device)
 
 
+def _persistent_bn(m: int, n: int, batch: int, device: torch.device) -> int:
+    """128 x 64 tiles while every phase still is a single wave of them."""
+    g = min(m, n)
+    tiles = max(_num_tiles(g, g, _BM, 64, True), _num_tiles(m, n, _BM, 64, False)) * batch
+    return 64 if tiles <= sm_count(device) else 128
+
+
 def ns_persistent(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs,
                   scale: Optional[Tensor], X2: Optional[Tensor] = None) -> Optional[Tensor]:
     """All iterations in one cooperative launch (csrc/ns_persistent_sm100.cu).  Returns the
@@ -444,11 +451,12 @@ def ns_persistent(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs,
     batch, m, n = X.shape
     dev = X.device
     g = min(m, n)
-    key = (m, n, dev.index)
+    bn = _persistent_bn(m, n, batch, dev)
+    key = (m, n, bn, dev.index)
     tab = _persist_tiles.get(key)
     if tab is None:
-        gg = tile_table(g, g, 128, True, dev)
-        mn = tile_table(m, n, 128, False, dev)
+        gg = tile_table(g, g, bn, True, dev)
+        mn = tile_table(m, n, bn, False, dev)
         tab = _persist_tiles[key] = (torch.cat([gg, mn]).contiguous(), gg.size(0), mn.size(0))
     tiles, n_gg, n_mn = tab
     idx = dev.index if dev.index is not None else torch.cuda.current_device()
@@ -460,7 +468,7 @@ def ns_persistent(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs,
     rc = _backend.lib("ns_persistent_sm100").dion_ns_persistent(
         _p(X), _p(Xalt), _p(X2), _p(A), _p(Bm), ctypes.c_int(batch), ctypes.c_int(m),
         ctypes.c_int(n), flat, ctypes.c_int(len(coeffs)), _p(scale), _p(tiles), ctypes.c_int(n_gg),
-        ctypes.c_int(n_mn), _p(counter), ctypes.c_int(sm_count(dev)), _p(st),
+        ctypes.c_int(n_mn), _p(counter), ctypes.c_int(sm_count(dev)), ctypes.c_int(bn), _p(st),
         ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
     if rc == -20:
         return None
