@@ -498,18 +498,16 @@ normalize_q_kernel(const T* R, const float* colsq, float eps, T* Qstack, const l
 
 
 // ---------------------------------------------------------------------------------------------
-// Blocked upper Cholesky factor (fp32), one CTA of 16 warps per matrix, r a multiple of 32 up to
-// 1024:  G = U^T U.  Right-looking over 32 x 32 blocks, all in the output buffer (which starts as
-// a copy of the upper blocks of G):
-//   for every block row k:  warp 0 factors the diagonal block in registers (lane l owns column
-//                           l; the row being eliminated travels by shuffles) and inverts the
-//                           factor;
-//                           block row:  U[k,j] = inv(U[k,k])^T G[k,j]          one block per warp
-//                           trailing:   G[i,j] -= U[k,i]^T U[k,j], k < i <= j  one block per warp
-// Every product is a 32 x 32 x 32 block operation with the left factor staged in the warp's own
-// shared-memory buffer and the right factor's column in registers.  A non-positive pivot gives
-// NaN, which propagates (the caller's clean-up turns the update into a no-op), as
-// torch.linalg.cholesky_ex does not raise either.
+// Blocked upper Cholesky factor (fp32), G = U^T U, r a multiple of 32 up to 1024: one launch per
+// block row k of 32 x 32 blocks, one CTA per block (k, j), j >= k, of every matrix.  Left-looking:
+//   J = G[k,j] - sum_{m < k} U[m,k]^T U[m,j],   D = G[k,k] - sum_{m < k} U[m,k]^T U[m,k],
+// the sums split over the CTA's warps and added in their order; warp 0 factors D in registers
+// (lane l owns column l, the row being eliminated travels by shuffles) and solves R^T X = J by
+// substitution.  Every CTA factors the same D: that is cheaper than another launch or a wait.
+// One CTA per matrix left a batch of 4 to 16 matrices on as many SMs: 512 x 512 took 780 us for 4
+// or 16 matrices and 853 us for 96 (now 292, 377 and 666 us), 1024 x 1024 4.3 ms for 2 (now 0.8).  A non-positive pivot gives NaN, which propagates (the
+// caller's clean-up turns the update into a no-op), as torch.linalg.cholesky_ex does not raise
+// either.
 // ---------------------------------------------------------------------------------------------
 // Copy the 32 x 32 block A[m0.., a0..] of a row-major matrix into the warp's staging buffer
 // (32 independent coalesced loads per lane).
@@ -543,106 +541,146 @@ __device__ __forceinline__ void mac_t_staged(const float* stage, const float (&x
   }
 }
 
-constexpr int kCholWarps = 16;
+constexpr int kCholWarps = 8;
+constexpr int kCholPart = 32 * 33;
+constexpr int kCholSmem = kCholWarps * (32 * kBlkPitch + kCholPart) * 4;
 
-__global__ void __launch_bounds__(kCholWarps * 32, 1)
-cholesky_blocked_kernel(const float* __restrict__ Gall, float* Uall, int r) {
+// Factor of a 32 x 32 block: lane l owns column l (a[i] = element (i, l)); zero below the diagonal.
+__device__ __forceinline__ void factor_block(float (&a)[32], int l) {
+#pragma unroll
+  for (int q = 0; q < 32; ++q) {
+    const float piv = sqrtf(__shfl_sync(0xffffffffu, a[q], q));   // NaN if not positive
+    const float rq = (l >= q) ? a[q] / piv : 0.f;                 // row q of the factor
+    a[q] = rq;
+#pragma unroll
+    for (int i = q + 1; i < 32; ++i) {
+      const float rqi = __shfl_sync(0xffffffffu, rq, i);
+      a[i] -= rqi * rq;                                           // meaningful for l >= i
+    }
+  }
+}
+
+// R^T X = J by substitution, every lane for its column g; row m of X goes to out[m * ld].
+__device__ __forceinline__ void solve_block(const float* R, float (&g)[32], float* out, int ld) {
+#pragma unroll
+  for (int m = 0; m < 32; ++m) {
+    const float* row = R + m * kBlkPitch;
+    const float y = g[m] / row[m];
+    out[(size_t)m * ld] = y;
+#pragma unroll
+    for (int i = m + 1; i < 32; ++i) g[i] -= row[i] * y;
+  }
+}
+
+__global__ void __launch_bounds__(kCholWarps * 32)
+cholesky_row_kernel(const float* __restrict__ Gall, float* Uall, int r, int k) {
   extern __shared__ __align__(16) float cb_smem[];
-  __shared__ __align__(16) float Yk[32 * kBlkPitch];   // inv(U[k,k]), row-major
-  const int NB = r >> 5;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int j = k + blockIdx.x, k0 = k * 32, j0 = j * 32;
   float* stage = cb_smem + (size_t)w * 32 * kBlkPitch;
-  const float* G = Gall + (size_t)blockIdx.x * r * r;
-  float* U = Uall + (size_t)blockIdx.x * r * r;
+  float* part = cb_smem + (size_t)kCholWarps * 32 * kBlkPitch;   // [warps][32][33]
+  const float* G = Gall + (size_t)blockIdx.y * r * r;
+  float* U = Uall + (size_t)blockIdx.y * r * r;
 
-  // U <- upper blocks of G, zero below.
-  for (int e = threadIdx.x; e < r * (r / 4); e += kCholWarps * 32) {
-    const int row = e / (r / 4), c4 = e - row * (r / 4);
-    const int col = c4 * 4;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if ((col >> 5) >= (row >> 5)) v = *reinterpret_cast<const float4*>(G + (size_t)row * r + col);
-    *reinterpret_cast<float4*>(U + (size_t)row * r + col) = v;
+  float acc[32];
+#pragma unroll
+  for (int a = 0; a < 32; ++a) acc[a] = 0.f;
+  const bool diag = w >= kCholWarps / 2;           // half of the warps for J, half for D
+  for (int m = w % (kCholWarps / 2); m < k; m += kCholWarps / 2) {
+    stage_block(U, r, m * 32, k0, stage, l);       // U[m,k]
+    float x[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q)
+      x[q] = diag ? stage[q * kBlkPitch + l] : U[(size_t)(m * 32 + q) * r + j0 + l];
+    mac_t_staged(stage, x, acc);
+  }
+#pragma unroll
+  for (int a = 0; a < 32; ++a) part[w * kCholPart + a * 33 + l] = acc[a];
+  __syncthreads();
+  float* pj = part;
+  float* pd = part + kCholWarps / 2 * kCholPart;
+  for (int e = threadIdx.x; e < 1024; e += kCholWarps * 32) {
+    const int row = e >> 5, col = e & 31;
+    float sj = 0.f, sd = 0.f;
+#pragma unroll
+    for (int q = 0; q < kCholWarps / 2; ++q) {
+      sj += pj[q * kCholPart + row * 33 + col];
+      sd += pd[q * kCholPart + row * 33 + col];
+    }
+    // (each element of part 0 is read and written by this thread alone)
+    pj[row * 33 + col] = G[(size_t)(k0 + row) * r + j0 + col] - sj;
+    pd[row * 33 + col] = G[(size_t)(k0 + row) * r + k0 + col] - sd;
   }
   __syncthreads();
-
-  for (int k = 0; k < NB; ++k) {
-    const int k0 = k * 32;
-    if (w == 0) {
-      // ---- factor the diagonal block: lane l owns column l (a[i] = element (i, l)) ----
-      float a[32];
+  if (w != 0) return;
+  float a[32];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) a[i] = U[(size_t)(k0 + i) * r + k0 + l];
+  for (int i = 0; i < 32; ++i) a[i] = pd[i * 33 + l];
+  factor_block(a, l);
+  if (j == k) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float piv = sqrtf(__shfl_sync(0xffffffffu, a[j], j));   // NaN if not positive
-        const float rj = (l >= j) ? a[j] / piv : 0.f;                 // row j of the factor
-        a[j] = rj;
-#pragma unroll
-        for (int i = j + 1; i < 32; ++i) {
-          const float rji = __shfl_sync(0xffffffffu, rj, i);
-          a[i] -= rji * rj;                                           // meaningful for l >= i
-        }
-      }
-      // write the factor (zero below the diagonal) and stage it for the inversion
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float v = (l >= i) ? a[i] : 0.f;
-        U[(size_t)(k0 + i) * r + k0 + l] = v;
-        stage[i * kBlkPitch + l] = v;
-      }
-      __syncwarp();
-      // ---- invert it: lane l solves R y = e_l by back substitution ----
-      float y[32];
-      const float* vs = stage;
-#pragma unroll
-      for (int i = 31; i >= 0; --i) {
-        float sacc = (i == l) ? 1.f : 0.f;
-#pragma unroll
-        for (int m = i + 1; m < 32; ++m) sacc -= vs[i * kBlkPitch + m] * y[m];
-        y[i] = sacc / vs[i * kBlkPitch + i];
-      }
-#pragma unroll
-      for (int i = 0; i < 32; ++i) Yk[i * kBlkPitch + l] = y[i];
-    }
-    __syncthreads();
-    // ---- block row: U[k,j] = Yk^T G[k,j] for j > k ----
-    for (int j = k + 1 + w; j < NB; j += kCholWarps) {
-      const int j0 = j * 32;
-      // Without this the 1024 loop-invariant reads of Yk are hoisted out of the loop and spilled.
-      asm volatile("" ::: "memory");
-      float g[32], acc[32];
-#pragma unroll
-      for (int m = 0; m < 32; ++m) {
-        g[m] = U[(size_t)(k0 + m) * r + j0 + l];
-        acc[m] = 0.f;
-      }
-      mac_t_staged(Yk, g, acc);          // acc[a] = sum_m Yk[m][a] * g[m]
-#pragma unroll
-      for (int a = 0; a < 32; ++a) U[(size_t)(k0 + a) * r + j0 + l] = acc[a];
-    }
-    __syncthreads();
-    // ---- trailing update: G[i,j] -= U[k,i]^T U[k,j] for k < i <= j ----
-    const int nt = NB - k - 1;              // trailing blocks per side
-    const int total = nt * (nt + 1) / 2;
-    for (int t = w; t < total; t += kCholWarps) {
-      // t -> (ii, jj) with ii <= jj over the upper triangle, row by row
-      int ii = 0, rem = t;
-      while (rem >= nt - ii) { rem -= nt - ii; ++ii; }
-      const int i = k + 1 + ii, j = i + rem;
-      const int i0 = i * 32, j0 = j * 32;
-      stage_block(U, r, k0, i0, stage, l);       // U[k,i]
-      float xm[32], acc[32];
-#pragma unroll
-      for (int m = 0; m < 32; ++m) {
-        xm[m] = U[(size_t)(k0 + m) * r + j0 + l];
-        acc[m] = 0.f;
-      }
-      mac_t_staged(stage, xm, acc);
-#pragma unroll
-      for (int a = 0; a < 32; ++a) U[(size_t)(i0 + a) * r + j0 + l] -= acc[a];
-    }
-    __syncthreads();
+    for (int i = 0; i < 32; ++i) U[(size_t)(k0 + i) * r + k0 + l] = (l >= i) ? a[i] : 0.f;
+    return;
   }
+#pragma unroll
+  for (int i = 0; i < 32; ++i) stage[i * kBlkPitch + l] = a[i];   // zero below the diagonal
+  __syncwarp();
+  float g[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) g[i] = pj[i * 33 + l];
+  solve_block(stage, g, U + (size_t)k0 * r + j0 + l, r);
+}
+
+// The same for batches that fill the GPU: a CTA takes up to four blocks (k, j) behind one factor of
+// D.  Warps 0 to 3 each accumulate one block in registers, warps 4 to 7 share D's sum.
+__global__ void __launch_bounds__(kCholWarps * 32)
+cholesky_row4_kernel(const float* __restrict__ Gall, float* Uall, int r, int k) {
+  extern __shared__ __align__(16) float cb_smem[];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int k0 = k * 32, j0 = (k + 1 + (int)blockIdx.x * 4 + w) * 32;   // j0: warps 0 to 3
+  const bool mine = w < 4 && j0 < r;
+  float* stage = cb_smem + (size_t)w * 32 * kBlkPitch;
+  float* part = cb_smem + (size_t)kCholWarps * 32 * kBlkPitch;   // [4][32][33]
+  const float* G = Gall + (size_t)blockIdx.y * r * r;
+  float* U = Uall + (size_t)blockIdx.y * r * r;
+  float acc[32];
+#pragma unroll
+  for (int a = 0; a < 32; ++a) acc[a] = 0.f;
+  for (int m = w < 4 ? 0 : w - 4; m < k && (mine || w >= 4); m += w < 4 ? 1 : 4) {
+    stage_block(U, r, m * 32, k0, stage, l);       // U[m,k]
+    float x[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q)
+      x[q] = w >= 4 ? stage[q * kBlkPitch + l] : U[(size_t)(m * 32 + q) * r + j0 + l];
+    mac_t_staged(stage, x, acc);
+  }
+  if (w >= 4) {
+#pragma unroll
+    for (int a = 0; a < 32; ++a) part[(w - 4) * kCholPart + a * 33 + l] = acc[a];
+  }
+  __syncthreads();
+  float* R = cb_smem + (size_t)4 * 32 * kBlkPitch;   // warp 4's staging block
+  if (w == 4) {
+    float a[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      float sd = 0.f;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) sd += part[q * kCholPart + i * 33 + l];
+      a[i] = G[(size_t)(k0 + i) * r + k0 + l] - sd;
+    }
+    factor_block(a, l);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      R[i * kBlkPitch + l] = a[i];
+      if (blockIdx.x == 0) U[(size_t)(k0 + i) * r + k0 + l] = (l >= i) ? a[i] : 0.f;
+    }
+  }
+  __syncthreads();
+  if (!mine) return;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) acc[i] = G[(size_t)(k0 + i) * r + j0 + l] - acc[i];
+  solve_block(R, acc, U + (size_t)k0 * r + j0 + l, r);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -652,8 +690,8 @@ cholesky_blocked_kernel(const float* __restrict__ Gall, float* Uall, int r) {
 //   * V  [kk, 32]: the reflectors, unit lower trapezoidal (kk = k - j rows),
 //   * VT [kk, 32] = V T^T, with T the 32 x 32 upper-triangular factor of
 //     H_0 ... H_31 = I - V T V^T,
-// so that the caller updates the columns to the right of the panel with two products on the
-// tensor cores:  W = V^T A[j:, j+32:],  A[j:, j+32:] -= VT W.
+// with which qr_update_kernel updates the columns to the right of the panel:
+//   W = V^T A[j:, j+32:],  A[j:, j+32:] -= VT W.
 // Within a column, lane = panel column: the dot products of column c with the columns to its
 // right are taken by all warps over interleaved rows, reduced through shared memory, and the
 // rank-one update follows; two block barriers per column.
@@ -667,8 +705,7 @@ __device__ __forceinline__ float qp_v(const float* P, int i, int a) {
 }
 
 __global__ void __launch_bounds__(kQpWarps * 32, 1)
-qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Vall, float* VTall,
-                float* Vlo_all, float* VTlo_all) {
+qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Vall, float* VTall) {
   extern __shared__ __align__(16) float qp_smem[];
   const int kk = k - j;
   float* P = qp_smem;                               // [kk][33]
@@ -682,8 +719,6 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
   float* A = Aall + (size_t)blockIdx.x * strideA + (size_t)j * ld + j;
   float* V = Vall + (size_t)blockIdx.x * k * 32;
   float* VT = VTall + (size_t)blockIdx.x * k * 32;
-  float* Vlo = Vlo_all + (size_t)blockIdx.x * k * 32;
-  float* VTlo = VTlo_all + (size_t)blockIdx.x * k * 32;
 
   for (int i = warp; i < kk; i += kQpWarps) P[i * kQpPitch + lane] = A[(size_t)i * ld + lane];
   for (int e = threadIdx.x; e < 32 * kQpPitch; e += kQpWarps * 32) G[e] = 0.f;
@@ -819,14 +854,101 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
       const float vv = qp_v(P, i, lane);
       V[(size_t)(j + i) * 32 + lane] = vv;
       VT[(size_t)(j + i) * 32 + lane] = acc;
-      // what a tf32 instruction does not see of them (second and third segment of the products)
-      Vlo[(size_t)(j + i) * 32 + lane] = vv - __uint_as_float(__float_as_uint(vv) & 0xFFFFE000u);
-      VTlo[(size_t)(j + i) * 32 + lane] = acc - __uint_as_float(__float_as_uint(acc) & 0xFFFFE000u);
     }
   }
   // the panel's part of R back into A (reflectors are not kept there)
   for (int i = warp; i < 32 && i < kk; i += kQpWarps)
     if (lane >= i) A[(size_t)i * ld + lane] = P[i * kQpPitch + lane];
+}
+
+// Trailing update behind a panel, one CTA per 32 columns of every matrix, lane = column:
+//   W = V^T A (rows split over the warps, the partial sums added in their order),  A -= VT W.
+// The products are 32 deep (or wide), 20 to 40 MFLOP a matrix and panel: as two split-operand tf32
+// products with their remainder passes they took five launches and 125 us a panel for 16 matrices
+// 640 x 512; here 25 us, in fp32 multiply-adds (R^T R off by 2.8e-7 instead of 1.4e-5), with the rows of V and VT as 16-byte broadcasts from shared
+// memory and A read twice, from L2.
+constexpr int kQuWarps = 8;
+constexpr int kQuRows = 64;    // rows of V / VT staged at a time
+
+__global__ void __launch_bounds__(kQuWarps * 32)
+qr_update_kernel(float* Aall, long long strideA, int ld, int k, int j, const float* Vall,
+                 const float* VTall) {
+  __shared__ __align__(16) float vs[kQuRows * 32];
+  __shared__ float part[kQuWarps][32 * 32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int kk = k - j;
+  float* A = Aall + (size_t)blockIdx.y * strideA + (size_t)j * ld + j + 32 + blockIdx.x * 32 + l;
+  const float* V = Vall + ((size_t)blockIdx.y * k + j) * 32;
+  const float* VT = VTall + ((size_t)blockIdx.y * k + j) * 32;
+  constexpr int kPer = kQuRows / kQuWarps;   // rows of a stage that one warp takes
+
+  auto stage = [&](const float* src, int i0) {
+    __syncthreads();
+    const int n4 = (kk - i0 < kQuRows ? kk - i0 : kQuRows) * 8;   // 16-byte pieces
+    for (int e = threadIdx.x; e < n4; e += kQuWarps * 32)
+      reinterpret_cast<float4*>(vs)[e] = __ldg(reinterpret_cast<const float4*>(src + (size_t)i0 * 32) + e);
+    __syncthreads();
+  };
+  float acc[32];
+#pragma unroll
+  for (int a = 0; a < 32; ++a) acc[a] = 0.f;
+  for (int i0 = 0; i0 < kk; i0 += kQuRows) {
+    float x[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int i = i0 + w * kPer + q;
+      x[q] = i < kk ? A[(size_t)i * ld] : 0.f;
+    }
+    stage(V, i0);
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      if (i0 + w * kPer + q >= kk) break;
+      const float4* row = reinterpret_cast<const float4*>(vs + (w * kPer + q) * 32);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float4 v = row[c];
+        acc[c * 4] += v.x * x[q];
+        acc[c * 4 + 1] += v.y * x[q];
+        acc[c * 4 + 2] += v.z * x[q];
+        acc[c * 4 + 3] += v.w * x[q];
+      }
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 32; ++a) part[w][a * 32 + l] = acc[a];
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < 32; ++a) {
+    float t = 0.f;
+#pragma unroll
+    for (int q = 0; q < kQuWarps; ++q) t += part[q][a * 32 + l];
+    acc[a] = t;                                  // W[a][column]
+  }
+  for (int i0 = 0; i0 < kk; i0 += kQuRows) {
+    float x[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int i = i0 + w * kPer + q;
+      x[q] = i < kk ? A[(size_t)i * ld] : 0.f;
+    }
+    stage(VT, i0);
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int i = i0 + w * kPer + q;
+      if (i >= kk) break;
+      const float4* row = reinterpret_cast<const float4*>(vs + (w * kPer + q) * 32);
+      float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float4 v = row[c];
+        s0 += v.x * acc[c * 4];
+        s1 += v.y * acc[c * 4 + 1];
+        s0 += v.z * acc[c * 4 + 2];
+        s1 += v.w * acc[c * 4 + 3];
+      }
+      A[(size_t)i * ld] = x[q] - (s0 + s1);
+    }
+  }
 }
 
 }  // namespace dion
@@ -882,14 +1004,29 @@ DION_EXPORT int dion_cholesky_upper(const void* G, void* U, int n, int r, void* 
       (reinterpret_cast<uintptr_t>(U) & 15) == 0) {
     // blocked kernel (the column-by-column kernel below serves the remaining sizes)
     static bool configured = false;
-    constexpr int kStage = dion::kCholWarps * 32 * dion::kBlkPitch * 4;
     if (!configured) {
-      if (cudaFuncSetAttribute(dion::cholesky_blocked_kernel,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, kStage) != cudaSuccess)
+      if (cudaFuncSetAttribute(dion::cholesky_row_kernel,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, dion::kCholSmem) !=
+              cudaSuccess ||
+          cudaFuncSetAttribute(dion::cholesky_row4_kernel,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, dion::kCholSmem) !=
+              cudaSuccess)
         return -3;
       configured = true;
     }
-    dion::cholesky_blocked_kernel<<<n, dion::kCholWarps * 32, kStage, S(stream)>>>(g, u, r);
+    if (n > 65535) return -2;
+    if (cudaMemsetAsync(u, 0, (size_t)n * r * r * sizeof(float), S(stream)) != cudaSuccess) return -1;
+    for (int k = 0; k < r / 32; ++k) {
+      const int blocks = r / 32 - k;
+      // One block per CTA while that is about two waves of CTAs (96 matrices 512 x 512 with one
+      // block per CTA throughout: 1070 us; with up to four: 666 us).
+      if ((long long)blocks * n <= 296)
+        dion::cholesky_row_kernel<<<dim3(blocks, n), dion::kCholWarps * 32, dion::kCholSmem,
+                                    S(stream)>>>(g, u, r, k);
+      else
+        dion::cholesky_row4_kernel<<<dim3(blocks > 1 ? (blocks + 2) / 4 : 1, n),
+                                     dion::kCholWarps * 32, dion::kCholSmem, S(stream)>>>(g, u, r, k);
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
   }
   if (r <= 256) return launch_chol<8>(g, u, n, r, S(stream));
@@ -975,23 +1112,31 @@ DION_EXPORT int dion_normalize_q(const void* R, const float* colsq, float eps, v
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-// One panel step of the blocked QR on every matrix of A [n][k][ld-pitched rows] (fp32, in
-// place): columns j .. j+31, rows j .. k-1.  V, VT and their tf32 remainders Vlo, VTlo:
-// [n][k][32] (rows j.. written).
-// Limits: j a multiple of 32, j + 32 <= min(k, columns), (k - j) * 33 * 4 bytes + 17 KB of
-// shared memory (k - j <= 1580).
-DION_EXPORT int dion_qr_panel(void* A, long long strideA, int ld, int n, int k, int j, void* V,
-                              void* VT, void* Vlo, void* VTlo, void* stream) {
-  if (n <= 0) return 0;
-  if (j < 0 || (j & 31) || j + 32 > k || j + 32 > ld) return -2;
-  const size_t smem = ((size_t)(k - j) * kQpPitch + kQpWarps * 32 + 96 + 2 * 32 * kQpPitch) *
-                      sizeof(float);
-  if (smem > 226 * 1024) return -2;
+// Upper-triangular factors of n dense fp32 matrices A [k, r] (k >= r, r a multiple of 32), in place:
+// the factor is left in the upper triangle of the first r rows, the rest of A is overwritten.
+// V and VT: [n, k, 32] fp32 scratch, 16-byte aligned.  Two launches per panel of 32 columns.
+DION_EXPORT int dion_qr_blocked(void* A, int n, int k, int r, void* V, void* VT, void* stream) {
+  if (n <= 0 || r <= 0) return 0;
+  if ((r & 31) || k < r || n > 65535 ||
+      ((reinterpret_cast<uintptr_t>(V) | reinterpret_cast<uintptr_t>(VT)) & 15))
+    return -2;
+  auto smem = [&](int j) {
+    return ((size_t)(k - j) * kQpPitch + kQpWarps * 32 + 96 + 2 * 32 * kQpPitch) * sizeof(float);
+  };
+  if (smem(0) > 226 * 1024) return -2;
   if (cudaFuncSetAttribute(dion::qr_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
+                           (int)smem(0)) != cudaSuccess)
     return -3;
-  dion::qr_panel_kernel<<<n, kQpWarps * 32, smem, S(stream)>>>(
-      static_cast<float*>(A), strideA, ld, k, j, static_cast<float*>(V), static_cast<float*>(VT),
-      static_cast<float*>(Vlo), static_cast<float*>(VTlo));
+  float* a = static_cast<float*>(A);
+  float* v = static_cast<float*>(V);
+  float* vt = static_cast<float*>(VT);
+  for (int j = 0; j < r; j += 32) {
+    dion::qr_panel_kernel<<<n, kQpWarps * 32, smem(j), S(stream)>>>(a, (long long)k * r, r, k, j, v,
+                                                                    vt);
+    const int blocks = (r - j) / 32 - 1;
+    if (blocks > 0)
+      dion::qr_update_kernel<<<dim3(blocks, n), dion::kQuWarps * 32, 0, S(stream)>>>(
+          a, (long long)k * r, r, k, j, v, vt);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

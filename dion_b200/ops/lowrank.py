@@ -301,7 +301,9 @@ def householder_q(P: Tensor) -> Tensor:
 
 _QR_PANEL = 32
 _QR_PANEL_MAX_ROWS = 1580      # shared memory of the panel kernel: (rows * 33 + ...) * 4 bytes
-_QR_BLOCKED_MIN_COLS = 256     # below this the single-kernel form wins (five launches per panel)
+# The single-kernel form takes 205 us for 16 matrices 160 x 128 and 424 us for 12 of 240 x 192, the
+# blocked one 174 and 316 us; narrower sketches are left to the former.
+_QR_BLOCKED_MIN_COLS = 128
 
 
 def blocked_qr_enabled() -> bool:
@@ -311,35 +313,23 @@ def blocked_qr_enabled() -> bool:
 def _qr_r_blocked(A32: Tensor) -> Tensor:
     """Blocked Householder QR of a private fp32 batch ``[B, k, r]`` (overwritten): per 32-column
     panel one kernel factors the panel in shared memory (one CTA per matrix) and emits the
-    reflectors ``V`` and ``V T^T`` of the compact WY form; the columns to the right are then
-    updated by two tensor-core products over the whole batch, ``W = V^T A_right`` and
-    ``A_right -= (V T^T) W`` (split operands: the factor is only as good as these)."""
+    reflectors ``V`` and ``V T^T`` of the compact WY form; a second one updates the columns to the
+    right, ``W = V^T A_right`` and ``A_right -= (V T^T) W``, in fp32."""
     B, k, r = A32.shape
     dev = A32.device
-    V, VT, Vlo, VTlo = torch.empty((4, B, k, _QR_PANEL), dtype=torch.float32, device=dev).unbind(0)
-    W = torch.empty((B, _QR_PANEL, r), dtype=torch.float32, device=dev)
-    lib = _backend.lib("lowrank_ops")
-    for j in range(0, r, _QR_PANEL):
-        rc = lib.dion_qr_panel(_ptr(A32), ctypes.c_longlong(k * r), r, B, k, j, _ptr(V), _ptr(VT),
-                               _ptr(Vlo), _ptr(VTlo), _stream(dev))
-        if rc != 0:
-            raise RuntimeError(f"dion_qr_panel launch failed (code {rc})")
-        nt = r - j - _QR_PANEL
-        if nt <= 0:
-            break
-        right = A32[:, j:, j + _QR_PANEL:]
-        Wv = W[:, :, :nt]
-        lr_gemm(V[:, j:, :], right, a_mn=True, b_mn=True, out=Wv, precise=True,
-                a_lo=Vlo[:, j:, :])
-        lr_gemm(VT[:, j:, :], Wv, b_mn=True, D=right, out=right, alpha=-1.0, beta=1.0,
-                precise=True, a_lo=VTlo[:, j:, :])
+    V, VT = torch.empty((2, B, k, _QR_PANEL), dtype=torch.float32, device=dev).unbind(0)
+    rc = _backend.lib("lowrank_ops").dion_qr_blocked(_ptr(A32), B, k, r, _ptr(V), _ptr(VT),
+                                                     _stream(dev))
+    if rc != 0:
+        raise RuntimeError(f"dion_qr_blocked launch failed (code {rc})")
+    _backend.add_launches(2 * (r // _QR_PANEL) - 2)
     return torch.triu(A32[:, :r, :r])
 
 
 def qr_r_factor(A: Tensor, overwrite: bool = False) -> Tensor:
     """Upper-triangular factor of every ``A[b]`` (``[B, k, r]``, ``k >= r``) in fp32.  On a GPU
-    all matrices of the batch are factored together: blocked Householder with the trailing
-    updates on the tensor cores when ``r`` is a multiple of 32 (at least 256), else one kernel
+    all matrices of the batch are factored together: blocked Householder, two kernels per panel,
+    when ``r`` is a multiple of 32 (at least 128), else one kernel
     with one CTA per matrix (up to 1024 rows).  The sign of a row of ``R`` may differ from
     LAPACK's.  ``overwrite``: ``A`` is a temporary of the caller and may be destroyed."""
     A32 = A.to(torch.float32)

@@ -234,17 +234,20 @@ def test_aol_rescale_matches_torch():
 @pytest.mark.parametrize("cautious", [False, True])
 def test_adamw_sizes_alignment_and_shared_counters(dtype, cautious):
     """Sizes around the 16-byte and 4096-element boundaries of the kernel, a tensor that starts off
-    a 16-byte boundary, counters shared by several parameters; against the PyTorch form on the CPU.
-    fp32 arithmetic in the same order on both sides: one unit in the last place of the dtype."""
-    from dion_b200.ops import foreach as F
+    a 16-byte boundary, counters shared by several parameters; against the PyTorch form on the CPU
+    in fp32.  The two may round differently in four places (fused multiply-adds), each 2^-24 of an
+    intermediate, and a bf16 result (8 significant bits) is half a unit, 2^-8, off."""
     torch.manual_seed(0)
     sizes = [8, 4096, 4096 + 8, 8192 + 12, 3, 40000]
-    make = lambda: [torch.randn(n) for n in sizes]  # noqa: E731
-    ref = [[t.to(dtype) for t in make()] for _ in range(3)] + [[t.square().to(dtype) for t in make()]]
+
     def moved(t):
         base = torch.empty(t.numel() + 1, dtype=dtype, device="cuda")
         out = base[1:] if t.numel() == 40000 else base[:-1]
         return out.copy_(t)
+
+    ref = [[torch.randn(n).to(dtype).float() for n in sizes] for _ in range(3)]
+    ref.append([torch.rand(n).to(dtype).float() for n in sizes])
+    scale = [2 * x.abs() + g.abs() + g.square() + m.abs() + v for x, g, m, v in zip(*ref)]
     dev = [[moved(t) for t in lst] for lst in ref]
     shared = torch.full((), 6.0)
     steps = [shared, torch.full((), 1.0), shared, shared, torch.full((), 300.0), shared]
@@ -254,8 +257,9 @@ def test_adamw_sizes_alignment_and_shared_counters(dtype, cautious):
     F.adamw(*dev, lr.cuda(), 0.9, 0.95, 0.1, 1e-8, state_steps=[on[id(s)] for s in steps],
             cautious_wd=cautious)
     assert all(on[id(s)].item() == s.item() for s in steps) and shared.item() == 7.0
-    ulp = 2.0 ** -22 if dtype == torch.float32 else 2.0 ** -7
+    half = 0.0 if dtype == torch.float32 else 2.0 ** -8
     for a, b in zip(ref, dev):
-        for x, y in zip(a, b):
-            err = (x.float() - y.float().cpu()).abs()
-            assert (err <= ulp * (x.float().abs() + 0.1)).all(), err.max()
+        for x, y, s in zip(a, b, scale):
+            err = (x - y.float().cpu()).abs()
+            bound = half * x.abs() + 4 * 2.0 ** -24 * (s + x.abs())
+            assert (err <= bound).all(), (err - bound).max()

@@ -89,6 +89,12 @@ def test_blocked_qr_equals_column_kernel_up_to_signs():
     assert (Rb.abs() - Rc.abs()).abs().max().item() < 1e-3 * Rc.abs().max().item()
 
 
+@pytest.mark.parametrize("shape", [(150, 96), (60, 160), (40, 512), (400, 64)])
+def test_cholesky_upper_of_large_batches(shape):
+    """More blocks than two waves: up to four of a block row per CTA, then one, every remainder."""
+    test_cholesky_upper(shape)
+
+
 @pytest.mark.parametrize("shape", [(3, 96), (5, 192), (2, 512), (2, 768), (4, 17), (2, 64), (1, 1024)])
 def test_cholesky_upper(shape):
     from dion_b200.ops import lowrank as LR
