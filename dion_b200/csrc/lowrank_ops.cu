@@ -697,7 +697,8 @@ cholesky_row4_kernel(const float* __restrict__ Gall, float* Uall, int r, int k) 
 // rank-one update follows; two block barriers per column.
 // ---------------------------------------------------------------------------------------------
 constexpr int kQpWarps = 16;
-constexpr int kQpPitch = 33;
+constexpr int kQpPitch = 32;   // the panel is only ever read along its rows
+constexpr int kQpSq = 36;      // pitch of the 32 x 32 factors: 16-byte rows, columns spread over banks
 
 // Reflector entry (i, a) of the panel held in P: zero above the diagonal, one on it.
 __device__ __forceinline__ float qp_v(const float* P, int i, int a) {
@@ -708,20 +709,20 @@ __global__ void __launch_bounds__(kQpWarps * 32, 1)
 qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Vall, float* VTall) {
   extern __shared__ __align__(16) float qp_smem[];
   const int kk = k - j;
-  float* P = qp_smem;                               // [kk][33]
+  float* P = qp_smem;                               // [kk][32]
   float* part = P + (size_t)kk * kQpPitch;          // [16][32]
   float* wv = part + kQpWarps * 32;                 // [32]  w of the current column
   float* taus = wv + 32;                            // [32]
   float* sc = taus + 32;                            // [32]  1 / (alpha - beta) per column
-  float* G = sc + 32;                               // [32][33]  V^T V (strictly upper part used)
-  float* T = G + 32 * kQpPitch;                     // [32][33]
+  float* G = sc + 32;                               // [32][36]  V^T V (strictly upper part used)
+  float* T = G + 32 * kQpSq;                        // [32][36]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* A = Aall + (size_t)blockIdx.x * strideA + (size_t)j * ld + j;
   float* V = Vall + (size_t)blockIdx.x * k * 32;
   float* VT = VTall + (size_t)blockIdx.x * k * 32;
 
   for (int i = warp; i < kk; i += kQpWarps) P[i * kQpPitch + lane] = A[(size_t)i * ld + lane];
-  for (int e = threadIdx.x; e < 32 * kQpPitch; e += kQpWarps * 32) G[e] = 0.f;
+  for (int e = threadIdx.x; e < 32 * kQpSq; e += kQpWarps * 32) G[e] = 0.f;
   __syncthreads();
 
   // Dot products of column 0 with every column, over the rows below the diagonal.
@@ -814,26 +815,35 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
 #pragma unroll
         for (int a = 0; a < 32; ++a) g[a] += qp_v(P, i, a) * vc;
       } else {
+        const float4* row = reinterpret_cast<const float4*>(P + i * kQpPitch);
 #pragma unroll
-        for (int a = 0; a < 32; ++a) g[a] += P[i * kQpPitch + a] * vc;
+        for (int a = 0; a < 8; ++a) {
+          const float4 u = row[a];
+          g[4 * a] += u.x * vc;
+          g[4 * a + 1] += u.y * vc;
+          g[4 * a + 2] += u.z * vc;
+          g[4 * a + 3] += u.w * vc;
+        }
       }
     }
 #pragma unroll
-    for (int a = 0; a < 32; ++a) atomicAdd(&G[a * kQpPitch + lane], g[a]);
+    for (int a = 0; a < 32; ++a) atomicAdd(&G[a * kQpSq + lane], g[a]);
   }
   __syncthreads();
   // T by columns (lane = row a):  T[a][c] = -tau_c * sum_{b = a}^{c-1} T[a][b] G[b][c],  T[c][c] = tau_c
+  // Column c is final once the columns before it have been subtracted: each is taken from all
+  // later sums at once, so the chain is 32 steps of independent multiply-adds.
   if (warp == 0) {
     float t[32];
 #pragma unroll
-    for (int c = 0; c < 32; ++c) {
-      float sacc = 0.f;
+    for (int c = 0; c < 32; ++c) t[c] = 0.f;
 #pragma unroll
-      for (int b = 0; b < 32; ++b)
-        if (b < c) sacc += (b >= lane ? t[b] : 0.f) * G[b * kQpPitch + c];
+    for (int c = 0; c < 32; ++c) {
       const float tc = taus[c];
-      t[c] = lane < c ? -tc * sacc : (lane == c ? tc : 0.f);
-      T[lane * kQpPitch + c] = t[c];
+      const float v = lane < c ? -tc * t[c] : (lane == c ? tc : 0.f);
+      T[lane * kQpSq + c] = v;
+#pragma unroll
+      for (int d = c + 1; d < 32; ++d) t[d] += v * G[c * kQpSq + d];
     }
   }
   __syncthreads();
@@ -841,15 +851,24 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
   {
     float trow[32];
 #pragma unroll
-    for (int c = 0; c < 32; ++c) trow[c] = T[lane * kQpPitch + c];
+    for (int c = 0; c < 32; ++c) trow[c] = T[lane * kQpSq + c];
     for (int i = warp; i < kk; i += kQpWarps) {
       float acc = 0.f;
       if (i < 32) {
 #pragma unroll
         for (int c = 0; c < 32; ++c) acc += qp_v(P, i, c) * trow[c];
       } else {
+        const float4* row = reinterpret_cast<const float4*>(P + i * kQpPitch);
+        float acc1 = 0.f;
 #pragma unroll
-        for (int c = 0; c < 32; ++c) acc += P[i * kQpPitch + c] * trow[c];
+        for (int c = 0; c < 8; ++c) {
+          const float4 u = row[c];
+          acc += u.x * trow[4 * c];
+          acc1 += u.y * trow[4 * c + 1];
+          acc += u.z * trow[4 * c + 2];
+          acc1 += u.w * trow[4 * c + 3];
+        }
+        acc += acc1;
       }
       const float vv = qp_v(P, i, lane);
       V[(size_t)(j + i) * 32 + lane] = vv;
@@ -865,8 +884,8 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
 //   W = V^T A (rows split over the warps, the partial sums added in their order),  A -= VT W.
 // The products are 32 deep (or wide), 20 to 40 MFLOP a matrix and panel: as two split-operand tf32
 // products with their remainder passes they took five launches and 125 us a panel for 16 matrices
-// 640 x 512; here 25 us, in fp32 multiply-adds (R^T R off by 2.8e-7 instead of 1.4e-5), with the rows of V and VT as 16-byte broadcasts from shared
-// memory and A read twice, from L2.
+// 640 x 512; here 25 us, in fp32 multiply-adds (R^T R off by 2.8e-7 instead of 1.4e-5), with the
+// rows of V and VT as 16-byte broadcasts from shared memory and A read twice, from L2.
 constexpr int kQuWarps = 8;
 constexpr int kQuRows = 64;    // rows of V / VT staged at a time
 
@@ -1121,7 +1140,7 @@ DION_EXPORT int dion_qr_blocked(void* A, int n, int k, int r, void* V, void* VT,
       ((reinterpret_cast<uintptr_t>(V) | reinterpret_cast<uintptr_t>(VT)) & 15))
     return -2;
   auto smem = [&](int j) {
-    return ((size_t)(k - j) * kQpPitch + kQpWarps * 32 + 96 + 2 * 32 * kQpPitch) * sizeof(float);
+    return ((size_t)(k - j) * kQpPitch + kQpWarps * 32 + 96 + 2 * 32 * kQpSq) * sizeof(float);
   };
   if (smem(0) > 226 * 1024) return -2;
   if (cudaFuncSetAttribute(dion::qr_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
