@@ -694,7 +694,11 @@ cholesky_row4_kernel(const float* __restrict__ Gall, float* Uall, int r, int k) 
 //   W = V^T A[j:, j+32:],  A[j:, j+32:] -= VT W.
 // Within a column, lane = panel column: the dot products of column c with the columns to its
 // right are taken by all warps over interleaved rows, reduced through shared memory, and the
-// rank-one update follows; two block barriers per column.
+// rank-one update follows; two block barriers per column.  A warp keeps its rows in registers while
+// they number at most NR (16 warps, so up to 16 * NR rows): a row then costs one shuffle and two
+// multiply-adds per column, where shared memory took four accesses, a shuffle and as many
+// multiply-adds (whole factorization of 16 matrices 640 x 512: 1421 -> 1131 us).  Taller panels
+// (NR = 0) stay in shared memory.
 // ---------------------------------------------------------------------------------------------
 constexpr int kQpWarps = 16;
 constexpr int kQpPitch = 32;   // the panel is only ever read along its rows
@@ -705,6 +709,7 @@ __device__ __forceinline__ float qp_v(const float* P, int i, int a) {
   return i > a ? P[i * kQpPitch + a] : (i == a ? 1.f : 0.f);
 }
 
+template <int NR>
 __global__ void __launch_bounds__(kQpWarps * 32, 1)
 qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Vall, float* VTall) {
   extern __shared__ __align__(16) float qp_smem[];
@@ -721,15 +726,33 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
   float* V = Vall + (size_t)blockIdx.x * k * 32;
   float* VT = VTall + (size_t)blockIdx.x * k * 32;
 
-  for (int i = warp; i < kk; i += kQpWarps) P[i * kQpPitch + lane] = A[(size_t)i * ld + lane];
+  // Row warp + 16 q of the panel in v[q], its entry in the current column in x[q].
+  float v[NR > 0 ? NR : 1], x[NR > 0 ? NR : 1];
+  if (NR > 0) {
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      const int i = warp + q * kQpWarps;
+      v[q] = i < kk ? A[(size_t)i * ld + lane] : 0.f;
+      x[q] = __shfl_sync(0xffffffffu, v[q], 0);
+      if (q < 2) P[i * kQpPitch + lane] = v[q];     // rows that become pivot rows (kk >= 32)
+    }
+  } else {
+    for (int i = warp; i < kk; i += kQpWarps) P[i * kQpPitch + lane] = A[(size_t)i * ld + lane];
+  }
   for (int e = threadIdx.x; e < 32 * kQpSq; e += kQpWarps * 32) G[e] = 0.f;
   __syncthreads();
 
   // Dot products of column 0 with every column, over the rows below the diagonal.
   {
     float acc = 0.f;
-    for (int i = 1 + warp; i < kk; i += kQpWarps)
-      acc += P[i * kQpPitch] * P[i * kQpPitch + lane];
+    if (NR > 0) {
+#pragma unroll
+      for (int q = 0; q < NR; ++q)
+        if (q > 0 || warp > 0) acc += x[q] * v[q];
+    } else {
+      for (int i = 1 + warp; i < kk; i += kQpWarps)
+        acc += P[i * kQpPitch] * P[i * kQpPitch + lane];
+    }
     part[warp * 32 + lane] = acc;
   }
   __syncthreads();
@@ -766,40 +789,62 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
     const float ws = wv[lane] * sc[c];
     const int cn = (c + 1) & 31;
     float a0 = 0.f, a1 = 0.f;
-    int i = c + 1 + warp;
-    for (; i + kQpWarps < kk; i += 2 * kQpWarps) {
-      float* p0 = P + i * kQpPitch;
-      float* p1 = p0 + kQpWarps * kQpPitch;
-      const float x0 = p0[c], x1 = p1[c];
-      float v0 = p0[lane], v1 = p1[lane];
-      if (lane > c) {
-        v0 -= x0 * ws;
-        v1 -= x1 * ws;
-        p0[lane] = v0;
-        p1[lane] = v1;
+    if (NR > 0) {
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        const int i = warp + q * kQpWarps;
+        if (q < 2 && i <= c) continue;               // pivot rows are finished (in P)
+        if (lane > c) v[q] -= x[q] * ws;
+        x[q] = __shfl_sync(0xffffffffu, v[q], cn);
+        if (q < 2) P[i * kQpPitch + lane] = v[q];
+        if (q >= 2 || i > c + 1) {
+          if (q & 1) a1 += x[q] * v[q];
+          else a0 += x[q] * v[q];
+        }
       }
-      const float n0 = __shfl_sync(0xffffffffu, v0, cn), n1 = __shfl_sync(0xffffffffu, v1, cn);
-      if (i > c + 1) a0 += n0 * v0;
-      a1 += n1 * v1;
-    }
-    if (i < kk) {
-      float* p0 = P + i * kQpPitch;
-      const float x0 = p0[c];
-      float v0 = p0[lane];
-      if (lane > c) {
-        v0 -= x0 * ws;
-        p0[lane] = v0;
+    } else {
+      int i = c + 1 + warp;
+      for (; i + kQpWarps < kk; i += 2 * kQpWarps) {
+        float* p0 = P + i * kQpPitch;
+        float* p1 = p0 + kQpWarps * kQpPitch;
+        const float x0 = p0[c], x1 = p1[c];
+        float v0 = p0[lane], v1 = p1[lane];
+        if (lane > c) {
+          v0 -= x0 * ws;
+          v1 -= x1 * ws;
+          p0[lane] = v0;
+          p1[lane] = v1;
+        }
+        const float n0 = __shfl_sync(0xffffffffu, v0, cn), n1 = __shfl_sync(0xffffffffu, v1, cn);
+        if (i > c + 1) a0 += n0 * v0;
+        a1 += n1 * v1;
       }
-      const float n0 = __shfl_sync(0xffffffffu, v0, cn);
-      if (i > c + 1) a0 += n0 * v0;
+      if (i < kk) {
+        float* p0 = P + i * kQpPitch;
+        const float x0 = p0[c];
+        float v0 = p0[lane];
+        if (lane > c) {
+          v0 -= x0 * ws;
+          p0[lane] = v0;
+        }
+        const float n0 = __shfl_sync(0xffffffffu, v0, cn);
+        if (i > c + 1) a0 += n0 * v0;
+      }
     }
     part[warp * 32 + lane] = a0 + a1;   // read by warp 0 only after the next barrier
     __syncthreads();
   }
-  // scale the reflector tails: V[i][a] = P[i][a] * sc[a] for i > a
+  if (NR > 0) {
+#pragma unroll
+    for (int q = 2; q < NR; ++q) {
+      const int i = warp + q * kQpWarps;
+      if (i < kk) P[i * kQpPitch + lane] = v[q];
+    }
+  }
+  // scale the reflector tails: V[i][a] = P[i][a] * sc[a] for i > a (a warp's own rows)
   {
     const float scl = sc[lane];
-    for (int i = 1 + warp; i < kk; i += kQpWarps)
+    for (int i = warp; i < kk; i += kQpWarps)
       if (i > lane) P[i * kQpPitch + lane] *= scl;
   }
   __syncthreads();
@@ -1143,15 +1188,21 @@ DION_EXPORT int dion_qr_blocked(void* A, int n, int k, int r, void* V, void* VT,
     return ((size_t)(k - j) * kQpPitch + kQpWarps * 32 + 96 + 2 * 32 * kQpSq) * sizeof(float);
   };
   if (smem(0) > 226 * 1024) return -2;
-  if (cudaFuncSetAttribute(dion::qr_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem(0)) != cudaSuccess)
-    return -3;
+  // Registers for 16, 32 or 48 rows per warp (256, 512, 768 rows), else shared memory.
+  typedef void (*Panel)(float*, long long, int, int, int, float*, float*);
+  const Panel panels[4] = {dion::qr_panel_kernel<16>, dion::qr_panel_kernel<32>,
+                           dion::qr_panel_kernel<48>, dion::qr_panel_kernel<0>};
+  for (Panel f : panels)
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(0)) !=
+        cudaSuccess)
+      return -3;
   float* a = static_cast<float*>(A);
   float* v = static_cast<float*>(V);
   float* vt = static_cast<float*>(VT);
   for (int j = 0; j < r; j += 32) {
-    dion::qr_panel_kernel<<<n, kQpWarps * 32, smem(j), S(stream)>>>(a, (long long)k * r, r, k, j, v,
-                                                                    vt);
+    const int rows = k - j;
+    const Panel panel = panels[rows <= 256 ? 0 : rows <= 512 ? 1 : rows <= 768 ? 2 : 3];
+    panel<<<n, kQpWarps * 32, smem(j), S(stream)>>>(a, (long long)k * r, r, k, j, v, vt);
     const int blocks = (r - j) / 32 - 1;
     if (blocks > 0)
       dion::qr_update_kernel<<<dim3(blocks, n), dion::kQuWarps * 32, 0, S(stream)>>>(
