@@ -4,17 +4,22 @@
 // dense embedding backward under its compiler (models/gpt_model.py:298-307: `nn.Embedding`), which
 // zero-fills the [V, C] gradient and scatters into it with atomics.
 //
-// Four launches, no host synchronisation, scratch supplied by the caller:
+// Five launches, no host synchronisation, scratch supplied by the caller:
 //   1. keys[i] = id (V for ids outside [0, V)), vals[i] = i as 32-bit integers;
 //   2. a stable radix sort of the (key, position) pairs over just the bits an id needs
 //      (CUB's device-wide sort; 16 bits for a 50 K vocabulary instead of the 64 of a sort of the
 //      id tensor itself), so that every id's positions are consecutive and ascending;
 //   3. starts[v] = first sorted index whose key is >= v, one thread per v (binary search) - the
 //      run of row v is [starts[v], starts[v+1]);
-//   4. one warp per row of GW sums the run in fp32 in position order, or writes zeros.  Runs
-//      longer than kEmbLongRun are split into contiguous segments over the block's warps and the
-//      partial sums added in segment order: real token streams have ids that occur thousands of
-//      times per batch, and one warp walking such a run alone would decide the kernel's duration.
+//   4. one block per chunk of sorted positions (64 up to 65536 tokens) sums the parts of runs longer
+//      than a chunk that lie in it.  Such a run covers the first or the last position of every
+//      chunk it meets, so a chunk has two slots;
+//   5. one warp per row of GW sums the run in fp32 in position order, or its parts in chunk order,
+//      or writes zeros.
+// Real token streams have ids that occur thousands of times per batch, and vocabularies are often
+// ordered by frequency, so that the longest runs are neighbours: with each of them summed by the
+// block of its row, 32768 tokens of rank-one-over-frequency text (768 columns) took 919 us, all but
+// a few of them in the first block.
 #include <cub/device/device_radix_sort.cuh>
 
 #include "common.cuh"
@@ -60,7 +65,7 @@ emb_starts_kernel(const int* __restrict__ sorted, int* __restrict__ starts, int 
 }
 
 constexpr int kEmbWarps = 8;
-constexpr int kEmbLongRun = 64;
+constexpr int kEmbChunk = 64;        // sorted positions per chunk, doubled until 1024 chunks suffice
 
 // acc += the rows perm[j] of DY for j in [j0, j1), columns [c8*8, c8*8+8), four loads in flight.
 __device__ __forceinline__ void emb_sum_run(const void* __restrict__ DY, int dy_dt,
@@ -84,54 +89,87 @@ __device__ __forceinline__ void emb_sum_run(const void* __restrict__ DY, int dy_
   }
 }
 
+// part[2 * c + slot][C] = sum over the positions of chunk c that belong to the long run covering its
+// first (slot 0) or its last position (slot 1, if that is another run).
 __global__ void __launch_bounds__(kEmbWarps * 32)
-embedding_bwd_kernel(const int* __restrict__ starts, const int* __restrict__ perm,
-                     const void* __restrict__ DY, int dy_dt, float* __restrict__ GW, int C,
-                     int V) {
+emb_parts_kernel(const int* __restrict__ sorted, const int* __restrict__ starts,
+                 const int* __restrict__ perm, const void* __restrict__ DY, int dy_dt,
+                 float* __restrict__ part, int n, int C, int V, int chunk) {
   extern __shared__ __align__(16) float emb_part[];          // [kEmbWarps][C]
-  __shared__ int run_lo[kEmbWarps], run_hi[kEmbWarps];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int C8 = C / 8;
-  // Every block walks whole groups of kEmbWarps rows so that its barriers stay uniform.
-  for (int base = blockIdx.x * kEmbWarps; base < V; base += gridDim.x * kEmbWarps) {
-    const int v = base + w;
-    int s = 0, e = 0;
-    if (v < V) { s = starts[v]; e = starts[v + 1]; }
-    if (lane == 0) { run_lo[w] = s; run_hi[w] = e; }
-    if (v < V && e - s <= kEmbLongRun) {
-      for (int c8 = lane; c8 < C8; c8 += 32) {
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        emb_sum_run(DY, dy_dt, perm, s, e, C, c8, acc);
-        float4* q = reinterpret_cast<float4*>(GW + (long long)v * C + c8 * 8);
-        q[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-        q[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
-      }
+  const int p0 = blockIdx.x * chunk, p1 = p0 + chunk < n ? p0 + chunk : n;
+  const int first = sorted[p0], last = sorted[p1 - 1];
+  for (int slot = 0; slot < 2; ++slot) {
+    const int v = slot == 0 ? first : last;
+    if (v >= V || (slot == 1 && first == last)) continue;    // ids outside the table sort last
+    const int s = starts[v], e = starts[v + 1];
+    if (e - s <= chunk) continue;                            // the same in every thread
+    const int lo = s > p0 ? s : p0, hi = e < p1 ? e : p1;
+    const int seg = (hi - lo + kEmbWarps - 1) / kEmbWarps;
+    const int j0 = lo + w * seg < hi ? lo + w * seg : hi, j1 = j0 + seg < hi ? j0 + seg : hi;
+    for (int c8 = lane; c8 < C / 8; c8 += 32) {
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      emb_sum_run(DY, dy_dt, perm, j0, j1, C, c8, acc);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) emb_part[(size_t)w * C + c8 * 8 + q] = acc[q];
     }
     __syncthreads();
-    for (int ww = 0; ww < kEmbWarps; ++ww) {
-      const int ls = run_lo[ww], le = run_hi[ww];
-      if (le - ls <= kEmbLongRun) continue;                  // same decision in every thread
-      const int seg = (le - ls + kEmbWarps - 1) / kEmbWarps;
-      int j0 = ls + w * seg, j1 = j0 + seg;
-      if (j0 > le) j0 = le;
-      if (j1 > le) j1 = le;
-      for (int c8 = lane; c8 < C8; c8 += 32) {
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        emb_sum_run(DY, dy_dt, perm, j0, j1, C, c8, acc);
+    float* out = part + (size_t)(2 * blockIdx.x + slot) * C;
+    for (int c = threadIdx.x; c < C; c += kEmbWarps * 32) {
+      float t = 0.f;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) emb_part[(size_t)w * C + c8 * 8 + q] = acc[q];
-      }
-      __syncthreads();
-      for (int c = threadIdx.x; c < C; c += kEmbWarps * 32) {
-        float t = 0.f;
-#pragma unroll
-        for (int q = 0; q < kEmbWarps; ++q) t += emb_part[(size_t)q * C + c];
-        GW[(long long)(base + ww) * C + c] = t;
-      }
-      __syncthreads();
+      for (int q = 0; q < kEmbWarps; ++q) t += emb_part[(size_t)q * C + c];
+      out[c] = t;
     }
-    __syncthreads();                                          // run_lo / run_hi are rewritten next
+    __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(kEmbWarps * 32)
+embedding_bwd_kernel(const int* __restrict__ starts, const int* __restrict__ perm,
+                     const void* __restrict__ DY, int dy_dt, const float* __restrict__ part,
+                     float* __restrict__ GW, int C, int V, int chunk) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int v = blockIdx.x * kEmbWarps + w; v < V; v += gridDim.x * kEmbWarps) {
+    const int s = starts[v], e = starts[v + 1];
+    const bool parts = e - s > chunk;
+    // The first chunk holds the run in slot 0 only if the run covers its first position.
+    const int c0 = s / chunk, c1 = (e - 1) / chunk;
+    for (int c8 = lane; c8 < C / 8; c8 += 32) {
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (parts) {
+        const float* p = part + c8 * 8;
+        emb_load8(p, DT_F32, (long long)(2 * c0 + (s % chunk != 0)) * C, acc);
+        int c = c0 + 1;
+        for (; c + 3 <= c1; c += 4) {
+          float u[4][8];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) emb_load8(p, DT_F32, (long long)(2 * (c + q)) * C, u[q]);
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int x = 0; x < 8; ++x) acc[x] += u[q][x];
+        }
+        for (; c <= c1; ++c) {
+          float u[8];
+          emb_load8(p, DT_F32, (long long)(2 * c) * C, u);
+#pragma unroll
+          for (int x = 0; x < 8; ++x) acc[x] += u[x];
+        }
+      } else {
+        emb_sum_run(DY, dy_dt, perm, s, e, C, c8, acc);
+      }
+      float4* q = reinterpret_cast<float4*>(GW + (long long)v * C + c8 * 8);
+      q[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+      q[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    }
+  }
+}
+
+static inline int emb_chunk(long long n) {
+  long long chunk = kEmbChunk;
+  while ((n + chunk - 1) / chunk > 1024) chunk *= 2;
+  return static_cast<int>(chunk);
 }
 
 static inline int key_bits(long long V) {   // bits needed for the values 0 .. V
@@ -157,13 +195,22 @@ DION_EXPORT long long dion_embedding_sort_bytes(long long n, long long V) {
   return static_cast<long long>(bytes);
 }
 
+// Rows of C floats that the partial sums of n tokens need.
+DION_EXPORT long long dion_embedding_part_rows(long long n) {
+  if (n <= 0) return 0;
+  const long long chunk = emb_chunk(n);
+  return 2 * ((n + chunk - 1) / chunk);
+}
+
 // ids: int64 [n].  DY: [n, C] fp32 or bf16 (dy_dt).  GW: fp32 [V, C], needs no initialisation.
 // Scratch: keys, vals int32 [2n] each (unsorted then sorted halves), starts int32 [V+1], temp of
-// at least dion_embedding_sort_bytes(n, V) bytes.  Limits: n, V < 2^31; 8*C*4 bytes of shared
+// at least dion_embedding_sort_bytes(n, V) bytes, part fp32 [dion_embedding_part_rows(n), C], 16-byte
+// aligned.  Limits: n, V < 2^31; 8*C*4 bytes of shared
 // memory (C <= 7168); C a multiple of 8.
 DION_EXPORT int dion_embedding_bwd(const void* ids, const void* DY, int dy_dt, float* GW,
                                    long long n, int C, long long V, int* keys, int* vals,
-                                   int* starts, void* temp, long long temp_bytes, void* stream) {
+                                   int* starts, void* temp, long long temp_bytes, float* part,
+                                   void* stream) {
   if (V <= 0) return 0;
   if (C % 8 || n < 0 || n >= (1LL << 31) - 256 || V >= (1LL << 31) - 256) return -2;
   const size_t smem = (size_t)kEmbWarps * C * sizeof(float);
@@ -179,12 +226,16 @@ DION_EXPORT int dion_embedding_bwd(const void* ids, const void* DY, int dy_dt, f
   }
   emb_starts_kernel<<<(Vi + 1 + 255) / 256, 256, 0, S(stream)>>>(keys + ni, starts, ni, Vi);
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(embedding_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute(emb_parts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
     return -3;
+  const int chunk = emb_chunk(n);
+  if (ni > chunk)   // else no run is longer than a chunk
+    emb_parts_kernel<<<(ni + chunk - 1) / chunk, kEmbWarps * 32, smem, S(stream)>>>(
+        keys + ni, starts, vals + ni, DY, dy_dt, part, ni, C, Vi, chunk);
   const int groups = (Vi + kEmbWarps - 1) / kEmbWarps;
   const int cap = 148 * 8;
-  embedding_bwd_kernel<<<groups < cap ? groups : cap, kEmbWarps * 32, smem, S(stream)>>>(
-      starts, vals + ni, DY, dy_dt, GW, C, Vi);
+  embedding_bwd_kernel<<<groups < cap ? groups : cap, kEmbWarps * 32, 0, S(stream)>>>(
+      starts, vals + ni, DY, dy_dt, part, GW, C, Vi, chunk);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

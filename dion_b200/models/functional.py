@@ -324,16 +324,18 @@ def qkv_rope(h: Tensor, wq: Tensor, wk: Tensor, wv: Tensor, cos: Tensor, sin: Te
 _sort_bytes: dict = {}
 
 
-def _embedding_sort_bytes(n: int, V: int) -> int:
+def _embedding_scratch(n: int, V: int) -> Tuple[int, int]:
+    """(bytes of temporary storage of the sort, rows of partial sums) for ``n`` tokens."""
     key = (n, V)
     b = _sort_bytes.get(key)
     if b is None:
-        fn = _backend.lib("embedding_ops")._dll.dion_embedding_sort_bytes
-        fn.restype = ctypes.c_longlong
-        b = int(fn(ctypes.c_longlong(n), ctypes.c_longlong(V)))
-        if b < 0:
+        dll = _backend.lib("embedding_ops")._dll
+        dll.dion_embedding_sort_bytes.restype = ctypes.c_longlong
+        dll.dion_embedding_part_rows.restype = ctypes.c_longlong
+        nbytes = int(dll.dion_embedding_sort_bytes(ctypes.c_longlong(n), ctypes.c_longlong(V)))
+        if nbytes < 0:
             raise RuntimeError("dion_embedding_sort_bytes failed")
-        _sort_bytes[key] = b
+        b = _sort_bytes[key] = nbytes, int(dll.dion_embedding_part_rows(ctypes.c_longlong(n)))
     return b
 
 
@@ -364,13 +366,14 @@ class _Embedding(torch.autograd.Function):
         dev = dy.device
         gw = torch.empty((V, C), dtype=torch.float32, device=dev)   # every row is written
         scratch = torch.empty(4 * n + V + 1, dtype=torch.int32, device=dev)
-        nbytes = _embedding_sort_bytes(n, V)
+        nbytes, part_rows = _embedding_scratch(n, V)
         temp = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=dev)
+        part = torch.empty((part_rows, C), dtype=torch.float32, device=dev)
         keys, vals, starts = scratch[:2 * n], scratch[2 * n:4 * n], scratch[4 * n:]
         _check(_backend.lib("embedding_ops").dion_embedding_bwd(
             _c(flat), _c(dy2), _DT[dy2.dtype], _c(gw), ctypes.c_longlong(n), C,
             ctypes.c_longlong(V), _c(keys), _c(vals), _c(starts), _c(temp),
-            ctypes.c_longlong(nbytes), _stream(dev)), "dion_embedding_bwd")
+            ctypes.c_longlong(nbytes), _c(part), _stream(dev)), "dion_embedding_bwd")
         return None, gw
 
 

@@ -110,6 +110,25 @@ def test_embedding_backward_matches_torch():
     assert w.grad[60:V - 1].abs().max().item() == 0.0
 
 
+@pytest.mark.parametrize("T", [1, 64, 65, 640, 70001])
+@pytest.mark.parametrize("C", [8, 264])
+def test_embedding_backward_runs_across_chunks(T, C):
+    """Skewed ids (neighbouring long runs), one id only, and a token count whose chunks are larger
+    than 64 positions; fp32 sums of T terms in another order than the fp64 ones."""
+    torch.manual_seed(1)
+    V = 97
+    g = torch.randn(T, C, device="cuda")
+    w = torch.randn(V, C, device="cuda", requires_grad=True)
+    u = torch.rand(T, device="cuda", dtype=torch.float64)
+    for idx in ((V ** u).long().sub_(1).clamp_(0, V - 1), torch.full((T,), V - 1, device="cuda")):
+        (gw,) = torch.autograd.grad(Fn.embedding(idx, w), w, g)
+        ref = torch.zeros(V, C, device="cuda", dtype=torch.float64).index_add_(0, idx, g.double())
+        mass = torch.zeros(V, C, device="cuda", dtype=torch.float64).index_add_(
+            0, idx, g.double().abs())
+        # each sum has at most T roundings of 2^-24 of a partial sum; far fewer in a tree of chunks
+        assert ((gw.double() - ref).abs() <= 2.0 ** -24 * 1100 * mass + 1e-30).all()
+
+
 def test_embedding_backward_long_runs_and_absent_rows():
     """Ids that occur hundreds of times (split over the block's warps), ids that occur once,
     rows that never occur (written as zeros, not left as allocated), a row count that is no
