@@ -697,7 +697,8 @@ cholesky_row4_kernel(const float* __restrict__ Gall, float* Uall, int r, int k) 
 // rank-one update follows; two block barriers per column.  A warp keeps its rows in registers while
 // they number at most NR (16 warps, so up to 16 * NR rows): a row then costs one shuffle and two
 // multiply-adds per column, where shared memory took four accesses, a shuffle and as many
-// multiply-adds (whole factorization of 16 matrices 640 x 512: 1421 -> 1131 us).  Taller panels
+// multiply-adds (whole factorization of 16 matrices 640 x 512: 1421 -> 1136 us;
+// one form of 48 rows that breaks off at the last row: 1444).  Taller panels
 // (NR = 0) stay in shared memory.
 // ---------------------------------------------------------------------------------------------
 constexpr int kQpWarps = 16;
@@ -1188,20 +1189,24 @@ DION_EXPORT int dion_qr_blocked(void* A, int n, int k, int r, void* V, void* VT,
     return ((size_t)(k - j) * kQpPitch + kQpWarps * 32 + 96 + 2 * 32 * kQpSq) * sizeof(float);
   };
   if (smem(0) > 226 * 1024) return -2;
-  // Registers for 16, 32 or 48 rows per warp (256, 512, 768 rows), else shared memory.
+  // Registers for 24 or 48 rows per warp (384, 768 rows), else shared memory.  Only the forms that
+  // this factorization uses are touched: loading a kernel takes milliseconds, once a process.
   typedef void (*Panel)(float*, long long, int, int, int, float*, float*);
-  const Panel panels[4] = {dion::qr_panel_kernel<16>, dion::qr_panel_kernel<32>,
-                           dion::qr_panel_kernel<48>, dion::qr_panel_kernel<0>};
-  for (Panel f : panels)
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(0)) !=
-        cudaSuccess)
+  auto panel_for = [&](int j) -> Panel {
+    const int rows = k - j;
+    if (rows <= 384) return dion::qr_panel_kernel<24>;
+    return rows <= 768 ? dion::qr_panel_kernel<48> : dion::qr_panel_kernel<0>;
+  };
+  for (int j = 0; j < r; j += 32)
+    if ((j == 0 || panel_for(j) != panel_for(j - 32)) &&
+        cudaFuncSetAttribute(panel_for(j), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem(j)) != cudaSuccess)
       return -3;
   float* a = static_cast<float*>(A);
   float* v = static_cast<float*>(V);
   float* vt = static_cast<float*>(VT);
   for (int j = 0; j < r; j += 32) {
-    const int rows = k - j;
-    const Panel panel = panels[rows <= 256 ? 0 : rows <= 512 ? 1 : rows <= 768 ? 2 : 3];
+    const Panel panel = panel_for(j);
     panel<<<n, kQpWarps * 32, smem(j), S(stream)>>>(a, (long long)k * r, r, k, j, v, vt);
     const int blocks = (r - j) / 32 - 1;
     if (blocks > 0)

@@ -302,7 +302,7 @@ def householder_q(P: Tensor) -> Tensor:
 _QR_PANEL = 32
 _QR_PANEL_MAX_ROWS = 1580      # shared memory of the panel kernel: (rows * 32 + ...) * 4 bytes
 # The single-kernel form takes 205 us for 16 matrices 160 x 128 and 424 us for 12 of 240 x 192, the
-# blocked one 157 and 256 us; narrower sketches are left to the former.
+# blocked one 162 and 268 us; narrower sketches are left to the former.
 _QR_BLOCKED_MIN_COLS = 128
 
 
