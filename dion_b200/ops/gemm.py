@@ -9,6 +9,7 @@ reference's three Triton kernels and its cuBLAS ``baddbmm`` call
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Dict, Optional, Tuple
 
@@ -200,6 +201,7 @@ def pair_exchange() -> bool:
     return os.environ.get("DION_B200_PAIR_EXCHANGE", "1") != "0"
 
 
+@functools.lru_cache(maxsize=1024)
 def _num_tiles(M: int, N: int, bm: int, bn: int, sym: bool) -> int:
     tm_n, tn_n = -(-M // bm), -(-N // bn)
     if not sym:
