@@ -245,8 +245,11 @@ def _ns_cuda(G: Tensor, coeffs: Coeffs, norm_mult: float, epsilon: float) -> Ten
 
 
 def buffer_form(ns_func: Optional[Callable], X_shape, device: torch.device) -> bool:
-    """Whether :func:`orthogonalize_buffer` stands in for ``ns_func`` on such a batch."""
-    return (getattr(ns_func, "ns_spec", None) is not None and device.type == "cuda"
+    """Whether :func:`orthogonalize_buffer` stands in for ``ns_func`` on such a batch.  Only for the
+    drivers themselves: a wrapper made with ``functools.wraps`` carries their attributes too, but has
+    to be called."""
+    return (any(ns_func is f for f in (newton_schulz_quintic, polar_express, newton_schulz_classic))
+            and device.type == "cuda"
             and len(X_shape) == 3 and all(X_shape) and X_shape[1] % 8 == 0 and X_shape[2] % 8 == 0)
 
 

@@ -43,6 +43,21 @@ def test_cpu_matches_reference(ref_dion):
     assert (NS.polar_express(G, 1e-6).float() - polar_express(G, 1e-6).float()).abs().max() < 2e-2
 
 
+def test_buffer_form_is_for_the_drivers_alone():
+    import functools
+
+    @functools.wraps(NS.polar_express)
+    def wrapped(X, epsilon=1e-6):
+        return NS.polar_express(X, epsilon)
+
+    cuda = torch.device("cuda", 0)
+    assert NS.buffer_form(NS.polar_express, (4, 64, 128), cuda)
+    assert not NS.buffer_form(wrapped, (4, 64, 128), cuda)
+    assert not NS.buffer_form(lambda X, epsilon=None: X, (4, 64, 128), cuda)
+    assert not NS.buffer_form(NS.polar_express, (4, 64, 100), cuda)
+    assert not NS.buffer_form(NS.polar_express, (4, 64, 128), torch.device("cpu"))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("form", ["dense", "odd", "two_dims", "four_dims", "transposed", "columns",
