@@ -281,6 +281,7 @@ ns_persistent_kernel(const __grid_constant__ PersistArgs p) {
         }
         if (!mbar_wait_bounded(&tfull_bar[aslot], aphase)) {
           if (lane == 0) atomicExch(p.status, kStatusTimeoutTmemFull);
+          grid_ok = 0;   // every epilogue warp leaves together, after the phase's barrier
           ok = false;
           break;
         }
