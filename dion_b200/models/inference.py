@@ -65,18 +65,24 @@ def _observed() -> bool:
 
 def _block_weights(block, types, C: int):
     """The block's six weights if its modules may be bypassed, else None."""
-    Block, Attention, MLP = types[:3]
+    Block, Attention, MLP, Rotary = types
+    if type(block) is not Block:
+        return None
     attn, mlp = block.attn, block.mlp
-    if not (type(block) is Block and type(attn) is Attention and type(mlp) is MLP
-            and _unhooked(block) and _unhooked(attn) and _unhooked(mlp)):
+    if not (type(attn) is Attention and type(mlp) is MLP and type(attn.rotary) is Rotary
+            and _unhooked(block) and _unhooked(attn) and _unhooked(mlp)
+            and _unhooked(attn.rotary)):
         return None
     linears = (attn.c_q, attn.c_k, attn.c_v, attn.c_proj, mlp.c_fc, mlp.c_proj)
+    if any(type(m) is not torch.nn.Linear for m in linears):
+        return None
     ws = tuple(m.weight for m in linears)
-    F = ws[4].size(0)
+    F = ws[4].size(0) if ws[4].ndim else 0
     shapes = ((C, C),) * 4 + ((F, C), (C, F))
     for m, w, s in zip(linears, ws, shapes):
         if not (_unhooked(m) and m.bias is None and is_plain_tensor(w) and w.is_cuda
-                and w.shape == s and w.dtype == ws[0].dtype and w.is_contiguous()
+                and w.shape == s and w.dtype == ws[0].dtype and w.device == ws[0].device
+                and w.is_contiguous()
                 and w.data_ptr() % 16 == 0):
             return None
     return ws
@@ -94,9 +100,11 @@ def hidden_states(model, idx: Tensor, types) -> Optional[Tensor]:
     replaced modules; fp32 embedding; dense fp32 or bf16 weights of one dtype) on the GPU of
     ``idx``, and nothing observes operators."""
     wte = model.transformer.wte
-    table = wte.weight
-    C = table.size(1)
     blocks = model.transformer.h
+    if type(wte) is not torch.nn.Embedding:
+        return None
+    table = wte.weight
+    C = table.size(-1)
     if (torch.is_grad_enabled() or not idx.is_cuda or not is_plain_tensor(idx) or idx.ndim != 2
             or idx.numel() == 0 or len(blocks) == 0
             or not torch.is_autocast_enabled("cuda")
@@ -105,25 +113,23 @@ def hidden_states(model, idx: Tensor, types) -> Optional[Tensor]:
             or table.device != idx.device or C % 8 or C > 4096 or not _unhooked(wte)
             or _observed()):
         return None
+    weights = [_block_weights(b, types, C) for b in blocks]
+    if any(w is None for w in weights):
+        return None
+    first = weights[0]
     B, T = idx.shape
     H = blocks[0].attn.n_head
-    D = C // H
-    if D not in (32, 64, 128, 256):
+    D, F = C // H, first[4].size(0)
+    if first[0].dtype not in (torch.float32, torch.bfloat16) or D not in (32, 64, 128, 256) \
+            or D * H != C:
         return None
-    weights = [_block_weights(b, types, C) for b in blocks]
-    first = weights[0]
-    if first is None or first[0].dtype not in (torch.float32, torch.bfloat16):
-        return None
-    F = first[4].size(0)
-    if F % 8 or any(w is None or w[4].size(0) != F or w[0].dtype != first[0].dtype
+    if F % 8 or any(w[4].size(0) != F or w[0].dtype != first[0].dtype
                     or w[0].device != idx.device for w in weights) \
             or any(b.attn.n_head != H for b in blocks):
         return None
     dev, rows = idx.device, B * T
     tables = []
     for b in blocks:
-        if type(b.attn.rotary) is not types[3] or not _unhooked(b.attn.rotary):
-            return None
         cos, sin = b.attn.rotary(idx)
         if any(not t.is_contiguous() or t.dtype != torch.bfloat16 or t.shape != (T, D // 2)
                or t.device != dev for t in (cos, sin)):

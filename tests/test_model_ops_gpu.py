@@ -308,3 +308,30 @@ def test_blocks_without_gradients_match_the_general_forward(B, T, heads, dim, dt
     for x in (got, hooked):
         assert ((x - ref).norm() / ref.norm()).item() < 2e-2
     assert ((last[:, 0] - ref[:, -1]).norm() / ref[:, -1].norm()).item() < 2e-2
+
+
+def test_replaced_modules_take_the_general_forward():
+    """A block, a linear layer or an embedding of another type may look nothing like the original:
+    the path without gradients leaves such a model to the modules."""
+    from dion_b200.models.gpt import GPT, GPTConfig
+
+    class Twice(torch.nn.Module):
+        def forward(self, x, h=None):
+            return 2 * x, Fn.rms_norm(2 * x)
+
+    class Scaled(torch.nn.Linear):
+        def forward(self, x):
+            return 0.5 * super().forward(x)
+
+    torch.manual_seed(0)
+    ids = torch.randint(0, 512, (2, 24), device="cuda")
+    for change in (lambda m: m.transformer.h.__setitem__(0, Twice()),
+                   lambda m: setattr(m.transformer.h[1].mlp, "c_fc", Scaled(128, 512, bias=False).cuda())):
+        model = GPT(GPTConfig(sequence_len=24, vocab_size=512, n_layer=2, n_head=2, n_embd=128)).cuda()
+        model.init_weights()
+        change(model)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            ref = model(ids, ids, return_logits=True).detach()
+            with torch.no_grad():
+                got = model(ids, ids, return_logits=True)
+        assert torch.equal(got, ref)
