@@ -860,9 +860,9 @@ normuon_rowstats_kernel(const long long* raw, const __nv_bfloat16* U, int rows, 
   }
 }
 
-// sum of squares per matrix of a contiguous bf16 batch [n][numel] -> out[n] (atomic accumulate)
+// sums of squares of a contiguous bf16 batch [n][numel], one per chunk: part[t][blockIdx.x]
 __global__ void __launch_bounds__(kThreads)
-sumsq_kernel(const __nv_bfloat16* X, long long numel, float* out) {
+sumsq_kernel(const __nv_bfloat16* X, long long numel, float* part) {
   const int t = blockIdx.y;
   const __nv_bfloat16* x = X + (long long)t * numel;
   float acc = 0.f;
@@ -882,16 +882,35 @@ sumsq_kernel(const __nv_bfloat16* X, long long numel, float* out) {
     }
   }
   const float s = block_sum(acc);
-  if (threadIdx.x == 0) atomicAdd(&out[t], s);
+  if (threadIdx.x == 0) part[(size_t)t * gridDim.x + blockIdx.x] = s;
+}
+
+enum { kSumWrite = 0, kSumAdd = 1, kSumScale = 2 };
+
+// The sum of part[t][0 .. blocks), one block per matrix: written to out[t], added to it, or turned
+// into the scale 1 / (sqrt(sum) * mult + eps).  Always in the same order: a norm that depends on the
+// order in which blocks finish (atomic adds: 4 to 12 different values in 12 calls on one matrix
+// 768 x 768 or four) flips roundings of the first product, which the iteration carries on to 0.7 %
+// between two calls on the same input.
+__global__ void __launch_bounds__(kThreads)
+sum_parts_kernel(const float* part, int blocks, float* out, int mode, float mult, float eps) {
+  const float* p = part + (size_t)blockIdx.x * blocks;
+  float acc = 0.f;
+  for (int i = threadIdx.x; i < blocks; i += kThreads) acc += p[i];
+  const float s = block_sum(acc);
+  if (threadIdx.x == 0) {
+    float* o = out + blockIdx.x;
+    *o = mode == kSumScale ? 1.f / (sqrtf(s) * mult + eps) : mode == kSumAdd ? *o + s : s;
+  }
 }
 
 // Newton-Schulz input of a dense fp32 or bf16 batch G [B][m][n]: rounded to bf16 into
 // X [B][mp][np] (mp >= m, np >= n multiples of 8, the padding zero), and the squares of the rounded
-// values added to ss[b].  One pass, bound by memory; it stands for a cast, a zero fill, a strided
-// copy and a norm pass (6 x 997 x 1531 fp32: 41 -> 9 us).
+// values summed per chunk in part[b][blockIdx.x].  One pass, bound by memory; it stands for a cast, a
+// zero fill, a strided copy and a norm pass (6 x 997 x 1531 fp32: 41 -> 9 us).
 __global__ void __launch_bounds__(kThreads)
 ns_prepare_kernel(const void* G, int g_dt, int m, int n, __nv_bfloat16* X, int mp, int np,
-                  float* ss) {
+                  float* part) {
   const int b = blockIdx.y;
   const long long per = (long long)mp * np;
   const long long gofs = (long long)b * m * n;
@@ -926,7 +945,7 @@ ns_prepare_kernel(const void* G, int g_dt, int m, int n, __nv_bfloat16* X, int m
     st8b(x, i, v);
   }
   const float s = block_sum(acc);
-  if (threadIdx.x == 0) atomicAdd(&ss[b], s);
+  if (threadIdx.x == 0) part[(size_t)b * gridDim.x + blockIdx.x] = s;
 }
 
 // scale[t] = 1 / (sqrt(sumsq[t]) * mult + eps)
@@ -1094,23 +1113,38 @@ DION_EXPORT int dion_normuon_rowstats(const void* table, const void* U, int n_ma
   return rc();
 }
 
-DION_EXPORT int dion_sumsq(const void* X, int n, long long numel, float* out, void* stream) {
+// part: fp32 [n, chunks of numel], written; out (optional): fp32 [n], the sums, written or added to.
+DION_EXPORT int dion_sumsq(const void* X, int n, long long numel, float* part, float* out,
+                           int accumulate, void* stream) {
   if (n <= 0 || numel <= 0) return 0;
   dim3 grid((unsigned)((numel + kChunk - 1) / kChunk), (unsigned)n);
-  sumsq_kernel<<<grid, kThreads, 0, S(stream)>>>(static_cast<const __nv_bfloat16*>(X), numel, out);
+  sumsq_kernel<<<grid, kThreads, 0, S(stream)>>>(static_cast<const __nv_bfloat16*>(X), numel, part);
+  if (out)
+    sum_parts_kernel<<<n, kThreads, 0, S(stream)>>>(part, (int)grid.x, out,
+                                                    accumulate ? kSumAdd : kSumWrite, 0.f, 0.f);
   return rc();
 }
 
 // G: dense [batch, m, n] fp32 (0) or bf16 (1); X: bf16 [batch, mp, np], 16-byte aligned, mp and np
-// multiples of 8; ss: fp32 [batch], accumulated into.
+// multiples of 8; part: fp32 [batch, chunks of mp * np], written; ss (optional): fp32 [batch], written.
 DION_EXPORT int dion_ns_prepare(const void* G, int g_dt, int batch, int m, int n, void* X, int mp,
-                                int np, float* ss, void* stream) {
+                                int np, float* part, float* ss, void* stream) {
   if (batch <= 0 || m <= 0 || n <= 0) return 0;
   if (mp < m || np < n || (np & 7) || batch > 65535 || (reinterpret_cast<uintptr_t>(X) & 15))
     return -2;
   dim3 grid((unsigned)(((long long)mp * np + kChunk - 1) / kChunk), (unsigned)batch);
-  ns_prepare_kernel<<<grid, kThreads, 0, S(stream)>>>(G, g_dt, m, n,
-                                                      static_cast<__nv_bfloat16*>(X), mp, np, ss);
+  ns_prepare_kernel<<<grid, kThreads, 0, S(stream)>>>(G, g_dt, m, n, static_cast<__nv_bfloat16*>(X),
+                                                      mp, np, part);
+  if (ss)
+    sum_parts_kernel<<<batch, kThreads, 0, S(stream)>>>(part, (int)grid.x, ss, kSumWrite, 0.f, 0.f);
+  return rc();
+}
+
+// scale[t] = 1 / (sqrt(sum of part[t][0 .. blocks)) * mult + eps)
+DION_EXPORT int dion_parts_scale(const float* part, int blocks, float* scale, int n, float mult,
+                                 float eps, void* stream) {
+  if (n <= 0) return 0;
+  sum_parts_kernel<<<n, kThreads, 0, S(stream)>>>(part, blocks, scale, kSumScale, mult, eps);
   return rc();
 }
 

@@ -21,7 +21,7 @@ from torch import Tensor
 
 from . import _backend
 from ..utils.tensors import is_plain_tensor
-from .tables import RawPointer, build_table
+from .tables import CHUNK, RawPointer, build_table
 
 Scalar = Union[float, Tensor]
 _DT = {torch.float32: 0, torch.bfloat16: 1}
@@ -499,34 +499,67 @@ def normuon_rowstats(
     return rinv, normU2, normNew2
 
 
+def _partials(batch: int, numel: int, device: torch.device) -> Tensor:
+    return torch.empty((batch, -(-numel // CHUNK)), dtype=torch.float32, device=device)
+
+
+def sumsq_parts(X: Tensor, out: Optional[Tensor] = None, accumulate: bool = False) -> Tensor:
+    """``[N, chunks]`` fp32: the sums of squares of a dense CUDA bf16 batch chunk by chunk; their
+    totals go to ``out`` ``[N]`` (or are added to it)."""
+    N, numel = X.size(0), X[0].numel()
+    part = _partials(N, numel, X.device)
+    _check(
+        _backend.lib("foreach_ops").dion_sumsq(
+            _c(X.data_ptr()), N, ctypes.c_longlong(numel), _c(part.data_ptr()),
+            _c(out.data_ptr() if out is not None else 0), int(accumulate), _stream(X.device)),
+        "dion_sumsq")
+    if out is not None:
+        _backend.add_launches(1)
+    return part
+
+
 def sumsq(X: Tensor, out: Optional[Tensor] = None) -> Tensor:
-    """Squared Frobenius norm of every matrix of a bf16 batch ``[N, ...]`` (fp32 result)."""
+    """Squared Frobenius norm of every matrix of a bf16 batch ``[N, ...]`` (fp32 result), added to
+    ``out`` when given.  On the GPU always summed in the same order."""
     N = X.size(0)
+    if X.is_cuda and X.dtype == torch.bfloat16 and X.is_contiguous() and X.numel():
+        res = torch.empty(N, dtype=torch.float32, device=X.device) if out is None else out
+        sumsq_parts(X, res, accumulate=out is not None)
+        return res
     if out is None:
         out = torch.zeros(N, dtype=torch.float32, device=X.device)
-    if X.is_cuda and X.dtype == torch.bfloat16 and X.is_contiguous():
-        numel = X[0].numel() if N else 0
-        _check(
-            _backend.lib("foreach_ops").dion_sumsq(
-                _c(X.data_ptr()), N, ctypes.c_longlong(numel), _c(out.data_ptr()), _stream(X.device)),
-            "dion_sumsq")
-        return out
-    out.add_(X.to(torch.float32).reshape(N, -1).square().sum(dim=-1))
+    if X.numel():
+        out.add_(X.to(torch.float32).reshape(N, -1).square().sum(dim=-1))
     return out
 
 
-def ns_prepare(G: Tensor, mp: int, np_: int) -> Tuple[Tensor, Tensor]:
+def scale_of_parts(part: Tensor, mult: float, eps: float) -> Tensor:
+    """:func:`finalize_scale` of the totals of ``part`` (see :func:`sumsq_parts`), in one launch."""
+    out = torch.empty(part.size(0), dtype=torch.float32, device=part.device)
+    _check(
+        _backend.lib("foreach_ops").dion_parts_scale(
+            _c(part.data_ptr()), part.size(1), _c(out.data_ptr()), part.size(0),
+            ctypes.c_float(float(mult)), ctypes.c_float(float(eps)), _stream(part.device)),
+        "dion_parts_scale")
+    return out
+
+
+def ns_prepare(G: Tensor, mp: int, np_: int, totals: bool = True) -> Tuple[Tensor, Tensor]:
     """``(X, ss)`` of a dense CUDA batch ``G [B, m, n]`` (fp32 or bf16): ``X [B, mp, np_]`` is ``G``
-    rounded to bf16 with zeros beyond it, ``ss [B]`` the fp32 sums of squares of ``X``."""
+    rounded to bf16 with zeros beyond it, ``ss [B]`` the fp32 sums of squares of ``X``, or, without
+    ``totals``, these chunk by chunk (see :func:`sumsq_parts`)."""
     B, m, n = G.shape
     X = torch.empty((B, mp, np_), dtype=torch.bfloat16, device=G.device)
-    ss = torch.zeros(B, dtype=torch.float32, device=G.device)
+    part = _partials(B, mp * np_, G.device)
+    ss = torch.empty(B, dtype=torch.float32, device=G.device) if totals else None
     _check(
         _backend.lib("foreach_ops").dion_ns_prepare(
-            _c(G.data_ptr()), _DT[G.dtype], B, m, n, _c(X.data_ptr()), mp, np_, _c(ss.data_ptr()),
-            _stream(G.device)),
+            _c(G.data_ptr()), _DT[G.dtype], B, m, n, _c(X.data_ptr()), mp, np_,
+            _c(part.data_ptr()), _c(ss.data_ptr() if totals else 0), _stream(G.device)),
         "dion_ns_prepare")
-    return X, ss
+    if totals:
+        _backend.add_launches(1)
+    return X, ss if totals else part
 
 
 def aol_rescale_(X: Tensor, A: Tensor, eps: float) -> None:

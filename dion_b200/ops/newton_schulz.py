@@ -132,7 +132,7 @@ def _gram_torch(G: Tensor, coeffs: Coeffs, norm_mult: float, epsilon: float,
 # CUDA implementations on the tcgen05 GEMM
 # ------------------------------------------------------------------------------------------------
 def _prepare_cuda(G: Tensor, allow_tall: bool = False):
-    """-> (X [B, m, n] bf16 contiguous with m, n multiples of 8, sums of squares [B] or None,
+    """-> (X [B, m, n] bf16 contiguous with m, n multiples of 8, sums of squares by chunks or None,
     restore).  Tall inputs are transposed to wide unless ``allow_tall`` (the caller then iterates
     in right-multiply form).  ``X`` may be ``G`` itself: it is to be read only.  The sums are there
     where one pass could round, pad and add up."""
@@ -149,12 +149,12 @@ def _prepare_cuda(G: Tensor, allow_tall: bool = False):
     m, n = X.size(-2), X.size(-1)
     mp, np_ = (m + 7) // 8 * 8, (n + 7) // 8 * 8
     padded = (mp, np_) != (m, n)
-    ss: Optional[Tensor] = None
+    part: Optional[Tensor] = None
     if (not padded and X.dtype == torch.bfloat16 and X.is_contiguous()
             and X.data_ptr() % 16 == 0):
         pass
     elif X.is_contiguous() and X.dtype in (torch.float32, torch.bfloat16) and X.size(0) < 65536:
-        X, ss = F.ns_prepare(X, mp, np_)
+        X, part = F.ns_prepare(X, mp, np_, totals=False)
     else:
         X = X.to(torch.bfloat16)
         if padded:
@@ -171,13 +171,11 @@ def _prepare_cuda(G: Tensor, allow_tall: bool = False):
             Y = Y.mT
         return Y.reshape(shape)
 
-    return X, ss, restore
+    return X, part, restore
 
 
-def _norm_scale(X: Tensor, norm_mult: float, epsilon: float, ss: Optional[Tensor]) -> Tensor:
-    if ss is None:
-        ss = F.sumsq(X)
-    return F.finalize_scale(ss, norm_mult, epsilon, out=ss)
+def _norm_scale(X: Tensor, norm_mult: float, epsilon: float, part: Optional[Tensor]) -> Tensor:
+    return F.scale_of_parts(F.sumsq_parts(X) if part is None else part, norm_mult, epsilon)
 
 
 def _iterate_cuda(X: Tensor, coeffs: Coeffs, scale: Optional[Tensor], hooks=None,
@@ -239,8 +237,8 @@ def _iterate_cuda(X: Tensor, coeffs: Coeffs, scale: Optional[Tensor], hooks=None
 
 def _ns_cuda(G: Tensor, coeffs: Coeffs, norm_mult: float, epsilon: float) -> Tensor:
     with trace.span("newton_schulz"):
-        X, ss, restore = _prepare_cuda(G, allow_tall=True)
-        scale = _norm_scale(X, norm_mult, epsilon, ss)
+        X, part, restore = _prepare_cuda(G, allow_tall=True)
+        scale = _norm_scale(X, norm_mult, epsilon, part)
         return restore(_iterate_cuda(X, coeffs, scale))
 
 
@@ -289,8 +287,8 @@ def _gram_cuda(G: Tensor, coeffs: Coeffs, norm_mult: float, epsilon: float,
     read as it lies (a transposed copy of 8 x 8192 x 2048 took 555 us of 4.0 ms).  ``R`` is not
     brought forward where nothing reads it again: after the last step and before a reset (two of
     five steps, 0.2 ms each at that size)."""
-    X, ss, restore = _prepare_cuda(G, allow_tall=True)
-    scale = _norm_scale(X, norm_mult, epsilon, ss)
+    X, part, restore = _prepare_cuda(G, allow_tall=True)
+    scale = _norm_scale(X, norm_mult, epsilon, part)
     B_, m, n = X.shape
     tall = m > n
     g = min(m, n)

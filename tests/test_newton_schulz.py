@@ -111,6 +111,26 @@ def test_prepare_rounds_pads_and_sums(shape, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(1, 768, 768), (1, 104, 2048), (3, 517, 1031)])
+def test_cuda_driver_repeats_exactly(shape, dtype):
+    """The same input gives the same bits: one launch, padded, one matrix or several; the sum of
+    squares over tens of blocks included."""
+    from dion_b200.ops import foreach as F
+    torch.manual_seed(0)
+    G = (torch.randn(*shape, device="cuda") * 1e-3).to(dtype)
+    first = NS.polar_express(G)
+    X = G.bfloat16()
+    ss = F.sumsq(X)
+    assert ((ss - X.double().square().sum(dim=(1, 2))).abs() <= 1e-6 * ss).all()
+    for _ in range(24):
+        assert torch.equal(F.sumsq(X), ss)
+        assert torch.equal(NS.polar_express(G), first)
+    total = ss.clone()
+    assert torch.equal(F.sumsq(X, out=total), 2 * ss)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("variant", ["quintic", "classic", "polar_express", "aol", "gram"])
 @pytest.mark.parametrize("shape", [(6, 768, 768), (2, 768, 3072), (2, 3072, 768), (3, 192, 768),
                                    (1, 100, 52), (256, 256)])
