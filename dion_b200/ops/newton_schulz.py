@@ -133,9 +133,10 @@ def _gram_torch(G: Tensor, coeffs: Coeffs, norm_mult: float, epsilon: float,
 # ------------------------------------------------------------------------------------------------
 def _prepare_cuda(G: Tensor, allow_tall: bool = False):
     """-> (X [B, m, n] bf16 contiguous with m, n multiples of 8, sums of squares by chunks or None,
-    restore).  Tall inputs are transposed to wide unless ``allow_tall`` (the caller then iterates
-    in right-multiply form).  ``X`` may be ``G`` itself: it is to be read only.  The sums are there
-    where one pass could round, pad and add up."""
+    whether ``X`` is memory of this call, restore).  Tall inputs are transposed to wide unless
+    ``allow_tall`` (the caller then iterates in right-multiply form).  Where ``X`` is not of this
+    call it is the caller's tensor: to be read only.  The sums are there where one pass could
+    round, pad and add up."""
     G = unwrap(G)  # a pending functional collective must complete before its address is used
     shape = G.shape
     X = G
@@ -171,7 +172,7 @@ def _prepare_cuda(G: Tensor, allow_tall: bool = False):
             Y = Y.mT
         return Y.reshape(shape)
 
-    return X, part, restore
+    return X, part, X.data_ptr() != G.data_ptr(), restore
 
 
 def _norm_scale(X: Tensor, norm_mult: float, epsilon: float, part: Optional[Tensor]) -> Tensor:
@@ -237,7 +238,7 @@ def _iterate_cuda(X: Tensor, coeffs: Coeffs, scale: Optional[Tensor], hooks=None
 
 def _ns_cuda(G: Tensor, coeffs: Coeffs, norm_mult: float, epsilon: float) -> Tensor:
     with trace.span("newton_schulz"):
-        X, part, restore = _prepare_cuda(G, allow_tall=True)
+        X, part, _, restore = _prepare_cuda(G, allow_tall=True)
         scale = _norm_scale(X, norm_mult, epsilon, part)
         return restore(_iterate_cuda(X, coeffs, scale))
 
@@ -264,8 +265,8 @@ def orthogonalize_buffer(ns_func: Callable, X: Tensor, epsilon, sumsq: Tensor,
 
 
 def _aol_cuda(G: Tensor, epsilon: float) -> Tensor:
-    X, _, restore = _prepare_cuda(G)
-    if X.data_ptr() == G.data_ptr():
+    X, _, own, restore = _prepare_cuda(G)
+    if not own:
         X = X.clone()
     B_, m, n = X.shape
     A = torch.empty((B_, m, m), dtype=torch.bfloat16, device=X.device)
@@ -287,7 +288,7 @@ def _gram_cuda(G: Tensor, coeffs: Coeffs, norm_mult: float, epsilon: float,
     read as it lies (a transposed copy of 8 x 8192 x 2048 took 555 us of 4.0 ms).  ``R`` is not
     brought forward where nothing reads it again: after the last step and before a reset (two of
     five steps, 0.2 ms each at that size)."""
-    X, part, restore = _prepare_cuda(G, allow_tall=True)
+    X, part, _, restore = _prepare_cuda(G, allow_tall=True)
     scale = _norm_scale(X, norm_mult, epsilon, part)
     B_, m, n = X.shape
     tall = m > n

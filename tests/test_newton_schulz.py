@@ -58,6 +58,56 @@ def test_buffer_form_is_for_the_drivers_alone():
     assert not NS.buffer_form(NS.polar_express, (4, 64, 128), torch.device("cpu"))
 
 
+@pytest.fixture
+def products_on_cpu(monkeypatch):
+    """The CUDA drivers with their kernels replaced by plain torch, to follow their buffers."""
+    from dion_b200.ops import foreach as F
+    from dion_b200.ops import gemm
+
+    def ns_gemm(A, B, out=None, a_is_km=False, b_is_kn=False, D=None, alpha=1.0, beta=0.0,
+                scale=None, alpha_pow=0, beta_pow=0, sym=False, extra=None):
+        A, B = A.float(), B.float()
+        s = scale.view(-1, 1, 1) if scale is not None else 1.0
+        r = alpha * s ** alpha_pow * ((A.mT if a_is_km else A) @ (B if b_is_kn else B.mT))
+        if D is not None:
+            r = r + beta * s ** beta_pow * D.float()
+        r = r.to(torch.bfloat16)
+        return r if out is None else out.copy_(r)
+
+    def aol_rescale_(X, A, eps):
+        s = A.float().abs().sum(-1).clamp_min(eps).rsqrt()
+        X.copy_(X.float() * s.unsqueeze(-1))
+        A.copy_(A.float() * s.unsqueeze(-1) * s.unsqueeze(-2))
+
+    monkeypatch.setattr(gemm, "ns_gemm", ns_gemm)
+    monkeypatch.setattr(F, "aol_rescale_", aol_rescale_)
+    for name in ("persistent_fits", "iterate_in_one_call"):
+        monkeypatch.setattr(gemm, name, lambda *a: False)
+    monkeypatch.setattr(NS, "_norm_scale", lambda X, mult, eps, part: 1.0 / (
+        X.float().square().sum(dim=(1, 2)).sqrt() * mult + eps))
+    monkeypatch.setattr(NS, "_use_cuda", lambda G: True)
+
+
+_DRIVERS = {"polar_express": NS.polar_express, "aol": NS.newton_schulz_aol,
+            "gram": NS.gram_newton_schulz}
+
+
+@pytest.mark.parametrize("pending", [False, True])
+@pytest.mark.parametrize("shape", [(2, 16, 40), (2, 40, 16), (24, 24)])
+@pytest.mark.parametrize("variant", list(_DRIVERS))
+def test_input_is_kept_and_not_returned(products_on_cpu, variant, shape, pending):
+    """Dense bf16 input is read in place: a plain tensor, and the pending result of a functional
+    collective, whose own address is not that of its data."""
+    from torch.distributed._functional_collectives import AsyncCollectiveTensor
+    torch.manual_seed(0)
+    G = torch.randn(shape).bfloat16()
+    before = G.clone()
+    got = _DRIVERS[variant](AsyncCollectiveTensor(G) if pending else G)
+    assert torch.equal(G, before)
+    assert got.untyped_storage().data_ptr() != G.untyped_storage().data_ptr()
+    assert torch.equal(got, _DRIVERS[variant](before))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("form", ["dense", "odd", "two_dims", "four_dims", "transposed", "columns",
