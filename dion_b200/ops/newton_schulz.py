@@ -188,6 +188,8 @@ def _iterate_cuda(X: Tensor, coeffs: Coeffs, scale: Optional[Tensor], hooks=None
     otherwise goes to and fro between two buffers of its own; these come from ``alloc(like)``
     where the caller wants the result in memory of its own.  ``hooks`` (fused exchange) may supply per-launch coupling to other GPUs:
     ``hooks.first_gram()``, ``hooks.after_first_iteration()``, ``hooks.last_update()``."""
+    if not coeffs:
+        return X if overwrite else X.clone()
     B_, m, n = X.shape
     tall = m > n
     g = n if tall else m

@@ -108,6 +108,14 @@ def test_input_is_kept_and_not_returned(products_on_cpu, variant, shape, pending
     assert torch.equal(got, _DRIVERS[variant](before))
 
 
+@pytest.mark.parametrize("shape", [(2, 16, 40), (40, 16)])
+def test_no_steps_give_a_copy(products_on_cpu, shape):
+    G = torch.randn(shape).bfloat16()
+    got = NS.newton_schulz_classic(G, steps=0)
+    assert torch.equal(got, G)
+    assert got.untyped_storage().data_ptr() != G.untyped_storage().data_ptr()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("form", ["dense", "odd", "two_dims", "four_dims", "transposed", "columns",
