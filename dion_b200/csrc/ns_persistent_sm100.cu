@@ -57,7 +57,7 @@ struct PersistArgs {
   long long ld[5], stride[5];
   const int2* tiles;
   const float* scale;          // one fp32 per matrix or nullptr
-  unsigned int* counter;       // grid barrier, zero at launch; left at zero
+  unsigned int* counter;       // grid barrier of this launch, zero at its start
   int* status;
 };
 
@@ -394,15 +394,6 @@ ns_persistent_kernel(const __grid_constant__ PersistArgs p) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   }
-  // Leave the barrier counter at zero for the next launch: the last CTA to pass resets it.
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned done = atomicAdd(p.counter + 1, 1u);
-    if (done == gridDim.x - 1) {
-      p.counter[0] = 0u;
-      p.counter[1] = 0u;
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -466,6 +457,7 @@ static int launch_persistent(PersistArgs& a, int max_tiles, int num_sms, cudaStr
   int grid = max_tiles < num_sms ? max_tiles : num_sms;
   if (grid > max_blocks) grid = max_blocks;
   if (grid <= 0) return 0;
+  if (cudaMemsetAsync(a.counter, 0, sizeof(unsigned int), stream) != cudaSuccess) return -4;
   void* kargs[] = {&a};
   cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kernel), dim3(grid),
                                               dim3(kPThreads), kargs, kDyn, stream);
@@ -480,8 +472,9 @@ static int launch_persistent(PersistArgs& a, int max_tiles, int num_sms, cudaStr
 
 // All iterations (a, b, c) = coeffs[3*i .. 3*i+2] of the Newton-Schulz loop on the dense bf16 batch
 // X [batch, m, n] in one cooperative launch.  Xalt and X2 [batch, m, n], A and Bm [batch, g, g]
-// (g = min(m, n)) are work buffers; `counter` points to two zero-initialised unsigned ints in
-// device memory that the kernel leaves at zero.  tiles_all: (tile_m, tile_n) pairs in units of
+// (g = min(m, n)) are work buffers; `counter` points to an unsigned int of this launch alone in
+// device memory (one that launches on two streams share would let a phase of the one begin on the
+// arrivals of the other); it is cleared here.  tiles_all: (tile_m, tile_n) pairs in units of
 // 128 x bn, first the n_tiles_gg tiles on or above the diagonal of the symmetric g x g products,
 // then the n_tiles_mn tiles of the m x n update.  The result lies in Xalt when
 // `iters` is odd, else in X, or in X2 where that is given (X is then only read).  Returns 0 on success,

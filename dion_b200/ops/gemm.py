@@ -398,7 +398,6 @@ def ns_iterate(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs, scale: Op
 
 
 _persist_tiles: Dict[Tuple, Tensor] = {}
-_persist_counter: Dict[int, Tensor] = {}
 
 
 def persistent_enabled() -> bool:
@@ -461,10 +460,7 @@ def ns_persistent(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs,
         mn = tile_table(m, n, bn, False, dev)
         tab = _persist_tiles[key] = (torch.cat([gg, mn]).contiguous(), gg.size(0), mn.size(0))
     tiles, n_gg, n_mn = tab
-    idx = dev.index if dev.index is not None else torch.cuda.current_device()
-    counter = _persist_counter.get(idx)
-    if counter is None:
-        counter = _persist_counter[idx] = torch.zeros(2, dtype=torch.int32, device=dev)
+    counter = torch.empty(1, dtype=torch.int32, device=dev)   # of this launch alone
     flat = (ctypes.c_float * (3 * len(coeffs)))(*[float(v) for abc in coeffs for v in abc])
     st = status_tensor(dev)
     rc = _backend.lib("ns_persistent_sm100").dion_ns_persistent(

@@ -116,6 +116,57 @@ def test_no_steps_give_a_copy(products_on_cpu, shape):
     assert got.untyped_storage().data_ptr() != G.untyped_storage().data_ptr()
 
 
+def test_one_launch_loops_in_flight_have_their_own_counters(monkeypatch):
+    """A second launch issued while the first one is running (another stream or thread of the same
+    device) counts its barrier elsewhere."""
+    from dion_b200.ops import _backend, gemm
+    seen = []
+
+    class Lib:
+        def dion_ns_persistent(self, *args):
+            seen.append(args[14].value)
+            if len(seen) == 1:
+                launch()
+            return 0
+
+    def launch():
+        X, A = torch.zeros(1, 64, 128), torch.zeros(1, 64, 64)
+        gemm.ns_persistent(X, torch.zeros_like(X), A, torch.zeros_like(A), NS.QUINTIC_COEFFS, None)
+
+    monkeypatch.setattr(_backend, "lib", lambda stem: Lib())
+    monkeypatch.setattr(gemm, "sm_count", lambda dev: 148)
+    monkeypatch.setattr(gemm, "status_tensor", lambda dev: torch.zeros(4, dtype=torch.int32))
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "current_stream",
+                        lambda dev=None: type("Stream", (), {"cuda_stream": 0})())
+    launch()
+    assert len(seen) == 2 and 0 not in seen and seen[0] != seen[1]
+
+
+@pytest.mark.gpu
+def test_one_launch_loops_on_two_streams():
+    """Grids that fit the GPU together, of different sizes and phase lengths: the bits of the same
+    calls one after the other."""
+    from dion_b200.ops import gemm
+    torch.manual_seed(0)
+    Gs = [torch.randn(1, m, n, device="cuda").bfloat16()
+          for m, n in ((256, 256), (384, 512), (256, 1024), (512, 384))]
+    for G in Gs:
+        assert gemm.persistent_fits(G, *G.shape, 5)
+    alone = [NS.polar_express(G) for G in Gs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for _ in range(20):
+        outs = []
+        for i, G in enumerate(Gs):
+            with torch.cuda.stream(streams[i % 2]):
+                outs.append(NS.polar_express(G))
+        torch.cuda.synchronize()
+        for a, b in zip(alone, outs):
+            assert torch.equal(a, b)
+    gemm.check_status()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("form", ["dense", "odd", "two_dims", "four_dims", "transposed", "columns",
