@@ -23,6 +23,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include "common.cuh"
+#include "embedding_chunks.h"
 
 namespace dion {
 
@@ -58,14 +59,13 @@ emb_starts_kernel(const int* __restrict__ sorted, int* __restrict__ starts, int 
   if (v > V) return;
   int lo = 0, hi = n;                      // first index with sorted[idx] >= v
   while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
+    const int mid = emb_mid(lo, hi);
     if (sorted[mid] < v) lo = mid + 1; else hi = mid;
   }
   starts[v] = lo;
 }
 
 constexpr int kEmbWarps = 8;
-constexpr int kEmbChunk = 64;        // sorted positions per chunk, doubled until 1024 chunks suffice
 
 // acc += the rows perm[j] of DY for j in [j0, j1), columns [c8*8, c8*8+8), four loads in flight.
 __device__ __forceinline__ void emb_sum_run(const void* __restrict__ DY, int dy_dt,
@@ -97,7 +97,7 @@ emb_parts_kernel(const int* __restrict__ sorted, const int* __restrict__ starts,
                  float* __restrict__ part, int n, int C, int V, int chunk) {
   extern __shared__ __align__(16) float emb_part[];          // [kEmbWarps][C]
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p0 = blockIdx.x * chunk, p1 = p0 + chunk < n ? p0 + chunk : n;
+  const int p0 = blockIdx.x * chunk, p1 = emb_chunk_end(p0, chunk, n);
   const int first = sorted[p0], last = sorted[p1 - 1];
   for (int slot = 0; slot < 2; ++slot) {
     const int v = slot == 0 ? first : last;
@@ -130,7 +130,7 @@ embedding_bwd_kernel(const int* __restrict__ starts, const int* __restrict__ per
                      const void* __restrict__ DY, int dy_dt, const float* __restrict__ part,
                      float* __restrict__ GW, int C, int V, int chunk) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int v = blockIdx.x * kEmbWarps + w; v < V; v += gridDim.x * kEmbWarps) {
+  for (long long v = blockIdx.x * kEmbWarps + w; v < V; v += gridDim.x * kEmbWarps) {
     const int s = starts[v], e = starts[v + 1];
     const bool parts = e - s > chunk;
     // The first chunk holds the run in slot 0 only if the run covers its first position.
@@ -159,17 +159,11 @@ embedding_bwd_kernel(const int* __restrict__ starts, const int* __restrict__ per
       } else {
         emb_sum_run(DY, dy_dt, perm, s, e, C, c8, acc);
       }
-      float4* q = reinterpret_cast<float4*>(GW + (long long)v * C + c8 * 8);
+      float4* q = reinterpret_cast<float4*>(GW + v * C + c8 * 8);
       q[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
       q[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
     }
   }
-}
-
-static inline int emb_chunk(long long n) {
-  long long chunk = kEmbChunk;
-  while ((n + chunk - 1) / chunk > 1024) chunk *= 2;
-  return static_cast<int>(chunk);
 }
 
 static inline int key_bits(long long V) {   // bits needed for the values 0 .. V
@@ -198,8 +192,7 @@ DION_EXPORT long long dion_embedding_sort_bytes(long long n, long long V) {
 // Rows of C floats that the partial sums of n tokens need.
 DION_EXPORT long long dion_embedding_part_rows(long long n) {
   if (n <= 0) return 0;
-  const long long chunk = emb_chunk(n);
-  return 2 * ((n + chunk - 1) / chunk);
+  return 2LL * emb_num_chunks(n, emb_chunk(n));
 }
 
 // ids: int64 [n].  DY: [n, C] fp32 or bf16 (dy_dt).  GW: fp32 [V, C], needs no initialisation.
@@ -231,7 +224,7 @@ DION_EXPORT int dion_embedding_bwd(const void* ids, const void* DY, int dy_dt, f
     return -3;
   const int chunk = emb_chunk(n);
   if (ni > chunk)   // else no run is longer than a chunk
-    emb_parts_kernel<<<(ni + chunk - 1) / chunk, kEmbWarps * 32, smem, S(stream)>>>(
+    emb_parts_kernel<<<emb_num_chunks(n, chunk), kEmbWarps * 32, smem, S(stream)>>>(
         keys + ni, starts, vals + ni, DY, dy_dt, part, ni, C, Vi, chunk);
   const int groups = (Vi + kEmbWarps - 1) / kEmbWarps;
   const int cap = 148 * 8;
