@@ -1020,6 +1020,7 @@ qr_update_kernel(float* Aall, long long strideA, int ld, int k, int j, const flo
 
 using namespace dion;
 static inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
+constexpr int kMaxGridY = 65535;   // matrices per launch where they are the grid's second index
 
 template <int KPL>
 static int launch_qr(const float* A, float* V, float* tau, float* R, int n, int k, int r,
@@ -1079,18 +1080,23 @@ DION_EXPORT int dion_cholesky_upper(const void* G, void* U, int n, int r, void* 
         return -3;
       configured = true;
     }
-    if (n > 65535) return -2;
     if (cudaMemsetAsync(u, 0, (size_t)n * r * r * sizeof(float), S(stream)) != cudaSuccess) return -1;
-    for (int k = 0; k < r / 32; ++k) {
-      const int blocks = r / 32 - k;
-      // One block per CTA while that is about two waves of CTAs (96 matrices 512 x 512 with one
-      // block per CTA throughout: 1070 us; with up to four: 666 us).
-      if ((long long)blocks * n <= 296)
-        dion::cholesky_row_kernel<<<dim3(blocks, n), dion::kCholWarps * 32, dion::kCholSmem,
-                                    S(stream)>>>(g, u, r, k);
-      else
-        dion::cholesky_row4_kernel<<<dim3(blocks > 1 ? (blocks + 2) / 4 : 1, n),
-                                     dion::kCholWarps * 32, dion::kCholSmem, S(stream)>>>(g, u, r, k);
+    const int total = n;
+    for (int first = 0; first < total; first += kMaxGridY) {
+      n = total - first < kMaxGridY ? total - first : kMaxGridY;
+      for (int k = 0; k < r / 32; ++k) {
+        const int blocks = r / 32 - k;
+        // One block per CTA while that is about two waves of CTAs (96 matrices 512 x 512 with one
+        // block per CTA throughout: 1070 us; with up to four: 666 us).
+        if ((long long)blocks * n <= 296)
+          dion::cholesky_row_kernel<<<dim3(blocks, n), dion::kCholWarps * 32, dion::kCholSmem,
+                                      S(stream)>>>(g, u, r, k);
+        else
+          dion::cholesky_row4_kernel<<<dim3(blocks > 1 ? (blocks + 2) / 4 : 1, n),
+                                       dion::kCholWarps * 32, dion::kCholSmem, S(stream)>>>(g, u, r, k);
+      }
+      g += (size_t)n * r * r;
+      u += (size_t)n * r * r;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
   }
@@ -1182,7 +1188,7 @@ DION_EXPORT int dion_normalize_q(const void* R, const float* colsq, float eps, v
 // V and VT: [n, k, 32] fp32 scratch, 16-byte aligned.  Two launches per panel of 32 columns.
 DION_EXPORT int dion_qr_blocked(void* A, int n, int k, int r, void* V, void* VT, void* stream) {
   if (n <= 0 || r <= 0) return 0;
-  if ((r & 31) || k < r || n > 65535 ||
+  if ((r & 31) || k < r ||
       ((reinterpret_cast<uintptr_t>(V) | reinterpret_cast<uintptr_t>(VT)) & 15))
     return -2;
   auto smem = [&](int j) {
@@ -1209,9 +1215,11 @@ DION_EXPORT int dion_qr_blocked(void* A, int n, int k, int r, void* V, void* VT,
     const Panel panel = panel_for(j);
     panel<<<n, kQpWarps * 32, smem(j), S(stream)>>>(a, (long long)k * r, r, k, j, v, vt);
     const int blocks = (r - j) / 32 - 1;
-    if (blocks > 0)
-      dion::qr_update_kernel<<<dim3(blocks, n), dion::kQuWarps * 32, 0, S(stream)>>>(
-          a, (long long)k * r, r, k, j, v, vt);
+    for (int first = 0; blocks > 0 && first < n; first += kMaxGridY)
+      dion::qr_update_kernel<<<dim3(blocks, n - first < kMaxGridY ? n - first : kMaxGridY),
+                               dion::kQuWarps * 32, 0, S(stream)>>>(
+          a + (size_t)first * k * r, (long long)k * r, r, k, j, v + (size_t)first * k * 32,
+          vt + (size_t)first * k * 32);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -89,6 +89,23 @@ def test_blocked_qr_equals_column_kernel_up_to_signs():
     assert (Rb.abs() - Rc.abs()).abs().max().item() < 1e-3 * Rc.abs().max().item()
 
 
+@pytest.mark.parametrize("kind", ["cholesky", "qr"])
+def test_factorizations_of_more_matrices_than_a_grid_has_rows(kind):
+    """65535 matrices fit one launch; those behind them are factored like any other."""
+    from dion_b200.ops import lowrank as LR
+    torch.manual_seed(0)
+    n, k, r = 65535 + 3, (64 if kind == "cholesky" else 128), (64 if kind == "cholesky" else 128)
+    few = torch.randn(7, k, r, device="cuda")
+    if kind == "cholesky":
+        few = few.mT @ few + 8 * torch.eye(r, device="cuda")
+    A = few[torch.arange(n, device="cuda") % 7]
+    f = LR.cholesky_upper if kind == "cholesky" else (lambda x: LR.qr_r_factor(x, overwrite=True))
+    got, one = f(A), f(few.clone())
+    rel = lambda i: ((got[i] - one[i % 7]).norm() / one[i % 7].norm()).item()  # noqa: E731
+    # the batch decides how a block's sums are split over warps: fp32 sums of at most 128 terms
+    assert max(rel(i) for i in (0, 1, 65533, 65534, 65535, 65536, 65537)) < 1e-5
+
+
 @pytest.mark.parametrize("shape", [(150, 96), (60, 160), (40, 512), (400, 64)])
 def test_cholesky_upper_of_large_batches(shape):
     """More blocks than two waves: up to four of a block row per CTA, then one, every remainder."""
