@@ -218,9 +218,13 @@ DION_EXPORT int dion_embedding_bwd(const void* ids, const void* DY, int dy_dt, f
       return -4;
   }
   emb_starts_kernel<<<(Vi + 1 + 255) / 256, 256, 0, S(stream)>>>(keys + ni, starts, ni, Vi);
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(emb_parts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
+  // The same limit in every call: a smaller one, set by another thread, could come between it and
+  // the launch.
+  constexpr size_t kMost = (size_t)kEmbWarps * 7168 * sizeof(float);
+  if (smem > kMost ||
+      (smem > 48 * 1024 &&
+       cudaFuncSetAttribute(emb_parts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)kMost) != cudaSuccess))
     return -3;
   const int chunk = emb_chunk(n);
   if (ni > chunk)   // else no run is longer than a chunk

@@ -1022,13 +1022,23 @@ using namespace dion;
 static inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
 constexpr int kMaxGridY = 65535;   // matrices per launch where they are the grid's second index
 
+// Lets a kernel use up to `most` bytes of dynamic shared memory.  `most` is the same in every call for
+// a kernel: a limit that follows the call's own size is lowered by a smaller one on another thread
+// between its setting and the launch, which is then refused.
+template <class K>
+static int allow_dynamic_smem(K kernel, size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) !=
+         cudaSuccess;
+}
+
 template <int KPL>
 static int launch_qr(const float* A, float* V, float* tau, float* R, int n, int k, int r,
                      cudaStream_t s) {
-  const size_t smem = ((size_t)k * kTilePitch + 2 * (size_t)k + (size_t)kPanel * k) * sizeof(float);
-  if (cudaFuncSetAttribute(qr_r_kernel<KPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    return -3;
+  auto smem_for = [](int rows) {
+    return ((size_t)rows * kTilePitch + 2 * (size_t)rows + (size_t)kPanel * rows) * sizeof(float);
+  };
+  const size_t smem = smem_for(k);
+  if (allow_dynamic_smem(qr_r_kernel<KPL>, smem_for(KPL * 32))) return -3;
   qr_r_kernel<KPL><<<n, kLrThreads, smem, s>>>(A, V, tau, R, k, r);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -1052,9 +1062,7 @@ DION_EXPORT int dion_qr_r_factor(const void* A, void* V, void* tau, void* R, int
 template <int KPL>
 static int launch_chol(const float* G, float* U, int n, int r, cudaStream_t s) {
   const size_t smem = (2 + kPanel) * (size_t)r * sizeof(float);
-  if (cudaFuncSetAttribute(cholesky_upper_kernel<KPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    return -3;
+  if (allow_dynamic_smem(cholesky_upper_kernel<KPL>, (2 + kPanel) * KPL * 32 * sizeof(float))) return -3;
   cholesky_upper_kernel<KPL><<<n, kLrThreads, smem, s>>>(G, U, r);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -1194,7 +1202,8 @@ DION_EXPORT int dion_qr_blocked(void* A, int n, int k, int r, void* V, void* VT,
   auto smem = [&](int j) {
     return ((size_t)(k - j) * kQpPitch + kQpWarps * 32 + 96 + 2 * 32 * kQpSq) * sizeof(float);
   };
-  if (smem(0) > 226 * 1024) return -2;
+  constexpr size_t kMost = 226 * 1024;
+  if (smem(0) > kMost) return -2;
   // Registers for 24 or 48 rows per warp (384, 768 rows), else shared memory.  Only the forms that
   // this factorization uses are touched: loading a kernel takes milliseconds, once a process.
   typedef void (*Panel)(float*, long long, int, int, int, float*, float*);
@@ -1204,9 +1213,7 @@ DION_EXPORT int dion_qr_blocked(void* A, int n, int k, int r, void* V, void* VT,
     return rows <= 768 ? dion::qr_panel_kernel<48> : dion::qr_panel_kernel<0>;
   };
   for (int j = 0; j < r; j += 32)
-    if ((j == 0 || panel_for(j) != panel_for(j - 32)) &&
-        cudaFuncSetAttribute(panel_for(j), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem(j)) != cudaSuccess)
+    if ((j == 0 || panel_for(j) != panel_for(j - 32)) && allow_dynamic_smem(panel_for(j), kMost))
       return -3;
   float* a = static_cast<float*>(A);
   float* v = static_cast<float*>(V);

@@ -89,6 +89,43 @@ def test_blocked_qr_equals_column_kernel_up_to_signs():
     assert (Rb.abs() - Rc.abs()).abs().max().item() < 1e-3 * Rc.abs().max().item()
 
 
+def test_factorizations_on_two_threads():
+    """Different sizes at the same time, which differ in the shared memory of the same kernels:
+    every launch is accepted and gives what it gives alone."""
+    import threading
+
+    from dion_b200.ops import lowrank as LR
+    torch.manual_seed(0)
+    sizes = [(768, 256), (416, 160), (640, 128), (400, 384), (200, 100), (130, 90)]
+    As = [torch.randn(2, k, r, device="cuda") for k, r in sizes]
+    alone = [LR.qr_r_factor(A) for A in As]
+    torch.cuda.synchronize()
+    errors, start = [], threading.Barrier(2)
+
+    def work(which):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait()
+                for _ in range(150):
+                    for i in which:
+                        R = LR.qr_r_factor(As[i])
+                for i in which:
+                    R = LR.qr_r_factor(As[i])
+                    torch.cuda.current_stream().synchronize()
+                    # atomics order the sums of V^T V: fp32 roundings of at most 768 terms
+                    err = (R.abs() - alone[i].abs()).norm() / alone[i].norm()
+                    assert err.item() < 1e-4, (sizes[i], err.item())
+        except Exception as e:                                   # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(w,)) for w in ((0, 2, 4), (1, 3, 5))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+
+
 @pytest.mark.parametrize("kind", ["cholesky", "qr"])
 def test_factorizations_of_more_matrices_than_a_grid_has_rows(kind):
     """65535 matrices fit one launch; those behind them are factored like any other."""
