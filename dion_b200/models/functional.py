@@ -374,6 +374,8 @@ class _Embedding(torch.autograd.Function):
             _c(flat), _c(dy2), _DT[dy2.dtype], _c(gw), ctypes.c_longlong(n), C,
             ctypes.c_longlong(V), _c(keys), _c(vals), _c(starts), _c(temp),
             ctypes.c_longlong(nbytes), _c(part), _stream(dev)), "dion_embedding_bwd")
+        if n > 64:      # a run can be longer than a chunk: the kernel that sums parts runs too
+            _backend.add_launches(1)
         return None, gw
 
 

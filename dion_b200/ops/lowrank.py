@@ -299,6 +299,7 @@ def householder_q(P: Tensor) -> Tensor:
     return Q
 
 
+_MAX_GRID_Y = 65535            # matrices per launch of the update and Cholesky kernels
 _QR_PANEL = 32
 _QR_PANEL_MAX_ROWS = 1580      # shared memory of the panel kernel: (rows * 32 + ...) * 4 bytes
 # The single-kernel form takes 205 us for 16 matrices 160 x 128 and 424 us for 12 of 240 x 192, the
@@ -312,9 +313,10 @@ def blocked_qr_enabled() -> bool:
 
 def _qr_r_blocked(A32: Tensor) -> Tensor:
     """Blocked Householder QR of a private fp32 batch ``[B, k, r]`` (overwritten): per 32-column
-    panel one kernel factors the panel in shared memory (one CTA per matrix) and emits the
-    reflectors ``V`` and ``V T^T`` of the compact WY form; a second one updates the columns to the
-    right, ``W = V^T A_right`` and ``A_right -= (V T^T) W``, in fp32."""
+    panel one kernel factors the panel (one CTA per matrix, up to 768 rows in registers, else in
+    shared memory) and emits the reflectors ``V`` and ``V T^T`` of the compact WY form; a second
+    one updates the columns to the right, ``W = V^T A_right`` and ``A_right -= (V T^T) W``, in
+    fp32."""
     B, k, r = A32.shape
     dev = A32.device
     V, VT = torch.empty((2, B, k, _QR_PANEL), dtype=torch.float32, device=dev).unbind(0)
@@ -322,7 +324,8 @@ def _qr_r_blocked(A32: Tensor) -> Tensor:
                                                      _stream(dev))
     if rc != 0:
         raise RuntimeError(f"dion_qr_blocked launch failed (code {rc})")
-    _backend.add_launches(2 * (r // _QR_PANEL) - 2)
+    panels = r // _QR_PANEL     # one launch was counted
+    _backend.add_launches(panels - 1 + (panels - 1) * -(-B // _MAX_GRID_Y))
     return torch.triu(A32[:, :r, :r])
 
 
@@ -357,7 +360,8 @@ def qr_r_factor(A: Tensor, overwrite: bool = False) -> Tensor:
 
 def cholesky_upper(G: Tensor) -> Tensor:
     """Upper Cholesky factor without raising on failure (NaNs propagate and are handled by
-    :func:`fix_all_zero_or_nan`).  GPU batches of fp32 matrices go to one kernel."""
+    :func:`fix_all_zero_or_nan`).  GPU batches of fp32 matrices are factored together: one launch
+    per 32 rows for sizes that are a multiple of 32 (at least 64), else one kernel."""
     if (G.is_cuda and G.dtype == torch.float32 and G.ndim == 3
             and G.size(-1) == G.size(-2) <= _MAX_FACTOR_DIM):
         Gc = G.contiguous()
@@ -366,6 +370,8 @@ def cholesky_upper(G: Tensor) -> Tensor:
             _ptr(Gc), _ptr(U), Gc.size(0), Gc.size(-1), _stream(Gc.device))
         if rc != 0:
             raise RuntimeError(f"dion_cholesky_upper launch failed (code {rc})")
+        if Gc.size(-1) % 32 == 0 and Gc.size(-1) >= 64 and Gc.data_ptr() % 16 == 0:
+            _backend.add_launches(Gc.size(-1) // 32 * -(-Gc.size(0) // _MAX_GRID_Y) - 1)
         return U
     return torch.linalg.cholesky_ex(G, upper=True)[0]
 

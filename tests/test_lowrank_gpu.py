@@ -149,6 +149,16 @@ def test_cholesky_upper_of_large_batches(shape):
     test_cholesky_upper(shape)
 
 
+@pytest.mark.parametrize("r,launches", [(17, 1), (32, 1), (64, 2), (512, 16)])
+def test_cholesky_counts_its_launches(r, launches):
+    from dion_b200.ops import _backend
+    from dion_b200.ops import lowrank as LR
+    G = torch.eye(r, device="cuda").repeat(2, 1, 1)
+    before = _backend.launch_count()
+    LR.cholesky_upper(G)
+    assert _backend.launch_count() - before == launches
+
+
 @pytest.mark.parametrize("shape", [(3, 96), (5, 192), (2, 512), (2, 768), (4, 17), (2, 64), (1, 1024)])
 def test_cholesky_upper(shape):
     from dion_b200.ops import lowrank as LR
