@@ -256,7 +256,7 @@ def adamw(
             else None
         _check(
             _backend.lib("foreach_ops").dion_adamw(
-                _c(tb.device_tensor.data_ptr()), ctypes.c_longlong(tb.n_chunks),
+                _c(tb.device_tensor.data_ptr()), ctypes.c_longlong(tb.n_chunks), n,
                 _c(lr_t.data_ptr()), _c(wd_t.data_ptr() if wd_t is not None else 0),
                 ctypes.c_float(wd_f), ctypes.c_float(beta1), ctypes.c_float(beta2),
                 ctypes.c_float(epsilon), int(bool(cautious_wd)),
@@ -264,6 +264,8 @@ def adamw(
                 int(state_steps is not None), ctypes.c_float(float(step or 0)),
                 _c(corr.data_ptr() if corr is not None else 0), _stream(dev)),
             "dion_adamw")
+        if state_steps is not None:     # counters: one launch, two beyond 256 tensors
+            _backend.add_launches(1 if n <= 256 else 2)
         return
     # PyTorch path
     if state_steps is not None:
