@@ -174,7 +174,7 @@ class GPT(nn.Module):
                 return_logits: bool = False):
         x = None
         if not torch.is_grad_enabled():
-            x = inference.hidden_states(self, idx, (Block, CausalSelfAttention, MLP, Rotary))
+            x = inference.hidden_states(self, idx, _FORWARDS)
         if x is None:
             wte = self.transformer.wte
             x = Fn.embedding(idx, wte.weight) if _is_plain(wte) else wte(idx)
@@ -209,6 +209,10 @@ class GPT(nn.Module):
             nxt = torch.multinomial(tF.softmax(logits, dim=-1), num_samples=1)
             idx = torch.cat([idx, nxt], dim=1)
         return idx
+
+
+# The modules that the path without gradients stands in for, with the forwards that it computes.
+_FORWARDS = tuple((c, c.forward) for c in (Block, CausalSelfAttention, MLP, Rotary))
 
 
 # ------------------------------------------------------------------------------------------------

@@ -50,8 +50,17 @@ def _entry_points() -> tuple:
     return _entries
 
 
+_MODULE_CALL = torch.nn.Module.__call__
+
+
 def _unhooked(m) -> bool:
-    return not (m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__)
+    return not (m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__
+                or m._compiled_call_impl is not None)
+
+
+def _replaced(forwards) -> bool:
+    """A class of the blocks' modules has been given another ``forward`` or ``__call__``."""
+    return any(c.forward is not f or c.__call__ is not _MODULE_CALL for c, f in forwards)
 
 
 def _observed() -> bool:
@@ -94,25 +103,27 @@ def _config(rows: int, N: int, K: int, dev: torch.device) -> _Gemm:
     return _Gemm(tiles.data_ptr(), tiles.size(0), 0 if pair else bn)
 
 
-def hidden_states(model, idx: Tensor, types) -> Optional[Tensor]:
+def hidden_states(model, idx: Tensor, forwards) -> Optional[Tensor]:
     """``[B, T, C]`` bf16: the residual stream after the last block, normalized.  None unless
     gradients are off, bf16 autocast is on, the model is a plain GPT (no hooks, no shards, no
-    replaced modules; fp32 embedding; dense fp32 or bf16 weights of one dtype) on the GPU of
-    ``idx``, and nothing observes operators."""
+    replaced modules or forwards; fp32 embedding; dense fp32 or bf16 weights of one dtype) on the
+    GPU of ``idx``, and nothing observes operators.  ``forwards``: the classes of block, attention,
+    MLP and rotary embedding, each with its own ``forward``."""
     wte = model.transformer.wte
     blocks = model.transformer.h
     if type(wte) is not torch.nn.Embedding:
         return None
     table = wte.weight
     C = table.size(-1)
-    if (torch.is_grad_enabled() or not idx.is_cuda or not is_plain_tensor(idx) or idx.ndim != 2
+    if (torch.is_grad_enabled() or not is_plain_tensor(idx) or not idx.is_cuda or idx.ndim != 2
             or idx.numel() == 0 or len(blocks) == 0
             or not torch.is_autocast_enabled("cuda")
             or torch.get_autocast_dtype("cuda") != torch.bfloat16
             or not is_plain_tensor(table) or table.dtype != torch.float32
             or table.device != idx.device or C % 8 or C > 4096 or not _unhooked(wte)
-            or _observed()):
+            or _observed() or _replaced(forwards)):
         return None
+    types = tuple(c for c, _ in forwards)
     weights = [_block_weights(b, types, C) for b in blocks]
     if any(w is None for w in weights):
         return None

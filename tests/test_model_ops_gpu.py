@@ -335,3 +335,30 @@ def test_replaced_modules_take_the_general_forward():
             with torch.no_grad():
                 got = model(ids, ids, return_logits=True)
         assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("name", ["Block", "CausalSelfAttention", "MLP", "Rotary"])
+def test_replaced_forward_of_a_class_is_called(name, monkeypatch):
+    """A ``forward`` put on the class (as instrumentation and adapters do) counts without gradients
+    too."""
+    from dion_b200.models import gpt
+    cls = getattr(gpt, name)
+    torch.manual_seed(0)
+    ids = torch.randint(0, 512, (2, 24), device="cuda")
+    model = gpt.GPT(gpt.GPTConfig(sequence_len=24, vocab_size=512, n_layer=2, n_head=2,
+                                  n_embd=128)).cuda()
+    model.init_weights()
+    own, seen = cls.forward, []
+
+    def forward(self, *args):
+        seen.append(1)
+        return own(self, *args)
+
+    monkeypatch.setattr(cls, "forward", forward)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        ref = model(ids, ids, return_logits=True).detach()
+        with torch.no_grad():
+            seen.clear()
+            got = model(ids, ids, return_logits=True)
+    assert len(seen) == 2
+    assert torch.equal(got, ref)
