@@ -116,32 +116,37 @@ def sm_count(device: torch.device) -> int:
     return n
 
 
+def _tile_pairs(tm_n: int, tn_n: int, bm: int, bn: int, sym: bool) -> Tensor:
+    pairs = torch.cartesian_prod(torch.arange(tm_n, dtype=torch.int32),
+                                 torch.arange(tn_n, dtype=torch.int32))
+    return pairs[(pairs[:, 1] + 1) * bn > pairs[:, 0] * bm] if sym else pairs
+
+
+def _upload(host: Tensor, device: torch.device) -> Tensor:
+    return host.to(device, non_blocking=host.is_pinned())
+
+
+def _capturing(device: torch.device) -> bool:
+    return device.type == "cuda" and torch.cuda.is_current_stream_capturing()
+
+
 def tile_table(M: int, N: int, bn: int, sym: bool, device: torch.device,
                bm: int = _BM) -> Tensor:
     """Device array of (tile_m, tile_n) pairs.  For ``sym`` only tiles that intersect the
-    upper triangle (column range reaching the tile's first row) are listed."""
-    key = (M, N, bn, sym, device.index, bm)
+    upper triangle (column range reaching the tile's first row) are listed.  Kept by the numbers
+    of tiles, which text of growing length changes once in 128 or 256 tokens."""
+    tm_n, tn_n = -(-M // bm), -(-N // bn)
+    key = (tm_n, tn_n, bm if sym else 0, bn if sym else 0, device.index)
     t = _tile_cache.get(key)
     if t is not None:
         return t
-    tm_n = (M + bm - 1) // bm
-    tn_n = (N + bn - 1) // bn
-    pairs = []
-    for tm in range(tm_n):
-        for tn in range(tn_n):
-            if sym and (tn + 1) * bn - 1 < tm * bm:
-                continue
-            pairs.append((tm, tn))
-    host = torch.tensor(pairs, dtype=torch.int32)
-    if device.type == "cuda" and torch.cuda.is_current_stream_capturing():
+    if _capturing(device):
         # First use of this shape inside a graph capture: the copy is recorded, so it has to
         # read pinned memory that stays alive as long as the table does.
-        host = host.pin_memory()
-        _tile_hosts[key] = host
-        t = host.to(device, non_blocking=True)
-    else:
-        t = host.to(device)
-    _tile_cache[key] = t
+        host = _tile_hosts[key] = _tile_pairs(tm_n, tn_n, bm, bn, sym).contiguous().pin_memory()
+        t = _tile_cache[key] = _upload(host, device)
+        return t
+    t = _tile_cache[key] = _upload(_tile_pairs(tm_n, tn_n, bm, bn, sym).contiguous(), device)
     return t
 
 
@@ -239,6 +244,8 @@ def _choose_config(M: int, N: int, K: int, batch: int, sym: bool, pair_ok: bool,
         t = -(-tiles // units) * size * (K / eff + fixed)
         if best_t is None or t < best_t - 1e-9:
             best, best_t = (is_pair, bn), t
+    if len(_config_cache) >= 4096:      # every length of a text is a shape of its own
+        _config_cache.clear()
     _config_cache[key] = best
     return best
 
@@ -453,7 +460,7 @@ def ns_persistent(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs,
     dev = X.device
     g = min(m, n)
     bn = _persistent_bn(m, n, batch, dev)
-    key = (m, n, bn, dev.index)
+    key = (-(-m // _BM), -(-n // bn), -(-g // _BM), -(-g // bn), bn, dev.index)
     tab = _persist_tiles.get(key)
     if tab is None:
         gg = tile_table(g, g, bn, True, dev)

@@ -82,3 +82,23 @@ def test_tensor_map_cache_hits_only_on_identical_keys(tmp_path):
                         text=True, check=True).stdout.split()
     assert off == ["3", "6", "0", "1", "1"]      # every call encodes
     assert on == ["1", "3", "1", "1", "1"]       # repeats hit, other box / address miss
+
+
+def test_tile_tables_are_kept_by_tile_counts(monkeypatch):
+    """A text that grows token by token uploads a table once per 128 or 256 rows, and the choices
+    that are kept per length are bounded."""
+    from dion_b200.ops import gemm
+    dev = torch.device("cpu")
+    for name in ("_tile_cache", "_config_cache"):
+        monkeypatch.setattr(gemm, name, {})
+    monkeypatch.setattr(gemm, "sm_count", lambda d: 148)
+    for M in range(1, 1025):
+        for N in (768, 2304, 3072):
+            for bm, bn in ((128, 128), (128, 256), (256, 256)):
+                t = gemm.tile_table(M, N, bn, False, dev, bm=bm)
+                assert t.size(0) == -(-M // bm) * -(-N // bn)
+    assert len(gemm._tile_cache) <= 8 * 6 + 4 * 3
+    for M in range(1, 20001):
+        gemm._choose_config(M, 768, 768, 1, False, True, dev)
+    assert len(gemm._config_cache) <= 4096
+
