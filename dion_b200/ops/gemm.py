@@ -141,11 +141,12 @@ def tile_table(M: int, N: int, bn: int, sym: bool, device: torch.device,
     if t is not None:
         return t
     if _capturing(device):
-        # First use of this shape inside a graph capture: the copy is recorded, so it has to
-        # read pinned memory that stays alive as long as the table does.
-        host = _tile_hosts[key] = _tile_pairs(tm_n, tn_n, bm, bn, sym).contiguous().pin_memory()
-        t = _tile_cache[key] = _upload(host, device)
-        return t
+        # The copy is recorded: it reads pinned memory that stays, and what it writes is there only
+        # once that graph has run, so no other call may find it.
+        host = _tile_hosts.get(key)
+        if host is None:
+            host = _tile_hosts[key] = _tile_pairs(tm_n, tn_n, bm, bn, sym).contiguous().pin_memory()
+        return _upload(host, device)
     t = _tile_cache[key] = _upload(_tile_pairs(tm_n, tn_n, bm, bn, sym).contiguous(), device)
     return t
 
@@ -465,7 +466,9 @@ def ns_persistent(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs,
     if tab is None:
         gg = tile_table(g, g, bn, True, dev)
         mn = tile_table(m, n, bn, False, dev)
-        tab = _persist_tiles[key] = (torch.cat([gg, mn]).contiguous(), gg.size(0), mn.size(0))
+        tab = (torch.cat([gg, mn]).contiguous(), gg.size(0), mn.size(0))
+        if not _capturing(dev):
+            _persist_tiles[key] = tab
     tiles, n_gg, n_mn = tab
     counter = torch.empty(1, dtype=torch.int32, device=dev)   # of this launch alone
     flat = (ctypes.c_float * (3 * len(coeffs)))(*[float(v) for abc in coeffs for v in abc])

@@ -102,3 +102,24 @@ def test_tile_tables_are_kept_by_tile_counts(monkeypatch):
         gemm._choose_config(M, 768, 768, 1, False, True, dev)
     assert len(gemm._config_cache) <= 4096
 
+
+def test_tile_tables_of_a_capture_are_its_own(monkeypatch):
+    """What a captured copy writes is there only once that graph has run: neither an eager call nor
+    another capture may find it."""
+    from dion_b200.ops import gemm
+    monkeypatch.setattr(gemm, "_tile_cache", {})
+    monkeypatch.setattr(gemm, "_tile_hosts", {})
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda t: t)
+    uploads = []
+    monkeypatch.setattr(gemm, "_upload", lambda host, dev: uploads.append(host) or host.clone())
+    dev, capturing = torch.device("cuda", 0), [True]
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    first = gemm.tile_table(300, 300, 128, True, dev)
+    second = gemm.tile_table(300, 300, 128, True, dev)
+    assert first is not second and uploads[0] is uploads[1]      # one host copy serves every graph
+    capturing[0] = False
+    eager = gemm.tile_table(300, 300, 128, True, dev)
+    assert eager is not first and len(uploads) == 3
+    assert gemm.tile_table(300, 300, 128, True, dev) is eager
+    capturing[0] = True
+    assert gemm.tile_table(300, 300, 128, True, dev) is eager    # filled before: graphs may use it

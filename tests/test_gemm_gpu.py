@@ -332,3 +332,28 @@ def test_exchange_coupling_by_columns_on_one_gpu(pair, tall):
     assert (got.float() - want).abs().max().item() < 2e-2 * want.abs().max().item()
     for b_ in bufs:
         assert float(b_[0].abs().max()) == 0 and float(b_[4].abs().max()) == 0
+
+
+def test_shape_first_met_in_a_capture():
+    """A product whose tile table is first needed while a graph is captured: right when that graph
+    runs, when another one does, and in an eager call made before either has run."""
+    from dion_b200.ops import gemm
+    torch.manual_seed(0)
+    A = torch.randn(3, 872, 136, device="cuda").bfloat16()
+    B = torch.randn(3, 1112, 136, device="cuda").bfloat16()
+    ref = A.float() @ B.float().mT
+    gemm.ns_gemm(A[:, :8].contiguous(), B[:, :8].contiguous())       # libraries are loaded
+    torch.cuda.synchronize()
+    graphs, outs = [], []
+    for _ in range(2):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs.append(gemm.ns_gemm(A, B))
+        graphs.append(g)
+    eager = gemm.ns_gemm(A, B)
+    assert _rel_err(eager, ref) < 2.0 ** -8
+    for g, o in zip(reversed(graphs), reversed(outs)):
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(o, eager)
+    gemm.check_status()
