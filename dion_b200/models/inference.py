@@ -104,11 +104,24 @@ def _config(rows: int, N: int, K: int, dev: torch.device) -> _Gemm:
     return _Gemm(tiles.data_ptr(), tiles.size(0), 0 if pair else bn)
 
 
+def _pays(C: int, F: int, rows: int) -> bool:
+    """Whether a block of width ``C`` (``F`` in the MLP) is faster here for so many rows.
+
+    The general forward needs 0.4 ms of host time a block.  That is what a block takes on the device
+    here at (elements of its weights) x (rows + 512) = 1.7e11: rounding the weights weighs as much as
+    512 rows of products.  Beyond that the products decide, and for wide models the tcgen05 kernels
+    trail the library.  General against native, eight blocks: width 3072, 512 rows 3.50 / 2.88 ms, 2048
+    rows 4.51 / 5.61; width 2048, 2048 rows 3.50 / 2.45, 4096 rows 3.86 / 3.94, 65536 rows 50.8 / 52.2;
+    width 4096, 256 rows 3.56 / 3.59, 16384 rows 46.0 / 53.4.  Up to width 1536 the native blocks are
+    as fast or faster throughout (768, 65536 rows: 11.4 / 10.6; 1536, 8192 rows: 4.45 / 4.44)."""
+    return C <= 1536 or (4 * C * C + 2 * C * F) * (rows + 512) <= 1.7e11
+
+
 def hidden_states(model, idx: Tensor, forwards) -> Optional[Tensor]:
     """``[B, T, C]`` bf16: the residual stream after the last block, normalized.  None unless
     gradients are off, bf16 autocast is on, the model is a plain GPT (no hooks, no shards, no
     replaced modules or forwards; fp32 embedding; dense fp32 or bf16 weights of one dtype) on the
-    GPU of ``idx``, and nothing observes operators.  ``forwards``: the classes of block, attention,
+    GPU of ``idx``, nothing observes operators, and the size is one that gains (:func:`_pays`).  ``forwards``: the classes of block, attention,
     MLP and rotary embedding, each with its own ``forward``."""
     wte = model.transformer.wte
     blocks = model.transformer.h
@@ -135,8 +148,9 @@ def hidden_states(model, idx: Tensor, forwards) -> Optional[Tensor]:
     if first[0].dtype not in (torch.float32, torch.bfloat16) or D not in (32, 64, 128, 256) \
             or D * H != C:
         return None
-    if F % 8 or any(w[4].size(0) != F or w[0].dtype != first[0].dtype
-                    or w[0].device != idx.device for w in weights) \
+    if F % 8 or not _pays(C, F, B * T) or any(
+            w[4].size(0) != F or w[0].dtype != first[0].dtype or w[0].device != idx.device
+            for w in weights) \
             or any(b.attn.n_head != H for b in blocks):
         return None
     dev, rows = idx.device, B * T

@@ -138,3 +138,11 @@ def test_reference_import_names_forward_to_this_package():
                            env=dict(os.environ, PYTHONPATH=root), capture_output=True, text=True,
                            timeout=300)
     assert plain.stdout.strip() == "False"
+
+
+def test_native_blocks_are_chosen_by_size():
+    """Narrow models always; wide ones while the saved host time outweighs slower products."""
+    from dion_b200.models.inference import _pays
+    assert all(_pays(C, 4 * C, 1 << 20) for C in (64, 768, 1536))
+    for C, most in ((1792, 3899), (2048, 2865), (3072, 989), (4096, 332)):
+        assert _pays(C, 4 * C, 1) and _pays(C, 4 * C, most) and not _pays(C, 4 * C, most + 1)

@@ -362,3 +362,18 @@ def test_replaced_forward_of_a_class_is_called(name, monkeypatch):
             got = model(ids, ids, return_logits=True)
     assert len(seen) == 2
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("width,rows,native", [(768, 4096, True), (2048, 2048, True),
+                                               (2048, 4096, False), (3072, 512, True),
+                                               (3072, 2048, False)])
+def test_wide_models_with_many_rows_take_the_library_products(width, rows, native):
+    """Both sides of the line up to which the path without gradients gains (not how fast they are)."""
+    from dion_b200.models import gpt, inference
+    with torch.device("cuda"):
+        model = gpt.GPT(gpt.GPTConfig(sequence_len=512, vocab_size=64, n_layer=1,
+                                      n_head=width // 128, n_embd=width))
+    model.init_weights()
+    ids = torch.zeros(rows // 512, 512, dtype=torch.long, device="cuda")
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        assert (inference.hidden_states(model, ids, gpt._FORWARDS) is not None) == native
