@@ -19,9 +19,12 @@ static_assert(kChunk == kThreads * 16, "the vector paths read 16 elements per th
 
 enum : int { DT_F32 = 0, DT_BF16 = 1 };
 
+// [n | one_size << 32, chunk_prefix[n + 1], numel[n], ptr_0[n], ptr_1[n], ...]; one_size: n > 4 and
+// every tensor has as many chunks as the first.
 struct Table {
   const long long* raw;
   __device__ __forceinline__ int n() const { return (int)raw[0]; }
+  __device__ __forceinline__ bool one_size() const { return (raw[0] >> 32) != 0; }
   __device__ __forceinline__ const long long* prefix() const { return raw + 1; }
   __device__ __forceinline__ long long numel(int t) const { return raw[1 + (n() + 1) + t]; }
   __device__ __forceinline__ void* ptr(int which, int t) const {
@@ -29,15 +32,16 @@ struct Table {
   }
 };
 
+// The tensors of an optimizer's bucket mostly have one size: the tensor of a chunk is then a quotient,
+// and a block starts after one dependent read instead of one per bit of their number (48 x 2048^2:
+// bf16 momentum kernel 257 -> 243 us, fp32 492 -> 471 us).  Up to four tensors the search is as short
+// and the division costs more (one tensor of 30 M: 74 -> 76 us), so the host leaves the bit clear.
+// (A guess that is checked instead of known cost short lists and lists of several sizes 2 to 5 %.)
 __device__ __forceinline__ int find_tensor(const Table& tb, long long chunk) {
   const long long* pre = tb.prefix();
-  // The tensors of a bucket mostly have one size: then this guess is right, and a block starts
-  // after two dependent reads instead of one per bit of the number of tensors (48 x 2048^2: bf16
-  // momentum kernel 262 -> 253 us, fp32 499 -> 485 us).
-  const long long each = pre[1];
-  if (each > 0) {
-    const long long g = chunk / each;
-    if (g < tb.n() && pre[g] <= chunk && chunk < pre[g + 1]) return (int)g;
+  if (tb.one_size()) {
+    const unsigned each = (unsigned)pre[1];
+    return each > 0 ? (int)((unsigned)chunk / each) : 0;
   }
   int lo = 0, hi = tb.n();
   while (hi - lo > 1) {

@@ -1,6 +1,7 @@
 """Device-side tensor tables for the multi-tensor kernels.
 
-A table is one int64 device tensor ``[n, chunk_prefix[n+1], numel[n], ptr_0[n], ptr_1[n], ...]``.
+A table is one int64 device tensor ``[n, chunk_prefix[n+1], numel[n], ptr_0[n], ptr_1[n], ...]``;
+bit 32 of the first word says that there are more than four tensors, all of as many chunks.
 Tables are cached by the data pointers they describe, so a steady-state optimizer step (same
 parameter, gradient and state buffers every iteration) performs no host-to-device copy; when a
 gradient buffer moves (``zero_grad(set_to_none=True)``) the table is rebuilt.
@@ -124,7 +125,8 @@ def build_table(
     prefix = [0]
     for ne in numels:
         prefix.append(prefix[-1] + (ne + chunk - 1) // chunk)
-    flat: List[int] = [n] + prefix + list(numels)
+    one_size = n > 4 and all(b - a == prefix[1] for a, b in zip(prefix, prefix[1:]))
+    flat: List[int] = [n | int(one_size) << 32] + prefix + list(numels)
     for lst in lists:
         assert len(lst) == n
         flat.extend(_ptr(t) for t in lst)

@@ -286,6 +286,20 @@ def test_adamw_counters_of_many_tensors(n):
         assert (x - ref).abs().max().item() <= 1e-5 * abs(ref)
 
 
+@pytest.mark.parametrize("sizes", [[5000] * 4, [5000] * 5, [8193] * 9, [0] * 6, [1] * 300,
+                                   [8192, 4096, 12288] * 3, [5000] * 8 + [0], [0] + [5000] * 8,
+                                   [4096, 4097, 4095] * 2])
+def test_every_tensor_of_a_list_is_found(sizes):
+    """Lists of one size (a quotient) and of several (a search), some with the total that one size
+    would have, with empty tensors and remainders."""
+    g = torch.Generator().manual_seed(0)
+    G, M = [[torch.randn(n, generator=g) for n in sizes] for _ in range(2)]
+    Gd, Md = [t.cuda() for t in G], [t.cuda() for t in M]
+    F.muon_pre(G, M, 0.95, True)
+    F.muon_pre(Gd, Md, 0.95, True)
+    _close(M, Md, 1e-6)
+
+
 def test_adamw_counters_of_many_tensors_are_no_bottleneck():
     """4000 counters: the look for shared ones is spread over the GPU (0.4 ms; in one block 2 ms)."""
     n = 4000
