@@ -302,9 +302,23 @@ def householder_q(P: Tensor) -> Tensor:
 _MAX_GRID_Y = 65535            # matrices per launch of the update and Cholesky kernels
 _QR_PANEL = 32
 _QR_PANEL_MAX_ROWS = 1580      # shared memory of the panel kernel: (rows * 32 + ...) * 4 bytes
-# The single-kernel form takes 205 us for 16 matrices 160 x 128 and 424 us for 12 of 240 x 192, the
-# blocked one 162 and 268 us; narrower sketches are left to the former.
-_QR_BLOCKED_MIN_COLS = 128
+_QR_BLOCKED_MIN_COLS = 128     # narrower sketches are left to the single-kernel form
+
+
+def _blocked_qr_pays(B: int, k: int, r: int, sms: int) -> bool:
+    """Whether the blocked form is the faster one, for ``r >= 128`` columns.
+
+    From 256 columns it always is.  Below, the other form has one CTA per matrix do everything and a
+    GPU full of matrices hides its waits: single / blocked 205 / 162 us for 16 matrices 160 x 128, 216 /
+    224 for 148 of 256 x 128, 415 / 373 for 148 of 256 x 192, 1005 / 1379 for 1000 of 256 x 128; from
+    224 columns blocked again (2890 / 2428 for 600 of 384 x 224).  Panels of more than 768 rows do
+    not fit registers (48 of 1024 x 128: 508 / 645).  The single form ends at 1024 rows; the library,
+    which takes one matrix after the other, is the faster one for one (1536 x 128: 552 / 900 us)."""
+    if r >= 256:
+        return True
+    if k > _MAX_FACTOR_DIM:
+        return B > 1
+    return k <= 768 and (r >= 224 or (B <= sms and B * k <= 1.75 * r * r))
 
 
 def blocked_qr_enabled() -> bool:
@@ -332,14 +346,15 @@ def _qr_r_blocked(A32: Tensor) -> Tensor:
 def qr_r_factor(A: Tensor, overwrite: bool = False) -> Tensor:
     """Upper-triangular factor of every ``A[b]`` (``[B, k, r]``, ``k >= r``) in fp32.  On a GPU
     all matrices of the batch are factored together: blocked Householder, two kernels per panel,
-    when ``r`` is a multiple of 32 (at least 128), else one kernel
+    when ``r`` is a multiple of 32 (at least 128) and that is the faster form, else one kernel
     with one CTA per matrix (up to 1024 rows).  The sign of a row of ``R`` may differ from
     LAPACK's.  ``overwrite``: ``A`` is a temporary of the caller and may be destroyed."""
     A32 = A.to(torch.float32)
     if A32.is_cuda and A32.ndim == 3 and A32.size(-1) <= A32.size(-2):
         B, k, r = A32.shape
         if (blocked_qr_enabled() and r % _QR_PANEL == 0 and r >= _QR_BLOCKED_MIN_COLS
-                and k <= _QR_PANEL_MAX_ROWS and k % 4 == 0 and B > 0):
+                and k <= _QR_PANEL_MAX_ROWS and k % 4 == 0 and B > 0
+                and _blocked_qr_pays(B, k, r, gemm.sm_count(A32.device))):
             if not A32.is_contiguous():
                 A32 = A32.contiguous()
             elif A32.data_ptr() == A.data_ptr() and not overwrite:

@@ -104,3 +104,14 @@ def test_power_iteration_products_and_stacking():
     assert Mt.shape == (3, 9, 6) and Mt.is_contiguous() and torch.equal(Mt[1], M[1].T)
     mixed, q = LR.stack_for_power_iteration([m.bfloat16() for m in M], Qs, transposed=False)
     assert q.dtype == torch.bfloat16                         # Q follows the momentum dtype
+
+
+def test_qr_form_follows_columns_rows_and_matrices():
+    """The line between the two forms, on both sides as measured."""
+    from dion_b200.ops.lowrank import _blocked_qr_pays
+    for B, k, r in ((16, 160, 128), (96, 256, 128), (148, 256, 192), (600, 384, 224), (1, 640, 512),
+                    (1000, 384, 256), (2, 1536, 128)):
+        assert _blocked_qr_pays(B, k, r, 148), (B, k, r)
+    for B, k, r in ((148, 256, 128), (300, 256, 128), (1000, 256, 192), (48, 1024, 128),
+                    (1, 1536, 128)):
+        assert not _blocked_qr_pays(B, k, r, 148), (B, k, r)
