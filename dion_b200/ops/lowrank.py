@@ -15,7 +15,7 @@ from typing import List, Optional, Tuple
 import torch
 from torch import Tensor
 
-from . import _backend
+from . import _backend, gemm
 
 _MAX_FACTOR_DIM = 1024  # row limit of the batched factorization kernels (csrc/lowrank_ops.cu)
 
@@ -156,7 +156,6 @@ def lr_gemm(A: Tensor, B: Tensor, *, a_mn: bool = False, b_mn: bool = False,
     ``broadcast_to``: raw base addresses of buffers ``[slots, M, N]`` (``out_ld``,
     ``out_stride``) on every rank; matrix ``b`` is stored into slot ``slot0 + b`` of each - an
     all-gather."""
-    from . import gemm
 
     assert lr_gemm_ok(A, B), "operands violate the kernel's layout rules; see lr_gemm_ok()"
     batch = A.size(0)
