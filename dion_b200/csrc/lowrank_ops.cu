@@ -505,9 +505,9 @@ normalize_q_kernel(const T* R, const float* colsq, float eps, T* Qstack, const l
 // (lane l owns column l, the row being eliminated travels by shuffles) and solves R^T X = J by
 // substitution.  Every CTA factors the same D: that is cheaper than another launch or a wait.
 // One CTA per matrix left a batch of 4 to 16 matrices on as many SMs: 512 x 512 took 780 us for 4
-// or 16 matrices and 853 us for 96 (now 292, 377 and 666 us), 1024 x 1024 4.3 ms for 2 (now 0.8).  A non-positive pivot gives NaN, which propagates (the
-// caller's clean-up turns the update into a no-op), as torch.linalg.cholesky_ex does not raise
-// either.
+// or 16 matrices and 853 us for 96 (now 307, 336 and 638 us), 1024 x 1024 4.4 ms for 4 (now 0.86).
+// A non-positive pivot gives NaN, which propagates (the caller's clean-up turns the update into a
+// no-op), as torch.linalg.cholesky_ex does not raise either.
 // ---------------------------------------------------------------------------------------------
 // Copy the 32 x 32 block A[m0.., a0..] of a row-major matrix into the warp's staging buffer
 // (32 independent coalesced loads per lane).
@@ -1020,6 +1020,7 @@ qr_update_kernel(float* Aall, long long strideA, int ld, int k, int j, const flo
 
 using namespace dion;
 static inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
+constexpr int kSms = 148;
 constexpr int kMaxGridY = 65535;   // matrices per launch where they are the grid's second index
 
 // Lets a kernel use up to `most` bytes of dynamic shared memory.  `most` is the same in every call for
@@ -1094,9 +1095,12 @@ DION_EXPORT int dion_cholesky_upper(const void* G, void* U, int n, int r, void* 
       n = total - first < kMaxGridY ? total - first : kMaxGridY;
       for (int k = 0; k < r / 32; ++k) {
         const int blocks = r / 32 - k;
-        // One block per CTA while that is about two waves of CTAs (96 matrices 512 x 512 with one
-        // block per CTA throughout: 1070 us; with up to four: 666 us).
-        if ((long long)blocks * n <= 296)
+        // One block per CTA up to one CTA per SM.  Every CTA factors the diagonal block, and these
+        // factorizations slow one another down: up to four blocks per CTA take longer alone (1 x 512^2
+        // 408 against 291 us) and less beside others.  With the line at 148, 296 CTAs and none:
+        // 16 x 512^2 336, 382, 381 us, 8 x 1024^2 957, 1044, 1043, 96 x 96^2 46, 56, 56, 96 x 128^2
+        // 61, 81, 89, 96 x 512^2 638, 665, more than 911.
+        if ((long long)blocks * n <= kSms)
           dion::cholesky_row_kernel<<<dim3(blocks, n), dion::kCholWarps * 32, dion::kCholSmem,
                                       S(stream)>>>(g, u, r, k);
         else
