@@ -5,8 +5,9 @@ models/gpt_model.py:64-193 of the reference (``transformer.wte``, ``transformer.
 
 The element-wise parts of the block (RMSNorm, RoPE + QK-norm, ReLU^2) and the loss go through
 ``dion_b200.models.functional``, which runs fused CUDA kernels with hand-written backward passes
-on the GPU and plain PyTorch elsewhere - there is no tracing compiler on this path.  The GEMMs
-are library calls and attention is PyTorch's fused SDPA.
+on the GPU and plain PyTorch elsewhere - there is no tracing compiler on this path.  Attention is
+PyTorch's fused SDPA.  The GEMMs are library calls, except without gradients, where the blocks of
+most sizes run on this package's kernels (``models/inference.py``).
 
 ``parallelize_gpt_model`` applies tensor parallelism (column/row-parallel linears), FSDP2
 (``fully_shard`` per block, then the root) and HSDP on a ``DeviceMesh`` exactly as
@@ -70,17 +71,22 @@ def apply_rotary_emb(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> t
     return torch.cat([x1 * c + x2 * s, x2 * c - x1 * s], 3).type_as(x)
 
 
+_LIBRARY_FORWARDS = (nn.Linear.forward, nn.Embedding.forward)
+
+
 def _is_plain(module: nn.Module) -> bool:
-    """True when ``module`` can be bypassed by a functional call on its weight: the weight is an
-    ordinary tensor (not a DTensor shard) and nothing hooks the module's forward (tensor
-    parallelism redistributes activations in such hooks)."""
+    """True when ``module`` can be bypassed by a functional call on its weight: its forward is that of
+    a linear layer or embedding, the weight is an ordinary tensor (not a DTensor shard) and nothing
+    hooks the module's forward (tensor parallelism redistributes activations in such hooks)."""
+    if type(module).forward not in _LIBRARY_FORWARDS or "forward" in module.__dict__:
+        return False
     w = module.weight
     return (type(w) in (torch.Tensor, nn.Parameter) and not module._forward_hooks
             and not module._forward_pre_hooks)
 
 
 def _linear(module: nn.Linear, x: torch.Tensor) -> torch.Tensor:
-    if module.bias is None and _is_plain(module):
+    if _is_plain(module) and module.bias is None:
         return Fn.linear(x, module.weight)
     return module(x)
 
@@ -122,8 +128,8 @@ class MLP(nn.Module):
         self.c_proj = nn.Linear(4 * config.n_embd, config.n_embd, bias=False)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        if (self.c_fc.bias is None and self.c_proj.bias is None and _is_plain(self.c_fc)
-                and _is_plain(self.c_proj)):
+        if (_is_plain(self.c_fc) and _is_plain(self.c_proj) and self.c_fc.bias is None
+                and self.c_proj.bias is None):
             return Fn.mlp_relu2(x, self.c_fc.weight, self.c_proj.weight)
         return _linear(self.c_proj, Fn.relu2(_linear(self.c_fc, x)))
 
@@ -212,7 +218,8 @@ class GPT(nn.Module):
 
 
 # The modules that the path without gradients stands in for, with the forwards that it computes.
-_FORWARDS = tuple((c, c.forward) for c in (Block, CausalSelfAttention, MLP, Rotary))
+_FORWARDS = tuple((c, c.forward) for c in (Block, CausalSelfAttention, MLP, Rotary, nn.Linear,
+                                           nn.Embedding))
 
 
 # ------------------------------------------------------------------------------------------------

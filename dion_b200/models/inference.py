@@ -122,7 +122,7 @@ def hidden_states(model, idx: Tensor, forwards) -> Optional[Tensor]:
     gradients are off, bf16 autocast is on, the model is a plain GPT (no hooks, no shards, no
     replaced modules or forwards; fp32 embedding; dense fp32 or bf16 weights of one dtype) on the
     GPU of ``idx``, nothing observes operators, and the size is one that gains (:func:`_pays`).  ``forwards``: the classes of block, attention,
-    MLP and rotary embedding, each with its own ``forward``."""
+    MLP, rotary embedding, linear layer and embedding, each with its own ``forward``."""
     wte = model.transformer.wte
     blocks = model.transformer.h
     if type(wte) is not torch.nn.Embedding:
@@ -137,7 +137,7 @@ def hidden_states(model, idx: Tensor, forwards) -> Optional[Tensor]:
             or table.device != idx.device or C % 8 or C > 4096 or not _unhooked(wte)
             or _observed() or _replaced(forwards)):
         return None
-    types = tuple(c for c, _ in forwards)
+    types = tuple(c for c, _ in forwards[:4])
     weights = [_block_weights(b, types, C) for b in blocks]
     if any(w is None for w in weights):
         return None

@@ -1,6 +1,7 @@
 """GPT model on CPU: shapes, generation, equivalence of the fused functional paths' fall-backs
 with the module-by-module composition, and parameter naming (checkpoint compatibility with the
 reference model: models/gpt_model.py:127-193)."""
+import pytest
 import torch
 
 from dion_b200.models import functional as Fn
@@ -146,3 +147,34 @@ def test_native_blocks_are_chosen_by_size():
     assert all(_pays(C, 4 * C, 1 << 20) for C in (64, 768, 1536))
     for C, most in ((1792, 3899), (2048, 2865), (3072, 989), (4096, 332)):
         assert _pays(C, 4 * C, 1) and _pays(C, 4 * C, most) and not _pays(C, 4 * C, most + 1)
+
+
+@pytest.mark.parametrize("where", ["class", "instance"])
+@pytest.mark.parametrize("name", ["attn.c_q", "attn.c_proj", "mlp.c_fc", "mlp.c_proj", "lm_head"])
+def test_a_linear_layer_with_its_own_forward_is_called(name, where):
+    """A layer whose forward is not that of ``nn.Linear`` (adapters, quantized layers) computes what
+    it says: here twice the product, which is what twice the weight gives, bit for bit."""
+    class Doubled(torch.nn.Linear):
+        def forward(self, x):
+            return 2 * torch.nn.functional.linear(x, self.weight)
+
+    cfg = GPTConfig(sequence_len=16, vocab_size=64, n_layer=1, n_head=2, n_embd=32)
+    torch.manual_seed(0)
+    model = GPT(cfg)
+    model.init_weights()
+    ids = torch.randint(0, 64, (2, 16))
+    path = name if name == "lm_head" else "transformer.h.0." + name
+    layer = model.get_submodule(path)
+    plain = model(ids, ids, return_logits=True)
+    with torch.no_grad():
+        layer.weight.mul_(2)
+    want = model(ids, ids, return_logits=True)
+    with torch.no_grad():
+        layer.weight.mul_(0.5)
+    if where == "class":
+        layer.__class__ = Doubled
+    else:
+        layer.forward = lambda x: 2 * torch.nn.functional.linear(x, layer.weight)
+    got = model(ids, ids, return_logits=True)
+    assert not torch.equal(got, plain) or name == "attn.c_q"     # queries are normalized
+    assert torch.allclose(got, want, rtol=1e-5, atol=1e-6)       # 2 (x W) and x (2 W) in fp32
