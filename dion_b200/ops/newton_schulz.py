@@ -137,7 +137,9 @@ def _prepare_cuda(G: Tensor, allow_tall: bool = False):
     ``allow_tall`` (the caller then iterates in right-multiply form).  Where ``X`` is not of this
     call it is the caller's tensor: to be read only.  The sums are there where one pass could
     round, pad and add up."""
-    G = unwrap(G)  # a pending functional collective must complete before its address is used
+    # A pending functional collective must complete and a lazy negation be carried out before the
+    # address is used.
+    G = unwrap(G).resolve_neg()
     shape = G.shape
     X = G
     if X.ndim == 2:

@@ -108,6 +108,16 @@ def test_input_is_kept_and_not_returned(products_on_cpu, variant, shape, pending
     assert torch.equal(got, _DRIVERS[variant](before))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_lazily_negated_input_is_resolved_before_its_address_is_used(dtype, monkeypatch):
+    from dion_b200.ops import foreach as F
+    G = torch.randn(2, 16, 40).to(dtype)
+    seen = []
+    monkeypatch.setattr(F, "ns_prepare", lambda X, *a, **kw: (seen.append(X) or X, None))
+    X = NS._prepare_cuda(torch._neg_view(G))[0]
+    assert not X.is_neg() and torch.equal(X, -G)
+
+
 @pytest.mark.parametrize("shape", [(2, 16, 40), (40, 16)])
 def test_no_steps_give_a_copy(products_on_cpu, shape):
     G = torch.randn(shape).bfloat16()
