@@ -11,7 +11,7 @@
 // barrier; no multicast).  The leader CTA's MMA thread issues the instructions for the pair and
 // releases stages / publishes accumulators in both CTAs with a cluster-multicast tcgen05.commit.
 // Each CTA drains its own half (128 TMEM lanes) of the accumulator in its epilogue warps, 64 columns
-// at a time through shared memory: D arrives by TMA (prefetched three sub-tiles ahead), each thread
+// at a time through shared memory: D arrives by TMA (each group's next sub-tile is in flight), each thread
 // combines its row in place in the 128-byte-swizzled buffer, and the buffer leaves by TMA store.
 // In symmetric mode only tiles on or above the diagonal are computed; an off-diagonal tile also
 // writes a transposed copy of each sub-tile that a second TMA store places at the mirrored

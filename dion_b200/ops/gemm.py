@@ -226,7 +226,9 @@ def _choose_config(M: int, N: int, K: int, batch: int, sym: bool, pair_ok: bool,
     smaller tiles (e.g. the 2048 x 2048 Gram matrix of one 2048 x 8192 input: 36 pair tiles for
     74 pairs, but 136 single-CTA 128 x 128 tiles for 148 SMs).  Efficiencies and the fixed cost
     per tile (pipeline fill + epilogue, expressed in K elements) are fitted to the timings of
-    ``benchmark/bench_newton_schulz.py --gemms``."""
+    ``benchmark/bench_newton_schulz.py --gemms``, those of the two-CTA kernel with one group of epilogue
+    warps; with two its tiles cost less, so it may be passed over for a single-CTA tiling now and
+    then."""
     key = (M, N, K, batch, sym, pair_ok, device.index)
     hit = _config_cache.get(key)
     if hit is not None:
@@ -417,7 +419,8 @@ def persistent_enabled() -> bool:
 def persistent_waves() -> float:
     """Largest GEMM of the loop, in waves of 128 x 128 tiles over the SMs, up to which the
     one-launch form is used (``DION_B200_PERSISTENT_WAVES``, default 1: beyond that the
-    256 x 256 two-CTA kernel's better efficiency outweighs the saved launches)."""
+    256 x 256 two-CTA kernel's better efficiency outweighs the saved launches; set before both forms
+    became faster)."""
     try:
         return float(os.environ.get("DION_B200_PERSISTENT_WAVES", "1"))
     except ValueError:
