@@ -374,8 +374,6 @@ class _Embedding(torch.autograd.Function):
             _c(flat), _c(dy2), _DT[dy2.dtype], _c(gw), ctypes.c_longlong(n), C,
             ctypes.c_longlong(V), _c(keys), _c(vals), _c(starts), _c(temp),
             ctypes.c_longlong(nbytes), _c(part), _stream(dev)), "dion_embedding_bwd")
-        if n > 64:      # a run can be longer than a chunk: the kernel that sums parts runs too
-            _backend.add_launches(1)
         return None, gw
 
 
@@ -462,9 +460,10 @@ def mlp_relu2(h: Tensor, wfc: Tensor, wproj: Tensor) -> Tensor:
     """The ReLU^2 MLP of the GPT block.  With ``DION_B200_FUSED_MLP=1``, bf16 activations with
     ordinary (non-DTensor) weights on a GPU take the fused form above; otherwise the plain
     composition (library GEMMs + element-wise kernels), which is the default: timed inside the
-    GPT-160M training step the fused form is slower (39.2 against 35.8 ms per step) although
-    it saves two element-wise passes, because at K = 768 the two-CTA kernel is bound by operand
-    traffic from L2 (no multicast loads) and trails the library GEMM by about 10 %."""
+    GPT-160M training step the fused form was slower (39.2 against 35.8 ms per step) although it saves
+    two element-wise passes.  That was with one group of epilogue warps in the two-CTA kernel, which
+    took up to 10 us to drain a tile whose products take 4 at K = 768; with two groups it has not
+    been timed."""
     h = materialize(h)
     if (is_plain_tensor(h) and h.is_cuda and h.dtype == torch.bfloat16 and is_plain_tensor(wfc)
             and is_plain_tensor(wproj)
