@@ -329,12 +329,107 @@ def test_replaced_modules_take_the_general_forward():
                    lambda m: setattr(m.transformer.h[1].mlp, "c_fc", Scaled(128, 512, bias=False).cuda())):
         model = GPT(GPTConfig(sequence_len=24, vocab_size=512, n_layer=2, n_head=2, n_embd=128)).cuda()
         model.init_weights()
-        change(model)
         with torch.autocast("cuda", dtype=torch.bfloat16):
+            plain = model(ids, ids, return_logits=True).detach()
+            change(model)
             ref = model(ids, ids, return_logits=True).detach()
+            assert not torch.equal(ref, plain)       # the replacement counts with gradients too
             with torch.no_grad():
                 got = model(ids, ids, return_logits=True)
         assert torch.equal(got, ref)
+
+
+def _small_gpt(**changes):
+    from dion_b200.models.gpt import GPT, GPTConfig
+    torch.manual_seed(0)
+    model = GPT(GPTConfig(**{**dict(sequence_len=32, vocab_size=512, n_layer=2, n_head=2, n_embd=128),
+                             **changes})).cuda()
+    model.init_weights()
+    return model, torch.randint(0, 512, (2, 24), device="cuda")
+
+
+def _native(model, ids, dtype=torch.bfloat16, enabled=True):
+    """What the path without gradients says to this call: its result, or None."""
+    from dion_b200.models import gpt, inference
+    with torch.no_grad(), torch.autocast("cuda", dtype=dtype, enabled=enabled):
+        return inference.hidden_states(model, ids, gpt._FORWARDS)
+
+
+def test_blocks_without_gradients_refuse_what_they_do_not_compute():
+    """Other types, shapes and settings than the native blocks are written for go to the general
+    forward, which gives a result for each of these."""
+    from torch import nn
+
+    from dion_b200.models import gpt, inference
+
+    def layer(m):
+        return m.transformer.h[1].attn.c_proj
+
+    def biased(m):
+        layer(m).bias = nn.Parameter(torch.zeros(128, device="cuda"))
+
+    def global_hook(m):
+        return nn.modules.module.register_module_forward_hook(lambda *a: None)
+
+    model, ids = _small_gpt()
+    assert _native(model, ids) is not None
+    assert _native(model, ids, dtype=torch.float16) is None
+    assert _native(model, ids, enabled=False) is None
+    assert _native(model, ids.cpu()) is None
+    assert _native(model, ids[0]) is None
+    assert _native(model, ids[:, :0]) is None
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert inference.hidden_states(model, ids, gpt._FORWARDS) is None
+    for change in (
+            biased,
+            lambda m: m.transformer.h[0].to(torch.bfloat16),                # mixed weight types
+            lambda m: m.transformer.h.to(torch.float16),
+            lambda m: m.transformer.wte.to(torch.bfloat16),
+            lambda m: setattr(layer(m), "weight", nn.Parameter(layer(m).weight.detach().t())),
+            lambda m: m.transformer.h[0].mlp.register_forward_pre_hook(lambda *a: None),
+            lambda m: m.transformer.wte.register_forward_hook(lambda *a: None),
+            lambda m: setattr(m.transformer.h[1].attn, "n_head", 4),
+            lambda m: setattr(m.transformer.h[1].mlp, "forward", lambda x: x),
+            global_hook):
+        model, ids = _small_gpt()
+        handle = change(model)
+        assert _native(model, ids) is None
+        if change is global_hook:
+            handle.remove()
+    model, ids = _small_gpt(n_embd=96)                                       # heads of 48
+    assert _native(model, ids) is None
+
+
+def test_blocks_without_gradients_are_seen_by_tracers_and_transforms():
+    """Whatever watches or transforms operators sees all of them: the general forward runs."""
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Pass(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class Count(TorchDispatchMode):
+        products = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            Count.products += "mm" in str(func)
+            return func(*args, **(kwargs or {}))
+
+    model, ids = _small_gpt()
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        want = model(ids, ids, return_logits=True)
+        with Count():
+            got = model(ids, ids, return_logits=True)
+        assert Count.products >= 9          # four products in each of two blocks, and the head
+        assert ((got - want).norm() / want.norm()).item() < 2e-2
+        with torch.autograd.forward_ad.dual_level():
+            assert _native(model, ids) is None
+        with Pass():
+            assert _native(model, ids) is None
+        seen = []
+        torch.func.vmap(lambda t: seen.append(_native(model, ids)) or t)(torch.zeros(2, device="cuda"))
+        assert seen == [None]
 
 
 @pytest.mark.parametrize("name", ["Block", "CausalSelfAttention", "MLP", "Rotary"])
