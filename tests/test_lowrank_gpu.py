@@ -46,8 +46,9 @@ def test_qr_r_factor_zero_column_is_finite():
                                    (2, 1408, 96)])
 @pytest.mark.parametrize("conditioning", ["random", "graded"])
 def test_blocked_qr_r_factor_matches_fp64(shape, conditioning, monkeypatch):
-    """Blocked Householder (panel kernel + tensor-core trailing updates): R is upper triangular,
-    R^T R reproduces A^T A, and |R| agrees with LAPACK's factor in fp64 - also for columns scaled
+    """Blocked Householder (panel kernel + fp32 trailing updates): R is upper triangular, R^T R
+    reproduces A^T A to fp32 rounding (2.8e-7 measured; the split tf32 products that the update
+    replaced left 1.4e-5), and |R| agrees with LAPACK's factor in fp64 - also for columns scaled
     over six orders of magnitude, where a factor of sloppy products would be useless as the
     preconditioner it is computed for."""
     from dion_b200.ops import lowrank as LR
@@ -69,7 +70,7 @@ def test_blocked_qr_r_factor_matches_fp64(shape, conditioning, monkeypatch):
     err = ((R.double().abs() - ref.abs()) / colmax).abs().max().item()
     assert err < 1e-3, err
     G = A.double().mT @ A.double()
-    assert ((R.double().mT @ R.double()) - G).abs().max().item() < 1e-4 * G.abs().max().item()
+    assert ((R.double().mT @ R.double()) - G).abs().max().item() < 2e-6 * G.abs().max().item()
     # as a preconditioner: A R^-1 has orthonormal columns
     Q = torch.linalg.solve_triangular(R.double(), A.double(), upper=True, left=False)
     eye = torch.eye(r, device="cuda", dtype=torch.float64)
