@@ -13,7 +13,7 @@
 //      run of row v is [starts[v], starts[v+1]);
 //      In the same launch one block per chunk of sorted positions (64 up to 65536 tokens) sums the
 //      parts of runs longer than a chunk that lie in it.  Such a run covers the first or the last
-//      position of every chunk it meets, so a chunk has two slots; the block searches for the run's
+//      position of every chunk it meets, so a chunk has two slots; the block looks for the run's
 //      ends itself (as a launch of its own behind the starts: 22 instead of 18 us for 512 tokens and
 //      512 rows of 64);
 //   4. one warp per row of GW sums the run in fp32 in position order, or its parts in chunk order,
@@ -55,15 +55,6 @@ emb_keys_kernel(const long long* __restrict__ ids, int* __restrict__ keys, int* 
   vals[i] = i;
 }
 
-// First index in [lo, hi) whose key is >= v, else hi.
-__device__ __forceinline__ int emb_lower_bound(const int* __restrict__ sorted, int v, int lo, int hi) {
-  while (lo < hi) {
-    const int mid = emb_mid(lo, hi);
-    if (sorted[mid] < v) lo = mid + 1; else hi = mid;
-  }
-  return lo;
-}
-
 constexpr int kEmbWarps = 8;
 
 // acc += the rows perm[j] of DY for j in [j0, j1), columns [c8*8, c8*8+8), four loads in flight.
@@ -98,7 +89,13 @@ emb_starts_parts_kernel(const int* __restrict__ sorted, int* __restrict__ starts
   extern __shared__ __align__(16) float emb_part[];          // [kEmbWarps][C]
   if ((int)blockIdx.x >= chunks) {
     const int v = ((int)blockIdx.x - chunks) * (kEmbWarps * 32) + threadIdx.x;
-    if (v <= V) starts[v] = emb_lower_bound(sorted, v, 0, n);
+    if (v > V) return;
+    int lo = 0, hi = n;                      // first index with sorted[idx] >= v
+    while (lo < hi) {
+      const int mid = emb_mid(lo, hi);
+      if (sorted[mid] < v) lo = mid + 1; else hi = mid;
+    }
+    starts[v] = lo;
     return;
   }
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -107,12 +104,18 @@ emb_starts_parts_kernel(const int* __restrict__ sorted, int* __restrict__ starts
   for (int slot = 0; slot < 2; ++slot) {
     const int v = slot == 0 ? first : last;
     if (v >= V || (slot == 1 && first == last)) continue;    // ids outside the table sort last
-    // A run longer than a chunk that covers p also covers p - chunk / 2 or p + chunk / 2.
-    const int p = slot == 0 ? p0 : p1 - 1, half = chunk / 2;
-    if (!(p >= half && sorted[p - half] == v) && !(n - p > half && sorted[p + half] == v)) continue;
-    const int s = emb_lower_bound(sorted, v, 0, p), e = emb_lower_bound(sorted, v + 1, p + 1, n);
-    if (e - s <= chunk) continue;                            // the same in every thread
-    const int lo = s > p0 ? s : p0, hi = e < p1 ? e : p1;
+    // The run's positions among the `chunk` on either side of the one it covers, and in this chunk.
+    const int p = slot == 0 ? p0 : p1 - 1;
+    const int from = p > chunk ? p - chunk : 0, to = n - p > chunk ? p + chunk : n - 1;
+    int near = 0, inside = 0;
+    for (int i0 = from; i0 <= to; i0 += kEmbWarps * 32) {
+      const int i = i0 + (int)threadIdx.x;
+      const bool here = i <= to && sorted[i] == v;
+      near += __syncthreads_count(here);
+      inside += __syncthreads_count(here && i >= p0 && i < p1);
+    }
+    if (near <= chunk) continue;                             // the same in every thread
+    const int lo = slot == 0 ? p0 : p1 - inside, hi = lo + inside;
     const int seg = (hi - lo + kEmbWarps - 1) / kEmbWarps;
     const int j0 = lo + w * seg < hi ? lo + w * seg : hi, j1 = j0 + seg < hi ? j0 + seg : hi;
     for (int c8 = lane; c8 < C / 8; c8 += 32) {
