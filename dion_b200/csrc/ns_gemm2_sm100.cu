@@ -10,12 +10,11 @@
 // (cp.async.bulk.tensor with .cta_group::2 so that both CTAs' transfers complete on the leader's
 // barrier; no multicast).  The leader CTA's MMA thread issues the instructions for the pair and
 // releases stages / publishes accumulators in both CTAs with a cluster-multicast tcgen05.commit.
-// Each CTA drains its own half (128 TMEM lanes) of the accumulator in its epilogue warps, 64 columns
-// at a time through shared memory: D arrives by TMA (each group's next sub-tile is in flight), each thread
-// combines its row in place in the 128-byte-swizzled buffer, and the buffer leaves by TMA store.
-// In symmetric mode only tiles on or above the diagonal are computed; an off-diagonal tile also
-// writes a transposed copy of each sub-tile that a second TMA store places at the mirrored
-// position, so both halves of the output are written with full-width bursts.
+// Each CTA drains its own half (128 TMEM lanes) of the accumulator in its epilogue warps, 64 or 32
+// columns at a time through shared memory: D arrives by TMA (each group's next sub-tile is in flight),
+// each thread combines its row in place in the swizzled buffer, and the buffer leaves by TMA store.
+// In symmetric mode only tiles on or above the diagonal are computed; the warps of an off-diagonal
+// tile also store their registers at the mirrored position, 64 bytes of a row at a time.
 //
 // Operand layouts and the epilogue arithmetic are the same as in the single-CTA kernel.  All waits
 // are bounded; the epilogue threads meet at a barrier that also ANDs their wait results, so a
@@ -28,34 +27,29 @@ namespace dion {
 constexpr int BM2 = 128;   // rows per CTA (256 per pair)
 constexpr int BN2 = 256;   // columns per pair (128 loaded by each CTA)
 constexpr int BK2 = 64;
-constexpr int kEpiGroups = 2;                       // groups of four epilogue warps
-constexpr int kThreads2 = 64 + kEpiGroups * 128;
-// Two groups of four warps drain a tile, each every second 64-column sub-tile through buffers of
-// its own.  One group alone needs 1.2 us per sub-tile (1.8 us with D: TMEM read, arithmetic,
-// shared-memory round trip, barrier, TMA store), 4.7 / 7.2 us a tile, more than the 3.3 us that
-// K = 768 multiplies for; two need 3.6 / 5.3 us (update of 64 matrices 768 x 3072: 256 -> 233 us,
-// 48 x 768^3: 62 -> 54 us, polynomial 64 x 768^3: 72.5 -> 65.7 us; K >= 2048 unchanged).
-// Shared memory is split between operand stages (32 KB), D/C sub-tile buffers and transposed
-// sub-tile buffers (16 KB each, half of them for each group).  A buffer is written again only after
-// its store has read it and, with D, the next D has arrived: with D a group has two buffers, so
-// that one D sub-tile is always in flight, at the expense of an operand stage (with two buffers in
-// all, the same update took 324 us).
-//   plain             5 stages + 4 D/C
-//   symmetric, no D   5 stages + 2 D/C + 2 transposed
-//   symmetric, D      4 stages + 4 D/C + 2 transposed
-struct CfgPlain { static constexpr int kStages = 5, kDC = 4, kT = 0; };
-struct CfgSym { static constexpr int kStages = 5, kDC = 2, kT = 2; };
-struct CfgSymD { static constexpr int kStages = 4, kDC = 4, kT = 2; };
+// Groups of four warps drain a tile in turn, each through two sub-tile buffers of its own: a buffer is
+// written again only after its store has read it and, with D, the next D has arrived, so that one D
+// sub-tile is always in flight.  A sub-tile is a chain of latencies (D, TMEM, arithmetic, barrier,
+// store): one group takes 4.7 us a tile (7.2 with D), more than the 3.3 us that K = 768 multiplies
+// for, two take 3.6 (5.3).  The mirrored copy of symmetric tiles doubles the instructions, so these
+// have four groups on half as wide sub-tiles: polynomial 64 x 768^3 66.5 -> 59.4 us, Gram 48 x 768^3 48 ->
+// 44 us.  Plain tiles gain nothing from that (update of 64 matrices 768 x 3072: 213 us either way).
+// With 32 KB per operand stage:
+//   plain       5 stages + 4 buffers of 128 x 64
+//   symmetric   5 stages + 8 buffers of 128 x 32
 constexpr int kABytes2 = BM2 * BK2 * 2;          // 16 KB
 constexpr int kBBytes2 = (BN2 / 2) * BK2 * 2;    // 16 KB
 constexpr int kStageBytes2 = kABytes2 + kBBytes2;
-constexpr int kSubCols = 64;                       // epilogue sub-tile: 128 rows x 64 columns
-constexpr int kEpiBufBytes = BM2 * kSubCols * 2;    // 16 KB: two 64 x 64 boxes of bf16
-// stages | D/C buffers | transposed buffers (symmetric mode) | alignment slack
-template <class CFG>
-constexpr int dyn_bytes2() {
-  return CFG::kStages * kStageBytes2 + (CFG::kDC + CFG::kT) * kEpiBufBytes + 1024;
-}
+template <int STAGES, int BUFS, int COLS, int GROUPS, bool SYM>
+struct Cfg2 {
+  static constexpr int kStages = STAGES, kDC = BUFS, kCols = COLS, kGroups = GROUPS;
+  static constexpr bool kSym = SYM;
+  static constexpr int kThreads = 64 + GROUPS * 128;   // producer, MMA, groups of four warps
+  static constexpr int kBufBytes = BM2 * COLS * 2;     // a sub-tile: two boxes of 64 rows
+  static constexpr int kDynBytes = STAGES * kStageBytes2 + BUFS * kBufBytes + 1024;
+};
+using CfgPlain = Cfg2<5, 4, 64, 2, false>;
+using CfgSym = Cfg2<5, 8, 32, 4, true>;
 constexpr uint32_t kTmemCols2 = 2 * BN2;
 
 // Epilogue forms: C = alpha*acc + beta*D | relu(alpha*acc)^2 | alpha*acc * 2*sqrt(D).
@@ -108,9 +102,9 @@ __device__ __forceinline__ float ld_volatile_f32_2(const float* p) {
   asm volatile("ld.volatile.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
   return v;
 }
-// Barrier over the 128 threads of an epilogue group without a predicate (barriers 3 and 4).
+// Barrier over the 128 threads of an epilogue group without a predicate (barriers 5 to 8).
 __device__ __forceinline__ void epi_barrier_plain(int group) {
-  asm volatile("barrier.cta.sync.aligned %0, 128;" ::"r"(3 + group) : "memory");
+  asm volatile("barrier.cta.sync.aligned %0, 128;" ::"r"(5 + group) : "memory");
 }
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -225,7 +219,7 @@ __device__ __forceinline__ void bulk_wait_group_read() {
 __device__ __forceinline__ void bulk_wait_group_all() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
-// Barrier over the 128 threads of an epilogue group (barriers 1 and 2) that also ANDs a predicate.
+// Barrier over the 128 threads of an epilogue group (barriers 1 to 4) that also ANDs a predicate.
 __device__ __forceinline__ bool epi_barrier_and(int group, bool mine) {
   uint32_t out;
   asm volatile(
@@ -248,13 +242,15 @@ __device__ __forceinline__ float ipow2(float s, int p) {
 }
 
 template <bool A_MN, bool B_MN, class CFG>
-__global__ void __launch_bounds__(kThreads2, 1)
+__global__ void __launch_bounds__(CFG::kThreads, 1)
 ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                 const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_d,
                 const Gemm2Args p) {
   constexpr int kStages2 = CFG::kStages, kDC = CFG::kDC;
-  constexpr int kGDC = CFG::kDC / kEpiGroups, kGT = CFG::kT / kEpiGroups;  // buffers per group
-  constexpr bool kSingle = kGT == 1 || kGDC == 1;   // a buffer is written by every sub-tile
+  constexpr int kEpiGroups = CFG::kGroups, kSubCols = CFG::kCols, kNSub = BN2 / kSubCols;
+  constexpr int kEpiBufBytes = CFG::kBufBytes;
+  constexpr int kGDC = CFG::kDC / kEpiGroups;       // buffers per group
+  static_assert(kGDC >= 2 && kNSub % kEpiGroups == 0, "");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -421,21 +417,23 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   } else {
     // ------------------------------ epilogue (both CTAs) ----------------------------------
-    // The 128 x 256 half-tile of this CTA is drained in sub-tiles of 64 columns, alternately by
-    // the two groups of warps.  D arrives by TMA into a shared-memory buffer (prefetched), each
-    // thread combines its row in place, and the buffer leaves by TMA store; with `sym`,
-    // off-diagonal tiles also write a transposed copy that a second TMA store places at the
-    // mirrored position.  g counts the sub-tiles of this group.
+    // The 128 x 256 half-tile of this CTA is drained in sub-tiles of 64 or 32 columns, in turn by the
+    // groups of warps.  D arrives by TMA into a shared-memory buffer (prefetched), each thread
+    // combines its row in place, and the buffer leaves by TMA store; with `sym`, off-diagonal tiles
+    // are also stored at the mirrored position.  g counts the sub-tiles of this group.
     const int grp = (warp - 2) >> 2;
     const int lane_grp = warp & 3;
     const int row_in_tile = lane_grp * 32 + lane;
     const bool elected = (warp == 2 + 4 * grp && lane == 0);
     const bool has_d = p.D != nullptr;
     const int epi = p.epi;
-    const uint32_t row_off = (uint32_t)(row_in_tile >> 6) * 8192u + (uint32_t)(row_in_tile & 63) * 128u;
-    const uint32_t row_sw = (uint32_t)(row_in_tile & 7);
+    constexpr uint32_t kBoxBytes = kEpiBufBytes / 2;
+    // Position of 16-byte piece c of row r in a box: r * row bytes + (c ^ swizzle(r)) * 16.
+    auto swizzle = [](uint32_t r) { return kSubCols == 64 ? r & 7u : (r >> 1) & 3u; };
+    const uint32_t row_off = (uint32_t)(row_in_tile >> 6) * kBoxBytes +
+                             (uint32_t)(row_in_tile & 63) * (kSubCols * 2);
+    const uint32_t row_sw = swizzle(row_in_tile);
     uint8_t* dc_base = smem + kStages2 * kStageBytes2 + grp * kGDC * kEpiBufBytes;
-    uint8_t* t_base = smem + kStages2 * kStageBytes2 + kDC * kEpiBufBytes + grp * kGT * kEpiBufBytes;
     uint64_t* dfull = dfull_bar + grp * kGDC;
 
     // Iterator over the sub-tiles this group will process, in order (used for the D prefetch).
@@ -444,7 +442,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     auto pf_skip = [&]() {   // to the next sub-tile of this group that exists
       while (pf_t < p.total_tiles) {
         const int2 tt = p.tiles[pf_t % p.tiles_per_mat];
-        if (pf_s < 4 && tt.y * BN2 + pf_s * kSubCols < p.N) break;
+        if (pf_s < kNSub && tt.y * BN2 + pf_s * kSubCols < p.N) break;
         pf_s = grp;
         pf_t += tile_step;
       }
@@ -470,7 +468,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       uint8_t* dst = dc_base + buf * kEpiBufBytes;
       mbar_expect_tx(&dfull[buf], kEpiBufBytes);
       tma_load_3d(dst, &map_d, &dfull[buf], c0, r0, b);
-      tma_load_3d(dst + 8192, &map_d, &dfull[buf], c0, r0 + 64, b);
+      tma_load_3d(dst + kBoxBytes, &map_d, &dfull[buf], c0, r0 + 64, b);
     };
     if (elected && has_d) {
       for (uint32_t g0 = 0; g0 < kGDC && pf_valid(); ++g0) {
@@ -519,8 +517,9 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const float beta = p.beta * ipow2(sc, p.beta_pow);
       const int row0 = tt.x * 256 + (int)cta * BM2;
       const bool mirror = p.sym && tt.y > tt.x;
+      const int row = row0 + row_in_tile;
       int nsub = (p.N - tt.y * BN2 + kSubCols - 1) / kSubCols;
-      nsub = nsub > 4 ? 4 : nsub;
+      nsub = nsub > kNSub ? kNSub : nsub;
       // After this group's last read of the accumulator: hand the TMEM slot back to the MMA thread.
       auto release_accumulator = [&]() {
         tc_fence_before();
@@ -534,11 +533,10 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const int c0 = tt.y * BN2 + s * kSubCols;
         const uint32_t buf = g % kGDC;
         uint8_t* dc = dc_base + buf * kEpiBufBytes;
-        uint8_t* tb = kGT ? t_base + (g % (kGT ? kGT : 1)) * kEpiBufBytes : nullptr;
-        if (elected && (has_d || kSingle)) {
+        if (elected && has_d) {
           // The stores of sub-tile g-1 have read their buffers: the next D may land there.
           bulk_wait_group_read<0>();
-          if (mine_ok && has_d && g > 0 && pf_valid()) {
+          if (mine_ok && g > 0 && pf_valid()) {
             issue_d(g + kGDC - 1);
             pf_advance();
           }
@@ -548,77 +546,84 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                                mbar_wait_bounded(&dfull[buf], (g / kGDC) & 1));
           if (!mine_ok && lane == 0) atomicExch(p.status, kStatusTimeoutFull);
         }
-        // 32 columns at a time: 64 accumulators in registers would spill at 320 threads.
-        float v[32];
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(lane_grp * 32) << 16) +
                                aslot * BN2 + s * kSubCols;
         if (mine_ok) {
-          tmem_ld_32x32(taddr, v);
-          tmem_ld_wait();
-        }
-        if (kSingle) epi_barrier_plain(grp);   // ... and so may this sub-tile
-        if (mine_ok) {
-          uint8_t* rowp = dc + row_off;
+          // 32 columns at a time: everything is requested first, and the form is chosen once, so
+          // that a warp has many instructions in flight.
 #pragma unroll
-          for (int j = 0; j < kSubCols / 8; ++j) {
-            if (j == 4) {
-              tmem_ld_32x32(taddr + 32, v);
-              tmem_ld_wait();
-              if (s + kEpiGroups >= nsub) release_accumulator();
-            }
-            uint4* cell = reinterpret_cast<uint4*>(rowp + (((uint32_t)j ^ row_sw) << 4));
-            float* vj = v + (j & 3) * 8;
+          for (int half = 0; half < kSubCols / 32; ++half) {
+            const int ch = c0 + half * 32;
+            float v[32];
+            tmem_ld_32x32(taddr + half * 32, v);
+            auto cell = [&](int q) {
+              return reinterpret_cast<uint4*>(dc + row_off +
+                                              (((uint32_t)(half * 4 + q) ^ row_sw) << 4));
+            };
+            uint4 d[4];
             if (has_d) {
-              const uint4 u = *cell;
-              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-              if (epi == kEpiMul2Sqrt) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) d[q] = *cell(q);
+            }
+            tmem_ld_wait();
+            if (half == kSubCols / 32 - 1 && s + kEpiGroups >= nsub) release_accumulator();
+            // f(i, D's element) for every element i of the row piece
+            auto with_d = [&](auto f) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const uint32_t w[4] = {d[q].x, d[q].y, d[q].z, d[q].w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                  const float2 f = unpack_bf16x2(w[e]);
-                  vj[2 * e] = alpha * vj[2 * e] * (2.f * sqrtf(f.x));
-                  vj[2 * e + 1] = alpha * vj[2 * e + 1] * (2.f * sqrtf(f.y));
-                }
-              } else {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float2 f = unpack_bf16x2(w[e]);
-                  vj[2 * e] = alpha * vj[2 * e] + beta * f.x;
-                  vj[2 * e + 1] = alpha * vj[2 * e + 1] + beta * f.y;
+                  const float2 x = unpack_bf16x2(w[e]);
+                  f(q * 8 + 2 * e, x.x);
+                  f(q * 8 + 2 * e + 1, x.y);
                 }
               }
-            } else if (epi == kEpiRelu2) {
+            };
+            if (has_d && !CFG::kSym && epi == kEpiMul2Sqrt) {
+              with_d([&](int i, float x) { v[i] = alpha * v[i] * (2.f * sqrtf(x)); });
+            } else if (has_d) {
+              with_d([&](int i, float x) { v[i] = alpha * v[i] + beta * x; });
+            } else if (!CFG::kSym && epi == kEpiRelu2) {
 #pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const float t = fmaxf(alpha * vj[e], 0.f);
-                vj[e] = t * t;
+              for (int i = 0; i < 32; ++i) {
+                const float t = fmaxf(alpha * v[i], 0.f);
+                v[i] = t * t;
               }
             } else {
 #pragma unroll
-              for (int e = 0; e < 8; ++e) vj[e] *= alpha;
+              for (int i = 0; i < 32; ++i) v[i] *= alpha;
             }
-            uint32_t pk[4];
+            uint32_t pk[16];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) pk[e] = pack_bf16x2(vj[2 * e], vj[2 * e + 1]);
-            *cell = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            if (kGT && mirror) {
-              // Transposed copy: element (row, c0 + c) goes to row c, column `row` of two
-              // 64 x 64 boxes (128-byte swizzled like every other buffer).
-              const uint32_t tcol = (uint32_t)(row_in_tile >> 6) * 8192u +
-                                    ((uint32_t)(row_in_tile & 7) << 1);
-              const uint32_t tchunk = (uint32_t)(row_in_tile & 63) >> 3;
+            for (int i = 0; i < 16; ++i) pk[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
 #pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const uint32_t c = (uint32_t)(j * 8 + e);
-                const uint32_t w = pk[e >> 1];
-                const uint16_t h = (e & 1) ? (uint16_t)(w >> 16) : (uint16_t)(w & 0xFFFF);
-                *reinterpret_cast<uint16_t*>(tb + tcol + c * 128u + ((tchunk ^ (c & 7)) << 4)) = h;
+            for (int q = 0; q < 4; ++q)
+              *cell(q) = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
+            if (CFG::kSym && mirror) {
+              // Mirrored copy, two columns at a time: neighbouring lanes swap so that each holds
+              // one column of its own and the other's row, 64 bytes of C's row per half-warp.
+              const int c = ch + (lane & 1), r2 = row & ~1;
+              const uint32_t sel = (lane & 1) ? 0x3276u : 0x5410u;
+              uint8_t* dst = reinterpret_cast<uint8_t*>(p.C + (long long)b * p.strideC +
+                                                        (long long)c * p.ldc + r2);
+              const long long step = 4 * p.ldc;   // two rows of C in bytes
+              const bool whole = ch + 32 <= p.N && row - lane + 32 <= p.M;
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const uint32_t w =
+                    __byte_perm(pk[i], __shfl_xor_sync(0xffffffffu, pk[i], 1), sel);
+                if (whole || (c + 2 * i < p.N && r2 + 1 < p.M))
+                  *reinterpret_cast<uint32_t*>(dst + i * step) = w;
+                else if (c + 2 * i < p.N && r2 < p.M)
+                  *reinterpret_cast<uint16_t*>(dst + i * step) = (uint16_t)w;
               }
             }
           }
           fence_proxy_async();
         }
-        // Two buffers and no D: sub-tile g+1 overwrites what the store of g-1 reads.
-        if (elected && !has_d && !kSingle) bulk_wait_group_read<0>();
+        // No D: sub-tile g+1 overwrites what the store of g+1-kGDC reads.
+        if (elected && !has_d) bulk_wait_group_read<kGDC - 2>();
         // Every epilogue thread reaches this barrier (all waits above are bounded); it also
         // tells whether any of them gave up.
         ok = epi_barrier_and(grp, mine_ok);
@@ -626,15 +631,17 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         if (remote) {
           // Rows leave for the ranks that own them: 16-byte stores over NVLink, eight
           // consecutive threads per 128-byte row segment of the (swizzled) sub-tile.
-          const int chunk = epi_tid & 7;
+          constexpr int kChunks = kSubCols / 8;
+          const int chunk = epi_tid % kChunks;
           if (c0 + chunk * 8 < p.N) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int rr = (epi_tid >> 3) + 16 * i;     // row of the 128-row half-tile
+            for (int i = 0; i < kChunks; ++i) {
+              const int rr = epi_tid / kChunks + (128 / kChunks) * i;     // row of the 128-row half-tile
               const int grow = row0 + rr;
               if (grow < p.M) {
-                const uint8_t* src = dc + (uint32_t)(rr >> 6) * 8192u + (uint32_t)(rr & 63) * 128u +
-                                     (((uint32_t)chunk ^ (uint32_t)(rr & 7)) << 4);
+                const uint8_t* src = dc + (uint32_t)(rr >> 6) * kBoxBytes +
+                                     (uint32_t)(rr & 63) * (kSubCols * 2) +
+                                     (((uint32_t)chunk ^ swizzle(rr)) << 4);
                 __nv_bfloat16* out;
                 if (p.cols_per_dst > 0) {
                   const int col = c0 + chunk * 8;
@@ -658,11 +665,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         }
         if (elected) {
           if (row0 < p.M) tma_store_3d(&map_c, dc, c0, row0, b);
-          if (row0 + 64 < p.M) tma_store_3d(&map_c, dc + 8192, c0, row0 + 64, b);
-          if (kGT && mirror) {
-            if (row0 < p.N) tma_store_3d(&map_c, tb, row0, c0, b);
-            if (row0 + 64 < p.N) tma_store_3d(&map_c, tb + 8192, row0 + 64, c0, b);
-          }
+          if (row0 + 64 < p.M) tma_store_3d(&map_c, dc + kBoxBytes, c0, row0 + 64, b);
           bulk_commit_group();
         }
       }
@@ -730,14 +733,14 @@ static int launch2(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorM
   static bool configured = false;
   static int max_clusters = 0;
   auto kernel = ns_gemm2_kernel<A_MN, B_MN, CFG>;
-  constexpr int kDynBytes2 = dyn_bytes2<CFG>();
+  constexpr int kDynBytes2 = CFG::kDynBytes;
   if (!configured) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynBytes2) !=
         cudaSuccess)
       return -3;
     cudaLaunchConfig_t probe = {};
     probe.gridDim = dim3(2 * 74, 1, 1);
-    probe.blockDim = dim3(kThreads2, 1, 1);
+    probe.blockDim = dim3(CFG::kThreads, 1, 1);
     probe.dynamicSmemBytes = kDynBytes2;
     cudaLaunchAttribute pattr[1];
     pattr[0].id = cudaLaunchAttributeClusterDimension;
@@ -758,7 +761,7 @@ static int launch2(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorM
   if (clusters <= 0) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters, 1, 1);
-  cfg.blockDim = dim3(kThreads2, 1, 1);
+  cfg.blockDim = dim3(CFG::kThreads, 1, 1);
   cfg.dynamicSmemBytes = kDynBytes2;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -831,17 +834,18 @@ DION_EXPORT int dion_ns_gemm2_ex(const void* A, long long lda, long long strideA
   } else {
     if (make_map2(&mb, B, batch, K, N, ldb, strideB, 64, BK2) != 0) return -13;
   }
-  // C leaves (and D arrives) through TMA in 64 x 64 boxes.
+  // C leaves (and D arrives) through TMA in boxes of 64 rows.
   if (C && ((ldc & 7) || (strideC & 7) || (reinterpret_cast<uintptr_t>(C) & 15))) return -11;
   if (D && ((ldd & 7) || (strideD & 7) || (reinterpret_cast<uintptr_t>(D) & 15))) return -11;
   if (remote && (sym || (ldc & 7) || (N & 7) || (D == nullptr && C == nullptr))) return -15;
   CUtensorMap mc, md;
   // A map needs some valid tensor even where the kernel never uses it (no D / remote output).
   const void* c_for_map = C ? C : D;
-  if (make_map2(&mc, c_for_map, batch, M, N, C ? ldc : ldd, C ? strideC : strideD, kSubCols,
+  const int sub_cols = sym ? CfgSym::kCols : CfgPlain::kCols;
+  if (make_map2(&mc, c_for_map, batch, M, N, C ? ldc : ldd, C ? strideC : strideD, sub_cols,
                 64) != 0)
     return -14;
-  if (make_map2(&md, D ? D : C, batch, M, N, D ? ldd : ldc, D ? strideD : strideC, kSubCols,
+  if (make_map2(&md, D ? D : C, batch, M, N, D ? ldd : ldc, D ? strideD : strideC, sub_cols,
                 64) != 0)
     return -14;
   Gemm2Args a;
@@ -878,7 +882,6 @@ DION_EXPORT int dion_ns_gemm2_ex(const void* A, long long lda, long long strideA
   a.epi = epi;
   if (epi == kEpiMul2Sqrt && D == nullptr) return -16;
   if (epi == kEpiRelu2 && D != nullptr) return -16;
-  if (sym && D) return launch2_mode<CfgSymD>(a_mn, b_mn, ma, mb, mc, md, a, s);
   if (sym) return launch2_mode<CfgSym>(a_mn, b_mn, ma, mb, mc, md, a, s);
   return launch2_mode<CfgPlain>(a_mn, b_mn, ma, mb, mc, md, a, s);
 }

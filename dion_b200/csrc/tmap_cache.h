@@ -51,7 +51,8 @@ inline uint64_t tmap_hash(const TmapKey& k) {
   return h ^ (h >> 29);
 }
 
-// Encodes (or fetches) the 3-D bf16 map with 128-byte swizzle used throughout this library.
+// Encodes (or fetches) the 3-D bf16 map used throughout this library: 128-byte swizzle, 64-byte where
+// a row of the box has 64 bytes only.
 // `enc` is the driver's cuTensorMapEncodeTiled.  Returns 0, or -2 when the driver rejects the map.
 template <typename EncodeFn>
 inline int encode_bf16_3d(EncodeFn enc, CUtensorMap* map, const void* ptr, const cuuint64_t dims[3],
@@ -76,7 +77,8 @@ inline int encode_bf16_3d(EncodeFn enc, CUtensorMap* map, const void* ptr, const
   }
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides,
-                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   box[0] == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return -2;
   if (cached) {

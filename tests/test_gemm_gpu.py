@@ -128,6 +128,29 @@ def test_pair_symmetric(shape):
     assert (C - C.mT).abs().max().item() == 0.0
 
 
+@pytest.mark.parametrize("with_d", [False, True])
+@pytest.mark.parametrize("M", [257, 288, 519, 777])
+def test_pair_symmetric_ragged_rows(M, with_d):
+    """The mirrored copy leaves the registers two rows at a time, 32 rows to a warp: odd sizes, sizes
+    that end inside a warp's rows, and rows of C further apart than they are long."""
+    from dion_b200.ops import gemm
+    torch.manual_seed(5)
+    ld, K, b = (M + 7) // 8 * 8 + 8, 136, 2
+    X = torch.randn(b, M, K, device="cuda").bfloat16()
+    D = torch.randn(b, M, ld, device="cuda").bfloat16()[:, :, :M]
+    D = (D + D.mT).new_zeros(b, M, ld)[:, :, :M].copy_(D + D.mT)
+    out = torch.full((b, M + 2, ld), -7.0, device="cuda", dtype=torch.bfloat16)
+    C = out[:, :M, :M]
+    kw = dict(D=D, alpha=0.5, beta=2.0) if with_d else dict(alpha=0.5)
+    gemm.ns_gemm(X, X, out=C, sym=True, pair=True, **kw)
+    torch.cuda.synchronize()
+    gemm.check_status()
+    ref = 0.5 * (X.float() @ X.float().mT) + (2.0 * D.float() if with_d else 0.0)
+    assert _rel_err(C, ref) < 1e-2
+    assert torch.equal(C, C.mT)
+    assert (out[:, M:] == -7.0).all() and (out[:, :, ld - 8:] == -7.0).all()   # TMA: whole 16 bytes
+
+
 @pytest.mark.parametrize("sym", [False, True])
 @pytest.mark.parametrize("n", [256 + 8, 256 + 64, 256 + 72, 256 + 192, 512 + 136])
 def test_pair_narrow_last_tile(n, sym):
