@@ -40,16 +40,21 @@ constexpr int BK2 = 64;
 constexpr int kABytes2 = BM2 * BK2 * 2;          // 16 KB
 constexpr int kBBytes2 = (BN2 / 2) * BK2 * 2;    // 16 KB
 constexpr int kStageBytes2 = kABytes2 + kBBytes2;
-template <int STAGES, int BUFS, int COLS, int GROUPS, bool SYM>
+// The composed forms (see dion_ns_compose2) are kernels of their own, so that the vectors that
+// their addends are scaled with cost the others no registers.
+enum : int { kAddScalar = 0, kAddDiag = 1, kAddVector = 2 };
+template <int STAGES, int BUFS, int COLS, int GROUPS, int ADD, bool SYM>
 struct Cfg2 {
-  static constexpr int kStages = STAGES, kDC = BUFS, kCols = COLS, kGroups = GROUPS;
+  static constexpr int kStages = STAGES, kDC = BUFS, kCols = COLS, kGroups = GROUPS, kAdd = ADD;
   static constexpr bool kSym = SYM;
   static constexpr int kThreads = 64 + GROUPS * 128;   // producer, MMA, groups of four warps
   static constexpr int kBufBytes = BM2 * COLS * 2;     // a sub-tile: two boxes of 64 rows
   static constexpr int kDynBytes = STAGES * kStageBytes2 + BUFS * kBufBytes + 1024;
 };
-using CfgPlain = Cfg2<5, 4, 64, 2, false>;
-using CfgSym = Cfg2<5, 8, 32, 4, true>;
+using CfgPlain = Cfg2<5, 4, 64, 2, kAddScalar, false>;
+using CfgSym = Cfg2<5, 8, 32, 4, kAddScalar, true>;
+using CfgSymDiag = Cfg2<5, 8, 32, 4, kAddDiag, true>;
+using CfgPlainVec = Cfg2<5, 4, 64, 2, kAddVector, false>;
 constexpr uint32_t kTmemCols2 = 2 * BN2;
 
 // Epilogue forms: C = alpha*acc + beta*D | relu(alpha*acc)^2 | alpha*acc * 2*sqrt(D).
@@ -90,6 +95,18 @@ struct Gemm2Args {
   // remote_c[c / cols_per_dst] + ((remote_slot + b) * M + r) * cols_per_dst + c % cols_per_dst
   // (a multiple of 8 columns, so a 16-byte piece has one destination).
   int cols_per_dst;
+  // ---- composed forms: symmetric matrices kept as bf16 off the diagonal and fp32 on it ----
+  // kAddVector: D is scaled by beta * row_vec[b*M + row], or by beta * col_vec[b*N + column].
+  // kAddDiag:   row_vec as above (null: ones).  With diag_out the diagonal leaves there as
+  //             result + diag_add and is stored as zero in C; with col_vec too, the right operand's
+  //             (and D's) diagonal is bf16(col_vec) and what the rounding took is added back.  With
+  //             `patch` (dense [batch, M, M]) the diagonal of that matrix becomes bf16(patch_vec).
+  const float* row_vec;
+  const float* col_vec;
+  float* diag_out;
+  float diag_add;
+  __nv_bfloat16* patch;
+  const float* patch_vec;
 };
 
 __device__ __forceinline__ int ld_acquire_sys2(const int* p) {
@@ -518,6 +535,9 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const int row0 = tt.x * 256 + (int)cta * BM2;
       const bool mirror = p.sym && tt.y > tt.x;
       const int row = row0 + row_in_tile;
+      float row_beta = beta;
+      if (CFG::kAdd != kAddScalar && p.row_vec != nullptr)
+        row_beta = row < p.M ? beta * p.row_vec[(long long)b * p.M + row] : 0.f;
       int nsub = (p.N - tt.y * BN2 + kSubCols - 1) / kSubCols;
       nsub = nsub > kNSub ? kNSub : nsub;
       // After this group's last read of the accumulator: hand the TMEM slot back to the MMA thread.
@@ -531,6 +551,11 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll 1
       for (int s = grp; s < nsub; s += kEpiGroups, ++g) {
         const int c0 = tt.y * BN2 + s * kSubCols;
+        // kAddDiag: a tile on the diagonal leaves exactly symmetric (products of matrices that
+        // commute but for their rounding are not), by blocks of a warp's 32 rows x 32 columns.
+        const bool diag_tile = CFG::kAdd == kAddDiag && tt.x == tt.y;
+        const bool on_diag = diag_tile && c0 == row - lane;
+        const bool above = diag_tile && c0 > row - lane;
         const uint32_t buf = g % kGDC;
         uint8_t* dc = dc_base + buf * kEpiBufBytes;
         if (elected && has_d) {
@@ -580,7 +605,19 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 }
               }
             };
-            if (has_d && !CFG::kSym && epi == kEpiMul2Sqrt) {
+            if (CFG::kAdd == kAddVector && p.col_vec != nullptr) {
+              float cv[32];   // N is a multiple of 8
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (ch + q * 4 < p.N)
+                  x = *reinterpret_cast<const float4*>(p.col_vec + (long long)b * p.N + ch + q * 4);
+                cv[q * 4] = x.x; cv[q * 4 + 1] = x.y; cv[q * 4 + 2] = x.z; cv[q * 4 + 3] = x.w;
+              }
+              with_d([&](int i, float x) { v[i] = alpha * v[i] + beta * cv[i] * x; });
+            } else if (CFG::kAdd != kAddScalar) {
+              with_d([&](int i, float x) { v[i] = alpha * v[i] + row_beta * x; });
+            } else if (has_d && !CFG::kSym && epi == kEpiMul2Sqrt) {
               with_d([&](int i, float x) { v[i] = alpha * v[i] * (2.f * sqrtf(x)); });
             } else if (has_d) {
               with_d([&](int i, float x) { v[i] = alpha * v[i] + beta * x; });
@@ -594,13 +631,34 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
               for (int i = 0; i < 32; ++i) v[i] *= alpha;
             }
+            if (CFG::kAdd == kAddDiag && on_diag && p.diag_out != nullptr) {
+              float mine = 0.f;
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                if (i == lane) {
+                  mine = v[i];
+                  v[i] = 0.f;
+                }
+              }
+              if (row < p.M) {
+                const long long at = (long long)b * p.M + row;
+                mine += p.diag_add;
+                if (p.col_vec != nullptr) {
+                  const float f = p.col_vec[at];
+                  mine += row_beta * (f - __bfloat162float(__float2bfloat16(f)));
+                }
+                p.diag_out[at] = mine;
+                if (p.patch != nullptr)
+                  p.patch[at * p.M + row] = __float2bfloat16(p.patch_vec[at]);
+              }
+            }
             uint32_t pk[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) pk[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
 #pragma unroll
             for (int q = 0; q < 4; ++q)
               *cell(q) = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-            if (CFG::kSym && mirror) {
+            if (CFG::kSym && (mirror || above)) {
               // Mirrored copy, two columns at a time: neighbouring lanes swap so that each holds
               // one column of its own and the other's row, 64 bytes of C's row per half-warp.
               const int c = ch + (lane & 1), r2 = row & ~1;
@@ -619,6 +677,18 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                   *reinterpret_cast<uint16_t*>(dst + i * step) = (uint16_t)w;
               }
             }
+          }
+          if (CFG::kAdd == kAddDiag && on_diag) {
+            // Below the diagonal of this 32 x 32 block: the elements above it.
+            __syncwarp();
+            uint8_t* blk = dc + (row_off - (uint32_t)(lane * kSubCols * 2));
+            auto cell2 = [&](uint32_t r, uint32_t c) {
+              return reinterpret_cast<uint16_t*>(blk + r * (kSubCols * 2) +
+                                                 (((c >> 3) ^ swizzle(r)) << 4) + (c & 7) * 2);
+            };
+#pragma unroll 4
+            for (int c = 0; c < 31; ++c)
+              if (c < lane) *cell2(lane, c) = *cell2(c, lane);
           }
           fence_proxy_async();
         }
@@ -664,8 +734,15 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           continue;
         }
         if (elected) {
-          if (row0 < p.M) tma_store_3d(&map_c, dc, c0, row0, b);
-          if (row0 + 64 < p.M) tma_store_3d(&map_c, dc + kBoxBytes, c0, row0 + 64, b);
+          if (CFG::kAdd == kAddDiag) {   // boxes of 32 rows; none below the diagonal
+#pragma unroll
+            for (int w = 0; w < 4; ++w)
+              if (row0 + w * 32 < p.M && !(diag_tile && c0 < row0 + w * 32))
+                tma_store_3d(&map_c, dc + w * (kEpiBufBytes / 4), c0, row0 + w * 32, b);
+          } else {
+            if (row0 < p.M) tma_store_3d(&map_c, dc, c0, row0, b);
+            if (row0 + 64 < p.M) tma_store_3d(&map_c, dc + kBoxBytes, c0, row0 + 64, b);
+          }
           bulk_commit_group();
         }
       }
@@ -862,6 +939,8 @@ DION_EXPORT int dion_ns_gemm2_ex(const void* A, long long lda, long long strideA
   a.scale_partials = nullptr; a.scale_mult = 1.f; a.scale_eps = 0.f;
   for (int i = 0; i < 8; ++i) a.remote_c[i] = 0;
   a.rows_per_dst = 1; a.remote_slot = 0; a.cols_per_dst = 0;
+  a.row_vec = a.col_vec = a.patch_vec = nullptr; a.diag_out = nullptr; a.diag_add = 0.f;
+  a.patch = nullptr;
   if (ex != nullptr) {
     if (ex->n_src > 8 || ex->n_src < 0) return -14;
     if ((ex->wait_flags != nullptr || ex->scale_partials != nullptr) &&
@@ -937,6 +1016,145 @@ DION_EXPORT int dion_ns_iterate2(void* X, void* Xalt, void* X2, void* A, void* B
     }
     if (rc != 0) return rc;
     void* t = cur; cur = nxt; nxt = it == 0 && X2 != nullptr ? X2 : t;
+  }
+  return 0;
+}
+
+namespace dion {
+
+// One product of the composed form; every operand is dense (leading dimension = its columns).
+struct ComposedProduct {
+  const void* A; int a_rows, a_cols, a_mn;
+  const void* B; int b_rows, b_cols, b_mn;
+  void* C;
+  const void* D;
+  int M, N, K;
+  float alpha, beta;
+  const float* scale;
+  int alpha_pow, beta_pow, sym;
+  const float *row_vec, *col_vec;
+  float* diag_out;
+  float diag_add;
+  void* patch;
+  const float* patch_vec;
+  const void* tiles; int n_tiles;
+};
+
+static int composed_product(const ComposedProduct& q, int batch, int* status, cudaStream_t stream) {
+  CUtensorMap ma, mb, mc, md;
+  const long long sa = (long long)q.a_rows * q.a_cols, sb = (long long)q.b_rows * q.b_cols;
+  const long long sc = (long long)q.M * q.N;
+  if (make_map2(&ma, q.A, batch, q.a_rows, q.a_cols, q.a_cols, sa, q.a_mn ? 64 : BK2,
+                q.a_mn ? BK2 : BM2) != 0)
+    return -12;
+  if (make_map2(&mb, q.B, batch, q.b_rows, q.b_cols, q.b_cols, sb, q.b_mn ? 64 : BK2,
+                q.b_mn ? BK2 : BN2 / 2) != 0)
+    return -13;
+  const int sub_cols = !q.sym ? CfgPlainVec::kCols : q.D ? CfgSymDiag::kCols : CfgSym::kCols;
+  const int box_rows = q.sym && q.D ? 32 : 64;   // see the stores of kAddDiag
+  if (make_map2(&mc, q.C, batch, q.M, q.N, q.N, sc, sub_cols, box_rows) != 0) return -14;
+  if (make_map2(&md, q.D ? q.D : q.C, batch, q.M, q.N, q.N, sc, sub_cols, 64) != 0) return -14;
+  Gemm2Args a = {};
+  a.batch = batch; a.M = q.M; a.N = q.N; a.K = q.K;
+  a.D = static_cast<const __nv_bfloat16*>(q.D); a.ldd = q.N; a.strideD = sc;
+  a.C = static_cast<__nv_bfloat16*>(q.C); a.ldc = q.N; a.strideC = sc;
+  a.alpha = q.alpha; a.beta = q.beta; a.scale = q.scale;
+  a.alpha_pow = q.alpha_pow; a.beta_pow = q.beta_pow; a.sym = q.sym;
+  a.tiles = static_cast<const int2*>(q.tiles); a.tiles_per_mat = q.n_tiles;
+  a.total_tiles = q.n_tiles * batch;
+  a.status = status; a.epi = kEpiAxpby;
+  a.rows_per_src = 1; a.rows_per_dst = 1;
+  a.row_vec = q.row_vec; a.col_vec = q.col_vec;
+  a.diag_out = q.diag_out; a.diag_add = q.diag_add;
+  a.patch = static_cast<__nv_bfloat16*>(q.patch); a.patch_vec = q.patch_vec;
+  if (q.sym && q.D == nullptr) return launch2_mode<CfgSym>(q.a_mn, q.b_mn, ma, mb, mc, md, a, stream);
+  if (q.sym) return launch2<false, false, CfgSymDiag>(ma, mb, mc, md, a, stream);
+  return q.b_mn ? launch2<false, true, CfgPlainVec>(ma, mb, mc, md, a, stream)
+                : launch2<false, false, CfgPlainVec>(ma, mb, mc, md, a, stream);
+}
+
+}  // namespace dion
+
+// The same loop as dion_ns_iterate2 with the steps of a group composed on the small matrix:
+//   A = s^2 X X^T;  Q = a I + b A + c A A;  with a second step:  A = Q A Q,  Q = (a I + b A + c A A) Q;
+//   X = s Q X.
+// All of these are polynomials of one symmetric matrix, so every small product is computed as a
+// half.  With g = min(m, n), rho = max(m, n) / g and products counted in g^3, a group of two costs
+// 3 rho + 5 where two plain steps cost 6 rho + 2: 17 against 26 at rho = 4, 53 against 98 at 16,
+// the same at rho = 1.
+// Z and Q are kept as bf16 off the diagonal and fp32 on it, and every small result is exactly
+// symmetric.  With a bf16 diagonal the rounding of Q alone doubled the result's error, with rounding
+// that differs above and below the diagonal it was a quarter larger; so it is smaller than the plain
+// loop's (which rounds X, A and B in every step): 0.6-0.9 of it on gradients, on spectra with a few
+// dominant directions and on decaying ones, from g = 512 and rho = 2.  Three steps in one group are
+// not: the rounding that a dominant direction leaves in A grows by the square of each step's slope
+// at zero (66, 16, ...) and diverges.
+// A group has one or two steps.  `work` holds three matrices [batch, g, g] bf16, `vecs` three vectors
+// [batch, g] fp32.  Buffers X, X2, Xalt as in dion_ns_iterate2, one swap a group; the result lies in
+// Xalt after an odd number of groups, else in X (X2).
+DION_EXPORT int dion_ns_compose2(void* X, void* Xalt, void* X2, void* work, float* vecs, int batch,
+                                 int m, int n, const float* coeffs, const int* groups, int n_groups,
+                                 const float* scale, const void* tiles_gg, int n_tiles_gg,
+                                 const void* tiles_mn, int n_tiles_mn, int* status, void* stream) {
+  using namespace dion;
+  const int tall = m > n;
+  const int g = tall ? n : m;
+  if (batch <= 0 || m <= 0 || n <= 0) return 0;
+  if ((m & 7) || (n & 7) || (reinterpret_cast<uintptr_t>(X) & 15)) return -10;
+  const size_t mat = (size_t)batch * g * g;
+  __nv_bfloat16* w = static_cast<__nv_bfloat16*>(work);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // C = alpha * Y B + beta * row_vec D, symmetric, all operands [g, g]
+  auto small = [&](const void* Y, const void* B, void* C, const void* D, float alpha, float beta,
+                   const float* row_vec, const float* col_vec, float* diag_out, float diag_add,
+                   void* patch, const float* patch_vec) {
+    ComposedProduct q = {Y, g, g, 0, B, g, g, 0, C, D, g, g, g, alpha, beta, nullptr, 0, 0, 1,
+                         row_vec, col_vec, diag_out, diag_add, patch, patch_vec, tiles_gg, n_tiles_gg};
+    return composed_product(q, batch, status, s);
+  };
+  void* cur = X;
+  void* nxt = Xalt;
+  for (int gr = 0, at = 0; gr < n_groups; ++gr) {
+    const float* sc = gr == 0 ? scale : nullptr;
+    if (groups[gr] != 1 && groups[gr] != 2) return -10;
+    void* A = w;
+    void* Q = w + mat;        // off the diagonal, with `q` on it
+    void* Y = w + 2 * mat;    // first Q A, then the second step's Z, with `y` on its diagonal
+    float* q = vecs;
+    float* y = vecs + (size_t)batch * g;
+    float* h = vecs + 2 * (size_t)batch * g;
+    // Gram matrix: wide X [g, K = n] against itself; tall X read as [K = m, g] on both sides.
+    ComposedProduct gram = {cur, m, n, tall, cur, m, n, tall, A, nullptr, g, g, tall ? m : n,
+                            1.f, 0.f, sc, sc ? 2 : 0, 0, 1, nullptr, nullptr, nullptr, 0.f,
+                            nullptr, nullptr, tiles_gg, n_tiles_gg};
+    int rc = composed_product(gram, batch, status, s);
+    if (rc != 0) return rc;
+    const float* co = coeffs + 3 * at;
+    at += groups[gr];
+    rc = small(A, A, Q, A, co[2], co[1], nullptr, nullptr, q, co[0], nullptr, nullptr);
+    if (rc != 0) return rc;
+    if (groups[gr] == 2) {
+      rc = small(Q, A, Y, A, 1.f, 1.f, q, nullptr, nullptr, 0.f, nullptr, nullptr);    // Q A
+      if (rc == 0)
+        rc = small(Q, Y, A, Y, 1.f, 1.f, q, nullptr, nullptr, 0.f, nullptr, nullptr);  // Q A Q
+      // On the way Q gets its diagonal back, rounded, to be read as a whole matrix below.
+      if (rc == 0) rc = small(A, A, Y, A, co[5], co[4], nullptr, nullptr, y, co[3], Q, q);
+      if (rc == 0) rc = small(Y, Q, A, Q, 1.f, 1.f, y, q, h, 0.f, nullptr, nullptr);   // Z Q
+      if (rc != 0) return rc;
+      Q = A;
+      q = h;
+    }
+    ComposedProduct up = {Q, g, g, 0, cur, m, n, 1, nxt, cur, m, n, g, 1.f, 1.f, sc, sc ? 1 : 0,
+                          sc ? 1 : 0, 0, q, nullptr, nullptr, 0.f, nullptr, nullptr, tiles_mn,
+                          n_tiles_mn};
+    if (tall) {    // X' = X Q, Q symmetric: given as [N, K]
+      up.A = cur; up.a_rows = m; up.a_cols = n;
+      up.B = Q; up.b_rows = g; up.b_cols = g; up.b_mn = 0;
+      up.row_vec = nullptr; up.col_vec = q;
+    }
+    rc = composed_product(up, batch, status, s);
+    if (rc != 0) return rc;
+    void* t = cur; cur = nxt; nxt = gr == 0 && X2 != nullptr ? X2 : t;
   }
   return 0;
 }

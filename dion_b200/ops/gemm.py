@@ -218,6 +218,23 @@ def _num_tiles(M: int, N: int, bm: int, bn: int, sym: bool) -> int:
 _config_cache: Dict[Tuple, Tuple[bool, int]] = {}
 
 
+def _config_costs(M: int, N: int, K: int, batch: int, sym: bool, pair_ok: bool, sms: int):
+    """``[(estimated time, (use the two-CTA kernel, BN of the single-CTA kernel))]``, see
+    :func:`_choose_config`; the unit is one 256-column tile of a single K element."""
+    cands = []
+    # (pair?, bn, execution units, tile size per unit, efficiency, fixed cost in K elements)
+    if pair_ok and M > 128 and N > 128:
+        cands.append((True, 256, sms // 2, 1.0, 1.0, 768.0))
+    if N > 128:
+        cands.append((False, 256, sms, 1.0, 0.7 if sym else 0.9, 2048.0 if sym else 1024.0))
+    cands.append((False, 128, sms, 0.5, 0.6 if sym else 0.8, 2048.0 if sym else 1024.0))
+    costs = []
+    for is_pair, bn, units, size, eff, fixed in cands:
+        tiles = _num_tiles(M, N, 256 if is_pair else _BM, bn, sym) * batch
+        costs.append((-(-tiles // units) * size * (K / eff + fixed), (is_pair, bn)))
+    return costs
+
+
 def _choose_config(M: int, N: int, K: int, batch: int, sym: bool, pair_ok: bool,
                    device: torch.device) -> Tuple[bool, int]:
     """-> (use the two-CTA kernel, BN of the single-CTA kernel).  Picks the tiling with the
@@ -233,20 +250,10 @@ def _choose_config(M: int, N: int, K: int, batch: int, sym: bool, pair_ok: bool,
     hit = _config_cache.get(key)
     if hit is not None:
         return hit
-    sms = sm_count(device)
-    cands = []
-    # (pair?, bn, execution units, tile size per unit, efficiency, fixed cost in K elements)
-    if pair_ok and M > 128 and N > 128:
-        cands.append((True, 256, sms // 2, 1.0, 1.0, 768.0))
-    if N > 128:
-        cands.append((False, 256, sms, 1.0, 0.7 if sym else 0.9, 2048.0 if sym else 1024.0))
-    cands.append((False, 128, sms, 0.5, 0.6 if sym else 0.8, 2048.0 if sym else 1024.0))
-    best, best_t = None, None
-    for is_pair, bn, units, size, eff, fixed in cands:
-        tiles = _num_tiles(M, N, 256 if is_pair else _BM, bn, sym) * batch
-        t = -(-tiles // units) * size * (K / eff + fixed)
+    best_t, best = None, None
+    for t, config in _config_costs(M, N, K, batch, sym, pair_ok, sm_count(device)):
         if best_t is None or t < best_t - 1e-9:
-            best, best_t = (is_pair, bn), t
+            best_t, best = t, config
     if len(_config_cache) >= 4096:      # every length of a text is a shape of its own
         _config_cache.clear()
     _config_cache[key] = best
@@ -405,6 +412,68 @@ def ns_iterate(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs, scale: Op
         raise RuntimeError(f"dion_ns_iterate2 failed with code {rc}")
     _backend.add_launches(3 * len(coeffs))
     return Xalt if len(coeffs) % 2 else (X if X2 is None else X2)
+
+
+@functools.lru_cache(maxsize=1024)
+def compose_groups(batch: int, m: int, n: int, steps: int, sms: int) -> Optional[Tuple[int, ...]]:
+    """Sizes of the groups in which the steps of a Newton-Schulz loop on ``[batch, m, n]`` are
+    composed on the small matrix (see ``dion_ns_compose2``), or None where the plain loop stays.
+
+    Pairs, from the first step on and with a single step at the end (without it the result is further
+    from the exact one than the plain loop's, 1.1 times; with it nearer), where the products of two steps are estimated at 0.825 of the plain
+    ones or less: the estimate is optimistic about the small products, which are bound by their
+    epilogue.  Composed / plain for five steps at an estimate of 0.57 (48 x 512 x 8192) 0.71, 0.68 (24 x
+    2048 x 8192) 0.79, 0.71-0.74 (64 x 768 x 3072, 96 x 512 x 2048) 0.87-0.92, 0.79-0.82 (16 x 1024 x 3072, 24
+    x 2048 x 4096) 0.89-0.91, 0.83 (6 x 768 x 3072, 12 x 512 x 2048) 1.00 and 0.93, 0.89 (64 x 768 x 1536, 2 x 4096 x 6144) 1.05 and
+    0.94, 0.95 and above 1.0-1.05.  And from ``min(m, n) = 512``: below, the composed result of a
+    spectrum that falls off as 1 / rank is further from the exact one (1.08 times at 384, 2.6 at 192)."""
+    g, long = min(m, n), max(m, n)
+    if g < 512 or steps < 3 or m % 8 or n % 8:
+        return None
+    products = {"gram": (g, g, long, True), "small": (g, g, g, True), "update": (m, n, g, False)}
+    plain = pairs = 0.0
+    for name, (M, N, K, sym) in products.items():
+        costs = _config_costs(M, N, K, batch, sym, True, sms)
+        plain += 2 * min(t for t, _ in costs)
+        pairs += (5 if name == "small" else 1) * costs[0][0]    # the two-CTA kernel comes first
+    if pairs > 0.825 * plain:
+        return None
+    count = (steps - 1) // 2
+    return (2,) * count + (1,) * (steps - 2 * count)
+
+
+def composed(X: Tensor, batch: int, m: int, n: int, steps: int) -> Optional[Tuple[int, ...]]:
+    """:func:`compose_groups` for a batch in memory that the two-CTA kernel can read."""
+    if not X.is_cuda or not pair_default() or not X.is_contiguous() or X.data_ptr() % 16:
+        return None
+    return compose_groups(batch, m, n, steps, sm_count(X.device))
+
+
+def ns_compose(X: Tensor, Xalt: Tensor, coeffs, groups: Tuple[int, ...], scale: Optional[Tensor],
+               X2: Optional[Tensor] = None) -> Tensor:
+    """:func:`ns_iterate` with the steps of each group composed on the small matrix; one swap of the
+    buffers a group."""
+    batch, m, n = X.shape
+    dev = X.device
+    g = min(m, n)
+    work = torch.empty((3, batch, g, g), dtype=torch.bfloat16, device=dev)
+    vecs = torch.empty((3, batch, g), dtype=torch.float32, device=dev)
+    tiles_gg = tile_table(g, g, 256, True, dev, bm=256)
+    tiles_mn = tile_table(m, n, 256, False, dev, bm=256)
+    flat = (ctypes.c_float * (3 * len(coeffs)))(*[float(v) for abc in coeffs for v in abc])
+    sizes = (ctypes.c_int * len(groups))(*groups)
+    assert sum(groups) == len(coeffs)
+    if scale is not None:
+        assert scale.dtype == torch.float32 and scale.numel() >= batch
+    rc = _backend.lib("ns_gemm2_sm100").dion_ns_compose2(
+        _p(X), _p(Xalt), _p(X2), _p(work), _p(vecs), ctypes.c_int(batch), ctypes.c_int(m),
+        ctypes.c_int(n), flat, sizes, ctypes.c_int(len(groups)), _p(scale), _p(tiles_gg),
+        ctypes.c_int(tiles_gg.size(0)), _p(tiles_mn), ctypes.c_int(tiles_mn.size(0)),
+        _p(status_tensor(dev)), ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+    if rc != 0:
+        raise RuntimeError(f"dion_ns_compose2 failed with code {rc}")
+    _backend.add_launches(sum(2 + k + 3 * (k - 1) for k in groups))
+    return Xalt if len(groups) % 2 else (X if X2 is None else X2)
 
 
 _persist_tiles: Dict[Tuple, Tensor] = {}

@@ -195,13 +195,19 @@ def _iterate_cuda(X: Tensor, coeffs: Coeffs, scale: Optional[Tensor], hooks=None
     B_, m, n = X.shape
     tall = m > n
     g = n if tall else m
+    alloc = alloc or torch.empty_like
+    persistent = hooks is None and gemm.persistent_fits(X, B_, m, n, len(coeffs))
+    groups = None if hooks is not None or persistent else gemm.composed(X, B_, m, n, len(coeffs))
+    if groups is not None:
+        C = alloc(X)
+        X2 = X if overwrite else alloc(X) if len(groups) > 1 else None
+        return gemm.ns_compose(X, C, coeffs, groups, scale, X2)
     A = torch.empty((B_, g, g), dtype=torch.bfloat16, device=X.device)
     Bm = torch.empty_like(A)
-    alloc = alloc or torch.empty_like
     C = alloc(X)
     if hooks is None:
         X2 = X if overwrite else alloc(X) if len(coeffs) > 1 else None
-        if gemm.persistent_fits(X, B_, m, n, len(coeffs)):
+        if persistent:
             done = gemm.ns_persistent(X, C, A, Bm, coeffs, scale, X2)
             if done is not None:
                 return done
