@@ -69,6 +69,10 @@ struct LrGemmArgs {
   // Optional: column sums of squares of the stored values, accumulated per matrix into
   // colsq[b * N + c] (fp32, pre-zeroed).
   float* colsq;
+  // Split K: matrix b's product is `splits` partial products over kb_per_split slabs each (of every
+  // segment), stored as matrices b * splits + s of C and added up by sum_splits_kernel.
+  int splits;
+  int kb_per_split;
 };
 
 enum : int { kOutStore = 0, kOutReduce = 1, kOutBroadcast = 2 };
@@ -232,13 +236,16 @@ lr_gemm_kernel(const __grid_constant__ LrMaps maps, const LrGemmArgs p) {
       for (int it = 0; ok; ++it) {
         const int t = post_tile(it);
         if (t < 0) break;
-        const int b = t / p.tiles_per_mat;
-        const int rem = t - b * p.tiles_per_mat;
+        const int bs = t / p.tiles_per_mat;
+        const int rem = t - bs * p.tiles_per_mat;
         const int tm = rem / p.tiles_n, tn = rem - tm * p.tiles_n;
+        const int b = bs / p.splits;
+        const int kb0 = (bs - b * p.splits) * p.kb_per_split;
+        const int kb1 = kb0 + p.kb_per_split < num_kb ? kb0 + p.kb_per_split : num_kb;
         for (int seg = 0; seg < p.nseg && ok; ++seg) {
           const CUtensorMap* ma = &maps.a[seg];
           const CUtensorMap* mb = &maps.b[seg];
-          for (int kb = 0; kb < num_kb; ++kb) {
+          for (int kb = kb0; kb < kb1; ++kb) {
             if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1)) {
               atomicExch(p.status, kStatusTimeoutEmpty);
               ok = false;
@@ -278,9 +285,11 @@ lr_gemm_kernel(const __grid_constant__ LrMaps maps, const LrGemmArgs p) {
       uint32_t stage = 0, phase = 0;
       uint32_t aslot = 0, aphase = 0;
       bool ok = true;
-      const int total_kb = num_kb * p.nseg;
       for (int it = 0; ok; ++it) {
-        if (take_tile(it, true, false) < 0) break;
+        const int t = take_tile(it, true, false);
+        if (t < 0) break;
+        const int left = num_kb - (t / p.tiles_per_mat) % p.splits * p.kb_per_split;
+        const int total_kb = (left < p.kb_per_split ? left : p.kb_per_split) * p.nseg;
         if (!mbar_wait_bounded(&tempty_bar[aslot], aphase ^ 1)) {
           atomicExch(p.status, kStatusTimeoutTmemEmpty);
           break;
@@ -663,6 +672,25 @@ __global__ void split_lo_view_kernel(const float* __restrict__ x, long long ld_x
   *reinterpret_cast<float4*>(lo + i * 4) = o;
 }
 
+// out[b] = the sum of matrices b * splits ... of `part`, in order; `n4` 16-byte pieces a matrix.
+__global__ void __launch_bounds__(256)
+sum_splits_kernel(const float4* __restrict__ part, float4* __restrict__ out, long long total4,
+                  long long n4, int splits) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= total4) return;
+  const long long b = i / n4;
+  const float4* p = part + b * (splits - 1) * n4 + i;   // (b * splits) * n4 + (i - b * n4)
+  float4 s = p[0];
+  for (int k = 1; k < splits; ++k) {
+    const float4 x = p[k * n4];
+    s.x += x.x;
+    s.y += x.y;
+    s.z += x.z;
+    s.w += x.w;
+  }
+  out[i] = s;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------------
@@ -751,6 +779,7 @@ struct DionLrExtra {
   int slot0;                  // mode 2: matrix b goes to slot slot0 + b
   float* colsq;               // [batch, N] column sums of squares of the result
   int* sched;                 // optional: two zeroed ints for the dynamic tile order (see LrGemmArgs)
+  int splits;                 // > 1: that many partial products per matrix (plain stores, no D)
 };
 
 // C[b] = alpha * sum_s A_s[b] op(B_s[b]) + beta * D[b].
@@ -801,6 +830,16 @@ DION_EXPORT int dion_lr_gemm(int elem_bytes, int nseg, const DionLrOperand* A,
   g.tiles_per_mat = ((M + LBM - 1) / LBM) * g.tiles_n;
   g.total_tiles = g.tiles_per_mat * batch;
   g.status = status;
+  const int num_kb = (K + bk - 1) / bk;
+  g.splits = 1;
+  g.kb_per_split = num_kb;
+  if (ex != nullptr && ex->splits > 1) {
+    if (ex->out_mode != 0 || ex->c_table || ex->d_table || ex->colsq || D || c_dt != 0) return -15;
+    g.kb_per_split = (num_kb + ex->splits - 1) / ex->splits;
+    if ((long long)g.kb_per_split * (ex->splits - 1) >= num_kb) return -15;   // an empty part
+    g.splits = ex->splits;
+    g.total_tiles *= g.splits;
+  }
   if (ex != nullptr) {
     g.c_table = ex->c_table;
     g.d_table = ex->d_table;
@@ -842,5 +881,19 @@ DION_EXPORT int dion_split_lo_view(const float* x, long long ld_x, long long bs_
   dion::split_lo_view_kernel<<<(unsigned)((total4 + 255) / 256), 256, 0,
                                static_cast<cudaStream_t>(stream)>>>(x, ld_x, bs_x, lo, total4, rows,
                                                                     cols / 4);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// `part` [batch * splits, n] -> out [batch, n], n a multiple of 4, both 16-byte aligned.
+DION_EXPORT int dion_sum_splits(const float* part, float* out, int batch, int splits, long long n,
+                                void* stream) {
+  if (batch <= 0 || n <= 0) return 0;
+  if ((n & 3) || splits < 1 || (reinterpret_cast<uintptr_t>(part) & 15) ||
+      (reinterpret_cast<uintptr_t>(out) & 15))
+    return -2;
+  const long long total4 = batch * (n / 4);
+  dion::sum_splits_kernel<<<(unsigned)((total4 + 255) / 256), 256, 0,
+                            static_cast<cudaStream_t>(stream)>>>(
+      reinterpret_cast<const float4*>(part), reinterpret_cast<float4*>(out), total4, n / 4, splits);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -36,7 +36,7 @@ class _LrExtra(ctypes.Structure):
     _fields_ = [("c_table", ctypes.c_void_p), ("d_table", ctypes.c_void_p),
                 ("out_mode", ctypes.c_int), ("targets", ctypes.c_longlong * 8),
                 ("n_targets", ctypes.c_int), ("slot0", ctypes.c_int),
-                ("colsq", ctypes.c_void_p), ("sched", ctypes.c_void_p)]
+                ("colsq", ctypes.c_void_p), ("sched", ctypes.c_void_p), ("splits", ctypes.c_int)]
 
 
 _sched_pairs: dict = {}
@@ -128,6 +128,18 @@ def split_lo(x: Tensor) -> Tensor:
     return lo
 
 
+def _k_splits(tiles: int, slabs: int, sms: int) -> int:
+    """Into how many partial products a product of ``tiles`` output tiles over ``slabs`` K slabs is
+    cut: as many as still fit one wave, eight at most, each of 16 slabs at least (a slab takes 0.3 us,
+    a tile's epilogue, the partial results and their sum about 4).  The Gram matrix of four factors
+    8192 x 512 has 32 tiles for 148 SMs, the sketch of four 8192 x 2048 matrices 40."""
+    splits = min(sms // max(tiles, 1), 8, slabs // 16)
+    if splits < 2:
+        return 1
+    per = -(-slabs // splits)
+    return -(-slabs // per)
+
+
 def lr_gemm(A: Tensor, B: Tensor, *, a_mn: bool = False, b_mn: bool = False,
             out: Optional[Tensor] = None, out_dtype: Optional[torch.dtype] = None,
             out_list: Optional[List[Tensor]] = None, D: Optional[Tensor] = None,
@@ -136,7 +148,8 @@ def lr_gemm(A: Tensor, B: Tensor, *, a_mn: bool = False, b_mn: bool = False,
             reduce_into: Optional[Tensor] = None, reduce_ld: int = 0,
             broadcast_to: Optional[List[int]] = None, slot0: int = 0, out_ld: int = 0,
             out_stride: int = 0, bn: Optional[int] = None,
-            a_lo: Optional[Tensor] = None, b_lo: Optional[Tensor] = None) -> Optional[Tensor]:
+            a_lo: Optional[Tensor] = None, b_lo: Optional[Tensor] = None,
+            split_k: bool = False) -> Optional[Tensor]:
     """``out[b] = alpha * A[b] @ op(B[b]) + beta * D[b]`` on the tensor cores (tf32 for fp32
     operands, bf16 otherwise; fp32 accumulation), see csrc/lowrank_gemm_sm100.cu.
 
@@ -146,6 +159,8 @@ def lr_gemm(A: Tensor, B: Tensor, *, a_mn: bool = False, b_mn: bool = False,
     ``precise`` (fp32 operands): three tf32 products recover fp32-level accuracy (``a_lo``,
     ``b_lo``: the tf32 remainders of ``A`` / ``B`` if the caller has them already; computed once
     when ``B`` is ``A``).
+    ``split_k``: a product of few tiles over a long K (see :func:`_k_splits`; fp32 result, no ``D``) is
+    computed as partial products, added up by a second launch.
     ``colsq [batch, N]`` (fp32, zeroed by the caller) receives the column sums of squares of the
     result.
 
@@ -223,6 +238,13 @@ def lr_gemm(A: Tensor, B: Tensor, *, a_mn: bool = False, b_mn: bool = False,
         use_ex = True
     if bn is None:
         bn = 256 if N > 128 else 128
+    splits = 1
+    if (split_k and c_ptr and c_dt == 0 and not d_ptr and colsq is None and out.is_contiguous()
+            and M * N % 4 == 0 and c_ptr % 16 == 0):
+        splits = _k_splits(-(-M // 128) * -(-N // bn) * batch, -(-K * eb // 128), gemm.sm_count(dev))
+        if splits > 1:
+            part = torch.empty((batch * splits, M, N), dtype=torch.float32, device=dev)
+            c_ptr, ex.splits, use_ex = part.data_ptr(), splits, True
     if dynamic_tiles_enabled() and not torch.cuda.is_current_stream_capturing():
         ex.sched = _sched_pair(dev).data_ptr()
         use_ex = True
@@ -235,6 +257,11 @@ def lr_gemm(A: Tensor, B: Tensor, *, a_mn: bool = False, b_mn: bool = False,
         _ptr(st), _stream(dev), ctypes.byref(ex) if use_ex else None)
     if rc != 0:
         raise RuntimeError(f"dion_lr_gemm launch failed (code {rc})")
+    if splits > 1:
+        rc = _backend.lib("lowrank_gemm_sm100").dion_sum_splits(
+            _ptr(part), _ptr(out), batch, splits, ctypes.c_longlong(M * N), _stream(dev))
+        if rc != 0:
+            raise RuntimeError(f"dion_sum_splits launch failed (code {rc})")
     return out
 
 
@@ -411,14 +438,15 @@ def right_solve_upper(R: Tensor, P: Tensor, p_lo: Optional[Tensor] = None,
 def gram(P: Tensor, p_lo: Optional[Tensor] = None) -> Tensor:
     """``P^T P`` in fp32 for ``P [B, m, r]`` fp32 (tensor cores with split operands on a GPU)."""
     if P.is_cuda and P.dtype == torch.float32 and P.ndim == 3 and lr_gemm_ok(P):
-        return lr_gemm(P, P, a_mn=True, b_mn=True, precise=True, a_lo=p_lo, b_lo=p_lo)
+        return lr_gemm(P, P, a_mn=True, b_mn=True, precise=True, a_lo=p_lo, b_lo=p_lo,
+                       split_k=True)
     return P.mT @ P
 
 
 def sketch_product(S: Tensor, P: Tensor) -> Tensor:
     """``S P`` for the sketch ``S [B, k, m]`` and ``P [B, m, r]`` (same dtype), fp32 result."""
     if lr_gemm_ok(S, P):
-        return lr_gemm(S, P, b_mn=True, out_dtype=torch.float32)
+        return lr_gemm(S, P, b_mn=True, out_dtype=torch.float32, split_k=True)
     return (S @ P).to(torch.float32)
 
 

@@ -284,7 +284,7 @@ class Dion(DeviceStatusMixin, Optimizer):
         dev = sample.device
         pool = self._side_streams.get(dev)
         if pool is None:
-            pool = self._side_streams[dev] = [torch.cuda.Stream(device=dev)
+            pool = self._side_streams[dev] = [torch.cuda.Stream(device=dev, priority=-1)
                                               for _ in range(self._SIDE_STREAMS)]
         side = pool[task_id % len(pool)]
         main = torch.cuda.current_stream(dev)

@@ -251,6 +251,43 @@ def test_lr_gemm_layouts_against_fp64(dtype, a_mn, b_mn, dims):
     assert lo.dtype == torch.bfloat16 and _rel(lo, A64 @ B64) < 1.5e-2
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, True), (True, True)])
+@pytest.mark.parametrize("dims", [(1, 128, 256, 1024), (2, 200, 136, 2056), (4, 512, 512, 8192),
+                                  (37, 128, 128, 4104)])
+def test_lr_gemm_with_few_tiles_and_long_k(dtype, a_mn, b_mn, dims):
+    """Few output tiles over a long K are computed as partial products, of uneven length and with a
+    ragged last slab, and added up in a fixed order."""
+    from dion_b200.ops import gemm, lowrank as LR
+    b, M, N, K = dims
+    torch.manual_seed(K)
+    A = torch.randn(b, K, M, device="cuda").to(dtype) if a_mn else \
+        torch.randn(b, M, K, device="cuda").to(dtype)
+    B = torch.randn(b, K, N, device="cuda").to(dtype)
+    parts = LR._k_splits(-(-M // 128) * -(-N // 256) * b, -(-K * A.element_size() // 128), 148)
+    assert parts > 1 or (K, dtype) == (1024, torch.bfloat16)
+    C = LR.lr_gemm(A, B, a_mn=a_mn, b_mn=b_mn, out_dtype=torch.float32, precise=True,
+                   split_k=True)
+    again = LR.lr_gemm(A, B, a_mn=a_mn, b_mn=b_mn, out_dtype=torch.float32, precise=True,
+                       split_k=True)
+    gemm.check_status()
+    ref = (A.double().mT if a_mn else A.double()) @ B.double()
+    # The tensor core truncates once per instruction (8 fp32 or 16 bf16 elements of K, three segments
+    # for fp32): half a unit of 2^-23 each, all one way; measured 0.49 of that, twice it is allowed.
+    steps = (3 * K / 8 if dtype == torch.float32 else K / 16) / parts
+    assert ((C - ref).norm() / ref.norm()).item() < 2e-6 + steps * 2.0 ** -24
+    assert torch.equal(C, again)
+
+
+@pytest.mark.parametrize("tiles,slabs,parts", [(32, 256, 4), (40, 256, 3), (74, 64, 2), (75, 512, 1),
+                                               (8, 31, 1), (8, 33, 2), (1, 512, 8), (148, 512, 1)])
+def test_k_splits(tiles, slabs, parts):
+    from dion_b200.ops import lowrank as LR
+    assert LR._k_splits(tiles, slabs, 148) == parts
+    per = -(-slabs // parts)
+    assert per * (parts - 1) < slabs          # no empty part
+
+
 def test_lr_gemm_split_operands_reach_fp32_accuracy():
     from dion_b200.ops import lowrank as LR
     torch.manual_seed(1)
