@@ -181,6 +181,7 @@ class GPT(nn.Module):
         x = None
         if not torch.is_grad_enabled():
             x = inference.hidden_states(self, idx, _FORWARDS)
+        native = x is not None
         if x is None:
             wte = self.transformer.wte
             x = Fn.embedding(idx, wte.weight) if _is_plain(wte) else wte(idx)
@@ -194,6 +195,9 @@ class GPT(nn.Module):
                 return logits.float()
             return Fn.cross_entropy(logits.view(-1, logits.size(-1)), targets.view(-1),
                                     ignore_index=-1)
+        logits = inference.next_token_logits(self.lm_head, x) if native else None
+        if logits is not None:
+            return logits if return_logits else None
         logits = self.lm_head(x[:, -1:, :] if x.size(1) else x[:, [-1], :]).float()
         return logits if return_logits else None
 

@@ -36,6 +36,15 @@ class _Infer(ctypes.Structure):
                 + [("eps_x", ctypes.c_float), ("eps_qk", ctypes.c_float), ("cfg", _Gemm * 4)])
 
 
+class _Stack(ctypes.Structure):
+    """Mirrors ``DionStack`` in csrc/infer_ops.cu."""
+
+    _fields_ = ([(n, ctypes.c_void_p) for n in
+                 ("norm", "weights", "cos", "sin", "x", "h", "xb", "qkv", "y", "act", "ss", "rstd", "status")]
+                + [(n, ctypes.c_int) for n in ("blocks", "B", "T", "H", "D", "F", "w_dt")]
+                + [("eps_x", ctypes.c_float), ("eps_qk", ctypes.c_float)])
+
+
 _entries: Optional[tuple] = None
 
 
@@ -78,24 +87,31 @@ def _block_weights(block, types, C: int):
     Block, Attention, MLP, Rotary = types
     if type(block) is not Block:
         return None
-    attn, mlp = block.attn, block.mlp
-    if not (type(attn) is Attention and type(mlp) is MLP and type(attn.rotary) is Rotary
-            and _unhooked(block) and _unhooked(attn) and _unhooked(mlp)
-            and _unhooked(attn.rotary)):
+    attn, mlp = block._modules.get("attn"), block._modules.get("mlp")
+    if not (type(attn) is Attention and type(mlp) is MLP and _unhooked(block) and _unhooked(attn)
+            and _unhooked(mlp)):
         return None
-    linears = (attn.c_q, attn.c_k, attn.c_v, attn.c_proj, mlp.c_fc, mlp.c_proj)
-    if any(type(m) is not torch.nn.Linear for m in linears):
+    am, mm = attn._modules, mlp._modules
+    rotary = am.get("rotary")
+    if type(rotary) is not Rotary or not _unhooked(rotary):
         return None
-    ws = tuple(m.weight for m in linears)
-    F = ws[4].size(0) if ws[4].ndim else 0
-    shapes = ((C, C),) * 4 + ((F, C), (C, F))
-    for m, w, s in zip(linears, ws, shapes):
-        if not (_unhooked(m) and m.bias is None and is_plain_tensor(w) and w.is_cuda
-                and w.shape == s and w.dtype == ws[0].dtype and w.device == ws[0].device
-                and w.is_contiguous()
-                and w.data_ptr() % 16 == 0):
+    linears = (am.get("c_q"), am.get("c_k"), am.get("c_v"), am.get("c_proj"), mm.get("c_fc"),
+               mm.get("c_proj"))
+    ws = []
+    for m in linears:
+        if type(m) is not torch.nn.Linear or not _unhooked(m):
             return None
-    return ws
+        w = m._parameters.get("weight")
+        if w is None or m.bias is not None:
+            return None
+        ws.append(w)
+    dt, dev = ws[0].dtype, ws[0].device
+    F = ws[4].size(0) if ws[4].ndim else 0
+    for w, s in zip(ws, ((C, C), (C, C), (C, C), (C, C), (F, C), (C, F))):
+        if not (is_plain_tensor(w) and w.is_cuda and w.shape == s and w.dtype == dt
+                and w.device == dev and w.is_contiguous() and w.data_ptr() % 16 == 0):
+            return None
+    return tuple(ws)
 
 
 def _config(rows: int, N: int, K: int, dev: torch.device) -> _Gemm:
@@ -115,6 +131,45 @@ def _pays(C: int, F: int, rows: int) -> bool:
     width 4096, 256 rows 3.56 / 3.59, 16384 rows 46.0 / 53.4.  Up to width 1536 the native blocks are
     as fast or faster throughout (768, 65536 rows: 11.4 / 10.6; 1536, 8192 rows: 4.45 / 4.44)."""
     return C <= 1536 or (4 * C * C + 2 * C * F) * (rows + 512) <= 1.7e11
+
+
+def _stack_fits(rows: int, T: int, C: int, F: int, D: int, blocks: int) -> bool:
+    """Whether ``dion_infer_stack`` takes these sizes and is the faster form.
+
+    It spares the host 60 us a block and rounds no weights, but reads them once per 128 rows, and its
+    attention, a chain over the keys, trails the library's for long texts.  Two native calls a block /
+    one in all, us: GPT-160M 128 tokens 1162 / 535, 256 1271 / 765, 512 1302 / 1165, 16 x 32 1228 / 1021;
+    eight blocks of width 448, 1024 tokens 780 / 744; twelve of 512 with heads of 128, 800 tokens 1114 /
+    1147; twelve of 1024, 2 x 256 tokens 1472 / 1770.  One or two blocks up to width 256 (370 / 163) keep
+    the two calls: the launches of that form are what its tests count."""
+    return (C <= 1024 and F <= 4096 and D in (32, 64, 128)
+            and rows * C * C / 4.0e8 + T * D / 131072.0 <= 1.07 and (blocks > 2 or C > 256))
+
+
+def _stack(x: Tensor, weights, tables, B: int, T: int, H: int, D: int, F: int) -> Tensor:
+    """All blocks on the embedded tokens ``x`` (overwritten) -> ``h``."""
+    dev, C, rows, n = x.device, H * D, B * T, len(weights)
+    h = torch.empty((B, T, C), dtype=torch.bfloat16, device=dev)
+    scratch = torch.empty(rows * (5 * C + F), dtype=torch.bfloat16, device=dev)
+    parts = -(-C // 32)
+    f32 = torch.empty(rows * (parts + 1), dtype=torch.float32, device=dev)
+    at = scratch.data_ptr()
+    step = 2 * rows * C
+    ptrs = ctypes.c_void_p * n
+    w = (ctypes.c_void_p * (6 * n))(*[t.data_ptr() for ws in weights for t in ws])
+    cos = ptrs(*[c.data_ptr() for c, _ in tables])
+    sin = ptrs(*[s.data_ptr() for _, s in tables])
+    p = _Stack(_entry_points()[2], ctypes.addressof(w), ctypes.addressof(cos), ctypes.addressof(sin),
+               x.data_ptr(), h.data_ptr(), at, at + step, at + 4 * step, at + 5 * step, f32.data_ptr(), f32.data_ptr() + 4 * rows * parts,
+               gemm.status_tensor(dev).data_ptr(), n, B, T, H, D, F,
+               0 if weights[0][0].dtype == torch.float32 else 1,
+               float(torch.finfo(torch.float32).eps), float(torch.finfo(torch.bfloat16).eps))
+    rc = _backend.lib("infer_ops").dion_infer_stack(
+        ctypes.byref(p), ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+    if rc != 0:
+        raise RuntimeError(f"dion_infer_stack failed with code {rc}")
+    _backend.add_launches(5 * n + 2)
+    return h
 
 
 def hidden_states(model, idx: Tensor, forwards) -> Optional[Tensor]:
@@ -150,18 +205,22 @@ def hidden_states(model, idx: Tensor, forwards) -> Optional[Tensor]:
         return None
     if F % 8 or not _pays(C, F, B * T) or any(
             w[4].size(0) != F or w[0].dtype != first[0].dtype or w[0].device != idx.device
-            for w in weights) \
-            or any(b.attn.n_head != H for b in blocks):
+            for w in weights):
         return None
     dev, rows = idx.device, B * T
-    tables = []
+    tables, shape = [], (T, D // 2)
     for b in blocks:
-        cos, sin = b.attn.rotary(idx)
-        if any(not t.is_contiguous() or t.dtype != torch.bfloat16 or t.shape != (T, D // 2)
-               or t.device != dev for t in (cos, sin)):
+        attn = b._modules["attn"]
+        if attn.n_head != H:
             return None
+        cos, sin = attn._modules["rotary"].forward(idx)
+        for t in (cos, sin):
+            if not t.is_contiguous() or t.dtype != torch.bfloat16 or t.shape != shape or t.device != dev:
+                return None
         tables.append((cos, sin))
     x = tF.embedding(idx, table)
+    if _stack_fits(rows, T, C, F, D, len(blocks)):
+        return _stack(x, weights, tables, B, T, H, D, F)
     x1 = torch.empty_like(x)
     bf16 = lambda *s: torch.empty(s, dtype=torch.bfloat16, device=dev)  # noqa: E731
     h, qkv, o, act = bf16(B, T, C), bf16(B, T, 3, H, D), bf16(rows, C), bf16(rows, F)
@@ -193,3 +252,27 @@ def hidden_states(model, idx: Tensor, forwards) -> Optional[Tensor]:
     if p.cfg[2].bn:     # the single-CTA kernel leaves relu^2 to one of its own
         _backend.add_launches(len(blocks))
     return h
+
+
+def next_token_logits(head, x: Tensor) -> Optional[Tensor]:
+    """``head(x[:, -1:]).float()`` for the result of :func:`hidden_states` (which has checked what
+    observes the call) and up to four sequences, reading the weights once as they are; None where
+    the head is not a plain linear layer or the sizes are others."""
+    if type(head) is not torch.nn.Linear or not _unhooked(head) or head.bias is not None:
+        return None
+    w = head.weight
+    B, T, C = x.shape
+    if (B > 4 or C > 1024 or C % 4 or not is_plain_tensor(w) or w.ndim != 2 or w.size(1) != C
+            or w.device != x.device or w.dtype not in (torch.float32, torch.bfloat16)
+            or not w.is_contiguous() or w.data_ptr() % 16):
+        return None
+    V = w.size(0)
+    out = torch.empty((B, 1, V), dtype=torch.float32, device=x.device)
+    ptr = ctypes.c_void_p
+    rc = _backend.lib("infer_ops").dion_infer_head(
+        ptr(x.data_ptr() + 2 * (T - 1) * C), ctypes.c_longlong(T * C), ptr(w.data_ptr()),
+        0 if w.dtype == torch.float32 else 1, ptr(out.data_ptr()), B, V, C, gemm.sm_count(x.device),
+        ptr(torch.cuda.current_stream(x.device).cuda_stream))
+    if rc != 0:
+        raise RuntimeError(f"dion_infer_head failed with code {rc}")
+    return out

@@ -110,8 +110,8 @@ def build(force: bool = False, verbose: bool = False) -> List[str]:
 # Kernels launched per exported entry point (default 1); used for the launch counter.
 _KERNELS_PER_CALL = {"dion_dion2_post_masked": 2, "dion_aol_rescale": 2,
                      "dion_embedding_bwd": 3, "dion_embedding_sort_bytes": 0,  # own kernels only
-                     "dion_infer_block_in": 3, "dion_infer_block_out": 5,
-                     "dion_ns_iterate2": 0, "dion_ns_compose2": 0}  # these two count themselves
+                     "dion_infer_block_in": 3, "dion_infer_block_out": 5, "dion_infer_stack": 0,
+                     "dion_ns_iterate2": 0, "dion_ns_compose2": 0}  # 0: these count themselves
 _launches = 0
 
 

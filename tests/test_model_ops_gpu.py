@@ -310,6 +310,88 @@ def test_blocks_without_gradients_match_the_general_forward(B, T, heads, dim, dt
     assert ((last[:, 0] - ref[:, -1]).norm() / ref[:, -1].norm()).item() < 2e-2
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,T,heads,dim", [(1, 1, 12, 64), (2, 63, 3, 128), (1, 129, 8, 64), (3, 65, 10, 32),
+                                           (1, 257, 5, 64), (2, 130, 8, 128), (5, 200, 2, 64)])
+def test_stack_of_blocks_matches_the_general_forward(B, T, heads, dim, dtype):
+    """One call for all blocks: rows and keys below, at and above their tiles, one to eight CTAs to a
+    cluster, column tiles of both widths, every head dimension.  Both sides round every product to
+    bf16 (2^-9 each, over three blocks)."""
+    from dion_b200.models import inference
+    from dion_b200.models.gpt import GPT, GPTConfig
+    from dion_b200.ops import _backend, gemm
+    torch.manual_seed(1)
+    model = GPT(GPTConfig(sequence_len=T, vocab_size=515, n_layer=3, n_head=heads,
+                          n_embd=heads * dim)).cuda()
+    model.init_weights()
+    model.transformer.h.to(dtype)
+    assert inference._stack_fits(B * T, T, heads * dim, 4 * heads * dim, dim, 3)
+    ids = torch.randint(0, 515, (B, T), device="cuda")
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        ref = model(ids, ids, return_logits=True).detach()
+        with torch.no_grad():
+            _backend.reset_launch_count()
+            got = model(ids, ids, return_logits=True)
+            assert _backend.launch_count() == 3 * 5 + 2
+            again = model(ids, ids, return_logits=True)
+            last = model(ids, return_logits=True)
+    gemm.check_status()
+    assert ((got - ref).norm() / ref.norm()).item() < 2e-2
+    assert torch.equal(got, again)
+    assert last.shape == (B, 1, 515)
+    assert ((last[:, 0] - ref[:, -1]).norm() / ref[:, -1].norm()).item() < 2e-2
+
+
+def test_stack_of_blocks_in_a_captured_graph_and_on_a_side_stream():
+    """The launches, which may start before their predecessors end, keep their order in a graph and
+    on another stream than the default one, and see weights changed just before."""
+    from dion_b200.models.gpt import GPT, GPTConfig
+    torch.manual_seed(2)
+    model = GPT(GPTConfig(sequence_len=96, vocab_size=512, n_layer=4, n_head=6, n_embd=384)).cuda()
+    model.init_weights()
+    ids = torch.randint(0, 512, (1, 96), device="cuda")
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        eager = model(ids, return_logits=True)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = model(ids, return_logits=True)
+        for _ in range(3):
+            out.zero_()
+            graph.replay()
+            assert torch.equal(out, eager)
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            for p in model.transformer.h.parameters():
+                p.mul_(0.5)
+            halved = model(ids, return_logits=True)
+        torch.cuda.current_stream().wait_stream(side)
+        graph.replay()
+        assert torch.equal(out, halved) and not torch.equal(out, eager)
+        with torch.enable_grad():
+            ref = model(ids, ids, return_logits=True)[:, -1:].detach()
+    assert ((halved - ref).norm() / ref.norm()).item() < 2e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,C,V", [(1, 768, 1003), (2, 100, 7), (3, 1024, 65), (4, 4, 1), (4, 640, 2053)])
+def test_next_token_logits(B, C, V, dtype):
+    """Exact products of bf16 numbers summed in fp32, then rounded to bf16 like the layer's result."""
+    from dion_b200.models import inference
+    torch.manual_seed(V)
+    head = torch.nn.Linear(C, V, bias=False, device="cuda", dtype=dtype)
+    h = torch.randn(B, 3, C, device="cuda").bfloat16()
+    got = inference.next_token_logits(head, h)
+    ref = h[:, -1:].double() @ head.weight.bfloat16().double().mT
+    assert got.shape == (B, 1, V) and got.dtype == torch.float32
+    assert torch.equal(got, got.bfloat16().float())
+    size = (h[:, -1:].double().abs() @ head.weight.bfloat16().double().abs().mT)
+    assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-6 * size).all()
+    assert inference.next_token_logits(torch.nn.Linear(C, V, device="cuda"), h) is None   # a bias
+    assert inference.next_token_logits(head, h.expand(3, -1, -1, -1).reshape(-1, 3, C)[:5]) is None \
+        if 3 * B >= 5 else True
+
+
 def test_replaced_modules_take_the_general_forward():
     """A block, a linear layer or an embedding of another type may look nothing like the original:
     the path without gradients leaves such a model to the modules."""
