@@ -134,6 +134,18 @@ __device__ __forceinline__ bool flag_wait_bounded(const int* flag, int want) {
   }
 }
 
+// ---- programmatic dependent launch --------------------------------------------------------
+// A kernel launched with programmatic stream serialization may start before the one ahead of it in
+// the stream has ended: whatever that one (or any before it) writes or reads is touched only
+// behind wait_for_previous_kernel(), which every CTA has to pass.
+__device__ __forceinline__ void wait_for_previous_kernel() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// From here on the next kernel's CTAs may take the room that this one's leave.
+__device__ __forceinline__ void let_next_kernel_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }

@@ -226,14 +226,6 @@ __device__ __forceinline__ float4 sk_ld_cluster(uint32_t local, uint32_t rank) {
                : "r"(a));      // volatile: stays behind the cluster barrier
   return v;
 }
-// Everything the preceding launches of the stream wrote is visible behind this.
-__device__ __forceinline__ void wait_for_previous() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void let_next_start() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // Y[rows, N] = X[rows, K] W^T for one tile of 128 rows x BN columns per cluster: grid (splits, column
 // tiles, row tiles), cluster (splits, 1, 1); CTA s of a cluster takes K slabs [s * slabs, ...), SLABS
 // at most.  A CTA's weights are all requested at once, into registers (96 to 128 of them), so nothing
@@ -263,7 +255,7 @@ skinny_kernel(const __grid_constant__ CUtensorMap map_x, const SkinnyArgs p) {
   const int ns = total_slabs - s0 < p.slabs ? total_slabs - s0 : p.slabs;   // 1 to SLABS
   const int n0 = blockIdx.y * BN;
   const int row0 = blockIdx.z * 128;
-  let_next_start();
+  let_next_kernel_start();
 
   float4 w[BN / 16][SLABS][2];
   const int t = (int)threadIdx.x - 32;     // 0..127 in warps 1 to 4
@@ -332,7 +324,7 @@ skinny_kernel(const __grid_constant__ CUtensorMap map_x, const SkinnyArgs p) {
 
   if (warp == 0) {
     if (lane == 0) {
-      wait_for_previous();
+      wait_for_previous_kernel();
       auto load = [&](int s) {
         mbar_expect_tx(&x_bar[s % kRing], kSkABytes);
         tma_load_3d(a_buf + (s % kRing) * kSkABytes, &map_x, &x_bar[s % kRing], (s0 + s) * 64, row0, 0);
@@ -391,7 +383,7 @@ skinny_kernel(const __grid_constant__ CUtensorMap map_x, const SkinnyArgs p) {
     fence_proxy_async();
     __syncwarp();
     if (lane == 0) mbar_arrive(&conv_bar);
-    wait_for_previous();    // from here on, what the preceding kernels wrote is read and written
+    wait_for_previous_kernel();    // from here on, what the preceding kernels wrote is read and written
     request_old(t / kLanes);
     if (p.ss != nullptr) {  // 1 / rms of every row of the tile
       float sum = 0.f;
@@ -557,8 +549,8 @@ short_attention_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat1
   const long long ld = 3LL * C;
   const __nv_bfloat16* base = qkv + (long long)b * T * ld + h * D;
   const int r_lo = q0 + warp * 16 + (lane >> 2), r_hi = r_lo + 8, cc = (lane & 3) * 2;
-  let_next_start();
-  wait_for_previous();
+  let_next_kernel_start();
+  wait_for_previous_kernel();
 
   // Rows [first, first + n) of a section of qkv, rotated and normalized, into `dst`.
   const int sub = (int)threadIdx.x % TPV;
@@ -775,7 +767,7 @@ static int map_rows(CUtensorMap* map, const void* ptr, int rows, int cols) {
   return encode_bf16_3d(enc, map, ptr, dims, strides, box);
 }
 
-// Launch with leave to start before the preceding kernel has ended (see wait_for_previous).
+// Launch with leave to start before the preceding kernel has ended (see wait_for_previous_kernel).
 template <class Kernel, class... Args>
 static int launch_early(Kernel kernel, dim3 grid, int threads, int dyn, int cluster,
                         cudaStream_t stream, const Args&... args) {

@@ -284,6 +284,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   const int num_kb = (p.K + BK2 - 1) / BK2;
   const int first_tile = (int)cluster_id_x();
   const int tile_step = (int)num_clusters_x();
+  let_next_kernel_start();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages2; ++s) {
@@ -318,6 +319,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       uint32_t ready_mask = 0;
+      wait_for_previous_kernel();
       const int seq = p.wait_flags ? *p.seq_ptr : 0;
       // Waits (bounded) until every source rank owning rows [r0, r1] has delivered.
       auto sources_ready = [&](int r0, int r1) -> bool {
@@ -452,6 +454,7 @@ ns_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const uint32_t row_sw = swizzle(row_in_tile);
     uint8_t* dc_base = smem + kStages2 * kStageBytes2 + grp * kGDC * kEpiBufBytes;
     uint64_t* dfull = dfull_bar + grp * kGDC;
+    wait_for_previous_kernel();
 
     // Iterator over the sub-tiles this group will process, in order (used for the D prefetch).
     // Only the last column of tiles can be narrower than 256 columns.
@@ -841,13 +844,20 @@ static int launch2(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorM
   cfg.blockDim = dim3(CFG::kThreads, 1, 1);
   cfg.dynamicSmemBytes = kDynBytes2;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  // CTAs may start as those of the preceding kernel leave their SMs, set up and wait for it to end:
+  // the launch gap, the ramp and the other kernel's last wave overlap.  Five iterations on 6 x 1000 x
+  // 1536: 328 -> 286 us, 48 x 192 x 768 201 -> 166, 4 x 1024^2 266 -> 230, 12 x 768 x 3072 444 -> 428; 24 x
+  // 2048^2 as before.  Launches that wait for other GPUs start in order.
+  cfg.numAttrs = args.wait_flags == nullptr && args.scale_partials == nullptr &&
+                 args.remote_c[0] == 0 ? 2 : 1;
   if (cudaLaunchKernelEx(&cfg, kernel, ma, mb, mc, md, args) != cudaSuccess) {
     cudaGetLastError();
     return -4;

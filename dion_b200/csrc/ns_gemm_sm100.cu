@@ -117,6 +117,7 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int num_kb = (p.K + BK - 1) / BK;
+  let_next_kernel_start();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -145,6 +146,7 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
+      wait_for_previous_kernel();
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       uint32_t ready_mask = 0;
@@ -274,6 +276,7 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else {
     // ------------------------------ epilogue ----------------------------------
+    wait_for_previous_kernel();
     const int lane_grp = warp & 3;  // TMEM lanes [32*lane_grp, +32) belong to this warp
     const int row_in_tile = lane_grp * 32 + lane;
     uint32_t aslot = 0, aphase = 0;
@@ -501,8 +504,24 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmArgs& 
   }
   int grid = args.total_tiles < num_sms ? args.total_tiles : num_sms;
   if (grid <= 0) return 0;
-  ns_gemm_kernel<BN, A_MN, B_MN><<<grid, kNumThreads, L::kDynBytes, stream>>>(ma, mb, args);
-  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(kNumThreads, 1, 1);
+  cfg.dynamicSmemBytes = L::kDynBytes;
+  cfg.stream = stream;
+  // As in ns_gemm2_sm100.cu: the next launch's set-up overlaps this one's end, unless it waits for
+  // other GPUs.
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = args.wait_flags == nullptr && args.scale_partials == nullptr &&
+                 args.remote_c[0] == 0 ? 1 : 0;
+  if (cudaLaunchKernelEx(&cfg, ns_gemm_kernel<BN, A_MN, B_MN>, ma, mb, args) != cudaSuccess) {
+    cudaGetLastError();
+    return -4;
+  }
+  return 0;
 }
 
 }  // namespace dion

@@ -380,3 +380,31 @@ def test_shape_first_met_in_a_capture():
         torch.cuda.synchronize()
         assert torch.equal(o, eager)
     gemm.check_status()
+
+
+@pytest.mark.parametrize("pair", [False, True])
+def test_products_that_follow_one_another_closely(pair):
+    """A launch may start before the one ahead of it has ended; it must see its result, and must not
+    overwrite what that one still reads.  Chains of products over three buffers, of one tile and of
+    several waves, as one burst and with a synchronization after each, give the same bits."""
+    from dion_b200.ops import gemm
+    torch.manual_seed(8)
+    for b, n in ((1, 136), (3, 264), (40, 512)):
+        X = (torch.randn(b, n, n, device="cuda") / n ** 0.5).bfloat16()
+
+        def chain(sync):
+            bufs = [X.clone(), torch.zeros_like(X), torch.zeros_like(X)]
+            for i in range(12):
+                A, B, C = (bufs[(i + k) % 3] for k in range(3))
+                gemm.ns_gemm(A, B if i else A, out=C, D=A, beta=0.5, pair=pair,
+                             bn=None if pair else 128)
+                if sync:
+                    torch.cuda.synchronize()
+            return bufs
+
+        ref = chain(True)
+        for _ in range(3):
+            got = chain(False)
+            torch.cuda.synchronize()
+            assert all(torch.equal(a, r) for a, r in zip(got, ref))
+    gemm.check_status()
