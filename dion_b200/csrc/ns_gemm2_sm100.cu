@@ -1168,3 +1168,100 @@ DION_EXPORT int dion_ns_compose2(void* X, void* Xalt, void* X2, void* work, floa
   }
   return 0;
 }
+
+namespace dion {
+
+// M[b][i][i] += a for a dense bf16 batch [batch, g, g], rounded once more.
+__global__ void __launch_bounds__(256)
+add_diagonal_kernel(__nv_bfloat16* M, int batch, int g, float a) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (long long)batch * g) return;
+  __nv_bfloat16* x = M + i * g + i % g;
+  *x = __float2bfloat16(__bfloat162float(*x) + a);
+}
+
+}  // namespace dion
+
+// Gram form of the loop from one host call: R = s^2 X X^T (X^T X for tall X); for every (a, b, c):
+//   Z = a I + b R + c R R,  Q = Z Q (Q = Z in the first),  R = (Z R) Z,
+// where reset[it] != 0 first applies Q to X and forms R anew.  R is not brought forward where nothing
+// reads it again.  `work` holds five matrices [batch, g, g]; the results go to and fro between Y0 and
+// Y1, X is only read.  Returns 0 or 1, the buffer that holds the result, or an error below zero.
+// 24 launches for five steps: issued one by one from Python they take 0.5 ms, more than the
+// products of anything up to 8 x 1024 x 2048.
+DION_EXPORT int dion_ns_gram2(const void* X, void* Y0, void* Y1, void* work, int batch, int m, int n,
+                              const float* coeffs, const int* reset, int iters, const float* scale,
+                              const void* tiles_sym, int n_tiles_sym, const void* tiles_gg,
+                              int n_tiles_gg, const void* tiles_mn, int n_tiles_mn, int* status,
+                              void* stream) {
+  using namespace dion;
+  const int tall = m > n;
+  const int g = tall ? n : m;
+  if (batch <= 0 || m <= 0 || n <= 0 || iters <= 0) return -10;
+  const long long sx = (long long)m * n, sg = (long long)g * g;
+  const size_t mat = (size_t)batch * g * g;
+  __nv_bfloat16* w = static_cast<__nv_bfloat16*>(work);
+  void *R = w, *T = w + mat, *zq[3] = {w + 2 * mat, w + 3 * mat, w + 4 * mat};
+  int qi = -1;                       // the one of zq that holds Q
+  const void* cur = X;
+  void* out[2] = {Y0, Y1};
+  int which = 0;
+  const float* sc = scale;           // X itself is unnormalized until Q has been applied to it
+  auto small = [&](const void* A, const void* B, int b_kn, void* C, const void* D, float alpha,
+                   float beta, int sym) {
+    return dion_ns_gemm2(A, g, sg, 0, B, g, sg, b_kn, C, g, sg, D, D ? g : 0, D ? sg : 0, batch, g, g,
+                         g, alpha, beta, nullptr, 0, 0, sym, sym ? tiles_sym : tiles_gg,
+                         sym ? n_tiles_sym : n_tiles_gg, 0, status, stream);
+  };
+  auto gram = [&]() {
+    return dion_ns_gemm2(cur, n, sx, tall, cur, n, sx, tall, R, g, sg, nullptr, 0, 0, batch, g, g,
+                         tall ? m : n, 1.f, 0.f, sc, sc ? 2 : 0, 0, 1, tiles_sym, n_tiles_sym, 0,
+                         status, stream);
+  };
+  auto apply = [&]() {
+    const void* Q = zq[qi];
+    int rc;
+    if (tall)
+      rc = dion_ns_gemm2(cur, n, sx, 0, Q, g, sg, 0, out[which], n, sx, nullptr, 0, 0, batch, m, n, g,
+                         1.f, 0.f, sc, sc ? 1 : 0, 0, 0, tiles_mn, n_tiles_mn, 0, status, stream);
+    else
+      rc = dion_ns_gemm2(Q, g, sg, 0, cur, n, sx, 1, out[which], n, sx, nullptr, 0, 0, batch, m, n, g,
+                         1.f, 0.f, sc, sc ? 1 : 0, 0, 0, tiles_mn, n_tiles_mn, 0, status, stream);
+    cur = out[which];
+    which ^= 1;
+    sc = nullptr;
+    qi = -1;
+    return rc;
+  };
+  int rc = gram();
+  for (int it = 0; it < iters && rc == 0; ++it) {
+    if (reset[it] && qi >= 0) {
+      rc = apply();
+      if (rc == 0) rc = gram();
+      if (rc != 0) break;
+    }
+    const float a = coeffs[3 * it], b = coeffs[3 * it + 1], c = coeffs[3 * it + 2];
+    const int zi = (qi + 1) % 3;
+    void* Z = zq[zi];
+    rc = small(R, R, 0, Z, R, c, b, 1);
+    if (rc != 0) break;
+    add_diagonal_kernel<<<(unsigned)(((long long)batch * g + 255) / 256), 256, 0,
+                          static_cast<cudaStream_t>(stream)>>>(static_cast<__nv_bfloat16*>(Z), batch,
+                                                               g, a);
+    if (cudaGetLastError() != cudaSuccess) return -4;
+    if (qi < 0) {
+      qi = zi;
+    } else {
+      const int next = 3 - qi - zi;
+      rc = small(Z, zq[qi], 1, zq[next], nullptr, 1.f, 0.f, 0);
+      if (rc != 0) break;
+      qi = next;
+    }
+    if (it + 1 < iters && !reset[it + 1]) {
+      rc = small(Z, R, 0, T, nullptr, 1.f, 0.f, 0);          // Z R   (R symmetric, so R^T = R)
+      if (rc == 0) rc = small(T, Z, 0, R, nullptr, 1.f, 0.f, 1);   // (Z R) Z  (Z symmetric)
+    }
+  }
+  if (rc == 0) rc = apply();
+  return rc != 0 ? (rc < 0 ? rc : -4) : which ^ 1;
+}

@@ -111,7 +111,7 @@ def build(force: bool = False, verbose: bool = False) -> List[str]:
 _KERNELS_PER_CALL = {"dion_dion2_post_masked": 2, "dion_aol_rescale": 2,
                      "dion_embedding_bwd": 3, "dion_embedding_sort_bytes": 0,  # own kernels only
                      "dion_infer_block_in": 3, "dion_infer_block_out": 5, "dion_infer_stack": 0,
-                     "dion_ns_iterate2": 0, "dion_ns_compose2": 0}  # 0: these count themselves
+                     "dion_ns_iterate2": 0, "dion_ns_compose2": 0, "dion_ns_gram2": 0}  # 0: these count themselves
 _launches = 0
 
 

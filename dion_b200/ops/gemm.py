@@ -374,17 +374,37 @@ def ns_gemm(
 
 
 def iterate_in_one_call(X: Tensor, batch: int, m: int, n: int) -> bool:
-    """True when all three GEMMs of a Newton-Schulz iteration on ``[batch, m, n]`` would go to the
-    two-CTA kernel, so that the whole iteration can be issued by one host call."""
-    if not pair_default() or not X.is_contiguous() or X.data_ptr() % 16 or m % 8 or n % 8:
-        return False
+    """True when the two-CTA kernel can read and write all of a Newton-Schulz iteration on ``[batch, m,
+    n]``, so that the whole loop is issued by one host call.  That is the faster form for every size:
+    chosen one by one the fifteen products of five steps take 340 us of host time, and on the device
+    (as graphs; chosen / two-CTA, us) 10 x 128 x 4096 285 / 250, 9 x 768^2 241 / 226, 1 x 2560^2 464 / 413, 1
+    x 2048 x 8192 695 / 658, 1 x 1280^2 221 / 225, 8 x 256 x 1024 139 / 146, 3 x 200 x 136 110 / 122."""
+    return (pair_default() and X.is_contiguous() and X.data_ptr() % 16 == 0 and m % 8 == 0
+            and n % 8 == 0)
+
+
+def ns_gram(X: Tensor, coeffs, resets, scale: Tensor) -> Tensor:
+    """The Gram form of the loop (``dion_ns_gram2``) on a batch that is only read."""
+    batch, m, n = X.shape
     dev = X.device
-    tall = m > n
-    g = n if tall else m
-    k_gram = m if tall else n
-    return (_choose_config(g, g, k_gram, batch, True, True, dev)[0]
-            and _choose_config(g, g, g, batch, True, True, dev)[0]
-            and _choose_config(m, n, g, batch, False, True, dev)[0])
+    g = min(m, n)
+    Y = [torch.empty_like(X) for _ in range(1 + any(0 < r < len(coeffs) for r in resets))]
+    work = torch.empty((5, batch, g, g), dtype=torch.bfloat16, device=dev)
+    flat = (ctypes.c_float * (3 * len(coeffs)))(*[float(v) for abc in coeffs for v in abc])
+    reset = (ctypes.c_int * len(coeffs))(*[int(i in resets) for i in range(len(coeffs))])
+    tables = [tile_table(g, g, 256, True, dev, bm=256), tile_table(g, g, 256, False, dev, bm=256),
+              tile_table(m, n, 256, False, dev, bm=256)]
+    sizes = [a for t in tables for a in (_p(t), ctypes.c_int(t.size(0)))]
+    rc = _backend.lib("ns_gemm2_sm100").dion_ns_gram2(
+        _p(X), _p(Y[0]), _p(Y[-1]), _p(work), ctypes.c_int(batch), ctypes.c_int(m), ctypes.c_int(n),
+        flat, reset, ctypes.c_int(len(coeffs)), _p(scale), *sizes, _p(status_tensor(dev)),
+        ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+    if rc < 0:
+        raise RuntimeError(f"dion_ns_gram2 failed with code {rc}")
+    steps, applied = len(coeffs), sum(0 < i and r for i, r in enumerate(reset))
+    forward = sum(i + 1 < steps and not reset[i + 1] for i in range(steps))
+    _backend.add_launches(2 * (1 + applied) + 2 * steps + (steps - 1 - applied) + 2 * forward)
+    return Y[rc]
 
 
 def ns_iterate(X: Tensor, Xalt: Tensor, A: Tensor, Bm: Tensor, coeffs, scale: Optional[Tensor],
@@ -420,22 +440,24 @@ def compose_groups(batch: int, m: int, n: int, steps: int, sms: int) -> Optional
     composed on the small matrix (see ``dion_ns_compose2``), or None where the plain loop stays.
 
     Pairs, from the first step on and with a single step at the end (without it the result is further
-    from the exact one than the plain loop's, 1.1 times; with it nearer), where the products of two steps are estimated at 0.825 of the plain
-    ones or less: the estimate is optimistic about the small products, which are bound by their
-    epilogue.  Composed / plain for five steps at an estimate of 0.57 (48 x 512 x 8192) 0.71, 0.68 (24 x
-    2048 x 8192) 0.79, 0.71-0.74 (64 x 768 x 3072, 96 x 512 x 2048) 0.87-0.92, 0.79-0.82 (16 x 1024 x 3072, 24
-    x 2048 x 4096) 0.89-0.91, 0.83 (6 x 768 x 3072, 12 x 512 x 2048) 1.00 and 0.93, 0.89 (64 x 768 x 1536, 2 x 4096 x 6144) 1.05 and
-    0.94, 0.95 and above 1.0-1.05.  And from ``min(m, n) = 512``: below, the composed result of a
-    spectrum that falls off as 1 / rank is further from the exact one (1.08 times at 384, 2.6 at 192)."""
+    from the exact one than the plain loop's, 1.1 times; with it nearer), where their products and
+    launches (2 us each, 300 of the estimate's units) are estimated at 0.825 of the plain ones or
+    less: the estimate is optimistic about the small products, which their epilogue bounds.  Composed /
+    plain for five steps at an estimate of 0.57-0.61 (24 x 8192 x 512, 12 x 512 x 8192) 0.72-0.77, 0.68-0.74
+    (24 x 2048 x 8192, 64 x 768 x 3072, 96 x 512 x 2048) 0.78-0.92, 0.77-0.82 (4 x 1024 x 4096, 16 x 1024 x 3072,
+    24 x 2048 x 4096) 0.89-0.96, 0.83-0.86 (4 x 512 x 4096, 6 x 768 x 3072, 12 x 512 x 2048) 1.01-1.02, 0.89 (64 x
+    768 x 1536, 2 x 4096 x 6144) 1.06 and 0.94.  And from ``min(m, n) = 512``: below, the composed result
+    of a spectrum that falls off as 1 / rank is further from the exact one (1.08 times at 384, 2.6 at
+    192)."""
     g, long = min(m, n), max(m, n)
     if g < 512 or steps < 3 or m % 8 or n % 8:
         return None
-    products = {"gram": (g, g, long, True), "small": (g, g, g, True), "update": (m, n, g, False)}
+    launch = 300.0
     plain = pairs = 0.0
-    for name, (M, N, K, sym) in products.items():
-        costs = _config_costs(M, N, K, batch, sym, True, sms)
-        plain += 2 * min(t for t, _ in costs)
-        pairs += (5 if name == "small" else 1) * costs[0][0]    # the two-CTA kernel comes first
+    for M, N, K, sym, count in ((g, g, long, True, 1), (g, g, g, True, 5), (m, n, g, False, 1)):
+        cost = _config_costs(M, N, K, batch, sym, True, sms)[0][0] + launch    # of the two-CTA kernel
+        plain += 2 * cost
+        pairs += count * cost
     if pairs > 0.825 * plain:
         return None
     count = (steps - 1) // 2
@@ -486,10 +508,9 @@ def persistent_enabled() -> bool:
 
 
 def persistent_waves() -> float:
-    """Largest GEMM of the loop, in waves of 128 x 128 tiles over the SMs, up to which the
-    one-launch form is used (``DION_B200_PERSISTENT_WAVES``, default 1: beyond that the
-    256 x 256 two-CTA kernel's better efficiency outweighs the saved launches; set before both forms
-    became faster)."""
+    """Largest GEMM of the loop, in waves over the SMs, up to which the one-launch form is used
+    (``DION_B200_PERSISTENT_WAVES``, default 1: beyond that the 256 x 256 two-CTA kernel's better
+    efficiency outweighs the saved launches, see :func:`persistent_fits`)."""
     try:
         return float(os.environ.get("DION_B200_PERSISTENT_WAVES", "1"))
     except ValueError:
@@ -503,8 +524,11 @@ def persistent_in_graphs() -> bool:
 
 
 def persistent_fits(X: Tensor, batch: int, m: int, n: int, iters: int) -> bool:
-    """The one-launch form pays when no GEMM of the loop has more 128 x 128 tiles than the GPU
-    has SMs (every phase is then a single wave and launch / fill / drain dominate)."""
+    """The one-launch form pays when no GEMM of the loop has more 128 x 64 tiles than the GPU has SMs
+    (every phase is then a single wave and launch / fill / drain dominate): one launch / fifteen, us, 256^2
+    96 / 127, 768^2 157 / 195, 512 x 2048 170 / 211.  With as many 128 x 128 tiles the two are level from
+    512 rows (8 x 512^2 173 / 177, 4 x 768^2 203 / 198, 1000 x 1536 232 / 245), below fifteen launches win (6 x
+    384 x 768 181 / 152, 8 x 256 x 1024 172 / 153, 64 x 128 x 256 143 / 122)."""
     if not persistent_enabled() or not X.is_contiguous() or X.data_ptr() % 16 or m % 8 or n % 8:
         return False
     if iters > 8:
@@ -512,7 +536,8 @@ def persistent_fits(X: Tensor, batch: int, m: int, n: int, iters: int) -> bool:
     if torch.cuda.is_current_stream_capturing() and not persistent_in_graphs():
         return False
     g = min(m, n)
-    tiles = max(_num_tiles(g, g, _BM, 128, True), _num_tiles(m, n, _BM, 128, False)) * batch
+    bn = 128 if g >= 512 else 64
+    tiles = max(_num_tiles(g, g, _BM, bn, True), _num_tiles(m, n, _BM, bn, False)) * batch
     return tiles <= persistent_waves() * sm_count(X.device)
 
 

@@ -303,6 +303,8 @@ def _gram_cuda(G: Tensor, coeffs: Coeffs, norm_mult: float, epsilon: float,
     B_, m, n = X.shape
     tall = m > n
     g = min(m, n)
+    if coeffs and X.is_cuda and gemm.iterate_in_one_call(X, B_, m, n):
+        return restore(gemm.ns_gram(X, coeffs, resets, scale))
     R = torch.empty((B_, g, g), dtype=torch.bfloat16, device=X.device)
 
     def gram(sc: Optional[Tensor]) -> None:

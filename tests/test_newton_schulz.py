@@ -376,3 +376,25 @@ def test_which_loops_are_composed():
     assert gemm.compose_groups(64, 768, 768, 5, 148) is None       # as many products either way
     assert gemm.compose_groups(64, 504, 8192, 5, 148) is None      # less exact below 512
     assert gemm.compose_groups(64, 772, 3072, 5, 148) is None      # not for TMA
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("resets", [(2,), (), (1, 3), (4,), (0, 2, 9)])
+@pytest.mark.parametrize("shape", [(1, 768, 768), (3, 136, 264), (2, 1032, 520), (4, 8, 64)])
+def test_gram_in_one_call_equals_its_products_one_by_one(shape, resets, monkeypatch):
+    """The same launches in the same order, so the same bits."""
+    from dion_b200.ops import gemm
+    torch.manual_seed(3)
+    G = torch.randn(shape, device="cuda").bfloat16()
+    keep = G.clone()
+    got = NS.gram_newton_schulz(G, reset_iterations=resets)
+    monkeypatch.setattr(gemm, "iterate_in_one_call", lambda *a: False)
+    product = gemm.ns_gemm
+    monkeypatch.setattr(gemm, "ns_gemm", lambda *a, **k: product(*a, **k, pair=True))
+    ref = NS.gram_newton_schulz(G, reset_iterations=resets)
+    gemm.check_status()
+    assert torch.equal(got, ref) and torch.equal(G, keep)
+    short = NS.gram_newton_schulz(G, reset_iterations=resets, coeffs=NS.POLAR_EXPRESS_COEFFS[:1])
+    monkeypatch.undo()
+    assert torch.equal(short, NS.gram_newton_schulz(G, reset_iterations=resets,
+                                                    coeffs=NS.POLAR_EXPRESS_COEFFS[:1]))
