@@ -300,6 +300,54 @@ def test_every_tensor_of_a_list_is_found(sizes):
     _close(M, Md, 1e-6)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("first", [0, 1])
+def test_whole_and_partial_chunks(dtype, first):
+    """Momentum and apply at the edges of the 4096-element chunks, on and off a 16-byte boundary,
+    against the PyTorch forms; the elements before and behind each tensor stay as they are.
+    The fp32 sums may round twice on one side and once on the other (fused multiply-add), 2^-23 of
+    the operands; a bf16 result is then one unit, 2^-7, off at most."""
+    g = torch.Generator().manual_seed(0)
+    shapes = [(1, 4092), (1, 4096), (1, 4100), (64, 128), (3, 4097), (5, 2456)]
+
+    def moved(t):
+        base = torch.full((t.numel() + first + 9,), 7.0, dtype=t.dtype, device="cuda")
+        view = base[first:first + t.numel()].view(t.shape)
+        return view.copy_(t), base
+
+    def check(host, dev, rel):
+        for h, (d, base) in zip(host, dev):
+            assert (base[:first] == 7.0).all() and (base[first + h.numel():] == 7.0).all()
+            a, b = h.float(), d.float().cpu()
+            assert ((a - b).abs() <= rel * (4 + a.abs())).all(), (h.shape, (a - b).abs().max())
+
+    G, M, X = [[torch.randn(s, generator=g).to(dtype) for s in shapes] for _ in range(3)]
+    rel = 2.0 ** -23 if dtype == torch.float32 else 2.0 ** -7
+    on = [[moved(t) for t in lst] for lst in (G, M, X)]
+    Gd, Md, Xd = [[d for d, _ in lst] for lst in on]
+    F.muon_pre(G, M, 0.95, True)
+    U = F.muon_pre(Gd, Md, 0.95, True)
+    check(G, on[0], 0.0)
+    check(M, on[1], rel)
+    lr = torch.full((), 0.02)
+    F.muon_post(X, [u.cpu() for u in U], lr, 0.1, 1.5, False)
+    F.muon_post(Xd, U, lr.cuda(), 0.1, 1.5, False)
+    check(X, on[2], rel)
+    for shape in ((64, 64), (64, 68), (3, 4097), (96, 128)):
+        for dim in (-2, -1):
+            X1 = torch.randn(shape, generator=g).to(dtype)
+            dev = moved(X1)
+            index = torch.randperm(shape[dim], generator=g)[:shape[dim] // 3]
+            where = torch.full((shape[dim],), -1, dtype=torch.int32)
+            where[index] = torch.arange(len(index), dtype=torch.int32)
+            part = (len(index), shape[1]) if dim == -2 else (shape[0], len(index))
+            u = torch.randn(part, generator=g).bfloat16()
+            F.dion2_post([X1], [u], [index], None, lr, 0.1, 1.5, dim)
+            F.dion2_post([dev[0]], [u.cuda()], [index.cuda()], [where.cuda()], lr.cuda(), 0.1, 1.5,
+                         dim)
+            check([X1], [dev], rel)
+
+
 def test_adamw_counters_of_many_tensors_are_no_bottleneck():
     """4000 counters: the look for shared ones is spread over the GPU (0.4 ms; in one block 2 ms)."""
     n = 4000
