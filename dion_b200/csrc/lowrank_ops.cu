@@ -687,11 +687,10 @@ cholesky_row4_kernel(const float* __restrict__ Gall, float* Uall, int r, int k) 
 // Panel step of a blocked Householder QR (compact WY form).  One CTA per matrix factors the
 // 32-column panel A[j:, j:j+32] in shared memory and leaves
 //   * the panel's part of R (upper triangle of its top 32 rows) in A,
-//   * V  [kk, 32]: the reflectors, unit lower trapezoidal (kk = k - j rows),
-//   * VT [kk, 32] = V T^T, with T the 32 x 32 upper-triangular factor of
-//     H_0 ... H_31 = I - V T V^T,
+//   * V [kk, 32]: the reflectors, unit lower trapezoidal (kk = k - j rows),
+//   * T^T, with T the 32 x 32 upper-triangular factor of H_0 ... H_31 = I - V T V^T,
 // with which qr_update_kernel updates the columns to the right of the panel:
-//   W = V^T A[j:, j+32:],  A[j:, j+32:] -= VT W.
+//   Y = T^T V^T A[j:, j+32:],  A[j:, j+32:] -= V Y.
 // Within a column, lane = panel column: the dot products of column c with the columns to its
 // right are taken by all warps over interleaved rows, reduced through shared memory, and the
 // rank-one update follows; two block barriers per column.  A warp keeps its rows in registers while
@@ -700,32 +699,31 @@ cholesky_row4_kernel(const float* __restrict__ Gall, float* Uall, int r, int k) 
 // multiply-adds (whole factorization of 16 matrices 640 x 512: 1421 -> 1136 us;
 // one form of 48 rows that breaks off at the last row: 1444).  Taller panels
 // (NR = 0) stay in shared memory.
+// V^T V, from which T is built, takes no pass of its own: the
+// dot products of column c with the finished columns to its left, which the lanes left of c would
+// otherwise compute for nothing, are its column c up to the reflectors' scales.
+// With that pass, its atomics, and the product V T^T that the update kernel was given instead of T,
+// panels of 640 to 385 rows took 51 us and shorter ones 34, now 33 and 23.
 // ---------------------------------------------------------------------------------------------
 constexpr int kQpWarps = 16;
 constexpr int kQpPitch = 32;   // the panel is only ever read along its rows
-constexpr int kQpSq = 36;      // pitch of the 32 x 32 factors: 16-byte rows, columns spread over banks
-
-// Reflector entry (i, a) of the panel held in P: zero above the diagonal, one on it.
-__device__ __forceinline__ float qp_v(const float* P, int i, int a) {
-  return i > a ? P[i * kQpPitch + a] : (i == a ? 1.f : 0.f);
-}
+constexpr int kQpSq = 36;      // pitch of V^T V: 16-byte rows, columns spread over banks
 
 template <int NR>
 __global__ void __launch_bounds__(kQpWarps * 32, 1)
-qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Vall, float* VTall) {
+qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Vall, float* TTall) {
   extern __shared__ __align__(16) float qp_smem[];
   const int kk = k - j;
-  float* P = qp_smem;                               // [kk][32]
-  float* part = P + (size_t)kk * kQpPitch;          // [16][32]
+  float* P = qp_smem;                               // [kk][32], or the 32 pivot rows alone
+  float* part = P + (size_t)(NR > 0 ? 32 : kk) * kQpPitch;   // [16][32]
   float* wv = part + kQpWarps * 32;                 // [32]  w of the current column
   float* taus = wv + 32;                            // [32]
   float* sc = taus + 32;                            // [32]  1 / (alpha - beta) per column
-  float* G = sc + 32;                               // [32][36]  V^T V (strictly upper part used)
-  float* T = G + 32 * kQpSq;                        // [32][36]
+  float* G = sc + 32;                               // [32][36]  V^T V (strictly upper part)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* A = Aall + (size_t)blockIdx.x * strideA + (size_t)j * ld + j;
   float* V = Vall + (size_t)blockIdx.x * k * 32;
-  float* VT = VTall + (size_t)blockIdx.x * k * 32;
+  float* TT = TTall + (size_t)blockIdx.x * 32 * 32;
 
   // Row warp + 16 q of the panel in v[q], its entry in the current column in x[q].
   float v[NR > 0 ? NR : 1], x[NR > 0 ? NR : 1];
@@ -740,7 +738,6 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
   } else {
     for (int i = warp; i < kk; i += kQpWarps) P[i * kQpPitch + lane] = A[(size_t)i * ld + lane];
   }
-  for (int e = threadIdx.x; e < 32 * kQpSq; e += kQpWarps * 32) G[e] = 0.f;
   __syncthreads();
 
   // Dot products of column 0 with every column, over the rows below the diagonal.
@@ -758,6 +755,7 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
   }
   __syncthreads();
 
+  float my_scale = 0.f;   // warp 0, lane a: sc[a]
   for (int c = 0; c < 32; ++c) {
     // part holds d[lane] = sum_{i > c} P[i][c] * P[i][lane]  (lane = c: the squared tail norm)
     if (warp == 0) {
@@ -774,8 +772,11 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
         rcc = beta;
       }
       // w[lane] = tau * v^T A[:, lane] with v = (1, scale * tail)
-      const float w = lane > c ? tau * (P[c * kQpPitch + lane] + scale * d) : 0.f;
+      const float top = P[c * kQpPitch + lane] + scale * d;
+      const float w = lane > c ? tau * top : 0.f;
       wv[lane] = w;
+      if (lane < c) G[lane * kQpSq + c] = my_scale * top;   // v_lane^T v_c
+      if (lane == c) my_scale = scale;
       if (lane > c) P[c * kQpPitch + lane] -= w;    // row c: v_c = 1
       if (lane == c) {
         taus[c] = tau;
@@ -835,47 +836,22 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
     part[warp * 32 + lane] = a0 + a1;   // read by warp 0 only after the next barrier
     __syncthreads();
   }
-  if (NR > 0) {
-#pragma unroll
-    for (int q = 2; q < NR; ++q) {
-      const int i = warp + q * kQpWarps;
-      if (i < kk) P[i * kQpPitch + lane] = v[q];
-    }
-  }
-  // scale the reflector tails: V[i][a] = P[i][a] * sc[a] for i > a (a warp's own rows)
+  // The reflectors, their tails scaled (lane = column), and the panel's part of R.
   {
     const float scl = sc[lane];
-    for (int i = warp; i < kk; i += kQpWarps)
-      if (i > lane) P[i * kQpPitch + lane] *= scl;
-  }
-  __syncthreads();
-
-  // G[a][lane] = sum_i V[i][a] V[i][lane]
-  {
-    float g[32];
+    if (NR > 0) {
 #pragma unroll
-    for (int a = 0; a < 32; ++a) g[a] = 0.f;
-    for (int i = warp; i < kk; i += kQpWarps) {
-      const float vc = qp_v(P, i, lane);
-      if (i < 32) {
-#pragma unroll
-        for (int a = 0; a < 32; ++a) g[a] += qp_v(P, i, a) * vc;
-      } else {
-        const float4* row = reinterpret_cast<const float4*>(P + i * kQpPitch);
-#pragma unroll
-        for (int a = 0; a < 8; ++a) {
-          const float4 u = row[a];
-          g[4 * a] += u.x * vc;
-          g[4 * a + 1] += u.y * vc;
-          g[4 * a + 2] += u.z * vc;
-          g[4 * a + 3] += u.w * vc;
-        }
+      for (int q = 2; q < NR; ++q) {
+        const int i = warp + q * kQpWarps;
+        if (i < kk) V[(size_t)(j + i) * 32 + lane] = v[q] * scl;
       }
     }
-#pragma unroll
-    for (int a = 0; a < 32; ++a) atomicAdd(&G[a * kQpSq + lane], g[a]);
+    for (int i = warp; i < (NR > 0 ? 32 : kk); i += kQpWarps) {
+      const float p = P[i * kQpPitch + lane];
+      V[(size_t)(j + i) * 32 + lane] = i > lane ? p * scl : (i == lane ? 1.f : 0.f);
+      if (i <= lane) A[(size_t)i * ld + lane] = p;
+    }
   }
-  __syncthreads();
   // T by columns (lane = row a):  T[a][c] = -tau_c * sum_{b = a}^{c-1} T[a][b] G[b][c],  T[c][c] = tau_c
   // Column c is final once the columns before it have been subtracted: each is taken from all
   // later sums at once, so the chain is 32 steps of independent multiply-adds.
@@ -887,133 +863,140 @@ qr_panel_kernel(float* Aall, long long strideA, int ld, int k, int j, float* Val
     for (int c = 0; c < 32; ++c) {
       const float tc = taus[c];
       const float v = lane < c ? -tc * t[c] : (lane == c ? tc : 0.f);
-      T[lane * kQpSq + c] = v;
+      TT[c * 32 + lane] = v;
 #pragma unroll
       for (int d = c + 1; d < 32; ++d) t[d] += v * G[c * kQpSq + d];
     }
   }
-  __syncthreads();
-  // V and VT = V T^T to global memory (lane = column a; row a of T in registers)
-  {
-    float trow[32];
-#pragma unroll
-    for (int c = 0; c < 32; ++c) trow[c] = T[lane * kQpSq + c];
-    for (int i = warp; i < kk; i += kQpWarps) {
-      float acc = 0.f;
-      if (i < 32) {
-#pragma unroll
-        for (int c = 0; c < 32; ++c) acc += qp_v(P, i, c) * trow[c];
-      } else {
-        const float4* row = reinterpret_cast<const float4*>(P + i * kQpPitch);
-        float acc1 = 0.f;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const float4 u = row[c];
-          acc += u.x * trow[4 * c];
-          acc1 += u.y * trow[4 * c + 1];
-          acc += u.z * trow[4 * c + 2];
-          acc1 += u.w * trow[4 * c + 3];
-        }
-        acc += acc1;
-      }
-      const float vv = qp_v(P, i, lane);
-      V[(size_t)(j + i) * 32 + lane] = vv;
-      VT[(size_t)(j + i) * 32 + lane] = acc;
-    }
-  }
-  // the panel's part of R back into A (reflectors are not kept there)
-  for (int i = warp; i < 32 && i < kk; i += kQpWarps)
-    if (lane >= i) A[(size_t)i * ld + lane] = P[i * kQpPitch + lane];
 }
 
 // Trailing update behind a panel, one CTA per 32 columns of every matrix, lane = column:
-//   W = V^T A (rows split over the warps, the partial sums added in their order),  A -= VT W.
+//   W = V^T A (rows split over the warps, the partial sums added in their order),  Y = T^T W,
+//   A -= V Y.
 // The products are 32 deep (or wide), 20 to 40 MFLOP a matrix and panel: as two split-operand tf32
 // products with their remainder passes they took five launches and 125 us a panel for 16 matrices
-// 640 x 512; here 25 us, in fp32 multiply-adds (R^T R off by 2.8e-7 instead of 1.4e-5), with the
-// rows of V and VT as 16-byte broadcasts from shared memory and A read twice, from L2.
+// 640 x 512; here 23 us, in fp32 multiply-adds (R^T R off by 2.8e-7 instead of 1.4e-5), with the
+// rows of V as 16-byte broadcasts from shared memory and A read twice, from L2.  The next stage's
+// rows are on their way while one is multiplied: with loads, barrier and products in turn a panel
+// took 25 us, most of it the latency of 20 stages.
 constexpr int kQuWarps = 8;
-constexpr int kQuRows = 64;    // rows of V / VT staged at a time
+constexpr int kQuRows = 64;    // rows of V staged at a time
 
 __global__ void __launch_bounds__(kQuWarps * 32)
 qr_update_kernel(float* Aall, long long strideA, int ld, int k, int j, const float* Vall,
-                 const float* VTall) {
-  __shared__ __align__(16) float vs[kQuRows * 32];
+                 const float* TTall) {
+  __shared__ __align__(16) float vs[2][kQuRows * 32];
   __shared__ float part[kQuWarps][32 * 32];
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   const int kk = k - j;
   float* A = Aall + (size_t)blockIdx.y * strideA + (size_t)j * ld + j + 32 + blockIdx.x * 32 + l;
-  const float* V = Vall + ((size_t)blockIdx.y * k + j) * 32;
-  const float* VT = VTall + ((size_t)blockIdx.y * k + j) * 32;
+  const float4* V = reinterpret_cast<const float4*>(Vall + ((size_t)blockIdx.y * k + j) * 32);
   constexpr int kPer = kQuRows / kQuWarps;   // rows of a stage that one warp takes
+  constexpr int kPieces = kQuRows * 8 / (kQuWarps * 32);   // 16-byte pieces of it per thread
+  const float4 tt = reinterpret_cast<const float4*>(TTall + (size_t)blockIdx.y * 32 * 32)[threadIdx.x];
 
-  auto stage = [&](const float* src, int i0) {
-    __syncthreads();
-    const int n4 = (kk - i0 < kQuRows ? kk - i0 : kQuRows) * 8;   // 16-byte pieces
-    for (int e = threadIdx.x; e < n4; e += kQuWarps * 32)
-      reinterpret_cast<float4*>(vs)[e] = __ldg(reinterpret_cast<const float4*>(src + (size_t)i0 * 32) + e);
-    __syncthreads();
+  float4 pv[kPieces];
+  float xn[kPer];
+  auto fetch = [&](int i0) {
+#pragma unroll
+    for (int e = 0; e < kPieces; ++e) {
+      const int piece = i0 * 8 + e * kQuWarps * 32 + threadIdx.x;
+      if (piece < kk * 8) pv[e] = __ldg(V + piece);
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int i = i0 + w * kPer + q;
+      xn[q] = i < kk ? A[(size_t)i * ld] : 0.f;
+    }
+  };
+  // Stages in turn: the fetched rows into buffer `s & 1`, whose last readers are two stages back and
+  // so behind the barrier of the stage between, then the next fetch, then body(row, x, i).
+  auto stages = [&](auto body) {
+    fetch(0);
+    for (int s = 0, i0 = 0; i0 < kk; ++s, i0 += kQuRows) {
+      float x[kPer];
+#pragma unroll
+      for (int q = 0; q < kPer; ++q) x[q] = xn[q];
+#pragma unroll
+      for (int e = 0; e < kPieces; ++e)
+        reinterpret_cast<float4*>(vs[s & 1])[e * kQuWarps * 32 + threadIdx.x] = pv[e];
+      __syncthreads();
+      if (i0 + kQuRows < kk) fetch(i0 + kQuRows);
+#pragma unroll
+      for (int q = 0; q < kPer; ++q) {
+        const int i = i0 + w * kPer + q;
+        if (i >= kk) break;
+        body(reinterpret_cast<const float4*>(vs[s & 1] + (w * kPer + q) * 32), x[q], i);
+      }
+    }
   };
   float acc[32];
 #pragma unroll
   for (int a = 0; a < 32; ++a) acc[a] = 0.f;
-  for (int i0 = 0; i0 < kk; i0 += kQuRows) {
-    float x[kPer];
+  stages([&](const float4* row, float x, int) {
 #pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      const int i = i0 + w * kPer + q;
-      x[q] = i < kk ? A[(size_t)i * ld] : 0.f;
+    for (int c = 0; c < 8; ++c) {
+      const float4 v = row[c];
+      acc[c * 4] += v.x * x;
+      acc[c * 4 + 1] += v.y * x;
+      acc[c * 4 + 2] += v.z * x;
+      acc[c * 4 + 3] += v.w * x;
     }
-    stage(V, i0);
-#pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      if (i0 + w * kPer + q >= kk) break;
-      const float4* row = reinterpret_cast<const float4*>(vs + (w * kPer + q) * 32);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float4 v = row[c];
-        acc[c * 4] += v.x * x[q];
-        acc[c * 4 + 1] += v.y * x[q];
-        acc[c * 4 + 2] += v.z * x[q];
-        acc[c * 4 + 3] += v.w * x[q];
-      }
-    }
-  }
+  });
 #pragma unroll
   for (int a = 0; a < 32; ++a) part[w][a * 32 + l] = acc[a];
   __syncthreads();
+  // Four rows of W per warp, over the partial sums of warp 0, and T^T behind the stages.
+  float* W = part[0];
+  float* Y = part[1];
+  float* TT = vs[0];
+  constexpr int kOwn = 32 / kQuWarps;
 #pragma unroll
-  for (int a = 0; a < 32; ++a) {
+  for (int q = 0; q < kOwn; ++q) {
+    const int a = w + q * kQuWarps;
     float t = 0.f;
 #pragma unroll
-    for (int q = 0; q < kQuWarps; ++q) t += part[q][a * 32 + l];
-    acc[a] = t;                                  // W[a][column]
+    for (int p = 0; p < kQuWarps; ++p) t += part[p][a * 32 + l];
+    W[a * 32 + l] = t;
   }
-  for (int i0 = 0; i0 < kk; i0 += kQuRows) {
-    float x[kPer];
+  reinterpret_cast<float4*>(TT)[threadIdx.x] = tt;
+  __syncthreads();
+  {
+    float y[kOwn];
 #pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      const int i = i0 + w * kPer + q;
-      x[q] = i < kk ? A[(size_t)i * ld] : 0.f;
-    }
-    stage(VT, i0);
+    for (int q = 0; q < kOwn; ++q) y[q] = 0.f;
 #pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      const int i = i0 + w * kPer + q;
-      if (i >= kk) break;
-      const float4* row = reinterpret_cast<const float4*>(vs + (w * kPer + q) * 32);
-      float s0 = 0.f, s1 = 0.f;
+    for (int a4 = 0; a4 < 8; ++a4) {
+      float wa[4];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float4 v = row[c];
-        s0 += v.x * acc[c * 4];
-        s1 += v.y * acc[c * 4 + 1];
-        s0 += v.z * acc[c * 4 + 2];
-        s1 += v.w * acc[c * 4 + 3];
+      for (int e = 0; e < 4; ++e) wa[e] = W[(a4 * 4 + e) * 32 + l];
+#pragma unroll
+      for (int q = 0; q < kOwn; ++q) {
+        const float4 t = reinterpret_cast<const float4*>(TT + (w + q * kQuWarps) * 32)[a4];
+        y[q] += t.x * wa[0];
+        y[q] += t.y * wa[1];
+        y[q] += t.z * wa[2];
+        y[q] += t.w * wa[3];
       }
-      A[(size_t)i * ld] = x[q] - (s0 + s1);
     }
+#pragma unroll
+    for (int q = 0; q < kOwn; ++q) Y[(w + q * kQuWarps) * 32 + l] = y[q];
   }
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < 32; ++a) acc[a] = Y[a * 32 + l];
+  stages([&](const float4* row, float x, int i) {
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float4 v = row[c];
+      s0 += v.x * acc[c * 4];
+      s1 += v.y * acc[c * 4 + 1];
+      s0 += v.z * acc[c * 4 + 2];
+      s1 += v.w * acc[c * 4 + 3];
+    }
+    A[(size_t)i * ld] = x - (s0 + s1);
+  });
 }
 
 }  // namespace dion
@@ -1197,14 +1180,16 @@ DION_EXPORT int dion_normalize_q(const void* R, const float* colsq, float eps, v
 
 // Upper-triangular factors of n dense fp32 matrices A [k, r] (k >= r, r a multiple of 32), in place:
 // the factor is left in the upper triangle of the first r rows, the rest of A is overwritten.
-// V and VT: [n, k, 32] fp32 scratch, 16-byte aligned.  Two launches per panel of 32 columns.
-DION_EXPORT int dion_qr_blocked(void* A, int n, int k, int r, void* V, void* VT, void* stream) {
+// V: [n, k, 32] and TT: [n, 32, 32] fp32 scratch, 16-byte aligned.  Two launches per panel of 32
+// columns.
+DION_EXPORT int dion_qr_blocked(void* A, int n, int k, int r, void* V, void* TT, void* stream) {
   if (n <= 0 || r <= 0) return 0;
   if ((r & 31) || k < r ||
-      ((reinterpret_cast<uintptr_t>(V) | reinterpret_cast<uintptr_t>(VT)) & 15))
+      ((reinterpret_cast<uintptr_t>(V) | reinterpret_cast<uintptr_t>(TT)) & 15))
     return -2;
   auto smem = [&](int j) {
-    return ((size_t)(k - j) * kQpPitch + kQpWarps * 32 + 96 + 2 * 32 * kQpSq) * sizeof(float);
+    const int rows = k - j <= 768 ? 32 : k - j;   // see panel_for
+    return ((size_t)rows * kQpPitch + kQpWarps * 32 + 96 + 32 * kQpSq) * sizeof(float);
   };
   constexpr size_t kMost = 226 * 1024;
   if (smem(0) > kMost) return -2;
@@ -1221,16 +1206,16 @@ DION_EXPORT int dion_qr_blocked(void* A, int n, int k, int r, void* V, void* VT,
       return -3;
   float* a = static_cast<float*>(A);
   float* v = static_cast<float*>(V);
-  float* vt = static_cast<float*>(VT);
+  float* tt = static_cast<float*>(TT);
   for (int j = 0; j < r; j += 32) {
     const Panel panel = panel_for(j);
-    panel<<<n, kQpWarps * 32, smem(j), S(stream)>>>(a, (long long)k * r, r, k, j, v, vt);
+    panel<<<n, kQpWarps * 32, smem(j), S(stream)>>>(a, (long long)k * r, r, k, j, v, tt);
     const int blocks = (r - j) / 32 - 1;
     for (int first = 0; blocks > 0 && first < n; first += kMaxGridY)
       dion::qr_update_kernel<<<dim3(blocks, n - first < kMaxGridY ? n - first : kMaxGridY),
                                dion::kQuWarps * 32, 0, S(stream)>>>(
           a + (size_t)first * k * r, (long long)k * r, r, k, j, v + (size_t)first * k * 32,
-          vt + (size_t)first * k * 32);
+          tt + (size_t)first * 32 * 32);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

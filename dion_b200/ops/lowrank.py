@@ -354,13 +354,13 @@ def blocked_qr_enabled() -> bool:
 def _qr_r_blocked(A32: Tensor) -> Tensor:
     """Blocked Householder QR of a private fp32 batch ``[B, k, r]`` (overwritten): per 32-column
     panel one kernel factors the panel (one CTA per matrix, up to 768 rows in registers, else in
-    shared memory) and emits the reflectors ``V`` and ``V T^T`` of the compact WY form; a second
-    one updates the columns to the right, ``W = V^T A_right`` and ``A_right -= (V T^T) W``, in
-    fp32."""
+    shared memory) and emits the reflectors ``V`` and ``T`` of the compact WY form; a second one
+    updates the columns to the right, ``A_right -= V (T^T (V^T A_right))``, in fp32."""
     B, k, r = A32.shape
     dev = A32.device
-    V, VT = torch.empty((2, B, k, _QR_PANEL), dtype=torch.float32, device=dev).unbind(0)
-    rc = _backend.lib("lowrank_ops").dion_qr_blocked(_ptr(A32), B, k, r, _ptr(V), _ptr(VT),
+    V = torch.empty((B, k, _QR_PANEL), dtype=torch.float32, device=dev)
+    T = torch.empty((B, _QR_PANEL, _QR_PANEL), dtype=torch.float32, device=dev)
+    rc = _backend.lib("lowrank_ops").dion_qr_blocked(_ptr(A32), B, k, r, _ptr(V), _ptr(T),
                                                      _stream(dev))
     if rc != 0:
         raise RuntimeError(f"dion_qr_blocked launch failed (code {rc})")

@@ -77,6 +77,25 @@ def test_blocked_qr_r_factor_matches_fp64(shape, conditioning, monkeypatch):
     assert (Q.mT @ Q - eye).abs().max().item() < (5e-3 if conditioning == "graded" else 1e-3)
 
 
+@pytest.mark.parametrize("shape", [(1, 64, 64), (2, 65, 64), (5, 127, 96), (3, 385, 96), (2, 769, 64),
+                                   (1, 1580, 64), (150, 97, 96)])
+def test_blocked_qr_at_the_edges_of_its_forms(shape, monkeypatch):
+    """Rows around the forms of the panel kernel (384, 768) and the 64-row stages of the update,
+    with a zero column (its reflector is the identity) and one that depends on another.  R^T R is off
+    by the rounding of 32 reflectors a panel at most, the bound of the test above."""
+    from dion_b200.ops import lowrank as LR
+    monkeypatch.setattr(LR, "_QR_BLOCKED_MIN_COLS", 64)
+    B, k, r = shape
+    torch.manual_seed(13)
+    A = torch.randn(B, k, r, device="cuda")
+    A[:, :, 5] = 0
+    A[:, :, 40] = A[:, :, 3]
+    R = LR._qr_r_blocked(A.clone()).double()
+    assert torch.equal(R, R.triu()) and R.isfinite().all()
+    G = A.double().mT @ A.double()
+    assert (R.mT @ R - G).abs().max().item() < 2e-6 * G.abs().max().item()
+
+
 def test_blocked_qr_equals_column_kernel_up_to_signs():
     from dion_b200.ops import lowrank as LR
     torch.manual_seed(12)
