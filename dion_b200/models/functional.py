@@ -460,9 +460,8 @@ def mlp_relu2(h: Tensor, wfc: Tensor, wproj: Tensor) -> Tensor:
     """The ReLU^2 MLP of the GPT block.  With ``DION_B200_FUSED_MLP=1``, bf16 activations with
     ordinary (non-DTensor) weights on a GPU take the fused form above; otherwise the plain
     composition (library GEMMs + element-wise kernels), which is the default: timed inside the
-    GPT-160M training step the fused form is slower (36.3 against 35.3 ms per step) although it saves
-    two element-wise passes: at K = 768 the epilogue of the two-CTA kernel takes longer than a tile's
-    products, and the library GEMM gains more than the passes cost."""
+    GPT-160M training step the fused form is slower (36.0-36.3 against 35.5 ms per step) although it saves
+    two element-wise passes: at K = 768 the library's products gain more than the passes cost."""
     h = materialize(h)
     if (is_plain_tensor(h) and h.is_cuda and h.dtype == torch.bfloat16 and is_plain_tensor(wfc)
             and is_plain_tensor(wproj)

@@ -1,11 +1,11 @@
-"""The GPT's blocks without gradients (``generate``, scoring under ``torch.no_grad``) as two native
-calls per block around the attention (``csrc/infer_ops.cu``).
+"""The GPT's blocks without gradients (``generate``, scoring under ``torch.no_grad``): those of a short
+text as one native call, others as two calls per block around the attention (``csrc/infer_ops.cu``).
 
 The general forward of ``gpt.py`` goes through modules and autograd functions, about fifteen calls
 and 400 us of host time per block, which for a short prompt is six times what the device needs.  The
 path here takes the same weights, hooks nothing and keeps nothing of a call but the products' tile
-tables, one per number of tiles (next-token logits of GPT-160M for 128 tokens: 4838 -> 1182 us;
-``generate``, where every token is another length, 6.2 -> 2.3 ms a token); whatever it does not
+tables, one per number of tiles (next-token logits of GPT-160M for 128 tokens: 4838 us with the general
+forward, 1145 with two calls per block, 526 with one for all); whatever it does not
 recognise (see :func:`hidden_states`) takes the general forward.
 """
 from __future__ import annotations
